@@ -160,6 +160,33 @@ __device__ __forceinline__ double fused_or_unfused(bool f, double alpha, double 
   if (!__any_sync(m, f)) return __dadd_rn(y, __dmul_rn(alpha, x));
   return f ? __fma_rn(alpha, x, y) : __dadd_rn(y, __dmul_rn(alpha, x));
 }
+// 1.0 / p, correctly rounded, mostly on the integer pipe.  GB300's FP64 pipe
+// takes ~70 cycles per dependent operation, so the division's chain costs 380
+// cycles (406 inside a panel kernel); two Newton steps for the reciprocal of
+// the 64-bit fixed-point significand m, from the FP32 reciprocal of its top 24
+// bits, take about 150.  With the seed within 2^-21 the steps leave
+// y = 2^127 / m (units 2^-64) within 4 units; the 53-bit rounding of y is then that
+// of 1/p unless y lies within 8 units of a midpoint between two doubles (0.8%
+// of all significands).  Those, powers of two, zero, subnormals, infinities
+// and NaN, and a subnormal quotient take the division itself.
+__device__ __forceinline__ double recip_rn(double p) {
+  const uint32_t hi = (uint32_t)__double2hiint(p), lo = (uint32_t)__double2loint(p);
+  const uint32_t e = (hi >> 20) & 0x7ffu;
+  const uint32_t mh = 0x80000000u | __funnelshift_l(lo, hi, 11), ml = lo << 11;  // m, in [2^63, 2^64)
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__uint_as_float(0x3f800000u | ((mh >> 8) & 0x7fffffu))));
+  const uint32_t rb = min(max(__float_as_uint(r), 0x3f000000u), 0x3f7fffffu);  // [0.5, 1)
+  const uint32_t y0 = (rb << 8) | 0x80000000u;                                  // units 2^-32
+  const uint64_t t = (uint64_t)mh * y0 + __umulhi(ml, y0);                      // m y0 / 2^32, about 2^63
+  const int32_t d0 = (int32_t)((int64_t)(0x8000000000000000ull - t) >> 11);
+  const uint64_t y1 = ((uint64_t)y0 << 32) + (uint64_t)(((int64_t)(int32_t)(y0 >> 1) * d0) >> 19);
+  const int32_t d1 = (int32_t)(0x8000000000000000ull - __umul64hi((uint64_t)mh << 32 | ml, y1));
+  const uint64_t y = y1 + (uint64_t)(((int64_t)(int32_t)(uint32_t)(y1 >> 33) * d1) >> 30);
+  const uint32_t tail = (uint32_t)y & 2047u;
+  if (e - 1u >= 2044u || ((hi & 0xfffffu) | lo) == 0 || tail - 1016u <= 16u) return 1.0 / p;
+  const uint64_t bits = ((uint64_t)(2044u - e) << 52) + ((y + 1024u) >> 11);
+  return __hiloint2double((int)((uint32_t)(bits >> 32) | (hi & 0x80000000u)), (int)(uint32_t)bits);
+}
 __device__ __forceinline__ bool stop_flag(const int32_t *info) {
   return info != nullptr && *(volatile const int32_t *)info != 0;
 }

@@ -2,12 +2,12 @@
 // (src/getrf.rs:37-101, src/getrf2.rs:39-185).
 //
 // Blocked right-looking LU with BOLA's NB = 32.  Per block column:
-//   1. panel_lu_split: one thread-block CLUSTER (up to 16 CTAs, the panel's
+//   1. panel_lu_cluster: one thread-block CLUSTER (up to 16 CTAs, the panel's
 //      rows spread over them and held in shared memory) factors the
-//      (m-j) x 32 panel column by column: warp-shuffle idamax under BOLA's
-//      lane order, candidate rows pushed through distributed shared memory,
-//      reciprocal scale and BOLA's pairwise rank-1 update — one split cluster
-//      barrier per column (panel_lu, rows in global memory, for taller panels).
+//      (m-j) x 32 panel column by column: idamax under BOLA's lane order,
+//      candidates and the pivot row exchanged through distributed shared
+//      memory, reciprocal scale and BOLA's pairwise rank-1 update by warps of
+//      their own (panel_lu, rows in global memory, for taller panels).
 //   2. step_swap_trsm: the 32 row interchanges applied to every other column
 //      (BOLA's two laswp calls) fused with BOLA's 32-row unit-lower trsm on
 //      the right block row.
@@ -18,6 +18,8 @@
 // come out bit-identical (for the SIMD width selected).
 #include <cooperative_groups.h>
 
+#include <atomic>
+#include <cstddef>
 #include <mutex>
 #include <vector>
 
@@ -50,7 +52,7 @@ constexpr size_t panel_base_bytes() {
 // Unblocked LU of an mp x nb panel (nb <= 32), iterative_getrf2 of
 // src/getrf2.rs:131-185, for panels too tall for the cluster's shared memory:
 // the rows stay in global memory (L2), one full cluster barrier per column.
-// Panels whose rows fit in shared memory take panel_lu_split below.
+// Panels whose rows fit in shared memory take panel_lu_cluster below.
 __global__ void __launch_bounds__(PT)
 panel_lu(double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *info, int32_t add_on_success,
          int32_t col0, int lanes, int64_t R) {
@@ -183,9 +185,8 @@ panel_lu(double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *inf
   cluster.sync();  // no CTA may leave while another can still read its shared memory
 }
 
-// BOLA's rank-1 step (src/getrf2.rs:152-164 with src/ger.rs:28-61) on one
-// element: row g (panel row), column c, by pivot p.  x is the row's scaled
-// multiplier, prow the pivot row.  ger walks columns p+1.. in pairs, skipping
+// BOLA's rank-1 step by pivot p (src/getrf2.rs:152-164 with src/ger.rs:28-61):
+// ger walks columns p+1.. in pairs, skipping
 // a pair whose two pivot-row entries are both zero, with the fused vector
 // body for rows below mr rounded down to the SIMD width and the unfused tail
 // after; an odd last column is always unfused (and skipped when zero).
@@ -200,227 +201,387 @@ __device__ __forceinline__ GerStep ger_step(int p, int nb, int64_t mp, int lanes
   s.vec_end = (mp - p - 1) & ~(int64_t)(lanes - 1);
   return s;
 }
-// -1: the column is skipped, 0: unfused, 1: fused body (rows permitting)
-__device__ __forceinline__ int ger_mode(const GerStep &s, const double *prow, int c) {
-  const int o = c - s.p - 1;
-  if (o < s.nun) {
-    const bool any = nonzero64(prow[c]) || nonzero64(prow[s.p + 1 + (o ^ 1)]);
-    return any ? 1 : -1;
-  }
-  return nonzero64(prow[c]) ? 0 : -1;
-}
-__device__ __forceinline__ double ger_apply(const GerStep &s, int mode, double a, double x, double pc, int64_t g) {
-  if (mode < 0) return a;
-  const double t = -pc;
-  return fused_or_unfused(mode == 1 && g - s.p - 1 < s.vec_end, x, t, a);
-}
-
-// What a CTA pushes into every CTA of the cluster for one column: its pivot
-// candidate and that row (left before pivot j-1's update of columns > j).
-struct XSlot {
-  long long v, key, g, pad;  // Cand (g: panel row, -1 if the CTA has none)
-  double row[PNB];
+// A warp's pivot candidate for one column, as every CTA of the cluster gets it.
+struct alignas(16) PivHdr {
+  uint32_t lo, hi;  // the candidate's value (bits)
+  uint32_t row;     // (row in its CTA's shared memory) << 16 | position in the panel; PIV_NONE: no candidate
+  uint32_t pad;
 };
+constexpr uint32_t PIV_NONE = 0xffffffffu;
 
-// The same unblocked LU as panel_lu (BOLA's iterative_getrf2), rows in shared
-// memory, with no cluster-wide barrier per column: the candidates travel by
-// asynchronous remote stores that count their bytes on the receiver's
-// mbarrier (st.async).  Per column j:
-//   (a) this CTA's candidate in column j is found (BOLA's lane-ordered idamax
-//       keys), one CTA barrier;
-//   (b) every warp pushes the CTA's candidate row (and row j, if owned) into
-//       its share of the cluster's CTAs, one CTA barrier;
-//   (c) the rank-1 update of pivot j-1 on columns j+1.. (deferred), while the
-//       pushes land; a bounded wait on this CTA's own mbarrier for all of
-//       them (a CTA pushes column j+1 only after it has read column j's
-//       slots, which keeps the double-buffered slots and mbarrier phases
-//       safe; a push that never lands stops the panel with
-//       *info = BOLA_INFO_WAIT_EXPIRED instead of hanging);
-//   (d) every CTA picks the same winner from its own slots and brings the
-//       pushed rows up to date (the owner's same operation for pivot j-1 on
-//       columns > j), one CTA barrier; zero pivot -> stop as BOLA does;
-//   (e) the swap, one CTA barrier, the multipliers of column j scaled and the
-//       update of column j+1 only (the next column searched).
-// Every element sees BOLA's operations in BOLA's order: A, ipiv and info are
-// bit-identical to panel_lu's.
-__global__ void __launch_bounds__(PT)
-panel_lu_split(double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *info, int32_t add_on_success,
-               int32_t col0, int lanes, int64_t R) {
+// BOLA's idamax order (make_cand) for one search, in pieces that one warp
+// reduction mostly decides: a larger major wins, then a larger low word of
+// |x|, then a smaller key.  Major 0: no candidate; 1: an element that idamax
+// never selects (NaN, and zero except in short searches).
+struct PivOrder {
+  int base, nch, sl;  // first searched position, chunks of BOLA's vector body, log2(lanes)
+  bool small;         // BOLA's scalar search
+};
+__device__ __forceinline__ PivOrder piv_order(int j, int mp, int lanes) {
+  PivOrder o;
+  o.base = j;
+  o.sl = lanes == 4 ? 2 : 1;
+  o.nch = (mp - j) >> (o.sl + 2);
+  o.small = o.nch == 0;
+  return o;
+}
+__device__ __forceinline__ uint32_t piv_major(const PivOrder &o, uint32_t hi, uint32_t lo) {
+  hi &= 0x7fffffffu;
+  const bool nan = hi > 0x7ff00000u || (hi == 0x7ff00000u && lo != 0);
+  return nan || ((hi | lo) == 0 && !o.small) ? 1u : hi + 2;
+}
+__device__ __forceinline__ uint32_t piv_key(const PivOrder &o, int pos) {
+  const int idx = pos - o.base, sc = o.sl + 2;
+  if (idx >= (o.nch << sc)) return (uint32_t)idx;
+  const int r = idx & ((1 << sc) - 1);
+  return (uint32_t)(((r & ((1 << o.sl) - 1)) * 4 + (r >> o.sl)) * o.nch + (idx >> sc));
+}
+__device__ __forceinline__ bool piv_better(const PivOrder &o, uint32_t ma, uint32_t la, int pa, uint32_t mb, uint32_t lb,
+                                           int pb) {
+  if (ma != mb) return ma > mb;
+  if (ma > 1 && la != lb) return la > lb;
+  return piv_key(o, pa) < piv_key(o, pb);
+}
+// The lane that holds the warp's best candidate.
+__device__ __forceinline__ int piv_best_lane(const PivOrder &o, uint32_t major, uint32_t lo, int pos) {
+  const unsigned FULL = 0xffffffffu;
+  const uint32_t mj = __reduce_max_sync(FULL, major);
+  unsigned m = __ballot_sync(FULL, major == mj);
+  if ((m & (m - 1)) && mj > 0) {
+    bool in = major == mj;
+    if (mj > 1) {
+      const uint32_t ml = __reduce_max_sync(FULL, in ? lo : 0u);
+      in = in && lo == ml;
+    }
+    const uint32_t key = in ? piv_key(o, pos) : PIV_NONE;
+    const uint32_t mk = __reduce_min_sync(FULL, key);
+    m = __ballot_sync(FULL, in && key == mk);
+  }
+  return __ffs(m) - 1;
+}
+
+constexpr int PIV_WARPS = 4;  // one per sub-partition
+constexpr int UPD_WARPS = 8;
+constexpr int PIV_T = 32 * PIV_WARPS;
+constexpr int PAN_T = 32 * (PIV_WARPS + UPD_WARPS);
+constexpr int PAN_ROWS = 32;  // rows per CTA aimed at
+enum { BAR_UPDATED = 1, BAR_SCALED = 2 };
+// Named barriers between the pivot warps and the update warps; a warp that
+// has diverged must be whole again before it takes part.
+__device__ __forceinline__ void bar_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(PAN_T) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(PAN_T) : "memory");
+}
+__host__ __device__ constexpr int panel_pitch(int R) { return R | 1; }  // odd: a row's columns lie in different banks
+inline size_t panel_smem(int64_t R) {
+  return sizeof(double) * PNB * (size_t)panel_pitch((int)R) + sizeof(int32_t) * (size_t)R;
+}
+
+// Unblocked LU of an mp x nb panel (BOLA's iterative_getrf2), the rows spread
+// over a cluster and held in shared memory.  What bounds it is the chain of
+// one column after the other: find the pivot, agree on it, divide by it, bring
+// the next column up to date.  So the chain has warps of its own and carries
+// nothing else:
+//  - rows never move; a row's position (where BOLA's interchanges would have
+//    put it) is kept beside it and decides its place in BOLA's idamax order
+//    and in the fused or unfused part of ger;
+//  - four pivot warps hold the current column in registers: they scale it,
+//    bring the next one up to date and search it, and each sends its candidate
+//    (16 bytes: value, row, position) to every CTA by st.async onto the
+//    receiver's mbarrier; every warp then knows the pivot and forms its
+//    reciprocal while the pivot's CTA sends the pivot row after it;
+//  - eight update warps apply pivot j to the columns right of j + 1 meanwhile;
+//    they are done before the next pivot's row is read.
+// Each exchange is double-buffered by the column's parity: a CTA sends its
+// candidates for column j + 2 only once it has everyone's for column j + 1,
+// and those are sent after column j's were read.  Waits are bounded: one that
+// runs out stops the panel with *info = BOLA_INFO_WAIT_EXPIRED.
+// Every element sees BOLA's operations in BOLA's order.  RPT: rows per pivot
+// thread (R <= 128 RPT).
+template <int RPT>
+__global__ void __launch_bounds__(PAN_T, 1)
+panel_lu_cluster(double *A, int64_t lda, int64_t mp64, int nb, int32_t *ipiv, int32_t *info, int32_t add_on_success,
+                 int32_t col0, int lanes, int64_t R64) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();
   const int cr = (int)cluster.block_rank();
-  __shared__ XSlot slots[2][MAXC];
-  __shared__ double rowj[2][PNB];
-  __shared__ double piv[2][PNB];  // pivot rows, up to date (piv[j & 1] = column j's)
-  __shared__ double oldj[PNB];    // the old row j, up to date (goes to the pivot's place)
-  __shared__ Cand wc[PT / 32];
-  __shared__ double sinv;
-  __shared__ uint64_t xbar[2];  // completes when every CTA's push for a column has landed here
-  __shared__ int sfail;
+  __shared__ PivHdr hdr[2][MAXC * PIV_WARPS];
+  __shared__ __align__(16) double prow[2][PNB];  // the pivot row (columns right of the pivot are used)
+  __shared__ uint64_t hbar[2], rbar[2];  // every candidate / the pivot row has landed
+  __shared__ int hfail[2], rfail[2], sstop;  // a wait for candidates / for a row ran out (by parity); the panel ends
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  double *data = reinterpret_cast<double *>(smem_raw);
+  const int mp = (int)mp64, R = (int)R64, RP = panel_pitch(R);
+  double *data = reinterpret_cast<double *>(smem_raw);  // column c of local row il: data[c * RP + il]
+  int32_t *spos = reinterpret_cast<int32_t *>(data + PNB * RP);
 
   // Uniform across the cluster: the only writer of *info here acts after
   // the cluster barrier that every CTA passes after this read.
   if (stop_flag(info)) return;
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t r0 = (int64_t)cr * R;
-  const int64_t r1 = imin(mp, r0 + R);
-  const int64_t nr = r1 > r0 ? r1 - r0 : 0;
-  auto el = [&](int c, int64_t il) -> double & { return data[(int64_t)c * R + il]; };
-  for (int64_t e = tid; e < nr * nb; e += PT) {
-    const int64_t il = e % nr;
-    const int c = (int)(e / nr);
-    el(c, il) = A[(r0 + il) + (int64_t)c * lda];
-  }
-  if (tid == 0) {
-    sm100::mbar_init(&xbar[0], 1);
-    sm100::mbar_init(&xbar[1], 1);
-    sm100::fence_mbar_init();
-    sfail = 0;
-  }
-  __syncthreads();
-  cluster.sync();  // every CTA runs, its mbarriers initialised, before the first push
-
-  // bytes that land in this CTA per column: a slot (header + row) from every
-  // CTA, row j from its owner
-  constexpr uint32_t SLOT_BYTES = 3 * 8 + PNB * 8, ROW_BYTES = PNB * 8;
-  const uint32_t xbytes = (uint32_t)C * SLOT_BYTES + ROW_BYTES;
-  const int steps = (int)imin(mp, nb);
-  bool failed = false;
-  double inv = 0.0;
-  for (int j = 0; j < steps; ++j) {
-    const int par = j & 1;
-    const double *pprev = piv[par ^ 1];
-    // this column's phase of xbar[par] (its previous phase, column j-2, was
-    // waited for by every thread): expect the pushes
-    if (tid == 0) sm100::mbar_arrive_expect_tx(&xbar[par], xbytes);
-    // (a)
-    Cand best = cand_none();
-    for (int64_t il = tid; il < nr; il += PT) {
-      const int64_t g = r0 + il;
-      if (g < j) continue;
-      const Cand c = make_cand(el(j, il), g - j, mp - j, lanes);
-      if (cand_better(c, best)) best = c;
-    }
-    best = warp_best(best);
-    if (lane == 0) wc[warp] = best;
-    __syncthreads();
-    // (b)
-    {
-      Cand cb = wc[0];
+  const int r0 = cr * R, nr = max(0, min(mp, r0 + R) - r0);
+  for (int il0 = 0; il0 < nr; il0 += 64) {
+    double t[3][2];
 #pragma unroll
-      for (int w = 1; w < PT / 32; ++w)
-        if (cand_better(wc[w], cb)) cb = wc[w];
-      const int64_t gl = cb.v > -2 ? j + cb.idx - r0 : -1;  // local row of the candidate
-      const bool own_j = j >= r0 && j < r1;
-      const double cv = (gl >= 0 && lane < nb) ? el(lane, gl) : 0.0;
-      const double jv = (own_j && lane < nb) ? el(lane, j - r0) : 0.0;
-      for (int d = warp; d < C; d += PT / 32) {
-        const uint32_t rbar = sm100::cluster_addr(&xbar[par], d);
-        const uint32_t rs = sm100::cluster_addr(&slots[par][cr], d);
-        if (lane == 0) {
-          sm100::st_async(rs + offsetof(XSlot, v), (long long)cb.v, rbar);
-          sm100::st_async(rs + offsetof(XSlot, key), (long long)cb.key, rbar);
-          sm100::st_async(rs + offsetof(XSlot, g), (long long)(gl >= 0 ? j + cb.idx : -1), rbar);
-        }
-        sm100::st_async(rs + (uint32_t)offsetof(XSlot, row) + 8u * lane, cv, rbar);
-        if (own_j) sm100::st_async(sm100::cluster_addr(&rowj[par][0], d) + 8u * lane, jv, rbar);
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = warp + q * (PAN_T / 32), il = il0 + 32 * h + lane;
+        t[q][h] = c < nb && il < nr ? A[(r0 + il) + (int64_t)c * lda] : 0.0;
       }
-    }
-    __syncthreads();  // the rows are read before the deferred update changes them
-    // (c) pivot j-1 on columns j+1.., rows >= j
-    if (j > 0 && j + 1 < nb && j - 1 < steps - 1) {
-      const GerStep gs = ger_step(j - 1, nb, mp, lanes);
-      for (int64_t il = tid; il < nr; il += PT) {
-        const int64_t g = r0 + il;
-        if (g < j) continue;
-        const double x = el(j - 1, il);
-        for (int c = j + 1; c < nb; ++c) {
-          const int mode = ger_mode(gs, pprev, c);
-          el(c, il) = ger_apply(gs, mode, el(c, il), x, pprev[c], g);
-        }
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int c = warp + q * (PAN_T / 32), il = il0 + 32 * h + lane;
+        if (c < nb && il < nr) data[c * RP + il] = t[q][h];
       }
-    }
-    // every CTA's push for this column has landed (bounded: a push that
-    // never lands stops the panel, never a hang)
-    if (!sm100::bounded_wait(&xbar[par], (uint32_t)(j >> 1) & 1u)) sfail = 1;
-    __syncthreads();
-    if (sfail) {
-      if (tid == 0) atomicCAS(info, 0, BOLA_INFO_WAIT_EXPIRED);
-      failed = true;
-      break;
-    }
-    // (d) the winner, identical in every CTA
-    Cand wk = cand_none();
-    int ws = 0;
-    {
-      Cand k = cand_none();
-      if (lane < C) {
-        k.v = slots[par][lane].v;
-        k.key = slots[par][lane].key;
-        k.idx = slots[par][lane].g;
-      }
-      wk = warp_best(k);
-      wk.v = __shfl_sync(0xffffffffu, wk.v, 0);
-      wk.key = __shfl_sync(0xffffffffu, wk.key, 0);
-      wk.idx = __shfl_sync(0xffffffffu, wk.idx, 0);
-      const unsigned m = __ballot_sync(0xffffffffu, lane < C && k.v == wk.v && k.key == wk.key && k.idx == wk.idx);
-      ws = m ? __ffs(m) - 1 : 0;
-    }
-    const int64_t jp = wk.v < 0 ? (int64_t)j : wk.idx;  // idamax -> 0 when nothing qualifies
-    const double *raw = jp == j ? rowj[par] : slots[par][ws].row;
-    double *pcur = piv[par];
-    if (tid < nb) {
-      double pv_ = raw[tid], ov = rowj[par][tid];
-      if (j > 0 && tid > j && j - 1 < steps - 1) {
-        const GerStep gs = ger_step(j - 1, nb, mp, lanes);
-        const int mode = ger_mode(gs, pprev, tid);
-        pv_ = ger_apply(gs, mode, pv_, raw[j - 1], pprev[tid], jp);
-        ov = ger_apply(gs, mode, ov, rowj[par][j - 1], pprev[tid], j);
-      }
-      pcur[tid] = pv_;
-      oldj[tid] = ov;
-      if (tid == j) sinv = 1.0 / pv_;  // once per CTA
-    }
-    __syncthreads();
-    const double pv = pcur[j];
-    if (cr == 0 && tid == 0) ipiv[j] = (int32_t)(jp + 1);
-    if (!nonzero64(pv)) {  // exact zero pivot: BOLA's "Matrix is singular" (src/getrf2.rs:166-168)
-      if (cr == 0 && tid == 0) *info = col0 + j + 1;
-      failed = true;
-      break;
-    }
-    inv = sinv;
-    // (e)
-    if (jp != j && tid < nb) {
-      if (j >= r0 && j < r1) el(tid, j - r0) = pcur[tid];
-      if (jp >= r0 && jp < r1) el(tid, jp - r0) = oldj[tid];
-    }
-    __syncthreads();
-    if (j < mp - 1) {
-      const bool next = j + 1 < nb && j < steps - 1;
-      const GerStep gs = ger_step(j, nb, mp, lanes);
-      const int mode = next ? ger_mode(gs, pcur, j + 1) : -1;
-      for (int64_t il = tid; il < nr; il += PT) {
-        const int64_t g = r0 + il;
-        if (g <= j) continue;
-        const double x = __dmul_rn(el(j, il), inv);
-        el(j, il) = x;
-        if (next) el(j + 1, il) = ger_apply(gs, mode, el(j + 1, il), x, pcur[j + 1], g);
-      }
-    }
   }
-  if (!failed && cr == 0 && add_on_success != 0)
-    for (int t = tid; t < steps; t += PT) ipiv[t] += add_on_success;
+  for (int il = tid; il < nr; il += PAN_T) spos[il] = r0 + il;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      sm100::mbar_init(&hbar[i], 1);
+      sm100::mbar_init(&rbar[i], 1);
+    }
+    sm100::fence_mbar_init();
+    hfail[0] = hfail[1] = rfail[0] = rfail[1] = sstop = 0;
+  }
   __syncthreads();
-  for (int64_t e = tid; e < nr * nb; e += PT) {
-    const int64_t il = e % nr;
-    const int c = (int)(e / nr);
-    A[(r0 + il) + (int64_t)c * lda] = el(c, il);
+  cluster.sync();  // every CTA runs, its mbarriers initialised and its rows loaded, before the first push
+
+  const int steps = min(mp, nb);
+  // log2 of the pivot warps per CTA that can hold rows
+  const int lsend = R <= 32 ? 0 : R <= 64 ? 1 : 2;
+  if (warp < PIV_WARPS) {
+    const bool sends = warp < (1 << lsend) && lane < C;
+    const uint32_t hdr_at = sm100::cluster_addr(&hdr[0][(cr << lsend) + (warp & ((1 << lsend) - 1))], min(lane, C - 1));
+    const uint32_t hbar_at = sm100::cluster_addr(&hbar[0], min(lane, C - 1));
+    const int S = C << lsend;
+    double a[RPT];  // column j of this thread's rows, up to date
+    int g[RPT];     // their positions; -1: no row
+#pragma unroll
+    for (int r = 0; r < RPT; ++r) {
+      const int il = tid + PIV_T * r;
+      g[r] = il < nr ? r0 + il : -1;
+      a[r] = il < nr ? data[il] : 0.0;
+    }
+    for (int j = 0; j < steps; ++j) {
+      const int par = j & 1;
+      const uint32_t phase = (uint32_t)(j >> 1) & 1u;
+      const bool next = j < steps - 1;  // then j + 1 < nb as well
+      const PivOrder o = piv_order(j, mp, lanes);
+      // -- this warp's candidate, to every CTA
+      if (warp < (1 << lsend)) {
+        uint32_t mj = 0, lo = 0, hi = 0, row = PIV_NONE;
+        int pos = -1;
+#pragma unroll
+        for (int r = 0; r < RPT; ++r) {
+          const uint32_t h = (uint32_t)__double2hiint(a[r]), l = (uint32_t)__double2loint(a[r]);
+          const uint32_t m = g[r] >= j ? piv_major(o, h, l) : 0u;
+          if (RPT == 1 || (m > 0 && piv_better(o, m, l, g[r], mj, lo, pos))) {
+            mj = m;
+            hi = h;
+            lo = l;
+            pos = g[r];
+            row = m > 0 ? (uint32_t)(tid + PIV_T * r) << 16 | (uint32_t)pos : PIV_NONE;
+          }
+        }
+        const int bl = piv_best_lane(o, mj, lo, pos);
+        hi = __shfl_sync(0xffffffffu, hi, bl);
+        lo = __shfl_sync(0xffffffffu, lo, bl);
+        row = __shfl_sync(0xffffffffu, row, bl);
+        if (sends)
+          sm100::st_async4(hdr_at + par * (uint32_t)sizeof(hdr[0]), lo, hi, row, 0u, hbar_at + par * 8u);
+      }
+      if (tid == PIV_T - 1) {  // (a warp that mostly sends nothing)
+        sm100::mbar_arrive_expect_tx(&hbar[par], (uint32_t)(S * sizeof(PivHdr)));
+        if (next) sm100::mbar_arrive_expect_tx(&rbar[par], (uint32_t)(PNB * sizeof(double)));
+      }
+      // -- the cluster's pivot, the same in every CTA
+      if (!sm100::bounded_wait(&hbar[par], phase)) hfail[par] = 1;
+      double pv;
+      uint32_t prw;
+      int wc;  // its CTA
+      {
+        PivHdr h;
+        h.row = PIV_NONE;
+        h.hi = h.lo = 0;
+        if (lane < S) h = hdr[par][lane];
+        uint32_t mj = h.row != PIV_NONE ? piv_major(o, h.hi, h.lo) : 0u;
+        int slot = lane;
+        if (S > 32) {
+          const int q = lane + 32;
+          PivHdr h2;
+          h2.row = PIV_NONE;
+          if (q < S) h2 = hdr[par][q];
+          const uint32_t m2 = h2.row != PIV_NONE ? piv_major(o, h2.hi, h2.lo) : 0u;
+          if (m2 > 0 &&
+              piv_better(o, m2, h2.lo, (int)(h2.row & 0xffffu), mj, h.lo, (int)(h.row & 0xffffu))) {
+            mj = m2;
+            h = h2;
+            slot = q;
+          }
+        }
+        const int wl = piv_best_lane(o, mj, h.lo, (int)(h.row & 0xffffu));
+        pv = __hiloint2double((int)__shfl_sync(0xffffffffu, h.hi, wl), (int)__shfl_sync(0xffffffffu, h.lo, wl));
+        prw = __shfl_sync(0xffffffffu, h.row, wl);
+        wc = __shfl_sync(0xffffffffu, slot, wl) >> lsend;
+      }
+      const int jp = (int)(prw & 0xffffu);
+      bar_sync(BAR_UPDATED);  // the update warps are done with pivot j - 1
+      const int lost = hfail[par] | rfail[par ^ 1];  // this column's candidates, the last one's row: written before it
+      if (lost || !nonzero64(pv)) {
+        // an exact zero pivot: BOLA's "Matrix is singular" (src/getrf2.rs:166-168)
+#pragma unroll
+        for (int r = 0; r < RPT; ++r)
+          if (g[r] >= j) data[j * RP + tid + PIV_T * r] = a[r];
+        if (tid == 0) {
+          sstop = 1;
+          if (lost) {
+            atomicCAS(info, 0, BOLA_INFO_WAIT_EXPIRED);
+          } else if (cr == 0) {
+            ipiv[j] = jp + 1;
+            *info = col0 + j + 1;
+          }
+        }
+        bar_arrive(BAR_SCALED);
+        break;
+      }
+      // -- the pivot's CTA sends the row; everyone forms the reciprocal
+      if (next && wc == cr) {
+        const int pil = (int)(prw >> 16), c = 2 * (tid & 15);
+        const double v0 = data[c * RP + pil], v1 = data[(c + 1) * RP + pil];
+        for (int d = tid >> 4; d < C; d += PIV_T / 16)
+          sm100::st_async4(sm100::cluster_addr(&prow[par][c], d), (uint32_t)__double2loint(v0),
+                           (uint32_t)__double2hiint(v0), (uint32_t)__double2loint(v1), (uint32_t)__double2hiint(v1),
+                           sm100::cluster_addr(&rbar[par], d));
+      }
+      // (src/getrf2.rs:152-164, src/ger.rs:28-61)
+      const double inv = recip_rn(pv);
+      double an[RPT];  // column j + 1
+#pragma unroll
+      for (int r = 0; r < RPT; ++r) {
+        if (RPT > 1 && PIV_T * r >= nr) break;
+        const int il = tid + PIV_T * r;
+        an[r] = next && il < nr ? data[(j + 1) * RP + il] : 0.0;
+        const double x = __dmul_rn(a[r], inv);
+        if (g[r] >= j) {
+          if (g[r] == j || g[r] == jp) {  // the interchange of positions j and jp
+            g[r] = g[r] == jp ? j : jp;
+            spos[il] = g[r];
+          }
+          data[j * RP + il] = g[r] == j ? a[r] : x;  // the pivot stays
+        }
+        a[r] = x;
+      }
+      if (next) {
+        if (!sm100::bounded_wait(&rbar[par], phase)) rfail[par] = 1;
+        bar_arrive(BAR_SCALED);  // the update warps may start
+        const GerStep gs = ger_step(j, nb, mp, lanes);
+        const double pn = prow[par][j + 1];
+        // j + 1 is ger's first column: paired with j + 2 unless it is the last
+        bool touch = nonzero64(pn);
+        if (gs.nun > 0) touch = touch || nonzero64(prow[par][j + 2]);
+        if (touch) {
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) {
+            if (RPT > 1 && PIV_T * r >= nr) break;
+            const bool body = gs.nun > 0 && g[r] - j - 1 < gs.vec_end;
+            const double u = __fma_rn(a[r], -pn, an[r]);
+            a[r] = __any_sync(0xffffffffu, !body && g[r] > j) && !body ? add_prod(an[r], a[r], -pn) : u;
+          }
+        } else {
+#pragma unroll
+          for (int r = 0; r < RPT; ++r) a[r] = an[r];
+        }
+      } else {
+        bar_arrive(BAR_SCALED);
+      }
+      if (cr == 0 && tid == 0) ipiv[j] = jp + 1;
+    }
+  } else {
+    // Update warps: pivot j on columns j + 2.., 32 rows of one group at a time;
+    // with fewer row groups than warps a group's columns are split.
+    const int uw = warp - PIV_WARPS;
+    const int groups = (nr + 31) / 32;
+    const int split = groups <= 1 ? 8 : groups <= 2 ? 4 : groups <= 4 ? 2 : 1;
+    const int ws = uw % split;
+    for (int j = 0; j < steps; ++j) {
+      const GerStep gs = ger_step(j, nb, mp, lanes);
+      const bool odd = (nb - j - 1) & 1;
+      const int cend = odd ? nb - 1 : nb, c0 = j + 2 + ws;
+      // first columns of ger's pairs
+      const unsigned first = gs.nun > 0 ? (0x55555555u << ((j + 1) & 1)) & (((1u << gs.nun) - 1u) << (j + 1)) : 0u;
+      const double *pr = prow[j & 1];
+      bar_arrive(BAR_UPDATED);
+      bar_sync(BAR_SCALED);
+      if (sstop) break;
+      if (j >= steps - 1) continue;
+      unsigned touch = 0;
+      for (int gr = uw / split; gr < groups; gr += UPD_WARPS / split) {
+        const int il = min(gr * 32 + lane, nr - 1);
+        const int g = gr * 32 + lane < nr ? spos[il] : -1;
+        const double x = data[j * RP + il];
+        constexpr int U = 4;  // independent updates in flight per warp
+        for (int cb = c0; cb < cend; cb += U * split) {
+          double v[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int c = cb + u * split;
+            if (c < cend) v[u] = __fma_rn(x, -pr[c], data[c * RP + il]);
+          }
+          if (cb == c0) {
+            // the columns that ger touches: a pair with a non-zero entry, a
+            // last odd column (always unfused) if non-zero
+            const unsigned nz = __ballot_sync(0xffffffffu, lane < nb && nonzero64(pr[lane]));
+            const unsigned pairs = (nz | nz >> 1) & first;
+            touch = pairs | pairs << 1 | (odd ? nz & (1u << (nb - 1)) : 0u);
+          }
+          const bool body = g > j && g - j - 1 < gs.vec_end;
+#pragma unroll
+          for (int u = 0; u < U; ++u) {
+            const int c = cb + u * split;
+            if (c < cend && body && (touch >> c & 1u)) data[c * RP + il] = v[u];
+          }
+        }
+        if (c0 >= cend) {  // no paired column of this warp's
+          const unsigned nz = __ballot_sync(0xffffffffu, lane < nb && nonzero64(pr[lane]));
+          touch = odd ? nz & (1u << (nb - 1)) : 0u;
+        }
+        const bool body = g > j && g - j - 1 < gs.vec_end;
+        if (odd && nb - 1 >= c0 && (nb - 1 - c0) % split == 0 && (touch >> (nb - 1) & 1u)) {
+          const double v = add_prod(data[(nb - 1) * RP + il], x, -pr[nb - 1]);
+          if (body) data[(nb - 1) * RP + il] = v;
+        }
+        // rows past the vector body (fewer than `lanes` of the whole panel): a
+        // lane per column, so that the other rows' warps issue only FMAs
+        unsigned tail = __ballot_sync(0xffffffffu, g > j && !body);
+        if (ws == split - 1 && tail) {
+          const unsigned nz = __ballot_sync(0xffffffffu, lane < nb && nonzero64(pr[lane]));
+          const unsigned pairs = (nz | nz >> 1) & first;
+          const unsigned all = pairs | pairs << 1 | (odd ? nz & (1u << (nb - 1)) : 0u);
+          do {
+            const int tl = gr * 32 + __ffs(tail) - 1;
+            tail &= tail - 1;
+            const double v = lane < nb ? add_prod(data[lane * RP + tl], data[j * RP + tl], -pr[lane]) : 0.0;
+            if (lane > j + 1 && lane < nb && (all >> lane & 1u)) data[lane * RP + tl] = v;
+          } while (tail);
+        }
+      }
+    }
   }
-  cluster.sync();  // no CTA may leave while another can still read its shared memory
+  __syncthreads();
+  if (!sstop && cr == 0 && add_on_success != 0)
+    for (int t = tid; t < steps; t += PAN_T) ipiv[t] += add_on_success;
+  // every row to its position (all but the rows that pivots displaced stay
+  // where they were: coalesced)
+  for (int c = warp; c < nb; c += PAN_T / 32)
+    for (int il = lane; il < nr; il += 32) A[spos[il] + (int64_t)c * lda] = data[c * RP + il];
+  cluster.sync();  // no CTA may leave while another can still push into it
 }
 
 // iterative_getrf2 for a short, wide matrix (m <= 32 rows, any n): one CTA,
@@ -544,29 +705,32 @@ step_swap_trsm(double *A, int64_t lda, int64_t n, int64_t j, int jb, const int32
 __global__ void zero_i32(int32_t *p) { *p = 0; }
 __global__ void copy_i32(const int32_t *src, int32_t *dst) { *dst = *src; }
 
-// Launches panel_lu with the largest cluster (<= 16 CTAs, ~256 rows each)
-// the device can co-schedule.
+// Launches a panel on the largest cluster (<= 16 CTAs) the device can
+// co-schedule: about 64 rows per CTA, so that the update warps (32 columns x
+// 64 rows, 0.25 us a column on average) stay behind the pivot warps' chain
+// (0.6 us); more rows per CTA once 16 CTAs are in use.  Rows that do not fit
+// in shared memory (mp > 12k) stay in global memory (panel_lu).
 int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *info,
                  int32_t add_on_success, int32_t col0) {
   double fl = 0.0;
   for (int j = 0; j < nb && j < mp; ++j) fl += (double)(mp - j - 1) * (1.0 + 2.0 * (nb - j - 1));
   ProfScope prof(s, "getrf_panel", fl, 16.0 * (double)mp * nb);
-  int C = (int)imin(MAXC, imax(1, cdiv(mp, 256)));
+  int C = (int)imin(MAXC, imax(1, cdiv(mp, PAN_ROWS)));
   for (;; C = C > 1 ? (C + 1) / 2 : 0) {
     if (C == 0) return fail(BOLA_ERR_CUDA, "panel_lu: no cluster size could be scheduled");
     const int64_t R = cdiv(mp, C);
-    // rows in shared memory: the split-barrier kernel; taller panels keep
-    // their rows in global memory (panel_lu)
-    const size_t rows_bytes = (size_t)R * nb * sizeof(double);
-    const bool use_smem = rows_bytes <= SMEM_DATA_LIMIT;
-    const size_t smem = use_smem ? rows_bytes : panel_base_bytes();
-    void (*kern)(double *, int64_t, int64_t, int, int32_t *, int32_t *, int32_t, int32_t, int, int64_t) =
-        use_smem ? panel_lu_split : panel_lu;
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DATA_LIMIT + 4096));
+    const bool use_smem = panel_smem(R) <= SMEM_DATA_LIMIT;
+    const size_t smem = use_smem ? panel_smem(R) : panel_base_bytes();
+    const int rpt = R <= PIV_T ? 0 : R <= 2 * PIV_T ? 1 : R <= 4 * PIV_T ? 2 : 3;
+    void (*const kerns[5])(double *, int64_t, int64_t, int, int32_t *, int32_t *, int32_t, int32_t, int, int64_t) = {
+        panel_lu_cluster<1>, panel_lu_cluster<2>, panel_lu_cluster<4>, panel_lu_cluster<7>, panel_lu};
+    const int ki = use_smem ? rpt : 4;
+    auto kern = kerns[ki];
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DATA_LIMIT));
     BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)C, 1, 1);
-    cfg.blockDim = dim3(PT, 1, 1);
+    cfg.blockDim = dim3(use_smem ? PAN_T : PT, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -576,11 +740,20 @@ int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) != cudaSuccess || nclusters < 1) {
+    // asked once per device, kernel and cluster size, for the largest shared memory
+    int dev = 0;
+    BOLA_TRY_CUDA(cudaGetDevice(&dev));
+    static std::atomic<int8_t> fits[64][5][MAXC + 1];
+    std::atomic<int8_t> &known = fits[dev & 63][ki][C];
+    if (known.load(std::memory_order_relaxed) == 0) {
+      cfg.dynamicSmemBytes = use_smem ? SMEM_DATA_LIMIT : smem;
+      int nclusters = 0;
+      const bool ok = cudaOccupancyMaxActiveClusters(&nclusters, kern, &cfg) == cudaSuccess && nclusters >= 1;
       cudaGetLastError();
-      continue;
+      known.store(ok ? 1 : -1, std::memory_order_relaxed);
+      cfg.dynamicSmemBytes = smem;
     }
+    if (known.load(std::memory_order_relaxed) < 0) continue;
     const int lanes_v = lanes();
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, kern, A, lda, mp, nb, ipiv, info, add_on_success, col0, lanes_v, R));
     return 0;
