@@ -1,7 +1,10 @@
 // api.cu — library-wide state: error messages, SIMD-width setting, device info.
+#include <cuda.h>
+
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "common.cuh"
 
@@ -37,6 +40,71 @@ int num_sms() {
     sms = v;
   }
   return sms;
+}
+
+namespace {
+
+// Unique id of the calling thread's current context (0 if none or unknown).
+// The driver functions are reached through the runtime's entry-point query,
+// so the library does not link the driver library directly.
+unsigned long long current_context_id() {
+  using GetCurrentFn = CUresult (*)(CUcontext *);
+  using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
+  static GetCurrentFn get_current = nullptr;
+  static GetIdFn get_id = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_current = reinterpret_cast<GetCurrentFn>(p);
+    p = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      get_id = reinterpret_cast<GetIdFn>(p);
+  });
+  CUcontext ctx = nullptr;
+  unsigned long long id = 0;
+  if (get_current == nullptr || get_id == nullptr || get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr ||
+      get_id(ctx, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
+constexpr int kMaxDevices = 64;
+constexpr uint64_t kScratchKept = uint64_t(64) << 20;
+std::mutex g_pool_mu;
+struct PoolSlot {
+  unsigned long long ctx_id = 0;  // the context the pool belongs to: a device reset ends it
+  cudaMemPool_t pool = nullptr;
+};
+PoolSlot g_pool_slot[kMaxDevices];
+
+}  // namespace
+
+cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
+  const unsigned long long id = current_context_id();
+  if (id == 0) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  PoolSlot &slot = g_pool_slot[dev];
+  if (slot.pool != nullptr && slot.ctx_id == id) return slot.pool;
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = kScratchKept;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  slot.pool = pool;
+  slot.ctx_id = id;
+  return pool;
 }
 
 }  // namespace bola
