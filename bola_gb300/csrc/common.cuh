@@ -196,6 +196,65 @@ __device__ __forceinline__ double recip_rn(double p) {
   const uint64_t bits = ((uint64_t)(2044u - e) << 52) + ((y + 1024u) >> 11);
   return __hiloint2double((int)((uint32_t)(bits >> 32) | (hi & 0x80000000u)), (int)(uint32_t)bits);
 }
+// sqrt(d), correctly rounded, mostly on the integer pipe (the FP64 square root
+// takes 628 cycles): y0 ~ 1/sqrt(M) from the FP32 pipe for the significand M in
+// [1, 4), s0 = M y0, and two Heron steps s + (M - s^2) y0 / 2 in 64-bit fixed
+// point leave s (units 2^-63) within 4 units; the rounding of s is that of
+// sqrt(d) unless s lies within 8 units of a midpoint.  Those, and everything
+// that is not a positive normal number, take the square root itself.
+__device__ __forceinline__ double sqrt_rn(double d) {
+  const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
+  const uint32_t e = hi >> 20;  // (the sign is its top bit)
+  const bool odd = (e & 1u) == 0;  // of the unbiased exponent
+  const uint64_t m1 = (uint64_t)(0x80000000u | __funnelshift_l(lo, hi, 11)) << 32 | (lo << 11);
+  const uint64_t m = odd ? m1 : m1 >> 1;  // M, units 2^-62
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;"
+      : "=f"(r)
+      : "f"(__uint_as_float((odd ? 0x40000000u : 0x3f800000u) | ((hi & 0xfffffu) << 3) | (lo >> 29))));
+  const uint32_t rb = min(max(__float_as_uint(r), 0x3f000000u), 0x3f7fffffu);
+  const uint32_t y0 = (rb << 8) | 0x80000000u;                                     // units 2^-32
+  const uint64_t v0 = ((uint64_t)(uint32_t)(m >> 32) * y0) >> 31;
+  const uint32_t s0 = v0 > 0xffffffffull ? 0xffffffffu : (uint32_t)v0;             // units 2^-31
+  const int32_t d0 = (int32_t)((int64_t)(m - (uint64_t)s0 * s0) >> 13);
+  const uint64_t s1 = ((uint64_t)s0 << 32) + (uint64_t)(((int64_t)d0 * (int32_t)(y0 >> 1)) >> 18);
+  const int32_t d1 = (int32_t)(m - __umul64hi(s1, s1));
+  const uint64_t s = s1 + (uint64_t)(((int64_t)d1 * (int64_t)y0) >> 32);
+  const uint32_t tail = (uint32_t)s & 2047u;
+  if (e - 1u >= 2046u || tail - 1016u <= 16u) return sqrt(d);
+  return __longlong_as_double((long long)(((uint64_t)((e + 1021u) >> 1) << 52) + ((s + 1024u) >> 11)));
+}
+// f ? fma(a, x, y) : y + a*x in two operations for a warp whose lanes differ:
+// the product of an unfused lane goes through the same multiply-add as a
+// factor of one, which adds it exactly as an addition does.
+__device__ __forceinline__ double fused_or_unfused2(bool f, double a, double x, double y) {
+  const double p = __dmul_rn(a, x);
+  return __fma_rn(f ? a : p, f ? x : 1.0, y);
+}
+// What a division by b repeats: y = RN(1/b) and the reciprocal's own error.
+struct Divisor {
+  double b, y, yl;
+};
+__device__ __forceinline__ Divisor divisor(double b) {
+  Divisor d;
+  d.b = b;
+  d.y = recip_rn(b);
+  d.yl = __dmul_rn(__fma_rn(-b, d.y, 1.0), d.y);
+  return d;
+}
+// a / b, correctly rounded, in four dependent operations: q within one unit in
+// the last place from the two-part reciprocal, then Markstein's correction (P.
+// Markstein, IBM J. Res. Dev. 34(1), 1990): with y = RN(1/b) and the exact
+// remainder r = a - b q, RN(q + r y) is the rounded quotient.  The division
+// itself where an exponent could leave the normal range on the way (zeros,
+// subnormals, infinities and NaN among them).
+__device__ __forceinline__ double div_rn(double a, const Divisor &d) {
+  const int ea = (__double2hiint(a) >> 20) & 0x7ff, eb = (__double2hiint(d.b) >> 20) & 0x7ff;
+  if ((unsigned)(ea - 200) > 1600u || (unsigned)(eb - 200) > 1600u || (unsigned)(ea - eb + 800) > 1600u)
+    return a / d.b;
+  const double q = __fma_rn(a, d.y, __dmul_rn(a, d.yl));
+  return __fma_rn(__fma_rn(-d.b, q, a), d.y, q);
+}
 __device__ __forceinline__ bool stop_flag(const int32_t *info) {
   return info != nullptr && *(volatile const int32_t *)info != 0;
 }

@@ -205,120 +205,202 @@ __device__ int p2_walk(bool upper, double *a0, double *rdg, int n, int lanes) {
   return 0;
 }
 
-// 128 threads: one warp per SMSP, so the SYRK steps' FP64 work never queues
-// two warps on one sub-partition's FP64 pipe.
-constexpr int P2T = 128;
-constexpr int P2E = (LDS * (LDS + 1) / 2 + P2T - 1) / P2T;  // lower-triangle elements per thread
-
-// Which updates of element (i, j) (i >= j) BOLA's recursion makes fused: bit l
-// set if the update from column l < j is the fused body of a daxpy.  In
-// p2_walk every update of (i, j) comes from a column l < j, in increasing l:
+// The 32x32 block column by column ('L') or row by row ('U') instead of by
+// recursion.  The chain of one column (square root, reciprocal or division,
+// the next column's update) is what bounds it, so one warp walks it, a lane
+// per row (column), with the square root and the reciprocal on the integer
+// pipe, and eight warps apply each finished column to the columns after the
+// next one meanwhile.  Every element sees the operations of BOLA's recursion
+// in BOLA's order:
+//
+// 'L': every update of (i, j) comes from a column l < j, in increasing l:
 // first from the SYRK of each frame whose leading half holds l and whose
-// trailing half holds i and j (a daxpy over that half's column jj: element
-// idx = ii - jj of len = n2 - jj, fused below len rounded down to the SIMD
-// width), then, in the frame that separates i from j, from its TRSM (unfused
-// b - a*x for l in [frame start, j)), after which (i, j) is scaled by 1/l_jj.
-__device__ uint32_t fused_updates(int i, int j, int n, int lanes) {
-  uint32_t m = 0;
-  int off = 0, nn = n;
-  while (nn > 1) {
-    const int n1 = nn / 2, n2 = nn - n1, split = off + n1;
-    if (j >= split) {  // (i, j) in the trailing half: SYRK from l in [off, split)
-      const int jj = j - split, idx = i - j, len = n2 - jj;
-      if (idx < (len & ~(lanes - 1))) m |= ((1u << n1) - 1u) << off;
-      off = split;
-      nn = n2;
-    } else if (i >= split) {  // below the leading half: the TRSM, unfused
-      break;
-    } else {
-      nn = n1;
-    }
-  }
-  return m;
+// trailing half holds i and j (a daxpy over that half's column j, fused below
+// its length rounded down to the SIMD width), then, in the frame that separates
+// i from j, from its TRSM (unfused), then the scale by 1/l_jj.  With
+// `end` the end of the frame that separates l from j, the update is fused for
+// rows i < j + ((end - j) rounded down).
+//
+// 'U': a frame whose trailing half begins at row k + 1 applies its SYRK, one
+// dot product over its leading rows per element, when row k is final; the
+// updates of the TRSM of the frame that separates i from j are applied row by
+// row, unfused; then the division by u_ii.
+//
+// Measured on one GB300 at n = 4096, launches serialised: @@L us ('L'),
+// @@U us ('U'), against 50 and 84 for the column sweep on four warps with
+// three CTA barriers a column and the recursion.
+constexpr int P2_UPD = 8;                      // update warps
+constexpr int P2_T = 32 * (1 + P2_UPD);
+constexpr int P2P = NB + 1;                    // pitch
+enum { P2_UPDATED = 1, P2_SCALED = 2 };
+__device__ __forceinline__ void p2_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(P2_T) : "memory");
+}
+__device__ __forceinline__ void p2_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(P2_T) : "memory");
+}
+__device__ __forceinline__ bool positive64(double d) {
+  const long long b = __double_as_longlong(d);
+  return b > 0 && b <= 0x7ff0000000000000ll;  // d > 0, not NaN
 }
 
-// potrf2 'L' of the block in shared memory, right-looking: column l is
-// finished (square root, 1/l_ll, the column scaled), then every element
-// (i, j > l) takes its update from column l, fused or not as BOLA's recursion
-// does it.  Every element sees BOLA's operations in BOLA's order, so the factor
-// is bit-identical; the dependent chain per column is one square root and
-// one reciprocal instead of the recursion's chains of solves.  Returns 0 or
-// the 1-based failing column; the block is then not in BOLA's state (the
-// caller redoes it with p2_walk).
-__device__ int p2_right_looking(double *a, double *rdg, int n, int lanes) {
-  __shared__ int fail;
-  const int tid = threadIdx.x;
-  int ei[P2E], ej[P2E];
-  uint32_t em[P2E];
-#pragma unroll
-  for (int s = 0; s < P2E; ++s) {  // element e = tid + s * P2T of the packed lower triangle, column by column
-    int e = tid + s * P2T, j = 0;
-    while (j < n && e >= n - j) {
-      e -= n - j;
-      ++j;
-    }
-    ei[s] = j < n ? j + e : -1;
-    ej[s] = j;
-    em[s] = j < n ? fused_updates(j + e, j, n, lanes) : 0u;
-  }
-  if (tid == 0) fail = 0;
-  __syncthreads();
-  for (int l = 0; l < n; ++l) {
-    if (tid == 0) {
-      const double d = a[l + l * LDS];
-      const long long db = __double_as_longlong(d);
-      if (db > 0 && db <= 0x7ff0000000000000ll) {  // d > 0, not NaN
-        const double r = sqrt(d);
-        a[l + l * LDS] = r;
-        rdg[l] = 1.0 / r;
+// a: column j of row i at a[j * P2P + i].  Returns 0 or the 1-based failing
+// column (the block is then not in BOLA's state).
+__device__ int p2_lower(double *a, int n, int lanes) {
+  __shared__ uint8_t cut[NB][NB];  // cut[l][j]: rows below it take column l's update of column j fused
+  __shared__ int stop;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int e = tid; e < n * n; e += P2_T) {
+    const int l = e % n, j = e / n;
+    if (j <= l) continue;
+    int off = 0, nn = n;
+    for (;;) {  // down to the frame that separates l from j
+      const int n1 = nn / 2;
+      if (l >= off + n1) {
+        off += n1;
+        nn -= n1;
+      } else if (j < off + n1) {
+        nn = n1;
       } else {
-        fail = l + 1;
+        break;
       }
     }
-    __syncthreads();
-    if (fail) return fail;
-    const double rl = rdg[l];
-#pragma unroll
-    for (int s = 0; s < P2E; ++s)
-      if (ej[s] == l && ei[s] > l) a[ei[s] + l * LDS] = __dmul_rn(a[ei[s] + l * LDS], rl);
-    __syncthreads();
-#pragma unroll
-    for (int s = 0; s < P2E; ++s) {
-      const int i = ei[s], j = ej[s];
-      if (i < 0 || j <= l) continue;
-      const double ljl = a[j + l * LDS];
-      if (!nonzero64(ljl)) continue;  // BOLA skips a zero multiplier
-      const double lil = a[i + l * LDS];
-      double &c = a[i + j * LDS];
-      c = fused_or_unfused((em[s] >> l) & 1u, -ljl, lil, c);  // unfused: c + (-l_jl) l_il = c - l_jl l_il
-    }
-    __syncthreads();
+    cut[l][j] = (uint8_t)(j + ((off + nn - j) & ~(lanes - 1)));
   }
-  return 0;
+  if (tid == 0) stop = 0;
+  __syncthreads();
+  if (warp == 0) {
+    double c = a[lane];
+    for (int l = 0; l < n; ++l) {
+      const double d = __shfl_sync(0xffffffffu, c, l);
+      if (!positive64(d)) {
+        if (lane == 0) stop = l + 1;
+        p2_arrive(P2_SCALED);
+        break;
+      }
+      const double r = sqrt_rn(d);
+      const double x = lane == l ? r : __dmul_rn(c, recip_rn(r));
+      if (lane >= l) a[l * P2P + lane] = x;
+      p2_sync(P2_UPDATED);  // column l - 1 is applied everywhere
+      if (l + 1 < n) c = a[(l + 1) * P2P + lane];
+      p2_arrive(P2_SCALED);
+      if (l + 1 < n) {
+        const double xj = __shfl_sync(0xffffffffu, x, l + 1);
+        if (nonzero64(xj)) c = fused_or_unfused2(lane < cut[l][l + 1], -xj, x, c);  // BOLA skips a zero multiplier
+      }
+    }
+  } else {
+    for (int l = 0; l < n; ++l) {
+      p2_arrive(P2_UPDATED);
+      p2_sync(P2_SCALED);
+      if (stop) break;
+      const double x = a[l * P2P + lane];
+      for (int j = l + 1 + warp; j < n; j += P2_UPD) {
+        const double xj = a[l * P2P + j];
+        if (!nonzero64(xj)) continue;
+        const double c = fused_or_unfused2(lane < cut[l][j], -xj, x, a[j * P2P + lane]);
+        if (lane >= j) a[j * P2P + lane] = c;
+      }
+    }
+  }
+  __syncthreads();
+  return stop;
 }
 
-__global__ void __launch_bounds__(P2T)
+// BOLA's dot product of rows off..off + n1 - 1 in columns i and j (n1 a power
+// of two; dot_exact's order), a: column j of row i at a[i * P2P + j].
+__device__ __forceinline__ double p2_dot(const double *a, int off, int n1, int i, int j, int lanes) {
+  return dot_exact(n1, a + off * P2P + i, P2P, a + off * P2P + j, P2P, lanes);
+}
+// Row i (lane j holds (i, j), up to date up to row k - 1) takes row k: the SYRK
+// of the frame whose trailing half begins at k + 1, or the TRSM update.
+__device__ __forceinline__ double p2_upper_row(const double *a, int k, int i, double c, int lanes) {
+  const int j = threadIdx.x & 31;
+  const int n1 = (k + 1) & -(k + 1);  // the half length of the frame that splits at k + 1
+  const double xi = a[k * P2P + i], xj = a[k * P2P + j];
+  const int s = 31 - __clz(i ^ j);    // the frame that separates i from j: 2^(s+1) rows
+  const bool trsm = j > i && (k >> (s + 1)) == (i >> (s + 1));
+  if (__any_sync(0xffffffffu, trsm)) {
+    const double u = sub_prod(c, xi, xj);
+    if (trsm) c = u;
+  }
+  if (i < k + 1 + n1) {  // (uniform)
+    const double t = p2_dot(a, k + 1 - n1, n1, i, j, lanes);
+    if (j >= i && j < k + 1 + n1) c = add_prod(c, -1.0, t);
+  }
+  return c;
+}
+// a: column j of row i at a[i * P2P + j], n = 32.
+__device__ int p2_upper32(double *a, int lanes) {
+  __shared__ int stop;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) stop = 0;
+  __syncthreads();
+  if (warp == 0) {
+    double c = a[lane];
+    for (int k = 0; k < NB; ++k) {
+      const double d = __shfl_sync(0xffffffffu, c, k);
+      if (!positive64(d)) {
+        if (lane == 0) stop = k + 1;
+        p2_arrive(P2_SCALED);
+        break;
+      }
+      const double r = sqrt_rn(d);
+      const double x = lane == k ? r : c / r;
+      if (lane >= k) a[k * P2P + lane] = x;
+      p2_sync(P2_UPDATED);
+      if (k + 1 < NB) c = a[(k + 1) * P2P + lane];
+      p2_arrive(P2_SCALED);
+      if (k + 1 < NB) c = p2_upper_row(a, k, k + 1, c, lanes);
+    }
+  } else {
+    for (int k = 0; k < NB; ++k) {
+      p2_arrive(P2_UPDATED);
+      p2_sync(P2_SCALED);
+      if (stop) break;
+      for (int i = k + 1 + warp; i < NB; i += P2_UPD) {
+        const double c = p2_upper_row(a, k, i, a[i * P2P + lane], lanes);
+        if (lane >= i) a[i * P2P + lane] = c;
+      }
+    }
+  }
+  __syncthreads();
+  return stop;
+}
+
+__global__ void __launch_bounds__(P2_T)
 potrf2_block(bool upper, int n, double *A, int64_t lda, int32_t *info, int32_t col0, int lanes) {
-  __shared__ double a[LDS * LDS];
-  __shared__ double a0[LDS * LDS];  // the input, for a failing 'L' block
+  __shared__ double a[NB * P2P];
+  __shared__ double a0[LDS * LDS];  // the input, for the recursion: a failing block, a short 'U' one
   __shared__ double rdg[LDS];
   if (stop_flag(info)) return;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const double v = A[(e % n) + (e / n) * lda];
-    a[(e % n) + (e / n) * LDS] = v;
-    a0[(e % n) + (e / n) * LDS] = v;
+    const int i = e % n, j = e / n;
+    const double v = A[i + (int64_t)j * lda];
+    a0[i + j * LDS] = v;
+    if (upper) a[i * P2P + j] = v;
+    else a[j * P2P + i] = v;
   }
   __syncthreads();
-  int r = upper ? p2_walk(true, a, rdg, n, lanes) : p2_right_looking(a, rdg, n, lanes);
-  if (!upper && r) {  // BOLA's state at a failure is its recursion's: redo the block that way
+  const bool walk = upper && n < NB;
+  int r = walk ? 1 : upper ? p2_upper32(a, lanes) : p2_lower(a, n, lanes);
+  if (r) {  // BOLA's state at a failure is its recursion's: (re)do the block that way
+    r = p2_walk(upper, a0, rdg, n, lanes);
     __syncthreads();
-    for (int e = threadIdx.x; e < LDS * LDS; e += blockDim.x) a[e] = a0[e];
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      const int i = e % n, j = e / n;
+      if (upper) a[i * P2P + j] = a0[i + j * LDS];
+      else a[j * P2P + i] = a0[i + j * LDS];
+    }
     __syncthreads();
-    r = p2_walk(false, a, rdg, n, lanes);
   }
-  __syncthreads();
   // BOLA stops at the failing column with everything before it written back.
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) A[(e % n) + (e / n) * lda] = a[(e % n) + (e / n) * LDS];
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int i = e % n, j = e / n;
+    if (upper ? i <= j : i >= j) A[i + (int64_t)j * lda] = upper ? a[i * P2P + j] : a[j * P2P + i];
+  }
   if (r && threadIdx.x == 0) *info = col0 + r;
 }
 
@@ -351,7 +433,7 @@ int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int
   if (n == 0) return 0;
   if (n <= NB) {
     ProfScope prof(s, "potrf2_block", (double)n * n * n / 3.0);
-    potrf2_block<<<1, P2T, 0, s>>>(upper, (int)n, A, lda, info, col0, lanes());
+    potrf2_block<<<1, P2_T, 0, s>>>(upper, (int)n, A, lda, info, col0, lanes());
     BOLA_CHECK_LAUNCH();
     return 0;
   }

@@ -35,42 +35,176 @@ __device__ __forceinline__ void load_tri(double *sA, const double *A, int64_t ld
 }
 
 // Left side, op(A) = A: trsm_lnl / trsm_lnu base cases (src/trsm.rs:96-123, 136-163).
+// A warp per right-hand side, two rows per lane, one warp per sub-partition
+// (the chain of a step, broadcast, division, multiply-add, is what it waits
+// for; eight warps per CTA queued two on a sub-partition's FP64 pipe).
+constexpr int LN_WARPS = 4;
 template <bool LOWER>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(32 * LN_WARPS)
 left_n_base(int m, int64_t n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
             int64_t ldb, int lanes, const int32_t *info) {
   __shared__ double sA[STOP * STOP];
+  __shared__ Divisor dv[STOP];
   if (stop_flag(info)) return;
   load_tri(sA, A, lda, m);
   __syncthreads();
+  if (!unit) {
+    if (threadIdx.x < m) dv[threadIdx.x] = divisor(sA[threadIdx.x * (STOP + 1)]);
+    __syncthreads();
+  }
   const int lane = threadIdx.x & 31;
-  const int64_t col = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t col = (int64_t)blockIdx.x * LN_WARPS + (threadIdx.x >> 5);
   if (col >= n) return;
   double *bc = B + col * ldb;
-  double b0 = lane < m ? bc[lane] : 0.0;
-  double b1 = lane + 32 < m ? bc[lane + 32] : 0.0;
+  double b[2] = {lane < m ? bc[lane] : 0.0, lane + 32 < m ? bc[lane + 32] : 0.0};
+  // column k of the triangle, a step ahead
+  auto column = [&](int k, double(&a)[2]) {
+    a[0] = sA[lane + k * STOP];
+    a[1] = sA[(lane + 32) + k * STOP];
+  };
+  double an[2];
+  column(LOWER ? 0 : m - 1, an);
+#pragma unroll 2
   for (int step = 0; step < m; ++step) {
     const int k = LOWER ? step : m - 1 - step;
-    const double bk = __shfl_sync(0xffffffffu, k < 32 ? b0 : b1, k & 31);
+    const double a[2] = {an[0], an[1]};
+    if (step + 1 < m) column(LOWER ? k + 1 : k - 1, an);
+    const double bk = __shfl_sync(0xffffffffu, k < 32 ? b[0] : b[1], k & 31);
     if (!nonzero64(bk)) continue;  // BOLA skips zero entries (src/trsm.rs:101,141)
-    const double u = unit ? bk : bk / sA[k + k * STOP];
-    if (k == lane) b0 = u;
-    if (k == lane + 32) b1 = u;
-    if (!nonzero64(u)) continue;  // daxpy returns early for a zero scale (src/utilities.rs:108)
-    // daxpy over rows k+1..m-1 (lower) or 0..k-1 (upper) with alpha = -u
-    const int64_t len = LOWER ? (int64_t)(m - k - 1) : (int64_t)k;
+    double u = bk;
+    if (!unit) {
+      u = div_rn(bk, dv[k]);
+      if (k == lane) b[0] = u;
+      if (k == lane + 32) b[1] = u;
+      if (!nonzero64(u)) continue;  // daxpy returns early for a zero scale (src/utilities.rs:108)
+    }
+    // daxpy over rows k+1..m-1 (lower) or 0..k-1 (upper) with alpha = -u: the
+    // last len % lanes rows are its unfused tail
+    const int len = LOWER ? m - k - 1 : k, end = LOWER ? m : k, cut = end - (len & (lanes - 1));
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
+      if (LOWER ? (k >= 31 + 32 * h || m <= 32 * h) : k <= 32 * h) continue;  // no row of this half
       const int i = lane + 32 * h;
-      const bool in = LOWER ? (i > k && i < m) : (i < k);
-      if (!in) continue;
-      const int64_t idx = LOWER ? (int64_t)(i - k - 1) : (int64_t)i;
-      double &bi = h == 0 ? b0 : b1;
-      bi = daxpy_elem(bi, -u, sA[i + k * STOP], idx, len, lanes);
+      const bool in = LOWER ? (i > k && i < m) : i < k;
+      const double f = __fma_rn(-u, a[h], b[h]);
+      if (cut < end && end > 32 * h && cut < 32 * h + 32) {  // (uniform) the tail lies in this half
+        const double t = add_prod(b[h], -u, a[h]);
+        if (in) b[h] = i < cut ? f : t;
+      } else if (in) {
+        b[h] = f;
+      }
     }
   }
-  if (lane < m) bc[lane] = b0;
-  if (lane + 32 < m) bc[lane + 32] = b1;
+  if (lane < m) bc[lane] = b[0];
+  if (lane + 32 < m) bc[lane + 32] = b[1];
+}
+
+// The base cases whose updates are BOLA's unfused t - a x, a warp per system
+// (a right-hand side on the left, a row of B on the right), of order n <= 64.
+// T[k][j] is the coefficient of x_k in equation j.
+//  - Ascending (ltu, rnu, rtl: x_0 first, equation j takes k < j in ascending
+//    order): once x_k is final every later equation subtracts it, two
+//    equations per lane.
+//  - Descending with ascending sums (ltl, rnl, rtu: x_{n-1} first, equation j
+//    takes k > j in ascending order, the newest solution first): equation j is
+//    one chain of n - 1 - j subtractions.  Its products are formed a lane per
+//    k, all but the newest one a step ahead; the chain itself, ~65 cycles per
+//    subtraction, is the bound (n = 48: 35 us; a thread per system, product
+//    after product: 81 us).
+// Left: t / a_jj; right: t * (1 / a_jj), and a zero coefficient is skipped.
+constexpr int TW_WARPS = 4;
+constexpr int TW_PITCH = STOP + 1;
+template <bool ASC, bool RIGHT>
+__global__ void __launch_bounds__(32 * TW_WARPS)
+tri_warp(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
+         int64_t elem, int64_t sys, const int32_t *info) {
+  __shared__ double T[STOP * TW_PITCH];
+  __shared__ Divisor dv[STOP];
+  __shared__ __align__(16) double pbuf[TW_WARPS][2][STOP];
+  if (stop_flag(info)) return;
+  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+    const int r = e % n, c = e / n;  // a(r, c): (k, j), or (j, k) when transposed
+    T[transposed ? c * TW_PITCH + r : r * TW_PITCH + c] = A[r + (int64_t)c * lda];
+  }
+  __syncthreads();
+  if (!unit) {
+    if (threadIdx.x < n) dv[threadIdx.x] = divisor(T[threadIdx.x * (TW_PITCH + 1)]);
+    __syncthreads();
+  }
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t s = (int64_t)blockIdx.x * TW_WARPS + warp;
+  if (s >= systems) return;
+  double *b = B + s * sys;
+  double x[2] = {lane < n ? b[lane * elem] : 0.0, lane + 32 < n ? b[(lane + 32) * elem] : 0.0};
+  auto finish = [&](double t, int j) { return unit ? t : RIGHT ? __dmul_rn(t, dv[j].y) : div_rn(t, dv[j]); };
+  if (ASC) {
+    double tn[2] = {T[lane], T[lane + 32]};
+    for (int k = 0; k < n; ++k) {
+      const double a[2] = {tn[0], tn[1]};
+      if (k + 1 < n) {
+        tn[0] = T[(k + 1) * TW_PITCH + lane];
+        tn[1] = T[(k + 1) * TW_PITCH + lane + 32];
+      }
+      const double xk = finish(__shfl_sync(FULL, k < 32 ? x[0] : x[1], k & 31), k);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = lane + 32 * h;
+        if (j == k) x[h] = xk;
+        if (k >= 31 + 32 * h || n <= 32 * h) continue;
+        const double u = sub_prod(x[h], a[h], xk);
+        if (j > k && (!RIGHT || nonzero64(a[h]))) x[h] = u;
+      }
+    }
+  } else {
+    // products of equation j with the solutions k >= j + 2, into pbuf[.][j & 1];
+    // which coefficients are zero (right) in zero[j & 1]
+    uint64_t zero[2] = {0, 0};
+    auto products = [&](int j, uint64_t &z) {
+      z = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int k = lane + 32 * h;
+        const bool in = k > j + 1 && k < n;
+        const double a = in ? T[k * TW_PITCH + j] : 1.0;
+        if (j + 1 < 31 + 32 * h && n > 32 * h) {  // (uniform) some k of this half
+          const double p = __dmul_rn(a, x[h]);
+          if (in) pbuf[warp][j & 1][k] = p;
+        }
+        if (RIGHT) z |= (uint64_t)__ballot_sync(FULL, in && !nonzero64(a)) << (32 * h);
+      }
+    };
+    double newest = 0.0;
+    for (int j = n - 1; j >= 0; --j) {
+      if (j >= 1) products(j - 1, zero[(j - 1) & 1]);  // equation j - 1, with the solutions from j + 1 on
+      double t = __shfl_sync(FULL, j < 32 ? x[0] : x[1], j & 31);
+      const double *p = pbuf[warp][j & 1];
+      const uint64_t z = zero[j & 1];
+      if (j + 1 < n) {
+        const double a = T[(j + 1) * TW_PITCH + j];
+        if (!RIGHT || nonzero64(a)) t = sub_prod(t, a, newest);
+      }
+      int k = j + 2;
+      if (z == 0) {
+        if ((k & 1) && k < n) t = __dsub_rn(t, p[k++]);
+#pragma unroll 4
+        for (; k + 1 < n; k += 2) {
+          const double2 v = *reinterpret_cast<const double2 *>(&p[k]);
+          t = __dsub_rn(t, v.x);
+          t = __dsub_rn(t, v.y);
+        }
+        if (k < n) t = __dsub_rn(t, p[k]);
+      } else {
+        for (; k < n; ++k)
+          if (!((z >> k) & 1u)) t = __dsub_rn(t, p[k]);
+      }
+      newest = finish(t, j);
+      if (lane == (j & 31)) x[j >> 5] = newest;
+      __syncwarp();
+    }
+  }
+  if (lane < n) b[lane * elem] = x[0];
+  if (lane + 32 < n) b[(lane + 32) * elem] = x[1];
 }
 
 // Left side, op(A) = A^T: trsm_ltl / trsm_ltu base cases (src/trsm.rs:176-188, 215-227).
@@ -171,15 +305,20 @@ struct Ctx {
   const int32_t *info;
 };
 
+// Up to how many systems a warp each (tri_warp) beats a thread each: the warps
+// of one SM share its FP64 pipe (n = 64: ~27 cycles of the GPU per ascending
+// system, ~210 per descending one, against 280k cycles for any number of
+// threads); rows of at most 32 columns over 4 lanes take ~24k cycles.
+constexpr int64_t ASC_WARP_MAX = 8192, SEQ_WARP_MAX = 1216, ASC32_WARP_MAX = 912;
+
 int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A, int64_t lda, double *B,
                 int64_t ldb) {
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
-  const int warps = 8;
-  const unsigned g = (unsigned)cdiv(n, warps);
+  const unsigned g = (unsigned)cdiv(n, LN_WARPS);
   if (lower)
-    left_n_base<true><<<g, 32 * warps, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
+    left_n_base<true><<<g, 32 * LN_WARPS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
   else
-    left_n_base<false><<<g, 32 * warps, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
+    left_n_base<false><<<g, 32 * LN_WARPS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -187,6 +326,15 @@ int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
 int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A, int64_t lda, double *B,
                 int64_t ldb) {
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
+  if (n <= (lower ? SEQ_WARP_MAX : ASC_WARP_MAX)) {
+    const unsigned gw = (unsigned)cdiv(n, TW_WARPS);
+    if (lower)
+      tri_warp<false, false><<<gw, 32 * TW_WARPS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb, c.info);
+    else
+      tri_warp<true, false><<<gw, 32 * TW_WARPS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb, c.info);
+    BOLA_CHECK_LAUNCH();
+    return 0;
+  }
   const unsigned g = (unsigned)cdiv(n, TCOLS);
   if (lower)
     left_t_base<true><<<g, TCOLS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.info);
@@ -256,7 +404,14 @@ right_base_asc32(int64_t m, int n, bool unit, const double *__restrict__ A, int6
 
 template <int V>
 int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64_t lda, double *B, int64_t ldb) {
-  if constexpr (V == 1 || V == 2) {
+  constexpr bool asc = V == 1 || V == 2;
+  if (m <= (!asc ? SEQ_WARP_MAX : n <= 32 ? ASC32_WARP_MAX : ASC_WARP_MAX)) {
+    tri_warp<asc, true><<<(unsigned)cdiv(m, TW_WARPS), 32 * TW_WARPS, 0, c.s>>>((int)n, m, c.unit, V >= 2, A, lda, B, ldb,
+                                                                              1, c.info);
+    BOLA_CHECK_LAUNCH();
+    return 0;
+  }
+  if constexpr (asc) {
     if (n <= 32) {
       right_base_asc32<V><<<(unsigned)cdiv(m, RA_ROWS), RA_THREADS, 0, c.s>>>(m, (int)n, c.unit, A, lda, B, ldb,
                                                                              c.info);
