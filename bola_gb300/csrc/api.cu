@@ -5,6 +5,8 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <set>
+#include <utility>
 
 #include "common.cuh"
 
@@ -82,6 +84,18 @@ struct PoolSlot {
 PoolSlot g_pool_slot[kMaxDevices];
 
 }  // namespace
+
+int roomy(const void *kern) {
+  int dev = 0;
+  BOLA_TRY_CUDA(cudaGetDevice(&dev));
+  static std::mutex mu;
+  static std::set<std::pair<int, const void *>> done;
+  std::lock_guard<std::mutex> lk(mu);
+  if (done.count({dev, kern})) return 0;
+  BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+  done.insert({dev, kern});
+  return 0;
+}
 
 cudaMemPool_t scratch_pool() {
   int dev = 0;

@@ -78,6 +78,17 @@ class Scratch {
   cudaStream_t stream_ = nullptr;
 };
 
+// Asks for all of an SM's shared memory as such for a kernel of the FP64 path
+// (once per kernel and device).  An SM that is set up for the shared memory
+// that one kernel's CTAs take has to run empty before it can take others': a
+// 32 x 32 solve beside a GEMM of 64x64 tiles, depth 64, started after 128 us
+// with each kernel's own setting, @@C us with this one.
+int roomy(const void *kern);
+template <typename... Args>
+int roomy(void (*kern)(Args...)) {
+  return roomy(reinterpret_cast<const void *>(kern));
+}
+
 // ---- internal launchers shared between translation units -------------------
 // Exact DGEMM: per output element, K is walked in chunks of `kc`; each chunk is
 // accumulated from zero with fused multiply-adds in increasing k and added to C
@@ -107,12 +118,11 @@ int getrf2_rec(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, int
 
 // Look-ahead resources of one blocked factorisation: a high-priority stream
 // for the critical path (panels, the next block's columns), a low-priority
-// stream for the rest of each trailing update, events, and two device ints.
+// stream for the rest of each trailing update, and events.
 // Pooled per device, so concurrent callers each take their own set.
 struct LookAhead {
   cudaStream_t sp = nullptr, su = nullptr;
   cudaEvent_t ev[8] = {};
-  int32_t *snap = nullptr;  // device int32[2]
 };
 LookAhead *la_acquire();  // nullptr if the resources cannot be created
 void la_release(LookAhead *la);

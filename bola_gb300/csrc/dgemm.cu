@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(EDGE_T) gemm_edges(const __grid_constant__ Gem
 // All of K in one CTA per tile: the first `big` cells of 64x64 as one tile
 // each, the others as 32x32 and, the last of them, 16x16 blocks.
 template <bool TA, bool TB>
-__global__ void __launch_bounds__(Tile<64>::NT, 2) gemm_grid64(const __grid_constant__ GemmArgs g) {
+__global__ void __maxnreg__(104) gemm_grid64(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) unsigned char smem[stage_bytes<64, 64>()];
   InParallel ip;
   if (stop_flag(g.info)) return;
@@ -693,6 +693,7 @@ int launch_plan(cudaStream_t s, TilePlan &p) {
       attr[cfg.numAttrs].val.clusterDim.y = 1;
       attr[cfg.numAttrs++].val.clusterDim.z = 1;
     }
+    BOLA_TRY(roomy(kern));
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, kern, g));
     beside = true;
     return 0;

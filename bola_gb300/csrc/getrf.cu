@@ -35,6 +35,7 @@ constexpr int PNB = 32;   // panel width: BOLA's NB (src/getrf.rs:11) / recursio
 constexpr int PT = 256;   // threads per CTA in the panel kernel
 constexpr int MAXC = 16;  // largest cluster (non-portable size on sm_103)
 constexpr size_t SMEM_DATA_LIMIT = 200 * 1024;
+constexpr int64_t LOOK_AHEAD_MIN = 512;
 
 struct PanelPub {  // what a CTA publishes to the rest of the cluster each column
   int64_t v;
@@ -185,6 +186,13 @@ panel_lu(double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *inf
   cluster.sync();  // no CTA may leave while another can still read its shared memory
 }
 
+// What a panel leaves for the kernels that follow: its interchanges composed
+// (position q < 32 takes old panel row SRC[q]; old row q < 32 goes to position
+// TO[q], or stays among the first 32 if -1) and the value of *info after it,
+// which those kernels stop on: the next panel, whose zero pivot must not stop
+// them, runs beside them.
+enum { PLAN_SRC = 0, PLAN_TO = PNB, PLAN_STOP = 2 * PNB, PLAN_INTS = 2 * PNB + 16 };
+
 // BOLA's rank-1 step by pivot p (src/getrf2.rs:152-164 with src/ger.rs:28-61):
 // ger walks columns p+1.. in pairs, skipping
 // a pair whose two pivot-row entries are both zero, with the fused vector
@@ -305,7 +313,7 @@ inline size_t panel_smem(int64_t R) {
 template <int RPT>
 __global__ void __launch_bounds__(PAN_T, 1)
 panel_lu_cluster(double *A, int64_t lda, int64_t mp64, int nb, int32_t *ipiv, int32_t *info, int32_t add_on_success,
-                 int32_t col0, int lanes, int64_t R64) {
+                 int32_t col0, int lanes, int64_t R64, int32_t *plan, bool fresh) {
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();
   const int cr = (int)cluster.block_rank();
@@ -319,10 +327,15 @@ panel_lu_cluster(double *A, int64_t lda, int64_t mp64, int nb, int32_t *ipiv, in
   int32_t *spos = reinterpret_cast<int32_t *>(data + PNB * RP);
 
   // Uniform across the cluster: the only writer of *info here acts after
-  // the cluster barrier that every CTA passes after this read.
-  if (stop_flag(info)) return;
+  // the cluster barrier that every CTA passes after this read.  (fresh: the
+  // first panel, which resets *info instead.)
+  if (!fresh && stop_flag(info)) {
+    if (plan != nullptr && cr == 0 && threadIdx.x == 0) plan[PLAN_STOP] = *info;
+    return;
+  }
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (fresh && cr == 0 && tid == 0) *info = 0;
   const int r0 = cr * R, nr = max(0, min(mp, r0 + R) - r0);
   for (int il0 = 0; il0 < nr; il0 += 64) {
     double t[3][2];
@@ -581,7 +594,15 @@ panel_lu_cluster(double *A, int64_t lda, int64_t mp64, int nb, int32_t *ipiv, in
   // where they were: coalesced)
   for (int c = warp; c < nb; c += PAN_T / 32)
     for (int il = lane; il < nr; il += 32) A[spos[il] + (int64_t)c * lda] = data[c * RP + il];
+  if (plan != nullptr) {
+    for (int il = tid; il < nr; il += PAN_T) {
+      const int was = r0 + il, is = spos[il];
+      if (is < steps) plan[PLAN_SRC + is] = was;
+      if (was < steps) plan[PLAN_TO + was] = is < steps ? -1 : is;
+    }
+  }
   cluster.sync();  // no CTA may leave while another can still push into it
+  if (plan != nullptr && cr == 0 && tid == 0) plan[PLAN_STOP] = *(volatile int32_t *)info;
 }
 
 // iterative_getrf2 for a short, wide matrix (m <= 32 rows, any n): one CTA,
@@ -654,56 +675,85 @@ panel_lu_wide(double *A, int64_t lda, int64_t m, int64_t n, int32_t *ipiv, int32
   }
 }
 
-// One getrf block step after the panel: the panel's interchanges applied to
-// all other columns (src/getrf.rs:64-70) and, on the right block row, BOLA's
-// unit-lower trsm base case with its daxpy (src/getrf.rs:78, src/trsm.rs:96-109).
-// A warp per column.
-__global__ void __launch_bounds__(256)
-step_swap_trsm(double *A, int64_t lda, int64_t n, int64_t j, int jb, const int32_t *ipiv,
-               const int32_t *info, int lanes) {
+// The same plan from the panel's ipiv (with its offset j added), for the
+// panel kernels that do not write one.  One warp.
+__global__ void plan_from_ipiv(int jb, const int32_t *ipiv, int32_t j, const int32_t *info, int32_t *plan) {
   __shared__ int64_t rows[2 * PNB], src[2 * PNB];
-  __shared__ double L[PNB * PNB];
-  __shared__ int cnt;
+  const int lane = threadIdx.x;
+  if (lane == 0) plan[PLAN_STOP] = *info;
   if (stop_flag(info)) return;
-  if (threadIdx.x < 32) {
-    SwapPlan p;
-    p.ix0 = j;
-    p.i1 = (int32_t)(j + 1);
-    p.i2 = (int32_t)(j + jb);
-    p.i_inc = 1;
-    p.incx = 1;
-    const int c = compose_swaps_warp(p, ipiv, rows, src);
-    if (threadIdx.x == 0) cnt = c;
+  SwapPlan p;
+  p.ix0 = 0;
+  p.i1 = j + 1;
+  p.i2 = j + jb;
+  p.i_inc = 1;
+  p.incx = 1;
+  const int cnt = compose_swaps_warp(p, ipiv, rows, src);
+  plan[PLAN_SRC + lane] = lane;
+  plan[PLAN_TO + lane] = -1;
+  __syncwarp();
+  for (int t = lane; t < cnt; t += 32) {
+    const int r = (int)(rows[t] - j), f = (int)(src[t] - j);
+    if (r < jb) plan[PLAN_SRC + r] = f;
+    else plan[PLAN_TO + f] = r;
   }
-  for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
-    const int r = e % jb, c = e / jb;
-    L[r + c * PNB] = A[(j + r) + (j + c) * lda];
+}
+
+// One getrf block step after the panel at column j: the panel's interchanges
+// applied to the columns [c0, c0 + ncols) but its own (src/getrf.rs:64-70) and,
+// right of it, BOLA's unit-lower trsm base case with its daxpy
+// (src/getrf.rs:78, src/trsm.rs:96-109).  A warp per column, a lane per row;
+// the chain of a step (broadcast, multiply-add) is what it waits for, with the
+// column's coefficients one step ahead.  Measured at n = 1024: @@S us for all
+// columns (26 with the interchanges composed by every CTA and the solve's votes
+// and loads inside the chain).
+constexpr int SW_WARPS = 4;
+__global__ void __launch_bounds__(32 * SW_WARPS)
+step_swap_trsm(double *A, int64_t lda, int64_t j, int jb, int64_t c0, int64_t ncols, const int32_t *plan, int lanes) {
+  __shared__ double L[PNB * PNB];
+  if (stop_flag(plan + PLAN_STOP)) return;
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * SW_WARPS + (threadIdx.x >> 5);
+  int64_t col = c0 + w;
+  if (col >= j && c0 <= j) col += jb;  // (a range that starts at or left of the panel skips it)
+  const bool on = w < ncols, right = col >= j + jb;
+  double *cp = A + col * lda + j;
+  double b = 0.0, mv = 0.0;
+  int to = -1;
+  if (on && lane < jb) {
+    b = cp[plan[PLAN_SRC + lane]];
+    to = plan[PLAN_TO + lane];
+    if (to >= 0) mv = cp[lane];
+  }
+  for (int e = threadIdx.x; e < PNB * PNB; e += 32 * SW_WARPS) {
+    const int r = e % PNB, c = e / PNB;
+    L[e] = r < jb && c < r ? A[(j + r) + (j + c) * lda] : 0.0;
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= n - jb) return;
-  const int64_t col = w < j ? w : w + jb;
-  double *cp = A + col * lda;
-  const double v0 = lane < cnt ? cp[src[lane]] : 0.0;
-  const double v1 = lane + 32 < cnt ? cp[src[lane + 32]] : 0.0;
-  __syncwarp();
-  if (lane < cnt) cp[rows[lane]] = v0;
-  if (lane + 32 < cnt) cp[rows[lane + 32]] = v1;
-  __syncwarp();
-  if (col < j + jb) return;
-  double b = lane < jb ? cp[j + lane] : 0.0;
-  for (int k = 0; k < jb; ++k) {
-    const double bk = __shfl_sync(0xffffffffu, b, k);
-    if (!nonzero64(bk)) continue;
-    if (lane > k && lane < jb)
-      b = daxpy_elem(b, -bk, L[lane + k * PNB], lane - k - 1, jb - k - 1, lanes);
+  if (!on) return;
+  if (to >= 0) cp[to] = mv;
+  if (right) {
+    double an = L[lane];
+    for (int k = 0; k < jb - 1; ++k) {
+      const double a = an;
+      an = L[lane + (k + 1) * PNB];
+      const double bk = __shfl_sync(0xffffffffu, b, k);
+      if (!nonzero64(bk)) continue;
+      // daxpy over rows k + 1.. with alpha = -b_k: its last len % lanes rows are the unfused tail
+      const int cut = jb - ((jb - k - 1) & (lanes - 1));
+      const double f = __fma_rn(-bk, a, b);
+      if (cut < jb) {
+        const double t = add_prod(b, -bk, a);
+        if (lane > k) b = lane < cut ? f : t;
+      } else if (lane > k) {
+        b = f;
+      }
+    }
   }
-  if (lane < jb) cp[j + lane] = b;
+  if (lane < jb) cp[lane] = b;
 }
 
 __global__ void zero_i32(int32_t *p) { *p = 0; }
-__global__ void copy_i32(const int32_t *src, int32_t *dst) { *dst = *src; }
 
 // Launches a panel on the largest cluster (<= 16 CTAs) the device can
 // co-schedule: about 64 rows per CTA, so that the update warps (32 columns x
@@ -711,7 +761,7 @@ __global__ void copy_i32(const int32_t *src, int32_t *dst) { *dst = *src; }
 // (0.6 us); more rows per CTA once 16 CTAs are in use.  Rows that do not fit
 // in shared memory (mp > 12k) stay in global memory (panel_lu).
 int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int32_t *ipiv, int32_t *info,
-                 int32_t add_on_success, int32_t col0) {
+                 int32_t add_on_success, int32_t col0, int32_t *plan = nullptr, bool fresh = false) {
   double fl = 0.0;
   for (int j = 0; j < nb && j < mp; ++j) fl += (double)(mp - j - 1) * (1.0 + 2.0 * (nb - j - 1));
   ProfScope prof(s, "getrf_panel", fl, 16.0 * (double)mp * nb);
@@ -721,11 +771,13 @@ int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int
     const int64_t R = cdiv(mp, C);
     const bool use_smem = panel_smem(R) <= SMEM_DATA_LIMIT;
     const size_t smem = use_smem ? panel_smem(R) : panel_base_bytes();
-    const int rpt = R <= PIV_T ? 0 : R <= 2 * PIV_T ? 1 : R <= 4 * PIV_T ? 2 : 3;
-    void (*const kerns[5])(double *, int64_t, int64_t, int, int32_t *, int32_t *, int32_t, int32_t, int, int64_t) = {
-        panel_lu_cluster<1>, panel_lu_cluster<2>, panel_lu_cluster<4>, panel_lu_cluster<7>, panel_lu};
-    const int ki = use_smem ? rpt : 4;
-    auto kern = kerns[ki];
+    void (*const cluster_kern)(double *, int64_t, int64_t, int, int32_t *, int32_t *, int32_t, int32_t, int, int64_t,
+                               int32_t *, bool) = R <= PIV_T       ? panel_lu_cluster<1>
+                                                  : R <= 2 * PIV_T ? panel_lu_cluster<2>
+                                                  : R <= 4 * PIV_T ? panel_lu_cluster<4>
+                                                                   : panel_lu_cluster<7>;
+    const void *kern = use_smem ? reinterpret_cast<const void *>(cluster_kern) : reinterpret_cast<const void *>(panel_lu);
+    const int ki = !use_smem ? 0 : R <= PIV_T ? 1 : R <= 2 * PIV_T ? 2 : R <= 4 * PIV_T ? 3 : 4;
     BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_DATA_LIMIT));
     BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     cudaLaunchConfig_t cfg = {};
@@ -755,7 +807,15 @@ int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int
     }
     if (known.load(std::memory_order_relaxed) < 0) continue;
     const int lanes_v = lanes();
-    BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, kern, A, lda, mp, nb, ipiv, info, add_on_success, col0, lanes_v, R));
+    if (use_smem) {
+      BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, cluster_kern, A, lda, mp, nb, ipiv, info, add_on_success, col0, lanes_v, R,
+                                       plan, fresh));
+      return 0;
+    }
+    if (fresh) zero_i32<<<1, 1, 0, s>>>(info);
+    BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, panel_lu, A, lda, mp, nb, ipiv, info, add_on_success, col0, lanes_v, R));
+    if (plan != nullptr) plan_from_ipiv<<<1, 32, 0, s>>>((int)imin(nb, mp), ipiv, add_on_success, info, plan);
+    BOLA_CHECK_LAUNCH();
     return 0;
   }
 }
@@ -815,8 +875,7 @@ LookAhead *la_acquire() {
   int least = 0, greatest = 0;
   bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
             cudaStreamCreateWithPriority(&la->sp, cudaStreamNonBlocking, greatest) == cudaSuccess &&
-            cudaStreamCreateWithPriority(&la->su, cudaStreamNonBlocking, least) == cudaSuccess &&
-            cudaMalloc(&la->snap, 2 * sizeof(int32_t)) == cudaSuccess;
+            cudaStreamCreateWithPriority(&la->su, cudaStreamNonBlocking, least) == cudaSuccess;
   for (cudaEvent_t &e : la->ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
   if (!ok) return nullptr;  // (leaks the partial set; only on a failing device)
   return la;
@@ -829,96 +888,94 @@ void la_release(LookAhead *la) {
   g_la_pool[dev & 63].push_back(la);
 }
 
-// BOLA's blocked getrf (src/getrf.rs:37-101) with look-ahead.  Per step k:
-// panel, swaps + trsm, and the update of the next panel's 32 columns on sp;
-// the update of the other columns on su, overlapping panel k+1 (whose swaps
-// wait for it).  Splitting the trailing DGEMM at a column multiple of 4 keeps
-// BOLA's 8x4 edge-tile classification, so every element is computed exactly
-// as in one call.  The wide update stops on its own step's snapshot of
-// *info: a zero pivot found by panel k+1 while it runs must not cut short
-// step k's update, which BOLA completes before factoring panel k+1.
+// BOLA's blocked getrf (src/getrf.rs:37-101) with look-ahead.  Per step k, on
+// the high-priority stream sp: the panel, then the interchanges, trsm and
+// update of the next panel's 32 columns; on su, once the panel is done: the
+// interchanges and trsm of all other columns and the update of those right of
+// the next panel, overlapping panel k + 1 (whose columns wait for it).
+// Splitting the trailing DGEMM at a column multiple of 4 keeps BOLA's 8x4
+// edge-tile classification, so every element is computed exactly as in one
+// call.  Everything after a panel stops on the panel's own record of *info
+// (PLAN_STOP): a zero pivot found by panel k + 1 while step k's wide update
+// runs must not cut that short, which BOLA completes before factoring panel
+// k + 1.
+int swap_columns(cudaStream_t s, double *A, int64_t lda, int64_t j, int jb, int64_t c0, int64_t ncols, int64_t nright,
+                 const int32_t *plan) {
+  if (ncols <= 0) return 0;
+  ProfScope prof(s, "getrf_swap_trsm", (double)jb * (jb - 1) * (double)nright, 32.0 * jb * (double)ncols);
+  BOLA_TRY(roomy(step_swap_trsm));
+  step_swap_trsm<<<(unsigned)cdiv(ncols, SW_WARPS), 32 * SW_WARPS, 0, s>>>(A, lda, j, jb, c0, ncols, plan, lanes());
+  BOLA_CHECK_LAUNCH();
+  return 0;
+}
+
 int getrf_blocked(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, int32_t *ipiv, int32_t *info) {
   const int64_t min_mn = imin(m, n);
+  if (m == 0 || n == 0 || PNB >= min_mn) {
+    ProfScope prof(s, "info_init");
+    zero_i32<<<1, 1, 0, s>>>(info);
+    BOLA_CHECK_LAUNCH();
+    return m == 0 || n == 0 ? 0 : getrf2_rec(s, m, n, A, lda, ipiv, info, 0);
+  }
+  Scratch plans;
+  BOLA_TRY(plans.alloc((size_t)cdiv(min_mn, PNB) * PLAN_INTS * sizeof(int32_t), s));
   // look-ahead pays from a few hundred columns on; below that its events and
   // the extra launches cost more than the overlap saves
-  LookAhead *la = (m > 0 && n > 0 && min_mn >= 512) ? la_acquire() : nullptr;
-  if (!la) {
-    {
-      ProfScope prof(s, "info_init");
-      zero_i32<<<1, 1, 0, s>>>(info);
-    }
-    BOLA_CHECK_LAUNCH();
-    if (m == 0 || n == 0) return 0;
-    if (PNB >= min_mn) return getrf2_rec(s, m, n, A, lda, ipiv, info, 0);
-    for (int64_t j = 0; j < min_mn; j += PNB) {
-      const int jb = (int)imin(PNB, min_mn - j);
-      BOLA_TRY(launch_panel(s, A + j + j * lda, lda, m - j, jb, ipiv + j, info, (int32_t)j, (int32_t)j));
-      const int64_t others = n - jb;
-      if (others > 0) {
-        ProfScope prof(s, "getrf_swap_trsm", (double)jb * (jb - 1) * (double)(n - j - jb), 32.0 * jb * (double)others);
-        step_swap_trsm<<<(unsigned)cdiv(others, 8), 256, 0, s>>>(A, lda, n, j, jb, ipiv, info, lanes());
-        BOLA_CHECK_LAUNCH();
-      }
-      if (j + jb < n && j + jb < m) {
-        BOLA_TRY(dgemm_exact(s, 'N', 'N', m - j - jb, n - j - jb, jb, -1.0, A + (j + jb) + j * lda, lda,
-                             A + j + (j + jb) * lda, lda, 1.0, A + (j + jb) + (j + jb) * lda, lda, 64, info, 0));
-      }
-    }
-    return 0;
-  }
-  int st = 0;
+  LookAhead *la = min_mn >= LOOK_AHEAD_MIN ? la_acquire() : nullptr;
+  cudaStream_t sp = la ? la->sp : s, su = la ? la->su : s;
   auto run = [&]() -> int {
-    BOLA_TRY_CUDA(cudaEventRecord(la->ev[0], s));
-    BOLA_TRY_CUDA(cudaStreamWaitEvent(la->sp, la->ev[0], 0));
-    BOLA_TRY_CUDA(cudaStreamWaitEvent(la->su, la->ev[0], 0));
-    {
-      ProfScope prof(la->sp, "info_init");
-      zero_i32<<<1, 1, 0, la->sp>>>(info);
+    if (la) {
+      BOLA_TRY_CUDA(cudaEventRecord(la->ev[0], s));
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(sp, la->ev[0], 0));
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(su, la->ev[0], 0));
     }
-    BOLA_CHECK_LAUNCH();
     bool wide_pending = false;
     for (int64_t j = 0, k = 0; j < min_mn; j += PNB, ++k) {
       const int jb = (int)imin(PNB, min_mn - j);
-      BOLA_TRY(launch_panel(la->sp, A + j + j * lda, lda, m - j, jb, ipiv + j, info, (int32_t)j, (int32_t)j));
-      if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(la->sp, la->ev[2], 0));
-      wide_pending = false;
-      const int64_t others = n - jb;
-      if (others > 0) {
-        ProfScope prof(la->sp, "getrf_swap_trsm", (double)jb * (jb - 1) * (double)(n - j - jb),
-                       32.0 * jb * (double)others);
-        step_swap_trsm<<<(unsigned)cdiv(others, 8), 256, 0, la->sp>>>(A, lda, n, j, jb, ipiv, info, lanes());
-        BOLA_CHECK_LAUNCH();
-      }
-      if (!(j + jb < n && j + jb < m)) continue;
+      int32_t *plan = plans.as<int32_t>() + k * PLAN_INTS, *stop = plan + PLAN_STOP;
+      BOLA_TRY(launch_panel(sp, A + j + j * lda, lda, m - j, jb, ipiv + j, info, (int32_t)j, (int32_t)j, plan, j == 0));
       const int64_t m2 = m - j - jb, n2 = n - j - jb;
-      const int64_t nb_next = imin((int64_t)PNB, n2);  // a multiple of 4 unless it is all of n2
       const double *A21 = A + (j + jb) + j * lda, *A12 = A + j + (j + jb) * lda;
       double *A22 = A + (j + jb) + (j + jb) * lda;
-      BOLA_TRY(dgemm_exact(la->sp, 'N', 'N', m2, nb_next, jb, -1.0, A21, lda, A12, lda, 1.0, A22, lda, 64, info, 0));
-      if (n2 > nb_next) {
-        int32_t *snap = la->snap + (k & 1);
-        copy_i32<<<1, 1, 0, la->sp>>>(info, snap);
-        BOLA_CHECK_LAUNCH();
-        BOLA_TRY_CUDA(cudaEventRecord(la->ev[1], la->sp));
-        BOLA_TRY_CUDA(cudaStreamWaitEvent(la->su, la->ev[1], 0));
-        BOLA_TRY(dgemm_exact(la->su, 'N', 'N', m2, n2 - nb_next, jb, -1.0, A21, lda, A12 + nb_next * lda, lda, 1.0,
-                             A22 + nb_next * lda, lda, 64, snap, 0));
-        BOLA_TRY_CUDA(cudaEventRecord(la->ev[2], la->su));
-        wide_pending = true;
+      if (!la) {
+        BOLA_TRY(swap_columns(s, A, lda, j, jb, 0, n - jb, n2, plan));
+        if (m2 > 0 && n2 > 0)
+          BOLA_TRY(dgemm_exact(s, 'N', 'N', m2, n2, jb, -1.0, A21, lda, A12, lda, 1.0, A22, lda, 64, stop, 0));
+        continue;
       }
+      BOLA_TRY_CUDA(cudaEventRecord(la->ev[1], sp));
+      const int64_t nn = imin((int64_t)PNB, n2);  // the next panel's columns: a multiple of 4 unless all of n2
+      if (n2 > 0) {
+        if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(sp, la->ev[2], 0));
+        BOLA_TRY(swap_columns(sp, A, lda, j, jb, j + jb, nn, nn, plan));
+        if (m2 > 0)
+          BOLA_TRY(dgemm_exact(sp, 'N', 'N', m2, nn, jb, -1.0, A21, lda, A12, lda, 1.0, A22, lda, 64, stop, 0));
+      }
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(su, la->ev[1], 0));
+      BOLA_TRY(swap_columns(su, A, lda, j, jb, j + jb + nn, n2 - nn, n2 - nn, plan));
+      if (n2 > nn && m2 > 0)
+        BOLA_TRY(dgemm_exact(su, 'N', 'N', m2, n2 - nn, jb, -1.0, A21, lda, A12 + nn * lda, lda, 1.0, A22 + nn * lda, lda,
+                             64, stop, 0));
+      BOLA_TRY_CUDA(cudaEventRecord(la->ev[2], su));
+      wide_pending = true;
+      BOLA_TRY(swap_columns(su, A, lda, j, jb, 0, j, 0, plan));  // the finished columns, read by nothing later
     }
-    if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(la->sp, la->ev[2], 0));
-    BOLA_TRY_CUDA(cudaEventRecord(la->ev[3], la->sp));
-    BOLA_TRY_CUDA(cudaStreamWaitEvent(s, la->ev[3], 0));
+    if (la) {
+      BOLA_TRY_CUDA(cudaEventRecord(la->ev[3], su));
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(sp, la->ev[3], 0));
+      BOLA_TRY_CUDA(cudaEventRecord(la->ev[4], sp));
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(s, la->ev[4], 0));
+    }
     return 0;
   };
-  st = run();
-  if (st != 0) {
-    // leave nothing of this call running on the look-ahead streams
-    cudaStreamSynchronize(la->sp);
-    cudaStreamSynchronize(la->su);
+  const int st = run();
+  if (la) {
+    if (st != 0) {  // leave nothing of this call running on the look-ahead streams
+      cudaStreamSynchronize(la->sp);
+      cudaStreamSynchronize(la->su);
+    }
+    la_release(la);
   }
-  la_release(la);
   return st;
 }
 

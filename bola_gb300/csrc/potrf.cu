@@ -423,6 +423,7 @@ int syrk_exact(cudaStream_t s, char uplo, char trans, int64_t n, int64_t k, doub
                          info, upper ? 1 : 2));
   }
   ProfScope prof(s, "syrk_diag", (double)imin(n, NB) * (imin(n, NB) + 1) * (double)k * (double)cdiv(n, NB));
+  BOLA_TRY(roomy(syrk_diag));
   syrk_diag<<<dim3(NB, (unsigned)cdiv(n, NB)), NB, 0, s>>>(upper, tt, n, k, alpha, A, lda, C, ldc, lanes(), info);
   BOLA_CHECK_LAUNCH();
   return 0;
@@ -433,6 +434,7 @@ int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int
   if (n == 0) return 0;
   if (n <= NB) {
     ProfScope prof(s, "potrf2_block", (double)n * n * n / 3.0);
+    BOLA_TRY(roomy(potrf2_block));
     potrf2_block<<<1, P2_T, 0, s>>>(upper, (int)n, A, lda, info, col0, lanes());
     BOLA_CHECK_LAUNCH();
     return 0;
@@ -459,6 +461,7 @@ int advance_diag(cudaStream_t s, bool upper, int64_t nt, const double *src, int6
                  const int32_t *info) {
   if (nt <= 0) return 0;
   ProfScope prof(s, "syrk_diag", (double)NB * (NB + 1) * (double)NB * (double)cdiv(nt, NB));
+  BOLA_TRY(roomy(syrk_diag));
   syrk_diag<<<dim3(NB, (unsigned)cdiv(nt, NB)), NB, 0, s>>>(upper, upper, nt, NB, -1.0, src, lda, C, lda, lan, info);
   BOLA_CHECK_LAUNCH();
   return 0;

@@ -298,6 +298,67 @@ right_base(int64_t m, int n, bool unit, const double *__restrict__ A, int64_t ld
   }
 }
 
+// The ascending base cases (ltu, rnu, rtl) for n <= 32 and many systems: as in
+// tri_warp, but eight lanes per system, lane q holding unknowns q, q + 8, ...
+// in registers, so that four systems share a warp's instructions.  (Four lanes
+// per system issue a quarter less in all, but 550 FP64 instructions on a
+// warp's path instead of 170; beside a GEMM, whose sixteen warps an SM queue on
+// the same pipe, that made 126 us of one block column's solve at n = 4096.)
+constexpr int AL = 8;  // lanes per system
+constexpr int AS_THREADS = 64;
+constexpr int AS_SYS = AS_THREADS / AL;
+
+template <bool RIGHT>
+__global__ void __launch_bounds__(AS_THREADS)
+tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
+          int64_t elem, int64_t sys, const int32_t *info) {
+  __shared__ double T[32 * 33];  // coefficient of x_k in equation j at T[k * 33 + j]
+  __shared__ Divisor dv[32];
+  if (stop_flag(info)) return;
+  for (int e = threadIdx.x; e < n * n; e += AS_THREADS) {
+    const int r = e % n, c = e / n;
+    T[transposed ? c * 33 + r : r * 33 + c] = A[r + (int64_t)c * lda];
+  }
+  __syncthreads();
+  if (!unit && threadIdx.x < n) dv[threadIdx.x] = divisor(T[threadIdx.x * 34]);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  // lanes of a system: consecutive along the elements where those are
+  // contiguous (left), else along the systems (right: the rows of B)
+  const int q = RIGHT ? lane / (32 / AL) : lane & (AL - 1), w = RIGHT ? lane & (32 / AL - 1) : lane / AL;
+  const int64_t s = (int64_t)blockIdx.x * AS_SYS + (threadIdx.x >> 5) * (32 / AL) + w;
+  const bool on = s < systems;  // lanes of a missing system still take part in the shuffles
+  double *b = B + s * sys;
+  double x[32 / AL];
+#pragma unroll
+  for (int c = 0; c < 32 / AL; ++c) x[c] = on && q + AL * c < n ? b[(q + AL * c) * elem] : 0.0;
+#pragma unroll
+  for (int k = 0; k < 32; ++k) {
+    if (k < n) {
+      if (!unit && q == (k & (AL - 1))) x[k / AL] = RIGHT ? __dmul_rn(x[k / AL], dv[k].y) : div_rn(x[k / AL], dv[k]);
+      const int src = RIGHT ? (k & (AL - 1)) * (32 / AL) + w : w * AL + (k & (AL - 1));
+      const double xk = __shfl_sync(0xffffffffu, x[k / AL], src);
+#pragma unroll
+      for (int c = k / AL; c < 32 / AL; ++c) {  // (earlier unknowns are done)
+        const int j = q + AL * c;
+        const double a = T[k * 33 + j];
+        const double u = sub_prod(x[c], a, xk);
+        if (j > k && j < n && (!RIGHT || nonzero64(a))) x[c] = u;  // right: BOLA skips a zero a
+      }
+    }
+  }
+  if (!on) return;
+#pragma unroll
+  for (int c = 0; c < 32 / AL; ++c)
+    if (q + AL * c < n) b[(q + AL * c) * elem] = x[c];
+}
+
+// Up to how many systems a warp each (tri_warp) beats a thread each: the warps
+// of one SM share its FP64 pipe (n = 64: ~27 cycles of the GPU per ascending
+// system, ~210 per descending one, against 280k cycles for any number of
+// threads; rows of at most 32 columns over 4 lanes take ~24k cycles.
+constexpr int64_t ASC_WARP_MAX = 8192, SEQ_WARP_MAX = 1216, ASC32_WARP_MAX = 912;
+
 struct Ctx {
   cudaStream_t s;
   bool unit;
@@ -305,16 +366,11 @@ struct Ctx {
   const int32_t *info;
 };
 
-// Up to how many systems a warp each (tri_warp) beats a thread each: the warps
-// of one SM share its FP64 pipe (n = 64: ~27 cycles of the GPU per ascending
-// system, ~210 per descending one, against 280k cycles for any number of
-// threads); rows of at most 32 columns over 4 lanes take ~24k cycles.
-constexpr int64_t ASC_WARP_MAX = 8192, SEQ_WARP_MAX = 1216, ASC32_WARP_MAX = 912;
-
 int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A, int64_t lda, double *B,
                 int64_t ldb) {
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
   const unsigned g = (unsigned)cdiv(n, LN_WARPS);
+  BOLA_TRY(roomy(lower ? left_n_base<true> : left_n_base<false>));
   if (lower)
     left_n_base<true><<<g, 32 * LN_WARPS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
   else
@@ -326,8 +382,16 @@ int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
 int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A, int64_t lda, double *B,
                 int64_t ldb) {
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
+  if (!lower && m <= 32 && n > ASC32_WARP_MAX) {
+    BOLA_TRY(roomy(tri_asc32<false>));
+    tri_asc32<false><<<(unsigned)cdiv(n, AS_SYS), AS_THREADS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb,
+                                                                        c.info);
+    BOLA_CHECK_LAUNCH();
+    return 0;
+  }
   if (n <= (lower ? SEQ_WARP_MAX : ASC_WARP_MAX)) {
     const unsigned gw = (unsigned)cdiv(n, TW_WARPS);
+    BOLA_TRY(roomy(lower ? tri_warp<false, false> : tri_warp<true, false>));
     if (lower)
       tri_warp<false, false><<<gw, 32 * TW_WARPS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb, c.info);
     else
@@ -344,68 +408,11 @@ int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
   return 0;
 }
 
-// The ascending right base cases (rnu, rtl) for n <= 32, right-looking: once
-// b_k is final it is subtracted from every later column of the row, so each
-// b_j still receives its updates in ascending k and then its scale, exactly as
-// in BOLA's column sweep.  A row is spread over RL = 4 lanes, lane q holding
-// columns q, q+4, ..., q+28 in registers: b_k is finished by its lane and
-// broadcast by a shuffle, and each lane updates its own later columns.  The
-// FP64 pipe retires a warp instruction in the same time whether 1 or 32 lanes
-// work, and a row's work is one dependent sweep; spreading a row over 4 lanes
-// cuts the instructions on a warp's path about 3.5-fold.
-constexpr int RL = 4;             // lanes per row
-constexpr int RA_THREADS = 64;    // 16 rows per CTA
-constexpr int RA_ROWS = RA_THREADS / RL;
-
-template <int V>
-__global__ void __launch_bounds__(RA_THREADS)
-right_base_asc32(int64_t m, int n, bool unit, const double *__restrict__ A, int64_t lda, double *B, int64_t ldb,
-                 const int32_t *info) {
-  static_assert(V == 1 || V == 2, "ascending variants only");
-  __shared__ double sA[32 * 33];  // a(r, c) at sA[r + 33 c]
-  __shared__ double rd[32];
-  if (stop_flag(info)) return;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) sA[(e % n) + (e / n) * 33] = A[(e % n) + (int64_t)(e / n) * lda];
-  __syncthreads();
-  if (!unit && threadIdx.x < n) rd[threadIdx.x] = 1.0 / sA[threadIdx.x * 34];
-  __syncthreads();
-  const int lane = threadIdx.x & 31, q = lane & (RL - 1), base = lane & ~(RL - 1);
-  const int64_t i = (int64_t)blockIdx.x * RA_ROWS + threadIdx.x / RL;
-  const bool row = i < m;  // lanes of a missing row still take part in the shuffles
-  double b[32 / RL];
-#pragma unroll
-  for (int c = 0; c < 32 / RL; ++c) {
-    const int j = q + RL * c;
-    b[c] = (row && j < n) ? B[i + (int64_t)j * ldb] : 0.0;
-  }
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    if (k < n) {
-      if (!unit && q == (k & (RL - 1))) b[k / RL] = __dmul_rn(b[k / RL], rd[k]);
-      const double bk = __shfl_sync(0xffffffffu, b[k / RL], base + (k & (RL - 1)));
-#pragma unroll
-      for (int c = 0; c < 32 / RL; ++c) {
-        const int j = q + RL * c;
-        if (j > k && j < n) {
-          const double a = (V == 1) ? sA[k + j * 33] : sA[j + k * 33];  // rnu: a(k, j); rtl: a(j, k)
-          const double u = sub_prod(b[c], a, bk);
-          b[c] = nonzero64(a) ? u : b[c];  // BOLA skips a zero a
-        }
-      }
-    }
-  }
-  if (!row) return;
-#pragma unroll
-  for (int c = 0; c < 32 / RL; ++c) {
-    const int j = q + RL * c;
-    if (j < n) B[i + (int64_t)j * ldb] = b[c];
-  }
-}
-
 template <int V>
 int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64_t lda, double *B, int64_t ldb) {
   constexpr bool asc = V == 1 || V == 2;
   if (m <= (!asc ? SEQ_WARP_MAX : n <= 32 ? ASC32_WARP_MAX : ASC_WARP_MAX)) {
+    BOLA_TRY(roomy(tri_warp<asc, true>));
     tri_warp<asc, true><<<(unsigned)cdiv(m, TW_WARPS), 32 * TW_WARPS, 0, c.s>>>((int)n, m, c.unit, V >= 2, A, lda, B, ldb,
                                                                               1, c.info);
     BOLA_CHECK_LAUNCH();
@@ -413,14 +420,16 @@ int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64
   }
   if constexpr (asc) {
     if (n <= 32) {
-      right_base_asc32<V><<<(unsigned)cdiv(m, RA_ROWS), RA_THREADS, 0, c.s>>>(m, (int)n, c.unit, A, lda, B, ldb,
-                                                                             c.info);
+      BOLA_TRY(roomy(tri_asc32<true>));
+      tri_asc32<true><<<(unsigned)cdiv(m, AS_SYS), AS_THREADS, 0, c.s>>>((int)n, m, c.unit, V >= 2, A, lda, B, ldb, 1,
+                                                                         c.info);
       BOLA_CHECK_LAUNCH();
       return 0;
     }
   }
   const size_t smem = right_base_smem((int)n);
   if (smem > 48 * 1024) BOLA_TRY_CUDA(cudaFuncSetAttribute(right_base<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  BOLA_TRY(roomy(right_base<V>));
   right_base<V><<<(unsigned)cdiv(m, RB_ROWS), RB_ROWS, smem, c.s>>>(m, (int)n, c.unit, A, lda, B, ldb, c.info);
   BOLA_CHECK_LAUNCH();
   return 0;
