@@ -29,7 +29,9 @@ namespace {
 constexpr int CNB = 64;  // panel width = update depth
 
 __device__ __forceinline__ float sqrtT(float x) { return sqrtf(x); }
-__device__ __forceinline__ double sqrtT(double x) { return sqrt(x); }
+__device__ __forceinline__ double sqrtT(double x) { return sqrt_rn(x); }
+__device__ __forceinline__ float recipT(float x) { return 1.f / x; }
+__device__ __forceinline__ double recipT(double x) { return recip_rn(x); }
 __device__ __forceinline__ bool positive(float x) { return x > 0.f && x <= 3.4e38f; }
 __device__ __forceinline__ bool positive(double x) { return x > 0.0 && x <= 1.7e308; }
 
@@ -42,55 +44,108 @@ __device__ __forceinline__ bool factor_stopped(const int32_t *info, const uint64
 // global 1-based column, and every later kernel of the factorisation returns
 // at once.  Tracks max/min of L_kk^2 (the U diagonal of the LU form) and
 // gives up as the LU panel does.
+//
+// Bound by the chain of a column (square root, reciprocal, scale, the next
+// column's update): one warp walks it, two rows per lane, while eight warps
+// apply each finished column to the columns after the next one.  Measured on
+// one GB300 with L21 of 1400 rows after it: @@D us a panel in FP32 (82 with
+// three CTA barriers a column and a division per updated element's index).
+constexpr int CH_UPD = 8;
+constexpr int CH_T = 32 * (1 + CH_UPD);
+constexpr int CHP = CNB + 1;  // pitch: column j of row i at a[j * CHP + i]
+enum { CH_UPDATED = 1, CH_SCALED = 2 };
+__device__ __forceinline__ void ch_sync(int id) {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(CH_T) : "memory");
+}
+__device__ __forceinline__ void ch_arrive(int id) {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(CH_T) : "memory");
+}
 template <typename T>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(CH_T)
 chol_dblock(T *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, uint64_t *track, double give_up) {
-  __shared__ T a[CNB][CNB + 1];
-  __shared__ T dinv;
+  __shared__ T a[CNB * CHP];
   __shared__ int stop;
-  if (threadIdx.x == 0) stop = factor_stopped(info, track) ? 1 : 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if (tid == 0) stop = factor_stopped(info, track) ? 1 : 0;
   __syncthreads();
   if (stop) return;
-  for (int e = threadIdx.x; e < CNB * CNB; e += blockDim.x) {
+  for (int e = tid; e < CNB * CNB; e += CH_T) {
     const int i = e % CNB, j = e / CNB;
-    a[i][j] = (i < jb && j < jb && i >= j) ? W[i + j * ldw] : T(0);
+    a[j * CHP + i] = (i < jb && j < jb && i >= j) ? W[i + j * ldw] : T(0);
   }
   __syncthreads();
-  double umax = 0.0, umin = INFINITY;
-  int k = 0;
-  for (; k < jb; ++k) {
-    if (threadIdx.x == 0) {
-      const T akk = a[k][k];
-      if (!positive(akk)) {
-        stop = 1;
-        atomicCAS(info, 0, col0 + k + 1);
-      } else {
-        const T d = sqrtT(akk);
-        a[k][k] = d;
-        dinv = T(1) / d;
-        umax = fmax(umax, (double)akk);
-        umin = fmin(umin, (double)akk);
+  T umax = T(0), umin = T(INFINITY);
+  if (warp == 0) {
+    T c[2] = {a[lane], a[lane + 32]};
+    for (int l = 0; l < jb; ++l) {
+      const T d = __shfl_sync(0xffffffffu, l < 32 ? c[0] : c[1], l & 31);
+      if (!positive(d)) {
+        if (lane == 0) {
+          stop = 1;
+          atomicCAS(info, 0, col0 + l + 1);
+        }
+        ch_arrive(CH_SCALED);
+        break;
+      }
+      const T r = sqrtT(d), inv = recipT(r);
+      T x[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int i = lane + 32 * h;
+        x[h] = i == l ? r : c[h] * inv;
+        if (i >= l) a[l * CHP + i] = x[h];
+      }
+      umax = d > umax ? d : umax;
+      umin = d < umin ? d : umin;
+      ch_sync(CH_UPDATED);  // column l - 1 is applied everywhere
+      const int nx = l + 1 < jb ? l + 1 : l;
+      c[0] = a[nx * CHP + lane];
+      c[1] = a[nx * CHP + lane + 32];
+      ch_arrive(CH_SCALED);
+      const T xj = __shfl_sync(0xffffffffu, nx < 32 ? x[0] : x[1], nx & 31);
+      c[0] = fmaT(-x[0], xj, c[0]);
+      c[1] = fmaT(-x[1], xj, c[1]);
+    }
+  } else {
+    for (int l = 0; l < jb; ++l) {
+      ch_arrive(CH_UPDATED);
+      ch_sync(CH_SCALED);
+      if (stop) break;
+      const T *xl = a + l * CHP;
+      const T x0 = xl[lane], x1 = xl[lane + 32];
+      for (int j0 = l + 1 + warp; j0 < jb; j0 += 4 * CH_UPD) {
+        T v[4], w[4], xj[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * CH_UPD < jb ? j0 + u * CH_UPD : jb - 1;
+          v[u] = a[j * CHP + lane];
+          w[u] = a[j * CHP + lane + 32];
+          xj[u] = xl[j];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * CH_UPD;
+          if (j >= jb) break;
+          if (j < 32) {
+            const T t = fmaT(-x0, xj[u], v[u]);
+            if (lane >= j) a[j * CHP + lane] = t;
+          }
+          const T t = fmaT(-x1, xj[u], w[u]);
+          if (lane + 32 >= j) a[j * CHP + lane + 32] = t;
+        }
       }
     }
-    __syncthreads();
-    if (stop) break;
-    const T di = dinv;
-    for (int i = k + 1 + (int)threadIdx.x; i < jb; i += blockDim.x) a[i][k] *= di;
-    __syncthreads();
-    const int m = jb - k - 1;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-      const int i = k + 1 + e % m, j = k + 1 + e / m;
-      if (i >= j) a[i][j] = fmaT(-a[i][k], a[j][k], a[i][j]);
-    }
-    __syncthreads();
   }
-  for (int e = threadIdx.x; e < jb * jb; e += blockDim.x) {
+  __syncthreads();
+  for (int e = tid; e < jb * jb; e += CH_T) {
     const int i = e % jb, j = e / jb;
-    if (i >= j) W[i + j * ldw] = a[i][j];
+    if (i >= j) W[i + j * ldw] = a[j * CHP + i];
   }
-  if (threadIdx.x == 0 && track != nullptr && !stop) {
+  if (tid == 0 && track != nullptr && !stop) {
     // the U diagonal of the LU form is L_kk^2 = the pivots: their running extent and the give-up test
-    const uint64_t mx = (uint64_t)__double_as_longlong(umax), mn = (uint64_t)__double_as_longlong(umin);
+    const uint64_t mx = (uint64_t)__double_as_longlong((double)umax), mn = (uint64_t)__double_as_longlong((double)umin);
     if (mx > track[0]) track[0] = mx;
     if (mn < track[1]) track[1] = mn;
     const double gmx = __longlong_as_double((long long)track[0]), gmn = __longlong_as_double((long long)track[1]);
@@ -99,41 +154,73 @@ chol_dblock(T *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, u
   }
 }
 
-// L21 = W21 L11^-T for the rows jb..mp-1 of the panel (one thread per row,
-// its 64 values in registers, L11 in shared memory), written back to W and
-// as row (row - jb) of the update's K-major operand.
-template <typename T, int CR>
-__global__ void __launch_bounds__(CR)
+// L21 = W21 L11^-T for the rows jb..mp-1 of the panel (one thread per row),
+// written back to W and as row (row - jb) of the update's K-major operand.
+// Eight columns at a time: their eight sums, in registers, take the earlier
+// columns in order from shared memory (one value of the row's and eight of
+// L11's per step), then each other; so eight chains are in flight and the loop
+// stays in the instruction cache, where 64 columns unrolled into one chain each
+// did neither.
+template <typename T>
+struct alignas(16) Vec8 {
+  T v[8];
+};
+constexpr int L21_T = 64;
+template <typename T>
+constexpr size_t l21_smem() {
+  return sizeof(T) * (CNB * CNB + CNB + CNB * L21_T);
+}
+template <typename T>
+__global__ void __launch_bounds__(L21_T)
 chol_l21(T *W, int64_t ldw, int64_t mp, int jb, int kind, void *aop, float *aop_lo, int32_t *aexp, int64_t cap,
          const int32_t *info, const uint64_t *track) {
-  __shared__ T L[CNB][CNB + 1];
-  __shared__ T rd[CNB];
+  extern __shared__ __align__(16) unsigned char l21_raw[];
+  T *Lt = reinterpret_cast<T *>(l21_raw);  // L(k, q) at Lt[q * CNB + k]
+  T *rd = Lt + CNB * CNB;
+  T *vs = rd + CNB + threadIdx.x;  // this thread's value k at vs[k * L21_T]
   __shared__ int stop;
   if (threadIdx.x == 0) stop = factor_stopped(info, track) ? 1 : 0;
   __syncthreads();
   if (stop) return;
-  for (int e = threadIdx.x; e < CNB * CNB; e += CR) {
+  for (int e = threadIdx.x; e < CNB * CNB; e += L21_T) {
     const int i = e % CNB, j = e / CNB;
-    L[i][j] = (i < jb && j < jb && i >= j) ? W[i + j * ldw] : T(0);
+    Lt[e] = (i < jb && j < jb && i >= j) ? W[i + j * ldw] : T(0);
   }
+  const int64_t row = jb + (int64_t)blockIdx.x * L21_T + threadIdx.x;
+#pragma unroll 16
+  for (int k = 0; k < CNB; ++k) vs[k * L21_T] = k < jb && row < mp ? W[row + k * ldw] : T(0);
   __syncthreads();
-  for (int k = threadIdx.x; k < CNB; k += CR) rd[k] = k < jb ? T(1) / L[k][k] : T(0);
+  for (int k = threadIdx.x; k < CNB; k += L21_T) rd[k] = k < jb ? recipT(Lt[k * (CNB + 1)]) : T(0);
   __syncthreads();
-  const int64_t row = jb + (int64_t)blockIdx.x * CR + threadIdx.x;
   if (row >= mp) return;
+#pragma unroll 1
+  for (int kb = 0; kb < CNB; kb += 8) {
+    T x[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) x[r] = vs[(kb + r) * L21_T];
+#pragma unroll 4
+    for (int q = 0; q < kb; ++q) {
+      const T vq = vs[q * L21_T];
+      const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + q * CNB + kb);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) x[r] = fmaT(-vq, l.v[r], x[r]);
+    }
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+      const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + (kb + p) * CNB + kb);
+      x[p] *= rd[kb + p];  // zero beyond jb (rd = 0 there)
+#pragma unroll
+      for (int r = p + 1; r < 8; ++r) x[r] = fmaT(-x[p], l.v[r], x[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 8; ++r) vs[(kb + r) * L21_T] = x[r];
+  }
   T v[CNB];
 #pragma unroll
-  for (int k = 0; k < CNB; ++k) v[k] = k < jb ? W[row + k * ldw] : T(0);
-#pragma unroll
   for (int k = 0; k < CNB; ++k) {
-    T x = v[k];
-#pragma unroll
-    for (int q = 0; q < k; ++q) x = fmaT(-v[q], L[k][q], x);
-    v[k] = x * rd[k];  // zero beyond jb (rd = 0 there)
-  }
-#pragma unroll
-  for (int k = 0; k < CNB; ++k)
+    v[k] = vs[k * L21_T];
     if (k < jb) W[row + k * ldw] = v[k];
+  }
   if (aop == nullptr) return;
   if constexpr (sizeof(T) == 4) {
     write_operand_row(kind, aop, aop_lo, row - jb, v);
@@ -209,10 +296,12 @@ int chol_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int32_t *info
     {
       ProfScope prof(lu.sp, fp64 ? "chol_panel64" : "chol_panel", (double)mp * jb * jb / 2.0,
                      2.0 * sizeof(T) * (double)mp * jb, 2);
-      chol_dblock<T><<<1, 256, 0, lu.sp>>>(Wp, ldw, jb, (int32_t)j, n, info, track, give_up);
+      chol_dblock<T><<<1, CH_T, 0, lu.sp>>>(Wp, ldw, jb, (int32_t)j, n, info, track, give_up);
       if (mp > jb) {
-        constexpr int CR = fp64 ? 64 : 128;
-        chol_l21<T, CR><<<(unsigned)cdiv(mp - jb, CR), CR, 0, lu.sp>>>(
+        if (l21_smem<T>() > 48 * 1024)
+          BOLA_TRY_CUDA(cudaFuncSetAttribute(chol_l21<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)l21_smem<T>()));
+        chol_l21<T><<<(unsigned)cdiv(mp - jb, L21_T), L21_T, l21_smem<T>(), lu.sp>>>(
             Wp, ldw, mp, jb, lu.kind, upd ? lu.aop[buf] : nullptr, fp64 ? nullptr : lu.aop_lo[buf],
             fp64 ? lu.ea[buf] : nullptr, lu.cap_n, info, track);
       }
