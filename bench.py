@@ -620,17 +620,14 @@ def run_serve(args, device):
 
 
 # DRAM bytes (read + write) per algorithmic byte, from the ncu captures
-# summarised under profiles/ (n=4096 cases): the tournament panel 0.82 MB read
-# for a 2816 x 64 FP32 panel whose algorithmic read + write is 1.44 MB;
-# tc_update 49.4 MB for a 3392 x 3328 step with 90.3 MB algorithmic (writes
+# summarised under profiles/ (n=4096 cases): tc_update 49.4 MB for a 3392 x 3328 step with 90.3 MB algorithmic (writes
 # still in L2); oz_update 129.4 MB for 180.6 MB.
-TRAFFIC_PER_ALGORITHMIC_BYTE = {"tpanel": 0.57, "tc_update": 0.55, "oz_update": 0.72}
+TRAFFIC_PER_ALGORITHMIC_BYTE = {"tc_update": 0.55, "oz_update": 0.72}
 
 
-# The tournament panels of the mixed LU as slu.cu schedules them: (mp, jb, C,
-# R) per panel of an n x n factorisation, 64 columns, CTAs of up to 256
-# threads x 2 rows.  The same kernel selects the FP64-accurate factor's
-# pivots (tselect64) on the same schedule.
+# The panels of the mixed LU as slu.cu schedules them: (mp, jb, C, R) per panel
+# of an n x n factorisation, 64 columns, a row per thread.  The same kernel
+# selects the FP64-accurate factor's pivots (select64) on the same schedule.
 def panel_schedule(n):
     out, j = [], 0
     while j < n:
@@ -642,22 +639,21 @@ def panel_schedule(n):
     return out
 
 
-TSLOT_BYTES = 16 + 64 * 4   # a tournament nominee pushed between CTAs
+CAND_BYTES, ROW_BYTES = 16, 64 * 4   # a column's candidate and its pivot's row, pushed between CTAs
 
 
 def panel_floor(n, exchange_us):
-    """Lower bound (us) of one factorisation's tournament panels and their
-    unit count: per group of 8 columns, the larger of one exchange round of 8
-    nominees at the panel's cluster size (measured) and the group's FP32 work
-    per CTA (rank-8 update of R rows over the remaining columns) at 128 FMA
-    per clock per SM, 2.07 GHz."""
+    """Lower bound (us) of one factorisation's panels and their unit count: per
+    column, the larger of its two exchange rounds at the panel's cluster size
+    (measured) and its FP32 work per CTA (rank-1 update of R rows over the
+    remaining columns) at 128 FMA per clock per SM, 2.07 GHz."""
     fma_sm = 128 * 2.07e9
     total, units = 0.0, 0
     sched = panel_schedule(n)
     for mp, jb, C, R in sched:
-        x = exchange_us(C, 8 * TSLOT_BYTES)
-        for g0 in range(0, jb, 8):
-            total += max(x, 1e6 * R * 8 * (64 - g0) / fma_sm)
+        x = exchange_us(C, CAND_BYTES) + exchange_us(C, ROW_BYTES)
+        for c in range(jb):
+            total += max(x, 1e6 * R * (64 - c) / fma_sm)
             units += 1
     return total, units, len(sched)
 
@@ -666,7 +662,7 @@ def roofline_for(name, v, peak_fp64_gflops, n=None, exchange_us=None):
     """The dominant kernel's achieved rate against its bounding peak.
     FP64 kernels: DFMA peak measured in this run.  Tensor-core update: HBM
     (it reads and writes the FP32 trailing matrix once per step).  Cluster
-    panels: latency-bound; time per column (or pivot group) against a floor
+    panels: latency-bound; time per column against a floor
     from measured exchange rounds and arithmetic rates, HBM fraction kept as
     a secondary field.  Others: HBM bytes of their algorithmic traffic."""
     peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
@@ -690,23 +686,24 @@ def roofline_for(name, v, peak_fp64_gflops, n=None, exchange_us=None):
         # algorithmic bytes of this run's average launch
         out["traffic"] = round(ratio * per_launch)
         out["algorithmic_bytes_per_launch"] = round(per_launch)
-    if name in ("tpanel", "tselect64") and n and exchange_us:
+    if name in ("ppanel", "select64") and n and exchange_us:
         floor_us, units, panels = panel_floor(n, exchange_us)
         facts = max(v["launches"], 1) / panels  # factorisations in the timed region
         ach_unit = 1e3 * v["ms"] / facts / units
         floor_unit = floor_us / units
         hbm_part = {k: out[k] for k in ("achieved", "peak", "unit", "frac", "traffic")}
         out = {"kernel": name, "bound": "latency", "achieved": round(ach_unit, 3), "peak": round(floor_unit, 3),
-               "unit": "us per pivot group of 8 columns", "frac": round(floor_unit / ach_unit, 4),
+               "unit": "us per column", "frac": round(floor_unit / ach_unit, 4),
                "traffic": hbm_part["traffic"],
-               "floor": ("per group: max(one cluster exchange round of 8 nominees (2176 bytes) at the panel's "
-                         "cluster size, measured by bola_measure_cluster_exchange; the group's FP32 work per CTA "
-                         "at 128 FMA/clock/SM)"),
-               "exchange_round_us": {str(c): round(exchange_us(c, 8 * TSLOT_BYTES), 3) for c in (2, 4, 8, 16)},
+               "floor": ("per column: max(cluster exchange rounds of its candidate (16 bytes) and its pivot's row "
+                         "(256 bytes) at the panel's cluster size, measured by bola_measure_cluster_exchange; its "
+                         "FP32 work per CTA at 128 FMA/clock/SM)"),
+               "exchange_round_us": {str(c): [round(exchange_us(c, b), 3) for b in (CAND_BYTES, ROW_BYTES)]
+                                    for c in (2, 4, 8, 16)},
                "factorisations": round(facts, 2), "hbm": hbm_part}
-        if name == "tpanel":
+        if name == "ppanel":
             out["note"] = ("launches of an abandoned 3xTF32 factorisation return at once and are averaged in, "
-                           "so the time per group of the factorisations that ran is somewhat higher")
+                           "so the time per column of the factorisations that ran is somewhat higher")
     return out
 
 

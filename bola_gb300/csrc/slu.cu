@@ -4,13 +4,10 @@
 // A (FP64) is scaled per 64-column block by a power of two (exact) and
 // rounded to the working matrix W: FP32 (factor kinds 0-2) or FP64 (kind 3).
 // Blocked right-looking LU, NB = 64 = the K of the tensor-core update:
-//   tpanel_kernel   FP32 W: the (n-j) x 64 panel on a cluster of <= 16 CTAs,
-//                   rows in shared memory, pivots chosen by tournament over
-//                   groups of 8 columns (one cluster exchange per group);
-//                   writes L21 as the update's K-major A operand (bf16 or
-//                   tf32 hi/lo).
-//   FP64 W (the FP64-accurate factor): the same tournament on FP32 copies
-//                   chooses the pivot rows (tpanel_kernel<double>), then
+//   ppanel_kernel   FP32 W: the (n-j) x 64 panel on a cluster of <= 16 CTAs,
+//                   a row per thread in registers, partial pivoting.
+//   FP64 W (the FP64-accurate factor): the same kernel on FP32 copies
+//                   chooses the pivot rows (ppanel_kernel<double>), then
 //                   panel_lu64 factors the panel in FP64 in that pivot order
 //                   on as many SMs as it has 64-row slices, writing L21's
 //                   exact bf16 slices as the A operand.
@@ -38,16 +35,6 @@ constexpr int SMAXC = 16;
 // a panel's moves of rows for the swap kernels: count, rows[128], src[128] (+ spare)
 constexpr int PLAN_STRIDE = 1 + 4 * SNB;
 
-// Bulk copy of `bytes` (a multiple of 16) from this CTA's shared memory into
-// another CTA's (cluster addresses dst and bar), completing on the
-// receiver's mbarrier; the issuing thread commits it as a bulk group.
-__device__ __forceinline__ void bulk_push(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "r"(sm100::smem_u32(src)), "r"(bytes), "r"(bar)
-      : "memory");
-}
-
 // Row pitch of a panel held in shared memory: at least R + 1 and a multiple
 // of the 16-byte vector (4 floats or 2 doubles), so that a lane can move V
 // consecutive rows of a column in one access.
@@ -56,116 +43,35 @@ __host__ __device__ constexpr int panel_pitch(int64_t R) {
   return (int)(((R + (int64_t)(16 / sizeof(T))) / (int64_t)(16 / sizeof(T))) * (int64_t)(16 / sizeof(T)));
 }
 
-// ---- tournament panel (the FP32 factors; pivot selection of the FP64 one) ----------------------------------------
-// Partial pivoting exchanges the pivot candidates of every CTA once per
-// column, so a cluster panel pays 64 cluster round trips.  The FP32 factors
-// (kinds 0-2) select their pivots by tournament instead (TSLU, the panel
-// step of communication-avoiding LU): per group of TG = 8 columns,
-//   1. every warp runs partial pivoting on its own rows over the group's
-//      columns (in registers, on scratch copies) and nominates TG rows;
-//   2. warp 0 runs it again on the CTA's 8 x TG nominees (their current
-//      values, not the warps' eliminated copies) and keeps TG;
-//   3. each CTA pushes its TG nominees into every CTA's shared memory
-//      (st.async onto the receiver's mbarrier: one exchange per group instead
-//      of one per column);
-//   4. while the pushes fly, each CTA applies the previous group's update to
-//      its rows' columns right of the current group (look-ahead: the previous
-//      group only updated the current group's columns before the search);
-//   5. every CTA runs partial pivoting on the same C x TG stacked nominees and
-//      so picks the same TG pivot rows, with their multipliers; the pivots' U
-//      rows right of the group come from the pushed rows, brought up to date
-//      with the previous group's update first (the pushed multipliers of that
-//      group travel with them);
-//   6. every CTA gives its rows the group's multipliers (forward substitution
-//      through the TG x TG block of U) and updates the next group's columns.
-// Rows never move during the panel (a per-row state records which column a
-// row is the pivot of); the interchanges (LAPACK ipiv) are derived at the end
-// and every row is written back once, to its final position.  The pivots are
-// not those of column-by-column partial pivoting; their growth is that of
-// tournament pivoting (CALU), and only the FP64 refinement decides accuracy.
-constexpr int TG = 8;     // columns per tournament group
-constexpr int TPT = 256;  // threads per panel CTA (8 warps)
-constexpr int TRPL = 2;   // panel rows per thread: R <= TPT * TRPL = 512
-
-struct alignas(16) TSlot {
-  uint32_t row, pad0, pad1, pad2;  // panel row of the nominee, or 0xFFFFFFFF (none)
-  float v[SNB];                    // its values from column pb on: v[k] = column pb + k
-};
-
-// Partial pivoting over gw <= TG columns of candidates held by the first NW
-// warps of the CTA: thread t (< 32 NW) holds candidate t + 32 NW r in row r
-// of v (r < RPL), the current column always in register slot 0 (the others
-// shift down after each step, which keeps the column loop rolled).  Pivot
-// key: |v| with its KB lowest bits replaced by (2^KB - 1 - candidate), so a
-// warp reduction and a maximum over the NW warps' results find the pivot
-// (the lowest mantissa bits do not matter for the pivot's quality; ties go
-// to the lowest candidate; a NaN never wins over a number).  Per step: the
-// warps' maxima meet in shared memory at one named barrier over the NW
-// warps, the pivot's owner publishes its row at a second, and every thread
-// updates its own candidates.  Writes the selected candidates in order to
-// sel[] and returns their count (the same in every thread).  RECORD: each
-// candidate's multipliers go to Lsm[candidate * TG + step], the selected
-// rows' ones to Lrec[t][s] (s < t), and the pivot rows' eliminated values in
-// group column t + k to Urec[(t + k) * uk + t].
-template <int RPL, int NW, bool RECORD>
-__device__ __forceinline__ int group_gepp(float (&v)[RPL][TG], bool (&live)[RPL], int gw, int32_t *sel, int bar,
-                                          uint32_t *wmax, float *prow, float *Lsm, float (*Lrec)[TG], float *Urec,
-                                          int uk) {
-  constexpr int NT = 32 * NW;
-  constexpr uint32_t MASK = RPL * NT <= 256 ? 0xFFu : 0x3FFu;  // candidate-index bits
-  static_assert(RPL * NT <= 1024, "too many candidates for the key");
-  const int t0 = threadIdx.x, lane = t0 & 31, w = t0 >> 5;
-  int cnt = 0;
-#pragma unroll 1
-  for (int t = 0; t < gw; ++t) {
-    uint32_t key = 0u;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const float x = fabsf(v[r][0]);
-      const uint32_t a = x == x ? __float_as_uint(x) : 0u;
-      const uint32_t k = (a & ~MASK) | (MASK - (uint32_t)(t0 + NT * r));
-      key = (live[r] && k > key) ? k : key;
-    }
-    key = __reduce_max_sync(0xffffffffu, key);
-    if (lane == 0) wmax[w] = key;
-    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(NT) : "memory");
-    uint32_t mk = wmax[0];
-#pragma unroll
-    for (int i = 1; i < NW; ++i) mk = wmax[i] > mk ? wmax[i] : mk;
-    if (mk == 0u) break;  // no live candidate left (a live one has a key > 0)
-    const int ci = (int)(MASK - (mk & MASK));
-    if (t0 == ci % NT) {  // the owner publishes the pivot row and retires it
-      const int ro = ci / NT;
-#pragma unroll
-      for (int r = 0; r < RPL; ++r)
-        if (r == ro) {
-#pragma unroll
-          for (int k = 0; k < TG; ++k) prow[k] = v[r][k];
-          live[r] = false;
-        }
-      sel[t] = ci;
-    }
-    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(NT) : "memory");
-    float pv[TG];
-#pragma unroll
-    for (int k = 0; k < TG; ++k) pv[k] = prow[k];
-    if (RECORD) {
-      if (t0 < t) Lrec[t][t0] = Lsm[ci * TG + t0];
-      if (t0 < TG && t0 < gw - t) Urec[(t + t0) * uk + t] = pv[t0];
-    }
-    const float inv = pv[0] != 0.f ? __frcp_rn(pv[0]) : 0.f;
-#pragma unroll
-    for (int r = 0; r < RPL; ++r) {
-      const float l = v[r][0] * inv;
-      if (RECORD && live[r]) Lsm[(t0 + NT * r) * TG + t] = l;
-#pragma unroll
-      for (int k = 1; k < TG; ++k) v[r][k - 1] = live[r] ? fmaf(-l, pv[k], v[r][k]) : v[r][k];
-      v[r][TG - 1] = 0.f;
-    }
-    ++cnt;
-  }
-  return cnt;
-}
+// ---- partial-pivoting panel (the FP32 factors; pivot selection of the FP64 one) ----
+// Column by column, a row per thread, the row's 64 values in registers; one
+// exchange of 16 bytes per CTA and column decides the pivot, and the pivot's
+// CTA then sends its row to every other.  What bounds it is that chain, so
+// everything else is placed in its shadow:
+//   1. every row's current column is brought up to date first; the largest
+//      |value| of a warp, of the CTA (shared memory, one CTA barrier), and of
+//      the cluster (st.async onto the receivers' mbarriers);
+//   2. while the candidates travel, the previous pivot's update of the other
+//      columns (the current column always sits in register slot 0, the others
+//      shift down with the update: the column loop stays rolled), and the
+//      CTA's candidate row is laid out in shared memory;
+//   3. the pivot's CTA sends that row (st.async, 256 bytes to every CTA);
+//      everyone scales its column and takes the update of the next one.
+// Rows never move during the panel (a state per row records which column it is
+// the pivot of); the interchanges (LAPACK ipiv) are derived beside it, and
+// every row is written back once, to its final position.  Pivots are compared
+// by |value| with the five lowest mantissa bits replaced by the lane.
+// Measured on one GB300 (n = 8192, mean over the panels): 76 us; tournament
+// pivoting over groups of eight columns, two dependent searches of eight steps
+// behind named barriers per group, took 86.  Other forms measured and slower:
+// eight columns' values beside the candidate (48 bytes) with the pivots' rows
+// exchanged once per group of eight, 88 (a longer combine and a group end of
+// two cluster barriers); the candidate's row pushed before the exchange, 86.
+constexpr int PP_MAXR = 512;   // rows per CTA at most (a thread each)
+// rows per CTA aimed at: fewer CTAs shorten the exchanges, more rows lengthen
+// the barrier and the update (n = 8192: 76 us with 256, 78 with 64, 80 with 512)
+constexpr int PP_CTA_ROWS = 256;
+constexpr int PP_MAXW = PP_MAXR / 32;
 
 // LAPACK's interchanges for a panel whose pivot of column j is panel row x
 // (j < jb), one column at a time in column order: interchange_step returns
@@ -240,36 +146,22 @@ __device__ __forceinline__ void list_panel_moves(const int32_t *pivl, const int3
   }
 }
 
-// Dynamic shared memory of the tournament panel: the rows (column-major,
-// pitch RP, 64 columns, zero beyond jb), the double-buffered nominee slots
-// (C x TG per buffer) and the row states.
-__host__ __device__ constexpr size_t tpanel_smem(int64_t R, int C) {
-  return sizeof(float) * (size_t)SNB * (size_t)panel_pitch<float>(R) + 2 * (size_t)C * TG * sizeof(TSlot) +
-         sizeof(int16_t) * (size_t)(R + 8);
-}
-
-// a -= sum_s l[s] u[s] (s = 0..7, in order)
-__device__ __forceinline__ float rank8(float a, const float (&l)[TG], const float4 &u0, const float4 &u1) {
-  a = fmaf(-l[0], u0.x, a);
-  a = fmaf(-l[1], u0.y, a);
-  a = fmaf(-l[2], u0.z, a);
-  a = fmaf(-l[3], u0.w, a);
-  a = fmaf(-l[4], u1.x, a);
-  a = fmaf(-l[5], u1.y, a);
-  a = fmaf(-l[6], u1.z, a);
-  a = fmaf(-l[7], u1.w, a);
-  return a;
+// Dynamic shared memory of the panel: the rows' finished values (column-major,
+// pitch RP, 64 columns) and the pivot rows (value k of row j at
+// u[j * 64 + k]: column j + k).
+__host__ __device__ constexpr size_t ppanel_smem(int64_t R) {
+  return sizeof(float) * ((size_t)SNB * (size_t)panel_pitch<float>(R) + (size_t)SNB * SNB);
 }
 
 // G = float: the FP32 factors' panel (factored in place).  G = double: the
-// FP64-accurate factor's pivot selection only — the tournament runs on FP32
-// copies of the panel's values and writes the jb pivot rows (panel rows, in
-// column order) to winout and their FP64 values (columns of the panel) to
-// sel, 64 x 64 row-major; W, ipiv, info and the operands are left to the
-// FP64 kernel that follows (panel_lu64).
+// FP64-accurate factor's pivot selection only — the panel is factored on FP32
+// copies of its values and the jb pivot rows (panel rows, in column order) go
+// to winout and their FP64 values (columns of the panel) to sel, 64 x 64
+// row-major; W, ipiv, info and the operands are left to the FP64 kernel that
+// follows (panel_lu64).
 template <typename G>
-__global__ void __launch_bounds__(TPT, 1)
-tpanel_kernel(G *W, int64_t ldw, int64_t mp, int jb, int32_t *ipiv, int32_t col0, int32_t *info, int64_t R,
+__global__ void __launch_bounds__(PP_MAXR, 1)
+ppanel_kernel(G *W, int64_t ldw, int64_t mp, int jb, int32_t *ipiv, int32_t col0, int32_t *info, int64_t R,
               int32_t *plan, uint64_t *track, double give_up, int32_t *err, int32_t *winout, G *sel) {
   constexpr bool SEL = std::is_same<G, double>::value;
   sm100::grid_dependency_wait();
@@ -283,395 +175,233 @@ tpanel_kernel(G *W, int64_t ldw, int64_t mp, int jb, int32_t *ipiv, int32_t col0
   }
   const int C = (int)cluster.num_blocks();
   const int cr = (int)cluster.block_rank();
-  __shared__ uint64_t xbar[2];             // completes when every CTA's nominees of a group have landed
-  __shared__ int32_t cand2[TG];            // the CTA's nominees (local rows, -1: none)
-  __shared__ uint32_t gwmax[TPT / 32];     // pivot searches: the warps' best keys
-  __shared__ float gprow[TG];              // pivot searches: the pivot row of the current step
-  __shared__ int32_t win[SNB];             // panel row of the pivot of each column
-  __shared__ int32_t wslot[TG];            // the group's pivots as slot indices
-  __shared__ float Lg[TG][TG];             // the group pivots' multipliers within the group
-  __shared__ __align__(16) float UgT[2][SNB][TG];  // U rows of a group's pivots, transposed (two groups)
-  __shared__ float invp[TG];
-  __shared__ int32_t posin[SNB], at_[SNB];  // interchange bookkeeping (CTA 0)
-  __shared__ int sfail;
-  __shared__ TSlot stage[TG];              // this CTA's nominees, as they are pushed
-  __shared__ int32_t selw[2][TG];          // pivot searches' outputs (candidate order): own rows, nominees
-  __shared__ float Lsm[SMAXC * TG * TG];   // multipliers of the stacked nominees, per step
-  __shared__ float Linv[TG][TG];           // inverse of the group's unit-lower 8 x 8 block of L
-  extern __shared__ __align__(16) unsigned char tp_raw[];
+  __shared__ uint64_t hbar[2], rbar[2];            // every CTA's candidate / the pivot row has landed
+  __shared__ __align__(16) uint4 hdr[2][SMAXC];    // key, value, local row
+  __shared__ uint2 wbest[2][PP_MAXW];              // a warp's best: key, value
+  __shared__ __align__(16) float stage[SNB];       // the CTA's candidate row, from the current column on
+  __shared__ int32_t win[SNB];                     // panel row of the pivot of each column
+  __shared__ int32_t posin[SNB], at_[SNB];         // interchange bookkeeping (CTA 0)
+  __shared__ int16_t rstate[PP_MAXR];              // -1: not a pivot; j: the pivot of column j
+  __shared__ int sfail[2];                         // a wait of a column of this parity ran out
+  extern __shared__ __align__(16) unsigned char pp_raw[];
   const int RP = panel_pitch<float>(R);
-  float *sp = reinterpret_cast<float *>(tp_raw);
-  TSlot *slots = reinterpret_cast<TSlot *>(tp_raw + sizeof(float) * (size_t)SNB * RP);
-  int16_t *rstate = reinterpret_cast<int16_t *>(tp_raw + sizeof(float) * (size_t)SNB * RP +
-                                                2 * (size_t)C * TG * sizeof(TSlot));
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float *sp = reinterpret_cast<float *>(pp_raw);
+  float *ub = sp + (size_t)SNB * RP;
+  const unsigned FULL = 0xffffffffu;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = (int)(blockDim.x >> 5), NT = (int)blockDim.x;
   const int r0 = (int)(cr * R);
   const int r1 = (int)imin(mp, r0 + R);
   const int nr = r1 > r0 ? r1 - r0 : 0;
+  const bool has = tid < nr;
 
-  // the panel into shared memory: a thread's rows, 32 columns at a time, with
-  // all of those loads in flight together (the copy is latency-bound otherwise)
+  float v[SNB];
 #pragma unroll
-  for (int c0 = 0; c0 < SNB; c0 += 32) {
-    float t[TRPL][32];
-#pragma unroll
-    for (int r = 0; r < TRPL; ++r) {
-      const int il = tid + TPT * r;
-#pragma unroll
-      for (int c = 0; c < 32; ++c)
-        t[r][c] = (il < nr && c0 + c < jb) ? (float)W[(r0 + il) + (int64_t)(c0 + c) * ldw] : 0.f;
-    }
-#pragma unroll
-    for (int r = 0; r < TRPL; ++r) {
-      const int il = tid + TPT * r;
-      if (il < nr)
-#pragma unroll
-        for (int c = 0; c < 32; ++c) sp[(c0 + c) * RP + il] = t[r][c];
-    }
-  }
-  for (int il = tid; il < nr; il += TPT) rstate[il] = -1;  // -1: not a pivot yet; j: the pivot of column j
+  for (int c = 0; c < SNB; ++c) v[c] = has && c < jb ? (float)W[(r0 + tid) + (int64_t)c * ldw] : 0.f;
+  if (tid < PP_MAXR) rstate[tid] = -1;
   if (tid == 0) {
-    sm100::mbar_init(&xbar[0], 1);
-    sm100::mbar_init(&xbar[1], 1);
+    for (int i = 0; i < 2; ++i) {
+      sm100::mbar_init(&hbar[i], 1);
+      sm100::mbar_init(&rbar[i], 1);
+      sfail[i] = 0;
+    }
     sm100::fence_mbar_init();
-    sfail = 0;
   }
   __syncthreads();
   cluster.sync();  // every CTA runs, its mbarriers initialised, before the first push
 
-  bool failed = false;
-  uint64_t umax = 0, umin = ~0ull;  // |u_jj| bits (CTA 0, thread 0)
-  const int ngroups = (int)cdiv(jb, TG);
-  for (int g = 0; g < ngroups; ++g) {
-    const int c0 = g * TG, gw = (int)imin(TG, jb - c0), par = g & 1, ub = g & 1;
-    const int pb = c0 >= TG ? c0 - TG : 0;  // first pushed column: the previous group's multipliers on
-    const int nv = SNB - pb;                // values pushed per nominee (a multiple of 8)
-    const int nq = 1 + nv / 4;
-    if (tid == 0) sm100::mbar_arrive_expect_tx(&xbar[par], (uint32_t)(C * gw * sizeof(TSlot)));
-    // -- 1-2. the CTA's nominees: partial pivoting over all of its rows on
-    // the group's columns (scratch copies in registers), every warp taking
-    // part in every step
+  bool live = has, failed = false;
+  float x = 0.f, cur = v[0];
+  uint32_t umax = 0, umin = ~0u;  // |u_jj| bits (CTA 0, thread 0)
+  const int bk = NT - 32;         // the thread that keeps the interchanges (the last warp's first lane)
+  if (!SEL && cr == 0 && tid == bk) interchanges_init(jb, posin, at_);
+  for (int j = 0; j < jb; ++j) {
+    const int par = j & 1;
+    const uint32_t phase = (uint32_t)(j >> 1) & 1u;
+    if (tid == 0) {
+      sm100::mbar_arrive_expect_tx(&hbar[par], (uint32_t)(C * sizeof(uint4)));
+      sm100::mbar_arrive_expect_tx(&rbar[par], (uint32_t)(SNB * sizeof(float)));
+    }
+    // -- 1. the CTA's candidate
     {
-      float v[TRPL][TG];
-      bool live[TRPL];
-#pragma unroll
-      for (int r = 0; r < TRPL; ++r) {
-        const int il = tid + TPT * r;
-        live[r] = il < nr && rstate[il] < 0;
-#pragma unroll
-        for (int k = 0; k < TG; ++k) v[r][k] = live[r] ? sp[(c0 + k) * RP + il] : 0.f;
-      }
-      const int cnt = group_gepp<TRPL, TPT / 32, false>(v, live, gw, selw[0], 1, gwmax, gprow, nullptr, nullptr,
-                                                        nullptr, 0);
-      if (tid < TG) cand2[tid] = tid < cnt ? selw[0][tid] : -1;
-      // the previous group's bulk pushes have read the staging slots
-      if (tid < C) sm100::bulk_wait_read0();
+      const uint32_t ab = __float_as_uint(cur) & 0x7fffffffu;
+      const uint32_t key = live ? ((ab <= 0x7f800000u ? ab : 0u) & ~31u) + 32u + (uint32_t)(31 - lane) : 0u;
+      const uint32_t mk = __reduce_max_sync(FULL, key);
+      if (key == mk && (mk != 0u || lane == 0)) wbest[par][warp] = make_uint2(mk, __float_as_uint(cur));
     }
     __syncthreads();
-    // -- 3. push the nominees (columns pb..63): staged as gw slots, then one
-    // bulk copy into every CTA (slots cr * gw .. of its buffer par)
-    for (int e = tid; e < gw * nq; e += TPT) {
-      const int q = e % nq, s2 = e / nq;
-      const int il = cand2[s2];
-      if (q == 0) {
-        stage[s2].row = il >= 0 ? (uint32_t)(r0 + il) : 0xFFFFFFFFu;
-      } else {
-        const int k = (q - 1) * 4;
-        float4 w4;
-        w4.x = il >= 0 ? sp[(pb + k) * RP + il] : 0.f;
-        w4.y = il >= 0 ? sp[(pb + k + 1) * RP + il] : 0.f;
-        w4.z = il >= 0 ? sp[(pb + k + 2) * RP + il] : 0.f;
-        w4.w = il >= 0 ? sp[(pb + k + 3) * RP + il] : 0.f;
-        *reinterpret_cast<float4 *>(&stage[s2].v[k]) = w4;
-      }
-    }
-    sm100::fence_proxy_async_smem();  // the staged slots, visible to the bulk copies
-    __syncthreads();
-    if (tid < C) {  // lane d of warp 0 pushes into CTA d
-      bulk_push(sm100::cluster_addr(&slots[(size_t)par * C * TG + cr * gw], tid), stage, (uint32_t)(gw * sizeof(TSlot)),
-                sm100::cluster_addr(&xbar[par], tid));
-      sm100::bulk_commit();
-    }
-    // -- 4. the previous group's update on the columns right of this group
-    // (a thread's rows and 4 columns at a time: 8 independent chains of the
-    // 8 dependent FMAs of rank8 in flight; SNB - c0 - TG is a multiple of 8)
-    if (g > 0) {
-      const float(*U)[TG] = UgT[ub ^ 1];
-      bool on[TRPL];
-      float l[TRPL][TG];
-#pragma unroll
-      for (int r = 0; r < TRPL; ++r) {
-        const int il = tid + TPT * r;
-        on[r] = il < nr && rstate[il] < 0;
-#pragma unroll
-        for (int s2 = 0; s2 < TG; ++s2) l[r][s2] = on[r] ? sp[(pb + s2) * RP + il] : 0.f;
-      }
-      for (int k0 = c0 + TG; k0 < SNB; k0 += 4) {
-        float x[TRPL][4];
-#pragma unroll
-        for (int r = 0; r < TRPL; ++r)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) x[r][j] = on[r] ? sp[(k0 + j) * RP + tid + TPT * r] : 0.f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 u0 = *reinterpret_cast<const float4 *>(&U[k0 + j][0]);
-          const float4 u1 = *reinterpret_cast<const float4 *>(&U[k0 + j][4]);
-#pragma unroll
-          for (int r = 0; r < TRPL; ++r) x[r][j] = rank8(x[r][j], l[r], u0, u1);
-        }
-#pragma unroll
-        for (int r = 0; r < TRPL; ++r)
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (on[r]) sp[(k0 + j) * RP + tid + TPT * r] = x[r][j];
-      }
-    }
-    // every CTA's nominees have landed (bounded: a missing push sets the
-    // error flag and ends the panel, never a hang)
-    if (!sm100::bounded_wait(&xbar[par], (uint32_t)(g >> 1) & 1u)) sfail = 1;
-    __syncthreads();
-    if (sfail) {
-      if (tid == 0) atomicExch(err, 5);
+    if (sfail[par ^ 1]) {  // a wait of the previous column ran out (written before the barrier above)
       failed = true;
       break;
     }
-    const TSlot *sl = slots + (size_t)par * C * TG;
-    // -- 5. the group's pivots from all nominees, the same in every CTA
-    // (warps 0-3, one candidate per lane)
-    if (warp < 4) {
-      float v[1][TG];
-      bool live[1];
-      live[0] = tid < C * gw && sl[tid].row != 0xFFFFFFFFu;
+    uint2 best;
+    int bw;
+    {
+      best = lane < nw ? wbest[par][lane] : make_uint2(0u, 0u);
+      const uint32_t mk = __reduce_max_sync(FULL, best.x);
+      bw = __ffs(__ballot_sync(FULL, best.x == mk)) - 1;
+      best.y = __shfl_sync(FULL, best.y, bw);
+      best.x = mk;
+    }
+    const int il = bw * 32 + 31 - (int)(best.x & 31u);  // the CTA's candidate (when best.x != 0)
+    if (warp == 0 && lane < C)
+      sm100::st_async4(sm100::cluster_addr(&hdr[par][cr], lane), best.x, best.y, (uint32_t)il, 0u,
+                       sm100::cluster_addr(&hbar[par], lane));
+    // -- 2. the previous pivot's update of the columns after this one; slot k
+    // takes column j + k (slots beyond the panel hold zeros or leftovers)
+    if (j > 0) {
+      const float *u = ub + (j - 1) * SNB;
+      v[0] = cur;
 #pragma unroll
-      for (int k = 0; k < TG; ++k) v[0][k] = live[0] ? sl[tid].v[c0 - pb + k] : 0.f;
-      const int cnt = group_gepp<1, 4, true>(v, live, gw, selw[1], 2, gwmax, gprow, Lsm, Lg, &UgT[ub][c0][0], TG);
-      if (warp == 0) {
-        // the panel always has at least gw rows that are not pivots yet, so
-        // cnt == gw; a shortfall would mean a corrupted exchange
-        if (cnt < gw && lane == 0) atomicExch(err, 6);
-        if (lane < gw) {
-          const int s2 = selw[1][lane];
-          wslot[lane] = lane < cnt ? s2 : -1;
-          win[c0 + lane] = lane < cnt ? (int32_t)sl[s2].row : -1;
-        }
-        // the inverse of the group's unit-lower block of L: lane q forms column q
-        __syncwarp();
-        if (lane < TG) {
-          float col[TG];
+      for (int kb = 0; kb < SNB; kb += 8) {
+        if (kb < SNB + 1 - j) {
+          const float4 a = *reinterpret_cast<const float4 *>(u + kb), b = *reinterpret_cast<const float4 *>(u + kb + 4);
+          const float p[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-          for (int t = 0; t < TG; ++t) {
-            float x = t == lane ? 1.f : 0.f;
-#pragma unroll
-            for (int p = 0; p < t; ++p) x = fmaf(-Lg[t][p], col[p], x);
-            col[t] = t < lane ? 0.f : x;
-          }
-#pragma unroll
-          for (int t = 0; t < TG; ++t) Linv[t][lane] = col[t];
+          for (int q = 0; q < 8; ++q)
+            if (kb + q >= 2) v[kb + q - 1] = fmaf(-x, p[q], v[kb + q]);
         }
       }
-    } else if (!SEL && cr == 0 && tid == TPT / 2) {
-      // meanwhile (warps 4-7 are idle): LAPACK's interchanges for the
-      // previous group's pivots
-      if (g == 0) interchanges_init(jb, posin, at_);
-      for (int j = c0 - TG; j >= 0 && j < c0; ++j) ipiv[j] = interchange_step(j, win[j], jb, col0, posin, at_);
     }
-    __syncthreads();
-    if (win[c0 + gw - 1] < 0) {  // (err is set) leave the group loop uniformly
-      failed = true;
-      break;
-    }
-    // the pivots' pushed rows, brought up to date on the columns right of the
-    // group with the previous group's update (their multipliers of that group
-    // are the first 8 pushed values), in place
-    if (g > 0) {
-      TSlot *slw = slots + (size_t)par * C * TG;
-      const float(*U)[TG] = UgT[ub ^ 1];
-      const int nk = SNB - c0 - gw;
-      for (int e = tid; e < gw * nk; e += TPT) {
-        const int ci = wslot[e / nk], k = c0 + gw + e % nk;
-        float l[TG];
+    if (tid == il && best.x != 0u) {
 #pragma unroll
-        for (int s2 = 0; s2 < TG; ++s2) l[s2] = slw[ci].v[s2];
-        slw[ci].v[k - pb] = rank8(slw[ci].v[k - pb], l, *reinterpret_cast<const float4 *>(&U[k][0]),
-                                  *reinterpret_cast<const float4 *>(&U[k][4]));
+      for (int k = 0; k < SNB; k += 4) *reinterpret_cast<float4 *>(&stage[k]) = make_float4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    }
+    if (!SEL && cr == 0 && tid == bk && j > 0) ipiv[j - 1] = interchange_step(j - 1, win[j - 1], jb, col0, posin, at_);
+    __syncwarp();
+    // -- the cluster's pivot, the same in every CTA
+    if (!sm100::bounded_wait(&hbar[par], phase)) sfail[par] = 1;
+    const uint4 h = lane < C ? hdr[par][lane] : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t ck = __reduce_max_sync(FULL, h.x);
+    const int ws = __ffs(__ballot_sync(FULL, h.x == ck)) - 1;
+    const float pv = __uint_as_float(__shfl_sync(FULL, h.y, ws));
+    const int pl = (int)__shfl_sync(FULL, h.z, ws);
+    // -- 3. its row to every CTA
+    if (ws == cr && warp == (pl >> 5)) {
+      const float4 q = *reinterpret_cast<const float4 *>(&stage[4 * (lane & 15)]);
+      for (int d = lane >> 4; d < C; d += 2)
+        sm100::st_async4(sm100::cluster_addr(ub + j * SNB + 4 * (lane & 15), d), __float_as_uint(q.x),
+                         __float_as_uint(q.y), __float_as_uint(q.z), __float_as_uint(q.w),
+                         sm100::cluster_addr(&rbar[par], d));
+      if (tid == pl) {
+        live = false;
+        rstate[tid] = (int16_t)j;
       }
-      __syncthreads();
     }
-    // the pivots' U rows right of the group: U = Linv A' over the up-to-date
-    // pushed rows A', one (row, column) element per thread
-    for (int e = tid; e < gw * (SNB - c0 - gw); e += TPT) {
-      const int t = e % gw, k = c0 + gw + e / gw;
-      float u = 0.f;
-#pragma unroll
-      for (int q = 0; q < TG; ++q)
-        if (q <= t) u = fmaf(Linv[t][q], sl[wslot[q]].v[k - pb], u);
-      UgT[ub][k][t] = u;
-    }
-    if (tid < gw) {
-      const float pv = UgT[ub][c0 + tid][tid];
-      invp[tid] = pv != 0.f ? __frcp_rn(pv) : 0.f;
-      const int row = win[c0 + tid];
-      if (row >= r0 && row < r1) rstate[row - r0] = (int16_t)(c0 + tid);
-    }
-    if (cr == 0 && tid == TPT - 1) {
-      for (int t = 0; t < gw; ++t) {
-        const float pv = UgT[ub][c0 + t][t];
-        if (!SEL && pv == 0.f) atomicCAS(info, 0, col0 + c0 + t + 1);
-        const uint64_t ab = __float_as_uint(pv) & 0x7fffffffu;
+    if (tid == 0) {
+      win[j] = (int32_t)(ws * R) + pl;
+      if (cr == 0) {
+        if (!SEL && pv == 0.f) atomicCAS(info, 0, col0 + j + 1);
+        const uint32_t ab = __float_as_uint(pv) & 0x7fffffffu;
         if (ab <= 0x7f800000u) {
           umax = ab > umax ? ab : umax;
           umin = ab < umin ? ab : umin;
         }
       }
     }
-    __syncthreads();
-    // -- 6. this CTA's pivot rows take their final values (all threads, an
-    // element each); the other rows their multipliers and the update of the
-    // next group's columns
-    for (int e = tid; e < gw * (SNB - c0); e += TPT) {
-      const int t = e / (SNB - c0), k = c0 + e % (SNB - c0);
-      const int row = win[c0 + t];
-      if (row < r0 || row >= r1) continue;
-      sp[k * RP + (row - r0)] = k < c0 + t ? Lg[t][k - c0] : UgT[ub][k][t];
-    }
-    // (a thread's rows side by side, so that their dependent chains overlap;
-    // pivot rows, of this group or earlier, are left as they are)
-    {
-      bool on[TRPL];
-      float l[TRPL][TG];
-#pragma unroll
-      for (int r = 0; r < TRPL; ++r) {
-        const int il = tid + TPT * r;
-        on[r] = il < nr && rstate[il] < 0;
-      }
-#pragma unroll
-      for (int s2 = 0; s2 < TG; ++s2) {
-#pragma unroll
-        for (int r = 0; r < TRPL; ++r) {
-          const int il = tid + TPT * r;
-          const bool live = on[r] && s2 < gw;
-          float a = live ? sp[(c0 + s2) * RP + il] : 0.f;
-#pragma unroll
-          for (int q = 0; q < s2; ++q) a = fmaf(-l[r][q], UgT[ub][c0 + s2][q], a);
-          l[r][s2] = live ? a * invp[s2] : 0.f;
-          if (live) sp[(c0 + s2) * RP + il] = l[r][s2];
-        }
-      }
-      if (c0 + TG < SNB) {  // the next group's 8 columns
-#pragma unroll
-        for (int j = 0; j < TG; ++j) {
-          const int k = c0 + TG + j;
-          const float4 u0 = *reinterpret_cast<const float4 *>(&UgT[ub][k][0]);
-          const float4 u1 = *reinterpret_cast<const float4 *>(&UgT[ub][k][4]);
-#pragma unroll
-          for (int r = 0; r < TRPL; ++r) {
-            const int il = tid + TPT * r;
-            if (on[r]) sp[k * RP + il] = rank8(sp[k * RP + il], l[r], u0, u1);
-          }
-        }
-      }
-    }
-    __syncthreads();
+    const float inv = pv != 0.f ? __frcp_rn(pv) : 0.f;
+    x = cur * inv;
+    if (has && (live || rstate[tid] == j)) sp[j * RP + tid] = live ? x : cur;
+    const float nx = v[1];
+    if (!sm100::bounded_wait(&rbar[par], phase)) sfail[par] = 1;
+    cur = fmaf(-x, ub[j * SNB + 1], nx);
   }
+  __syncthreads();
+  if (!failed && sfail[(jb - 1) & 1]) failed = true;
+  if (failed && tid == 0) atomicExch(err, 5);
   if (!failed) {
+    // this CTA's pivot rows: their U values beside their multipliers
+    for (int e = tid; e < jb * SNB; e += NT) {
+      const int t = e / SNB, c = e % SNB, row = win[t];
+      if (row >= r0 && row < r1 && c >= t) sp[c * RP + (row - r0)] = ub[t * SNB + (c - t)];
+    }
     if constexpr (SEL) {
       if (cr == 0)
-        for (int t = tid; t < jb; t += TPT) winout[t] = win[t];
+        for (int t = tid; t < jb; t += NT) winout[t] = win[t];
       // the pivot rows' FP64 values, each CTA its own rows
-      for (int e = tid; e < jb * jb; e += TPT) {
+      for (int e = tid; e < jb * jb; e += NT) {
         const int t = e / jb, c = e % jb, row = win[t];
         if (row >= r0 && row < r1) sel[t * SNB + c] = W[row + (int64_t)c * ldw];
       }
     } else {
-    // -- the last group's interchanges (CTA 0; the earlier groups' ran
-    // during the searches that followed them)
-    if (cr == 0 && tid == TPT / 2)
-      for (int j = (ngroups - 1) * TG; j < jb; ++j) ipiv[j] = interchange_step(j, win[j], jb, col0, posin, at_);
-    if (track != nullptr && cr == 0 && tid == TPT - 1) {
-      if (umin != ~0ull) {
-        const uint64_t mx = (uint64_t)__double_as_longlong((double)__uint_as_float((uint32_t)umax));
-        const uint64_t mn = (uint64_t)__double_as_longlong((double)__uint_as_float((uint32_t)umin));
-        if (mx > track[0]) track[0] = mx;
-        if (mn < track[1]) track[1] = mn;
+      // -- the last column's interchange (CTA 0; the earlier ones ran during the exchanges that followed them)
+      if (cr == 0 && tid == bk) ipiv[jb - 1] = interchange_step(jb - 1, win[jb - 1], jb, col0, posin, at_);
+      if (track != nullptr && cr == 0 && tid == 0) {
+        if (umin != ~0u) {
+          const uint64_t mx = (uint64_t)__double_as_longlong((double)__uint_as_float(umax));
+          const uint64_t mn = (uint64_t)__double_as_longlong((double)__uint_as_float(umin));
+          if (mx > track[0]) track[0] = mx;
+          if (mn < track[1]) track[1] = mn;
+        }
+        const double gmx = __longlong_as_double((long long)track[0]), gmn = __longlong_as_double((long long)track[1]);
+        const double spread = gmn > 0.0 ? gmx / gmn : INFINITY;
+        if (give_up_now(spread, give_up, col0 + jb, col0 + mp)) *(volatile int32_t *)(track + 2) = 1;
       }
-      const double gmx = __longlong_as_double((long long)track[0]), gmn = __longlong_as_double((long long)track[1]);
-      const double spread = gmn > 0.0 ? gmx / gmn : INFINITY;
-      if (give_up_now(spread, give_up, col0 + jb, col0 + mp)) *(volatile int32_t *)(track + 2) = 1;
-    }
-    __syncthreads();
-    // -- write back the panel: first every row where it started, as float4
-    // runs of 4 rows (a warp writes 512 contiguous bytes of a column; R is a
-    // multiple of 4, so runs start 16-byte aligned in W when W and ldw allow);
-    // the rows that move (the pivots, and CTA 0's first jb rows that are not
-    // pivots) are written again to their final positions after the cluster
-    // barrier below, so that those writes land last
-    const bool vec = (ldw & 3) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (R & 3) == 0;
-    if (vec) {
-      const int nq4 = nr / 4;
-      for (int e = tid; e < nq4 * jb; e += TPT) {
-        const int il0 = 4 * (e % nq4), c = e / nq4;
-        *reinterpret_cast<float4 *>(&W[(r0 + il0) + (int64_t)c * ldw]) =
-            *reinterpret_cast<const float4 *>(&sp[c * RP + il0]);
-      }
-      for (int e = tid; e < (nr - 4 * nq4) * jb; e += TPT) {
-        const int il = 4 * nq4 + e % (nr - 4 * nq4), c = e / (nr - 4 * nq4);
-        W[(r0 + il) + (int64_t)c * ldw] = sp[c * RP + il];
-      }
-    } else {
-#pragma unroll
-      for (int r = 0; r < TRPL; ++r) {
-        const int il = tid + TPT * r;
-        if (il >= nr) continue;
+      __syncthreads();
+      // -- write back the panel: first every row where it started, as float4
+      // runs of 4 rows (a warp writes 512 contiguous bytes of a column; R is a
+      // multiple of 4, so runs start 16-byte aligned in W when W and ldw allow);
+      // the rows that move (the pivots, and CTA 0's first jb rows that are not
+      // pivots) are written again to their final positions after the cluster
+      // barrier below, so that those writes land last
+      const bool vec = (ldw & 3) == 0 && (reinterpret_cast<uintptr_t>(W) & 15) == 0 && (R & 3) == 0;
+      if (vec) {
+        const int nq4 = nr / 4;
+        for (int e = tid; e < nq4 * jb; e += NT) {
+          const int il0 = 4 * (e % nq4), c = e / nq4;
+          *reinterpret_cast<float4 *>(&W[(r0 + il0) + (int64_t)c * ldw]) =
+              *reinterpret_cast<const float4 *>(&sp[c * RP + il0]);
+        }
+        for (int e = tid; e < (nr - 4 * nq4) * jb; e += NT) {
+          const int i2 = 4 * nq4 + e % (nr - 4 * nq4), c = e / (nr - 4 * nq4);
+          W[(r0 + i2) + (int64_t)c * ldw] = sp[c * RP + i2];
+        }
+      } else if (has) {
 #pragma unroll 8
-        for (int c = 0; c < jb; ++c) W[(r0 + il) + (int64_t)c * ldw] = sp[c * RP + il];
+        for (int c = 0; c < jb; ++c) W[(r0 + tid) + (int64_t)c * ldw] = sp[c * RP + tid];
       }
-    }
-    if (plan != nullptr && cr == 0 && warp == 0) list_panel_moves(win, posin, jb, col0, plan);
+      if (plan != nullptr && cr == 0 && warp == 0) list_panel_moves(win, posin, jb, col0, plan);
     }
   }
-  if (tid < C) sm100::bulk_wait_read0();  // this CTA's last pushes have read its staging slots
   cluster.sync();  // no CTA leaves while another may still push into it
   if constexpr (!SEL) {
     if (!failed) {
       // the rows that move, over their first write: the pivot of column t
       // (panel row win[t]) to position t, lanes on consecutive t; CTA 0's
       // first jb rows that are not pivots to where the interchanges put them
-      for (int e = tid; e < jb * jb; e += TPT) {
-        const int t = e % jb, c = e / jb, x = win[t];
-        if (x >= r0 && x < r1) W[t + (int64_t)c * ldw] = sp[c * RP + (x - r0)];
+      for (int e = tid; e < jb * jb; e += NT) {
+        const int t = e % jb, c = e / jb, row = win[t];
+        if (row >= r0 && row < r1) W[t + (int64_t)c * ldw] = sp[c * RP + (row - r0)];
       }
       if (cr == 0)
-        for (int e = tid; e < jb * jb; e += TPT) {
-          const int il = e % jb, c = e / jb;
-          if (rstate[il] < 0) W[posin[il] + (int64_t)c * ldw] = sp[c * RP + il];
+        for (int e = tid; e < jb * jb; e += NT) {
+          const int i2 = e % jb, c = e / jb;
+          if (rstate[i2] < 0) W[posin[i2] + (int64_t)c * ldw] = sp[c * RP + i2];
         }
     }
   }
 }
 
 template <typename G>
-int launch_tpanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t *ipiv, int32_t col0,
+int launch_ppanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t *ipiv, int32_t col0,
                   int32_t *info, int32_t *plan, uint64_t *track, double give_up, int32_t *err,
                   int32_t *winout = nullptr, G *sel = nullptr) {
-  const int C = (int)imin(SMAXC, imax(1, cdiv(mp, TPT)));
-  // rows per CTA, a multiple of 4 (the write-back's float4 runs); C <= 16
-  // keeps the last CTA's share positive: mp > 256 (C - 1) > 4 C (C - 1)
+  // (CTA 0 holds the panel's first jb rows: the interchange bookkeeping)
+  const int C = (int)imin(SMAXC, imax(1, cdiv(mp, PP_CTA_ROWS)));
+  // rows per CTA, a multiple of 4 (the write-back's float4 runs)
   const int64_t R = cdiv(cdiv(mp, C), 4) * 4;
-  // CTA 0 must hold the panel's first jb rows (the interchange bookkeeping)
-  if (R > (int64_t)TPT * TRPL || R < jb)
+  if (R > PP_MAXR || R < jb)
     return fail(BOLA_ERR_UNSUPPORTED, "mixed LU: panel of %lld x %d not supported", (long long)mp, jb);
-  const size_t smem = tpanel_smem(R, C);
   static bool attr = false;
   if (!attr) {
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(tpanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(tpanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)tpanel_smem(TPT * TRPL, SMAXC)));
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)ppanel_smem(PP_MAXR)));
     attr = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)C, 1, 1);
-  cfg.blockDim = dim3(TPT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.blockDim = dim3((unsigned)imax(64, cdiv(R, 32) * 32), 1, 1);
+  cfg.dynamicSmemBytes = ppanel_smem(R);
   cfg.stream = s;
   cudaLaunchAttribute at[2];  // the cluster; a programmatic dependent of the previous step's kernel
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -682,9 +412,9 @@ int launch_tpanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  ProfScope prof(s, std::is_same<G, double>::value ? "tselect64" : "tpanel", (double)mp * jb * jb,
+  ProfScope prof(s, std::is_same<G, double>::value ? "select64" : "ppanel", (double)mp * jb * jb,
                  8.0 * (double)mp * jb);
-  BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, tpanel_kernel<G>, W, ldw, mp, jb, ipiv, col0, info, R, plan, track,
+  BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, ppanel_kernel<G>, W, ldw, mp, jb, ipiv, col0, info, R, plan, track,
                                    give_up, err, winout, sel));
   return 0;
 }
@@ -694,10 +424,10 @@ int launch_tpanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t
 // exchange, four CTA barriers and the column's FP64 update confined to the
 // panel's CTAs.  The FP64-storage factor splits its panel instead, as
 // communication-avoiding LU (CALU) does:
-//   1. tpanel_kernel<double> chooses the jb pivot rows by tournament on FP32
+//   1. ppanel_kernel<double> chooses the jb pivot rows on FP32
 //      copies of the panel (W's column blocks are scaled to O(1), and FP32
 //      is ample for choosing pivots);
-//   2. panel_lu64 factors the panel in FP64 in the tournament's pivot order
+//   2. panel_lu64 factors the panel in FP64 in that pivot order
 //      without further pivoting (CALU's final step): the selected block and
 //      the rows below it, on one CTA per 64 rows, each factoring the block
 //      itself; it derives LAPACK's interchanges, puts the rows they displace
@@ -719,7 +449,7 @@ __device__ __forceinline__ double recip64(double p) {
 }
 
 // Steps 2 and 3 of the panel above in one launch (Wp: the panel's top-left,
-// rows col0.. of W).  The tournament has fixed the pivot order (row win[q]
+// rows col0.. of W).  The selection has fixed the pivot order (row win[q]
 // is the pivot of column q, chosen by partial pivoting among the nominees),
 // so the panel is factored without further pivoting, as CALU's last step
 // does: the selected block and every row below it go through the same 64
@@ -1292,11 +1022,11 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
     const int buf = (int)(k & 1);
     int32_t *plan_k = lu.plan + k * PLAN_STRIDE;  // this panel's moves, kept for apply_left_swaps
     if constexpr (fp64) {
-      // pivot rows by tournament on FP32 copies, then the FP64 factorisation
+      // pivot rows chosen on FP32 copies, then the FP64 factorisation
       // of the selected block and of the rows below it
       double *Wp = W + j + j * ldw;
       int32_t *win = lu.plan + (int64_t)PLAN_STRIDE * cdiv(lu.cap_n, SNB);
-      BOLA_TRY(launch_tpanel<double>(lu.sp, Wp, ldw, mp, jb, ipiv + j, (int32_t)j, info, nullptr, track, give_up,
+      BOLA_TRY(launch_ppanel<double>(lu.sp, Wp, ldw, mp, jb, ipiv + j, (int32_t)j, info, nullptr, track, give_up,
                                      lu.err, win, lu.sel));
       {
         ProfScope prof(lu.sp, "panel_lu64", (double)jb * jb * jb * 2.0 / 3.0 + (double)(mp - jb) * jb * jb,
@@ -1314,7 +1044,7 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
       }
       BOLA_CHECK_LAUNCH();
     } else
-      BOLA_TRY(launch_tpanel(lu.sp, W + j + j * ldw, ldw, mp, jb, ipiv + j, (int32_t)j, info, plan_k, track,
+      BOLA_TRY(launch_ppanel(lu.sp, W + j + j * ldw, ldw, mp, jb, ipiv + j, (int32_t)j, info, plan_k, track,
                              give_up, lu.err));
     // the row swaps reach every column: the previous wide update must be done
     if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(lu.sp, lu.ev_wide, 0));

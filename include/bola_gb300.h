@@ -80,7 +80,7 @@ int bola_measure_dmma_peak(double *gflops);
  * into every CTA of the cluster with bulk copies that complete on the
  * receiver's mbarrier, then wait for their own arrivals (bounded) and meet a
  * CTA barrier.  *us_per_round gets the time per round (microseconds), the
- * floor of the mixed LU panels' serial chain per pivot group.  Synchronises
+ * floor of the mixed LU panels' serial chain per exchange.  Synchronises
  * the device. */
 int bola_measure_cluster_exchange(int csize, int bytes, double *us_per_round);
 
@@ -173,9 +173,8 @@ int bola_sgemm_tc_update(int kind, int64_t m, int64_t n, const void *a, const vo
 /* The low-precision LU of bola_dgesv_mixed alone (no BOLA counterpart;
  * exposed for testing and profiling): W (n x n FP32, column-major, ld ldw,
  * n <= 8192) is replaced by P W = L U (unit-lower L below the diagonal, U on
- * and above), blocked right-looking with 64-column panels whose pivots are
- * chosen by tournament (8-column groups) and tcgen05 trailing updates of the
- * given kind (0 bf16, 1 tf32, 2 3xTF32).  ipiv (device, n entries) gets
+ * and above), blocked right-looking with partially pivoted 64-column panels
+ * and tcgen05 trailing updates of the given kind (0 bf16, 1 tf32, 2 3xTF32).  ipiv (device, n entries) gets
  * LAPACK-style 1-based interchanges, *info (device) the first exact-zero
  * pivot (1-based) or 0.  Synchronous. */
 int bola_sgetrf_mixed(int kind, int64_t n, float *w, int64_t ldw, int32_t *ipiv, int32_t *info,
