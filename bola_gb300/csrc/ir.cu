@@ -35,32 +35,39 @@ constexpr int TB = 64;      // triangular-solve block (= LU block)
 constexpr int MAXRHS = 32;  // right-hand sides per refinement sweep
 
 // ---- scaling and conversion -------------------------------------------------------
-// Per 64-column block the largest |a| (a CTA per block and slice of rows,
-// every thread's loads of 4 columns in flight together), folded with 64-bit
-// atomics into mbits as the bits of a non-negative double (they order like
-// the values; mbits starts at zero); colblock_finish then turns it in place
-// into the block's scale 2^-e with max|a| in [2^(e-1), 2^e).  A NaN is
-// passed over, as fmax does.
+// These kernels read A once and are bound by HBM: no FP64 instruction (16
+// cycles of an SM each, more than the element's bytes take) on the common
+// path, no index division, eight loads in flight per thread.  Measured at
+// n = 8192, launches serialised: colblock_max 106 us (280 with fmax), convert_scaled
+// to FP32 137 us (261 with a multiplication and a division per element).
+// Per 64-column block the largest |a| (a CTA per block and slice of rows),
+// compared as the bits of a non-negative double (they order like the values)
+// and folded with 64-bit atomics into mbits, which starts at zero;
+// colblock_finish then turns it in place into the block's scale 2^-e with
+// max|a| in [2^(e-1), 2^e).  A NaN is passed over.
 __global__ void __launch_bounds__(256)
 colblock_max(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *mbits) {
-  __shared__ double red[8];
+  __shared__ uint64_t red[8];
   const int64_t c0 = (int64_t)blockIdx.x * TB, c1 = imin(n, c0 + TB);
   const int64_t rs = cdiv(n, (int64_t)gridDim.y), r0 = (int64_t)blockIdx.y * rs, r1 = imin(n, r0 + rs);
-  double m = 0.0;
-  for (int64_t c = c0; c < c1; c += 4)
+  uint64_t m = 0;
+  for (int64_t c = c0; c < c1; c += 8)
     for (int64_t i = r0 + threadIdx.x; i < r1; i += 256) {
-      double v[4];
+      uint64_t v[8];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = c + u < c1 ? fabs(A[i + (c + u) * lda]) : 0.0;
+      for (int u = 0; u < 8; ++u) v[u] = c + u < c1 ? oz_mag(A[i + (c + u) * lda]) : 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) m = fmax(m, v[u]);
+      for (int u = 0; u < 8; ++u) m = v[u] > m && v[u] <= 0x7ff0000000000000ull ? v[u] : m;
     }
-  for (int off = 16; off > 0; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = 16; off > 0; off >>= 1) {
+    const uint64_t o = __shfl_xor_sync(0xffffffffu, m, off);
+    m = o > m ? o : m;
+  }
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < 8; ++w) m = fmax(m, red[w]);
-    atomicMax(mbits + blockIdx.x, (unsigned long long)__double_as_longlong(m));
+    for (int w = 1; w < 8; ++w) m = red[w] > m ? red[w] : m;
+    atomicMax(mbits + blockIdx.x, (unsigned long long)m);
   }
 }
 __global__ void colblock_finish(int64_t nb, double *scale) {
@@ -72,14 +79,54 @@ __global__ void colblock_finish(int64_t nb, double *scale) {
   scale[b] = (mm > 0.0 && isfinite(mm)) ? ldexp(1.0, -e) : 1.0;
 }
 
-// W = A S rounded to T (exact for T = double: S is a power of two per block).
+// The exponent k of a power of two 2^k that is a normal number; EXP_SLOW for any
+// other (no sum with it stays in range, so its products are multiplied out).
+constexpr int EXP_SLOW = 1 << 20;
+__device__ __forceinline__ int pow2_exponent(double p) {
+  const int e = (int)((uint64_t)__double_as_longlong(p) >> 52);
+  return e > 0 && e < 2047 ? e - 1023 : EXP_SLOW;
+}
+
+// (T)(v 2^k1 2^k2) for powers of two p1 = 2^k1, p2 = 2^k2, as the
+// multiplications and the conversion give it: on the exponent field, with the
+// significand rounded to nearest even for float, when v, the product after p1
+// and the result are normal numbers; a zero stays with scales that are; anything else
+// is multiplied out.
 template <typename T>
-__global__ void convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const double *scale,
-                               T *__restrict__ W, int64_t ldw) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n * n) return;
-  const int64_t i = e % n, j = e / n;
-  W[i + j * ldw] = (T)(A[i + j * lda] * scale[j / TB]);
+__device__ __forceinline__ T scaled_pow2(double v, int k1, double p1, int k2, double p2) {
+  const uint64_t bits = (uint64_t)__double_as_longlong(v), mag = bits & 0x7fffffffffffffffull;
+  const int e0 = (int)(mag >> 52), e1 = e0 + k1, e2 = e1 + k2;
+  constexpr bool F = std::is_same<T, float>::value;
+  const bool normal = e0 > 0 && e0 < 2047 && e1 > 0 && e1 < 2047 && e2 > (F ? 1023 - 127 : 0) &&
+                      e2 < (F ? 1023 + 128 : 2047);
+  if (!normal && (mag != 0 || k1 == EXP_SLOW || k2 == EXP_SLOW)) return (T)(v * p1 * p2);
+  if constexpr (F) {
+    const uint64_t t = normal ? mag + ((uint64_t)(int64_t)(k1 + k2 - (1023 - 127)) << 52) : 0;
+    const uint32_t cut = (uint32_t)t & 0x1fffffffu, keep = (uint32_t)(t >> 29);
+    const uint32_t f = keep + (cut + (keep & 1u) > 0x10000000u ? 1u : 0u);
+    return __uint_as_float(f | ((uint32_t)(bits >> 32) & 0x80000000u));
+  } else {
+    return __longlong_as_double((long long)(normal ? bits + ((uint64_t)(int64_t)(k1 + k2) << 52) : bits));
+  }
+}
+
+// W = A S rounded to T (exact for T = double: S is a power of two per block).
+// A thread: a row, CVT_COLS columns (of one block: CVT_COLS divides TB).
+constexpr int CVT_COLS = 8;
+template <typename T>
+__global__ void __launch_bounds__(256)
+convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const double *scale, T *__restrict__ W,
+               int64_t ldw) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
+  if (i >= n) return;
+  const double p = scale[j0 / TB];
+  const int k = pow2_exponent(p);
+  double v[CVT_COLS];
+#pragma unroll
+  for (int u = 0; u < CVT_COLS; ++u) v[u] = j0 + u < n ? A[i + (j0 + u) * lda] : 0.0;
+#pragma unroll
+  for (int u = 0; u < CVT_COLS; ++u)
+    if (j0 + u < n) W[i + (j0 + u) * ldw] = scaled_pow2<T>(v[u], k, p, 0, 1.0);
 }
 
 // max|u_ii| and min|u_ii| of the low-precision U (one CTA): a cheap lower
@@ -218,13 +265,22 @@ __global__ void sym_scale(int64_t n, const double *__restrict__ A, int64_t lda, 
 
 // W = fl(D A D), lower triangle only (the Cholesky reads no other part).
 template <typename T>
-__global__ void convert_sym_lower(int64_t n, const double *__restrict__ A, int64_t lda, const double *d,
-                                  T *__restrict__ W, int64_t ldw) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n * n) return;
-  const int64_t i = e % n, j = e / n;
-  if (i < j) return;
-  W[i + j * ldw] = (T)(A[i + j * lda] * d[i] * d[j]);
+__global__ void __launch_bounds__(256)
+convert_sym_lower(int64_t n, const double *__restrict__ A, int64_t lda, const double *d, T *__restrict__ W,
+                  int64_t ldw) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
+  if (i >= n || i < j0) return;
+  const double pi = d[i];
+  const int ki = pow2_exponent(pi);
+  double v[CVT_COLS];
+#pragma unroll
+  for (int u = 0; u < CVT_COLS; ++u) v[u] = j0 + u <= i ? A[i + (j0 + u) * lda] : 0.0;
+#pragma unroll
+  for (int u = 0; u < CVT_COLS; ++u)
+    if (j0 + u <= i) {
+      const double pj = d[j0 + u];
+      W[i + (j0 + u) * ldw] = scaled_pow2<T>(v[u], ki, pi, pow2_exponent(pj), pj);
+    }
 }
 
 __global__ void iota_perm(int64_t n, int32_t *perm) {
@@ -1281,14 +1337,15 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   double *nrm = w.norms;  // [0..nr): ||r||, [nr..2nr): ||x||, [2nr..3nr): ||b||, [3nr]: ||A||
 
   // scale, convert, factor
+  const dim3 cvt((unsigned)cdiv(n, 256), (unsigned)cdiv(n, CVT_COLS));
   if (chol) {
     // W = D A D (lower triangle), D a power of two per row making the diagonal O(1)
     ProfScope prof(s, "mixed_convert", 0.0, 6.0 * (double)n * n, 2);
     sym_scale<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, a, lda, w.dscale);
     if (fp64)
-      convert_sym_lower<double><<<(unsigned)cdiv(n * n, 256), 256, 0, s>>>(n, a, lda, w.dscale, (double *)w.W, ldW);
+      convert_sym_lower<double><<<cvt, 256, 0, s>>>(n, a, lda, w.dscale, (double *)w.W, ldW);
     else
-      convert_sym_lower<float><<<(unsigned)cdiv(n * n, 256), 256, 0, s>>>(n, a, lda, w.dscale, (float *)w.W, n);
+      convert_sym_lower<float><<<cvt, 256, 0, s>>>(n, a, lda, w.dscale, (float *)w.W, n);
   } else {
     ProfScope prof(s, "mixed_convert", 0.0, 12.0 * (double)n * n, 3);
     BOLA_TRY_CUDA(cudaMemsetAsync(w.scale, 0, sizeof(double) * cdiv(n, TB), s));
@@ -1296,9 +1353,9 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
         n, a, lda, reinterpret_cast<unsigned long long *>(w.scale));
     colblock_finish<<<(unsigned)cdiv(cdiv(n, TB), 256), 256, 0, s>>>(cdiv(n, TB), w.scale);
     if (fp64)
-      convert_scaled<double><<<(unsigned)cdiv(n * n, 256), 256, 0, s>>>(n, a, lda, w.scale, (double *)w.W, ldW);
+      convert_scaled<double><<<cvt, 256, 0, s>>>(n, a, lda, w.scale, (double *)w.W, ldW);
     else
-      convert_scaled<float><<<(unsigned)cdiv(n * n, 256), 256, 0, s>>>(n, a, lda, w.scale, (float *)w.W, n);
+      convert_scaled<float><<<cvt, 256, 0, s>>>(n, a, lda, w.scale, (float *)w.W, n);
   }
   BOLA_CHECK_LAUNCH();
   // A's digit planes and its row sums (once per call: a solve handed on to

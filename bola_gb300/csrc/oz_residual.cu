@@ -59,7 +59,7 @@ constexpr int32_t NONFINITE = 0x7fffffff;  // exponent marker of a row or column
 // X = round(v 2^(8 NS - 1 - e)), then signed base-256 digits, most
 // significant first: v ~ 2^(e - 7) sum_t s_t 2^(-8t), |s_t| <= 128.
 template <int NS>
-__device__ __forceinline__ void digits(double v, int e, int32_t (&s)[NS]) {
+__device__ __forceinline__ int64_t fixed_point(double v, int e) {  // X
   const uint64_t bits = (uint64_t)__double_as_longlong(v);
   const int ev = (int)((bits >> 52) & 0x7FF);
   int64_t X = 0;
@@ -70,6 +70,11 @@ __device__ __forceinline__ void digits(double v, int e, int32_t (&s)[NS]) {
     else if (k < 64) X = (int64_t)((M + (1ull << (k - 1))) >> k);
     if (bits >> 63) X = -X;
   }
+  return X;
+}
+template <int NS>
+__device__ __forceinline__ void digits(double v, int e, int32_t (&s)[NS]) {
+  int64_t X = fixed_point<NS>(v, e);
 #pragma unroll
   for (int t = NS - 1; t > 0; --t) {
     const int d = (int)((X + 128) & 255) - 128;
@@ -86,25 +91,34 @@ __device__ __forceinline__ int32_t exponent_of(uint64_t mag_bits) {
 }
 
 // Row statistics of A in one pass: max|a_ij| (as ordered bits, atomicMax)
-// and, per 512-column block, the partial row sums of |a_ij| (summed in a
+// and, per SCH-column block, the partial row sums of |a_ij| (summed in a
 // fixed order afterwards: the norm must not depend on scheduling).  CTA:
-// 128 rows x 512 columns, two column halves of 256 threads.
+// 128 rows x SCH columns, two column halves of 256 threads, eight loads in
+// flight each, so that small matrices fill the chip: measured at n = 1500
+// 14 us, at n = 8192 261; blocks of 512 columns, one load in flight, took
+// 55 and 275.
+constexpr int SCH = 128;
 __global__ void __launch_bounds__(256)
 oz_row_stats(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *rmax, double *psum) {
   __shared__ double red[128];
   __shared__ unsigned long long mred[128];
   const int r = threadIdx.x & 127, h = threadIdx.x >> 7;
   const int64_t i = (int64_t)blockIdx.x * 128 + r;
-  const int64_t c0 = (int64_t)blockIdx.y * KCH;
-  const int64_t c1 = imin(n, c0 + KCH);
+  const int64_t c0 = (int64_t)blockIdx.y * SCH;
+  const int64_t c1 = imin(n, c0 + SCH);
   double s = 0.0;
   uint64_t m = 0;
   if (i < n)
-    for (int64_t c = c0 + h; c < c1; c += 2) {
-      const double v = A[i + c * lda];
-      s += fabs(v);
-      const uint64_t b = oz_mag(v);
-      m = b > m ? b : m;
+    for (int64_t c = c0 + h; c < c1; c += 16) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = c + 2 * u < c1 ? A[i + (c + 2 * u) * lda] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        s += fabs(v[u]);
+        const uint64_t b = oz_mag(v[u]);
+        m = b > m ? b : m;
+      }
     }
   if (h == 1) {
     red[r] = s;
@@ -125,6 +139,7 @@ __global__ void oz_row_finish(int64_t n, int nblk, const unsigned long long *rma
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double s = 0.0;
+#pragma unroll 8
   for (int b = 0; b < nblk; ++b) s += psum[(int64_t)b * n + i];
   if (rowsum) rowsum[i] = s;
   e[i] = exponent_of(rmax[i]);
@@ -132,6 +147,9 @@ __global__ void oz_row_finish(int64_t n, int nblk, const unsigned long long *rma
 
 // A's digit planes, row-major: plane t, row i at ((t * mrows + i) * kp).
 // CTA: a 64 x 64 tile, staged through shared memory (column-major in, rows out).
+// Bound by HBM (2 SA bytes written per 8 read): measured at n = 8192 330 us,
+// of which the bytes take 210; with the digits peeled off one after the other
+// and converted one by one, 400.
 __global__ void __launch_bounds__(256)
 oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int32_t *__restrict__ e, int64_t mrows,
                 int64_t kp, __nv_bfloat16 *__restrict__ out) {
@@ -148,21 +166,24 @@ oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int3
     const int64_t i = i0 + r, j = j0 + 2 * p;
     if (i >= n || j >= n) continue;
     const int32_t ei = e[i];
-    int32_t d0[SA], d1[SA];
-    if (ei == NONFINITE) {
+    // all digits at once: X + 128 sum_t 256^t holds digit t + 128 in byte t
+    // (the leading one, up to 128 + 128, in the 16 bits above byte 5); each
+    // becomes the float 2^23 + byte - (2^23 + 128), exact, of eight
+    // significant bits at most: its upper half is the bf16
+    static_assert(SA == 7, "the digits fill seven bytes");
+    constexpr uint64_t BIAS = 0x0080808080808080ull;
+    const uint64_t x0 = BIAS + (ei == NONFINITE ? 0ull : (uint64_t)fixed_point<SA>(T[r][2 * p], ei));
+    const uint64_t x1 = BIAS + (ei == NONFINITE ? 0ull : (uint64_t)fixed_point<SA>(T[r][2 * p + 1], ei));
+    auto digit = [](uint64_t x, int t) {  // the float of digit t (0: the leading one)
+      const uint32_t word = t <= 2 ? (uint32_t)(x >> 32) : (uint32_t)x;
+      const uint32_t byte = (SA - 1 - t) & 3;
+      const uint32_t f = __byte_perm(word, 0x4b000000u, t == 0 ? 0x7432u : 0x7440u + byte);
+      return __uint_as_float(f) - 8388736.f;
+    };
 #pragma unroll
-      for (int t = 0; t < SA; ++t) d0[t] = d1[t] = 0;
-    } else {
-      digits<SA>(T[r][2 * p], ei, d0);
-      digits<SA>(T[r][2 * p + 1], ei, d1);
-    }
-#pragma unroll
-    for (int t = 0; t < SA; ++t) {
-      __nv_bfloat162 w;
-      w.x = __int2bfloat16_rn(d0[t]);
-      w.y = __int2bfloat16_rn(d1[t]);
-      *reinterpret_cast<__nv_bfloat162 *>(out + ((int64_t)t * mrows + i) * kp + j) = w;
-    }
+    for (int t = 0; t < SA; ++t)
+      *reinterpret_cast<uint32_t *>(out + ((int64_t)t * mrows + i) * kp + j) =
+          __byte_perm(__float_as_uint(digit(x0, t)), __float_as_uint(digit(x1, t)), 0x7632);
   }
 }
 
@@ -409,10 +430,10 @@ int OzMatrix::reserve(int64_t n_) {
   BOLA_TRY(al(reinterpret_cast<void **>(&e), sizeof(int32_t) * mr));
   BOLA_TRY(al(reinterpret_cast<void **>(&f), sizeof(int32_t) * NRB));
   BOLA_TRY(al(reinterpret_cast<void **>(&rmax), sizeof(unsigned long long) * mr));
-  BOLA_TRY(al(reinterpret_cast<void **>(&psum), sizeof(double) * cdiv(n_, KCH) * n_));
+  BOLA_TRY(al(reinterpret_cast<void **>(&psum), sizeof(double) * cdiv(n_, SCH) * n_));
   BOLA_TRY(al(reinterpret_cast<void **>(&acc), sizeof(unsigned long long) * 2 * NRB * mr));
   bytes = (int64_t)(sizeof(__nv_bfloat16) * (SA * mr * k + SX * NRB * k) + sizeof(int32_t) * (mr + NRB) +
-                    sizeof(unsigned long long) * 3 * mr + sizeof(double) * cdiv(n_, KCH) * n_);
+                    sizeof(unsigned long long) * 3 * mr + sizeof(double) * cdiv(n_, SCH) * n_);
   cap = n_;
   n = n_;
   mrows = mr;
@@ -434,7 +455,7 @@ void OzMatrix::release() {
 // Splits A into its digit planes (and ||A||_inf's row sums into rowsum, if given).
 int OzMatrix::split(cudaStream_t s, const double *A, int64_t lda, double *rowsum) {
   ProfScope prof(s, "oz_split", 0.0, 8.0 * 2.0 * n * n + 2.0 * SA * n * n, 4);
-  const int nblk = (int)cdiv(n, KCH);
+  const int nblk = (int)cdiv(n, SCH);
   BOLA_TRY_CUDA(cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * n, s));
   oz_row_stats<<<dim3((unsigned)cdiv(n, 128), (unsigned)nblk), 256, 0, s>>>(n, A, lda, rmax, psum);
   oz_row_finish<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, nblk, rmax, psum, rowsum, e);
