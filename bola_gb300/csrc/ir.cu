@@ -289,44 +289,75 @@ __global__ void iota_perm(int64_t n, int32_t *perm) {
 }
 
 // Inverses of the 64x64 diagonal blocks of L (unit lower) and U, once per
-// factorisation: block b -> Dl[b], Du[b] (column-major 64x64).  A thread per
-// column of the inverse, substitution down (L) or up (U) the block.
+// factorisation: block b -> Dl[b], Du[b] (column-major 64x64).  Substitution
+// down (L) or up (U) the block, four threads per column of the inverse (rows
+// i = part mod 4, in registers), a warp on eight columns: a solved row goes to
+// the column's other threads by shuffle and every row still open takes it at
+// once, so a step of the chain is a shuffle and a multiply-add.  Steps before
+// a warp's first column (after its last, for U) only see zeros and are left
+// out; U's column groups are dealt so that every sub-partition gets the same
+// FP64 work.  Measured, launches
+// serialised: FP32, n = 1500, 43 -> 18 us; FP64, n = 2000, 228 -> 80 us with
+// the pivots' extent beside it, against a thread per column with each row's
+// products one dependent chain.
+constexpr int DI_THREADS = 512;
+__device__ __forceinline__ float quotient(float t, float d, const Divisor &) { return t / d; }
+__device__ __forceinline__ double quotient(double t, double, const Divisor &q) { return div_rn(t, q); }
+
 template <typename T>
-__global__ void __launch_bounds__(64)
+__global__ void __launch_bounds__(DI_THREADS)
 diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du) {
   __shared__ T B[TB][TB + 1];
+  __shared__ Divisor dv[TB];
+  const unsigned FULL = 0xffffffffu;
   const int64_t k0 = (int64_t)blockIdx.x * TB;
   const int kb = (int)imin(TB, n - k0);
   // the whole tile is written: the substitutions below multiply entries
   // outside the kb x kb block by zeros, and 0 * (stale NaN) would be NaN
-  for (int e = threadIdx.x; e < TB * TB; e += blockDim.x) {
+  for (int e = threadIdx.x; e < TB * TB; e += DI_THREADS) {
     const int r = e % TB, c = e / TB;
     B[r][c] = (r < kb && c < kb) ? W[(k0 + r) + (k0 + c) * ldw] : T(0);
   }
   __syncthreads();
-  const int j = threadIdx.x;
-  T *L = Dl + (int64_t)blockIdx.x * TB * TB, *U = Du + (int64_t)blockIdx.x * TB * TB;
-  if (j >= TB) return;
-  T x[TB];
+  if (std::is_same<T, double>::value && threadIdx.x < TB) dv[threadIdx.x] = divisor((double)B[threadIdx.x][threadIdx.x]);
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane & 3;
+  const bool lower = warp < 8;
+  const int m = warp & 7;
+  const int grp = lower ? m : 4 + (m & 3) - (m & 4);  // 8 columns each; work falls (L) / grows (U) with it
+  const int j = 8 * grp + (lane >> 2);
+  T x[16];  // row part + 4 q of column j
 #pragma unroll
-  for (int i = 0; i < TB; ++i) {  // L x = e_j (unit diagonal)
-    T t = (i == j) ? T(1) : T(0);
+  for (int q = 0; q < 16; ++q) x[q] = part + 4 * q == j ? T(1) : T(0);
+  if (lower) {
 #pragma unroll
-    for (int k = 0; k < i; ++k) t = fmaT(-B[i][k], x[k], t);
-    x[i] = (i < kb) ? t : T(0);
+    for (int g = 0; g < 8; ++g)
+      if (g >= grp) {
+#pragma unroll
+        for (int k = 8 * g; k < 8 * g + 8; ++k) {
+          const T xk = __shfl_sync(FULL, x[k / 4], k & 3, 4);
+#pragma unroll
+          for (int q = k / 4; q < 16; ++q)
+            if (part + 4 * q > k) x[q] = fmaT(-B[part + 4 * q][k], xk, x[q]);
+        }
+      }
+  } else {
+#pragma unroll
+    for (int g = 7; g >= 0; --g)
+      if (g <= grp) {
+#pragma unroll
+        for (int k = 8 * g + 7; k >= 8 * g; --k) {
+          if (part == (k & 3)) x[k / 4] = (k < kb && j < kb) ? quotient(x[k / 4], B[k][k], dv[k]) : T(0);
+          const T xk = __shfl_sync(FULL, x[k / 4], k & 3, 4);
+#pragma unroll
+          for (int q = 0; q <= k / 4; ++q)
+            if (part + 4 * q < k) x[q] = fmaT(-B[part + 4 * q][k], xk, x[q]);
+        }
+      }
   }
+  T *out = (lower ? Dl : Du) + (int64_t)blockIdx.x * TB * TB;
 #pragma unroll
-  for (int i = 0; i < TB; ++i) L[i + j * TB] = (j < kb) ? x[i] : T(0);
-#pragma unroll
-  for (int ii = 0; ii < TB; ++ii) {  // U x = e_j
-    const int i = TB - 1 - ii;
-    T t = (i == j) ? T(1) : T(0);
-#pragma unroll
-    for (int k = i + 1; k < TB; ++k) t = fmaT(-B[i][k], x[k], t);
-    x[i] = (i < kb && j < kb) ? t / B[i][i] : T(0);
-  }
-#pragma unroll
-  for (int i = 0; i < TB; ++i) U[i + j * TB] = x[i];
+  for (int q = 0; q < 16; ++q) out[part + 4 * q + j * TB] = (j < kb && part + 4 * q < kb) ? x[q] : T(0);
 }
 
 __device__ __forceinline__ int ld_acquire(const int32_t *p) {
@@ -1410,10 +1441,10 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
     ProfScope prof(s, "diag_inverses");
     const unsigned nb = (unsigned)cdiv(n, TB);
     if (fp64) {
-      diag_block_inverses<double><<<nb, TB, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl, (double *)w.Du);
+      diag_block_inverses<double><<<nb, DI_THREADS, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl, (double *)w.Du);
       diag_extent<double><<<1, 1024, 0, s>>>(n, (const double *)w.W, ldW, w.norms + 5 * MAXRHS);
     } else {
-      diag_block_inverses<float><<<nb, TB, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du);
+      diag_block_inverses<float><<<nb, DI_THREADS, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du);
       BOLA_TRY(couple(s, n, (const float *)w.W, n, (const float *)w.Dl, (const float *)w.Du,
                       const_cast<float *>(w.ts.Cl), const_cast<float *>(w.ts.Cu)));
       diag_extent<float><<<1, 1024, 0, s>>>(n, (const float *)w.W, n, w.norms + 5 * MAXRHS);
