@@ -39,17 +39,136 @@ __device__ __forceinline__ bool factor_stopped(const int32_t *info, const uint64
   return *(volatile const int32_t *)info != 0 || (track != nullptr && *(volatile const int32_t *)(track + 2) != 0);
 }
 
+// The U diagonal of the LU form is L_kk^2 = the pivots: their running extent and the give-up test.
+__device__ __forceinline__ void track_pivots(uint64_t *track, double umax, double umin, double give_up, int64_t done,
+                                             int64_t n) {
+  const uint64_t mx = (uint64_t)__double_as_longlong(umax), mn = (uint64_t)__double_as_longlong(umin);
+  if (mx > track[0]) track[0] = mx;
+  if (mn < track[1]) track[1] = mn;
+  const double gmx = __longlong_as_double((long long)track[0]), gmn = __longlong_as_double((long long)track[1]);
+  const double spread = gmn > 0.0 ? gmx / gmn : INFINITY;
+  if (give_up_now(spread, give_up, done, n)) *(volatile int32_t *)(track + 2) = 1;
+}
+
 // The diagonal block W[0:jb, 0:jb] (lower) = L11 L11^T, one CTA.  A pivot
 // that is not positive (or not finite) stops the factorisation: *info = its
 // global 1-based column, and every later kernel of the factorisation returns
 // at once.  Tracks max/min of L_kk^2 (the U diagonal of the LU form) and
 // gives up as the LU panel does.
 //
-// Bound by the chain of a column (square root, reciprocal, scale, the next
+//
+// FP32: a thread per row and group of eight columns, its eight values in
+// registers throughout.  A group's two warps take its 8 x 8 block through
+// shared memory, every thread factors it for itself (no exchange on the
+// chain of square roots) while solving its own row against it, and the groups
+// right of it then take the eight columns at once.  Bound by the chain of the
+// 64 square roots and reciprocals.  Measured on one GB300, launches
+// serialised: 18.5 us; 36 with one warp on the chain, a column at a time.
+constexpr int CD_T = CNB * CNB / 8;
+constexpr int XP = 12;  // pitch of a row of eight values: float4 reads by row meet no bank twice
+__global__ void __launch_bounds__(CD_T)
+chol_dblock32(float *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, uint64_t *track,
+              double give_up) {
+  __shared__ __align__(16) float D[8][8], X[2][CNB][XP];
+  __shared__ float piv[CNB];
+  __shared__ int stop;
+  sm100::grid_dependency_wait();
+  const int tid = threadIdx.x, i = tid & (CNB - 1), grp = tid / CNB;
+  if (tid == 0) stop = factor_stopped(info, track) ? 1 : 0;
+  float v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = i < jb && 8 * grp + c <= i ? W[i + (8 * grp + c) * ldw] : 0.f;
+  __syncthreads();
+  if (stop) return;
+  const int ngroups = (jb + 7) / 8;
+#pragma unroll 1
+  for (int g = 0; g < ngroups; ++g) {
+    const int kb = 8 * g, w = jb - kb < 8 ? jb - kb : 8;
+    if (grp == g) {
+      if (i / 8 == g) {
+        *reinterpret_cast<float4 *>(&D[i & 7][0]) = make_float4(v[0], v[1], v[2], v[3]);
+        *reinterpret_cast<float4 *>(&D[i & 7][4]) = make_float4(v[4], v[5], v[6], v[7]);
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(CNB) : "memory");
+      float d[8][8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c <= r; c += 4) {
+          const float4 q = *reinterpret_cast<const float4 *>(&D[r][c]);
+          d[r][c] = q.x;
+          d[r][c + 1] = q.y;
+          d[r][c + 2] = q.z;
+          d[r][c + 3] = q.w;
+        }
+      bool ok = true;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) {
+        if (p >= w || !ok) continue;  // (the same in every thread)
+        const float dp = d[p][p];
+        if (!positive(dp)) {
+          ok = false;
+          if (i == kb) {
+            stop = 1;
+            atomicCAS(info, 0, col0 + kb + p + 1);
+          }
+          continue;
+        }
+        if (i == kb) piv[kb + p] = dp;
+        const float r = sqrtT(dp), inv = recipT(r);
+        v[p] = i == kb + p ? r : v[p] * inv;
+#pragma unroll
+        for (int q = p + 1; q < 8; ++q) {
+          d[q][p] *= inv;
+          v[q] = fmaT(-v[p], d[q][p], v[q]);
+        }
+#pragma unroll
+        for (int q = p + 1; q < 8; ++q)
+#pragma unroll
+          for (int t = p + 1; t <= q; ++t) d[q][t] = fmaT(-d[q][p], d[t][p], d[q][t]);
+        if (i >= kb + p && i < jb) W[i + (kb + p) * ldw] = v[p];
+      }
+      float *x = X[g & 1][i];
+      *reinterpret_cast<float4 *>(x) = make_float4(v[0], v[1], v[2], v[3]);
+      *reinterpret_cast<float4 *>(x + 4) = make_float4(v[4], v[5], v[6], v[7]);
+    }
+    __syncthreads();
+    if (stop) return;
+    if (grp > g && (i | 31) >= 8 * grp) {  // (warps wholly above the diagonal have no part)
+      const float4 xa = *reinterpret_cast<const float4 *>(X[g & 1][i]);
+      const float4 xb = *reinterpret_cast<const float4 *>(X[g & 1][i] + 4);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const float4 ya = *reinterpret_cast<const float4 *>(X[g & 1][8 * grp + c]);
+        const float4 yb = *reinterpret_cast<const float4 *>(X[g & 1][8 * grp + c] + 4);
+        v[c] = fmaT(-xa.x, ya.x, v[c]);
+        v[c] = fmaT(-xa.y, ya.y, v[c]);
+        v[c] = fmaT(-xa.z, ya.z, v[c]);
+        v[c] = fmaT(-xa.w, ya.w, v[c]);
+        v[c] = fmaT(-xb.x, yb.x, v[c]);
+        v[c] = fmaT(-xb.y, yb.y, v[c]);
+        v[c] = fmaT(-xb.z, yb.z, v[c]);
+        v[c] = fmaT(-xb.w, yb.w, v[c]);
+      }
+    }
+  }
+  if (tid < 32 && track != nullptr) {
+    float mx = 0.f, mn = INFINITY;
+    for (int k = tid; k < jb; k += 32) {
+      mx = fmaxf(mx, piv[k]);
+      mn = fminf(mn, piv[k]);
+    }
+    for (int off = 16; off > 0; off >>= 1) {
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+      mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, off));
+    }
+    if (tid == 0) track_pivots(track, mx, mn, give_up, col0 + jb, n);
+  }
+}
+
+// FP64: bound by the chain of a column (square root, reciprocal, scale, the next
 // column's update): one warp walks it, two rows per lane, while eight warps
-// apply each finished column to the columns after the next one.  Measured on
-// one GB300 with L21 of 1400 rows after it: @@D us a panel in FP32 (82 with
-// three CTA barriers a column and a division per updated element's index).
+// apply each finished column to the columns after the next one.
 constexpr int CH_UPD = 8;
 constexpr int CH_T = 32 * (1 + CH_UPD);
 constexpr int CHP = CNB + 1;  // pitch: column j of row i at a[j * CHP + i]
@@ -62,11 +181,12 @@ __device__ __forceinline__ void ch_arrive(int id) {
   __syncwarp();
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(CH_T) : "memory");
 }
-template <typename T>
 __global__ void __launch_bounds__(CH_T)
-chol_dblock(T *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, uint64_t *track, double give_up) {
+chol_dblock64(double *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, uint64_t *track, double give_up) {
+  using T = double;
   __shared__ T a[CNB * CHP];
   __shared__ int stop;
+  sm100::grid_dependency_wait();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   if (tid == 0) stop = factor_stopped(info, track) ? 1 : 0;
   __syncthreads();
@@ -143,32 +263,30 @@ chol_dblock(T *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *info, u
     const int i = e % jb, j = e / jb;
     if (i >= j) W[i + j * ldw] = a[j * CHP + i];
   }
-  if (tid == 0 && track != nullptr && !stop) {
-    // the U diagonal of the LU form is L_kk^2 = the pivots: their running extent and the give-up test
-    const uint64_t mx = (uint64_t)__double_as_longlong((double)umax), mn = (uint64_t)__double_as_longlong((double)umin);
-    if (mx > track[0]) track[0] = mx;
-    if (mn < track[1]) track[1] = mn;
-    const double gmx = __longlong_as_double((long long)track[0]), gmn = __longlong_as_double((long long)track[1]);
-    const double spread = gmn > 0.0 ? gmx / gmn : INFINITY;
-    if (give_up_now(spread, give_up, col0 + jb, n)) *(volatile int32_t *)(track + 2) = 1;
-  }
+  if (tid == 0 && track != nullptr && !stop) track_pivots(track, umax, umin, give_up, col0 + jb, n);
 }
 
-// L21 = W21 L11^-T for the rows jb..mp-1 of the panel (one thread per row),
-// written back to W and as row (row - jb) of the update's K-major operand.
-// Eight columns at a time: their eight sums, in registers, take the earlier
-// columns in order from shared memory (one value of the row's and eight of
-// L11's per step), then each other; so eight chains are in flight and the loop
-// stays in the instruction cache, where 64 columns unrolled into one chain each
-// did neither.
+// L21 = W21 L11^-T for the rows jb..mp-1 of the panel, written back to W and
+// as row (row - jb) of the update's K-major operand.  A lane per row (32 rows
+// per CTA), a warp per group of eight columns, its values in registers: the
+// groups solve in turn against L11's diagonal 8 x 8 blocks and the ones right
+// of them take the eight columns at once (a warp reads L11 by broadcast), so
+// the chain is 64 multiplications and eight barriers.  Measured on one GB300
+// with 1400 rows, launches serialised: FP32 7 us (21 with a thread per row),
+// FP64 38 (95).
 template <typename T>
 struct alignas(16) Vec8 {
   T v[8];
 };
-constexpr int L21_T = 64;
+constexpr int L21_R = 32;
+constexpr int L21_T = 8 * L21_R;
+template <typename T>
+__host__ __device__ constexpr int l21_pitch() {  // of a row of eight values: 16-byte reads by row meet no bank twice
+  return sizeof(T) == 4 ? 12 : 10;
+}
 template <typename T>
 constexpr size_t l21_smem() {
-  return sizeof(T) * (CNB * CNB + CNB + CNB * L21_T);
+  return sizeof(T) * (CNB * CNB + CNB + 2 * L21_R * l21_pitch<T>());
 }
 template <typename T>
 __global__ void __launch_bounds__(L21_T)
@@ -177,55 +295,76 @@ chol_l21(T *W, int64_t ldw, int64_t mp, int jb, int kind, void *aop, float *aop_
   extern __shared__ __align__(16) unsigned char l21_raw[];
   T *Lt = reinterpret_cast<T *>(l21_raw);  // L(k, q) at Lt[q * CNB + k]
   T *rd = Lt + CNB * CNB;
-  T *vs = rd + CNB + threadIdx.x;  // this thread's value k at vs[k * L21_T]
+  T *X = rd + CNB;  // the group's columns of row r at X[(g & 1) L21_R * XPT + r * XPT]
+  constexpr int XPT = l21_pitch<T>();
+  __shared__ uint64_t mag[8][L21_R];
   __shared__ int stop;
-  if (threadIdx.x == 0) stop = factor_stopped(info, track) ? 1 : 0;
-  __syncthreads();
-  if (stop) return;
-  for (int e = threadIdx.x; e < CNB * CNB; e += L21_T) {
+  sm100::grid_dependency_wait();
+  const int tid = threadIdx.x, r = tid & 31, grp = tid >> 5;
+  if (tid == 0) stop = factor_stopped(info, track) ? 1 : 0;
+  const int64_t row = jb + (int64_t)blockIdx.x * L21_R + r;
+  T v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) v[c] = 8 * grp + c < jb && row < mp ? W[row + (8 * grp + c) * ldw] : T(0);
+#pragma unroll 8
+  for (int e = tid; e < CNB * CNB; e += L21_T) {
     const int i = e % CNB, j = e / CNB;
     Lt[e] = (i < jb && j < jb && i >= j) ? W[i + j * ldw] : T(0);
   }
-  const int64_t row = jb + (int64_t)blockIdx.x * L21_T + threadIdx.x;
-#pragma unroll 16
-  for (int k = 0; k < CNB; ++k) vs[k * L21_T] = k < jb && row < mp ? W[row + k * ldw] : T(0);
   __syncthreads();
-  for (int k = threadIdx.x; k < CNB; k += L21_T) rd[k] = k < jb ? recipT(Lt[k * (CNB + 1)]) : T(0);
+  if (stop) return;
+  if (tid < CNB) rd[tid] = tid < jb ? recipT(Lt[tid * (CNB + 1)]) : T(0);
   __syncthreads();
-  if (row >= mp) return;
 #pragma unroll 1
-  for (int kb = 0; kb < CNB; kb += 8) {
-    T x[8];
+  for (int g = 0; g < 8; ++g) {
+    T *x = X + ((g & 1) * L21_R + r) * XPT;
+    if (grp == g) {
 #pragma unroll
-    for (int r = 0; r < 8; ++r) x[r] = vs[(kb + r) * L21_T];
-#pragma unroll 4
-    for (int q = 0; q < kb; ++q) {
-      const T vq = vs[q * L21_T];
-      const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + q * CNB + kb);
+      for (int p = 0; p < 8; ++p) {
+        const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + (8 * g + p) * CNB + 8 * g);
+        v[p] *= rd[8 * g + p];  // zero beyond jb (rd = 0 there)
 #pragma unroll
-      for (int r = 0; r < 8; ++r) x[r] = fmaT(-vq, l.v[r], x[r]);
+        for (int q = p + 1; q < 8; ++q) v[q] = fmaT(-v[p], l.v[q], v[q]);
+      }
+      Vec8<T> o;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) o.v[p] = v[p];
+      *reinterpret_cast<Vec8<T> *>(x) = o;
     }
+    __syncthreads();
+    if (grp > g) {
+      const Vec8<T> xr = *reinterpret_cast<const Vec8<T> *>(x);
 #pragma unroll
-    for (int p = 0; p < 8; ++p) {
-      const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + (kb + p) * CNB + kb);
-      x[p] *= rd[kb + p];  // zero beyond jb (rd = 0 there)
+      for (int p = 0; p < 8; ++p) {
+        const Vec8<T> l = *reinterpret_cast<const Vec8<T> *>(Lt + (8 * g + p) * CNB + 8 * grp);
 #pragma unroll
-      for (int r = p + 1; r < 8; ++r) x[r] = fmaT(-x[p], l.v[r], x[r]);
+        for (int q = 0; q < 8; ++q) v[q] = fmaT(-xr.v[p], l.v[q], v[q]);
+      }
     }
-#pragma unroll
-    for (int r = 0; r < 8; ++r) vs[(kb + r) * L21_T] = x[r];
   }
-  T v[CNB];
+  if (row < mp)
 #pragma unroll
-  for (int k = 0; k < CNB; ++k) {
-    v[k] = vs[k * L21_T];
-    if (k < jb) W[row + k * ldw] = v[k];
-  }
+    for (int c = 0; c < 8; ++c)
+      if (8 * grp + c < jb) W[row + (8 * grp + c) * ldw] = v[c];
   if (aop == nullptr) return;
   if constexpr (sizeof(T) == 4) {
-    write_operand_row(kind, aop, aop_lo, row - jb, v);
+    if (row < mp) write_operand_part(kind, aop, aop_lo, row - jb, 8 * grp, v);
   } else {
-    write_slices_row(v, row - jb, cap, static_cast<__nv_bfloat16 *>(aop), aexp);
+    uint64_t m = 0;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const uint64_t mc = oz_mag(v[c]);
+      m = mc > m ? mc : m;
+    }
+    mag[grp][r] = m;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) m = mag[q][r] > m ? mag[q][r] : m;
+    if (row < mp) {
+      const int e = oz_exponent(m);
+      if (grp == 0) aexp[row - jb] = e;
+      write_slices_part(v, e, row - jb, 8 * grp, cap, static_cast<__nv_bfloat16 *>(aop));
+    }
   }
 }
 
@@ -296,14 +435,17 @@ int chol_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int32_t *info
     {
       ProfScope prof(lu.sp, fp64 ? "chol_panel64" : "chol_panel", (double)mp * jb * jb / 2.0,
                      2.0 * sizeof(T) * (double)mp * jb, 2);
-      chol_dblock<T><<<1, CH_T, 0, lu.sp>>>(Wp, ldw, jb, (int32_t)j, n, info, track, give_up);
+      StepLaunch D(dim3(1), dim3(fp64 ? CH_T : CD_T), 0, lu.sp, true);
+      if constexpr (fp64)
+        BOLA_TRY_CUDA(cudaLaunchKernelEx(&D.cfg, chol_dblock64, Wp, ldw, jb, (int32_t)j, n, info, track, give_up));
+      else
+        BOLA_TRY_CUDA(cudaLaunchKernelEx(&D.cfg, chol_dblock32, Wp, ldw, jb, (int32_t)j, n, info, track, give_up));
       if (mp > jb) {
-        if (l21_smem<T>() > 48 * 1024)
-          BOLA_TRY_CUDA(cudaFuncSetAttribute(chol_l21<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)l21_smem<T>()));
-        chol_l21<T><<<(unsigned)cdiv(mp - jb, L21_T), L21_T, l21_smem<T>(), lu.sp>>>(
-            Wp, ldw, mp, jb, lu.kind, upd ? lu.aop[buf] : nullptr, fp64 ? nullptr : lu.aop_lo[buf],
-            fp64 ? lu.ea[buf] : nullptr, lu.cap_n, info, track);
+        StepLaunch L(dim3((unsigned)cdiv(mp - jb, L21_R)), dim3(L21_T), l21_smem<T>(), lu.sp, true);
+        BOLA_TRY_CUDA(cudaLaunchKernelEx(&L.cfg, chol_l21<T>, Wp, ldw, mp, jb, lu.kind, upd ? lu.aop[buf] : nullptr,
+                                         fp64 ? (float *)nullptr : lu.aop_lo[buf],
+                                         fp64 ? lu.ea[buf] : (int32_t *)nullptr, lu.cap_n, (const int32_t *)info,
+                                         (const uint64_t *)track));
       }
       BOLA_CHECK_LAUNCH();
     }
@@ -317,10 +459,10 @@ int chol_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int32_t *info
     auto update = [&](cudaStream_t st, int64_t cols, int64_t boff) -> int {
       if constexpr (fp64)
         return oz_update(st, m2, cols, lu.mapA[buf], lu.mapA64[buf], lu.cap_n, lu.cap_n, lu.ea[buf], lu.ea[buf],
-                         W22 + boff * ldw, ldw, lu.err, boff, abort, true);
+                         W22 + boff * ldw, ldw, lu.err, boff, abort, true, st == lu.sp);
       else
         return tc_update(st, lu.kind, m2, cols, lu.mapA[buf], lu.mapA64[buf], lu.mapAlo[buf], lu.mapAlo64[buf],
-                         W22 + boff * ldw, ldw, lu.err, boff, abort, true);
+                         W22 + boff * ldw, ldw, lu.err, boff, abort, true, st == lu.sp);
     };
     BOLA_TRY(update(lu.sp, nb_next, 0));  // the next panel's columns
     if (n2 > nb_next) {

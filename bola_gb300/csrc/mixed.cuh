@@ -114,64 +114,53 @@ __device__ __forceinline__ float tf32_round(float x) {
 }
 
 // Writes one 64-wide row of an update operand (K-major, row `r`).
-__device__ __forceinline__ void write_operand_row(int kind, void *op, float *op_lo, int64_t r, const float *v) {
+__device__ __forceinline__ void write_operand_part(int kind, void *op, float *op_lo, int64_t r, int c, const float *v) {
   if (kind == 0) {
-    __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(op) + r * 64;
+    __align__(16) __nv_bfloat16 t[8];
 #pragma unroll
-    for (int c = 0; c < 64; c += 8) {
-      __align__(16) __nv_bfloat16 t[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) t[u] = __float2bfloat16_rn(v[c + u]);
-      *reinterpret_cast<uint4 *>(d + c) = *reinterpret_cast<const uint4 *>(t);
-    }
+    for (int u = 0; u < 8; ++u) t[u] = __float2bfloat16_rn(v[u]);
+    *reinterpret_cast<uint4 *>(static_cast<__nv_bfloat16 *>(op) + r * 64 + c) = *reinterpret_cast<const uint4 *>(t);
   } else {
-    float *d = static_cast<float *>(op) + r * 64;
-    float *dl = op_lo + r * 64;
+    float *d = static_cast<float *>(op) + r * 64 + c;
+    float *dl = op_lo + r * 64 + c;
 #pragma unroll
-    for (int c = 0; c < 64; c += 4) {
+    for (int u = 0; u < 8; u += 4) {
       float4 h, l;
-      h.x = tf32_round(v[c]);
-      h.y = tf32_round(v[c + 1]);
-      h.z = tf32_round(v[c + 2]);
-      h.w = tf32_round(v[c + 3]);
-      *reinterpret_cast<float4 *>(d + c) = h;
+      h.x = tf32_round(v[u]);
+      h.y = tf32_round(v[u + 1]);
+      h.z = tf32_round(v[u + 2]);
+      h.w = tf32_round(v[u + 3]);
+      *reinterpret_cast<float4 *>(d + u) = h;
       if (kind == 2) {
-        l.x = tf32_round(v[c] - h.x);
-        l.y = tf32_round(v[c + 1] - h.y);
-        l.z = tf32_round(v[c + 2] - h.z);
-        l.w = tf32_round(v[c + 3] - h.w);
-        *reinterpret_cast<float4 *>(dl + c) = l;
+        l.x = tf32_round(v[u] - h.x);
+        l.y = tf32_round(v[u + 1] - h.y);
+        l.z = tf32_round(v[u + 2] - h.z);
+        l.w = tf32_round(v[u + 3] - h.w);
+        *reinterpret_cast<float4 *>(dl + u) = l;
       }
     }
   }
 }
+__device__ __forceinline__ void write_operand_row(int kind, void *op, float *op_lo, int64_t r, const float *v) {
+#pragma unroll
+  for (int c = 0; c < 64; c += 8) write_operand_part(kind, op, op_lo, r, c, v + c);
+}
 
-// Writes the exact bf16 slices of one 64-wide FP64 row (K-major row r of a
-// kind-3 operand with cap rows per slice plane) and its exponent.
-__device__ __forceinline__ void write_slices_row(const double (&v)[64], int64_t r, int64_t cap, __nv_bfloat16 *out,
-                                                 int32_t *ex) {
-  uint64_t mb = 0;
+// Columns c .. c + 7 of the exact bf16 slices of 64-wide FP64 row r of a
+// K-major operand with cap rows per slice plane; e: the row's exponent.
+__device__ __forceinline__ void write_slices_part(const double *v, int e, int64_t r, int c, int64_t cap,
+                                                  __nv_bfloat16 *out) {
+  __align__(16) __nv_bfloat16 q[OZ_SLICES][8];
 #pragma unroll
-  for (int c = 0; c < 64; ++c) {
-    const uint64_t mc = oz_mag(v[c]);
-    mb = mc > mb ? mc : mb;
+  for (int u = 0; u < 8; ++u) {
+    __nv_bfloat16 t8[OZ_SLICES];
+    oz_slices(v[u], e, t8);
+#pragma unroll
+    for (int t = 0; t < OZ_SLICES; ++t) q[t][u] = t8[t];
   }
-  const int e = oz_exponent(mb);
-  ex[r] = e;
 #pragma unroll
-  for (int c0 = 0; c0 < 64; c0 += 8) {
-    __align__(16) __nv_bfloat16 q[OZ_SLICES][8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      __nv_bfloat16 t8[OZ_SLICES];
-      oz_slices(v[c0 + u], e, t8);
-#pragma unroll
-      for (int t = 0; t < OZ_SLICES; ++t) q[t][u] = t8[t];
-    }
-#pragma unroll
-    for (int t = 0; t < OZ_SLICES; ++t)
-      *reinterpret_cast<uint4 *>(out + ((int64_t)t * cap + r) * 64 + c0) = *reinterpret_cast<const uint4 *>(q[t]);
-  }
+  for (int t = 0; t < OZ_SLICES; ++t)
+    *reinterpret_cast<uint4 *>(out + ((int64_t)t * cap + r) * 64 + c) = *reinterpret_cast<const uint4 *>(q[t]);
 }
 
 // W(m x n, FP64) -= A B^T from the slices of A (rows of capA per slice) and
