@@ -9,10 +9,11 @@
 // of persistent 256-thread CTAs pulls items from an atomic counter; the CTA
 // splits into 256/G groups, each factoring one system in place in global
 // memory (L2-resident: at most 512 KB per system) with partial pivoting (LU)
-// or Cholesky in panels of 8 columns (register-tiled trailing updates), and
-// then solving its right-hand sides.  A group synchronises
-// with its own named barrier, so a system's arithmetic never depends on which
-// systems share its CTA: every result is the same alone and in any mix.
+// or Cholesky in panels of 8 columns (a panel in registers, a row per thread;
+// register-tiled trailing updates), and then solving its right-hand sides, 8
+// rows at a time.  A group synchronises with its own named barrier, so a
+// system's arithmetic never depends on which systems share its CTA: every
+// result is the same alone and in any mix.
 // FP64 throughout; all waits are barriers (no spin loops).
 #include <algorithm>
 #include <cmath>
@@ -47,48 +48,22 @@ __device__ __forceinline__ void group_sync(int G, int g) {
   } else if (G == BT) {
     __syncthreads();
   } else {
+    __syncwarp();  // (the barrier counts a warp at its first arrival)
     asm volatile("bar.sync %0, %1;" ::"r"(1 + g), "r"(G) : "memory");
   }
 }
 
-// argmax |A[k:n, k]| within a group; ties -> lowest row; NaN never wins.
-// The comparisons run on the integer pipe: |v|'s bits order like |v| (a
-// double comparison would take a slot of the narrow FP64 pipe per element).
-// red: 2*MAXG scratch per group.
-__device__ int group_argmax(const double *col, int k, int n, int t, int G, int g, long long *redv, int *redi) {
-  long long best = -1;
-  int bi = k;
-  for (int i = k + t; i < n; i += G) {
-    const long long v = __double_as_longlong(col[i]) & 0x7fffffffffffffffll;
-    if (v <= 0x7ff0000000000000ll && v > best) {
-      best = v;
-      bi = i;
-    }
-  }
-  for (int off = 16; off > 0; off >>= 1) {
-    const long long ov = __shfl_down_sync(0xffffffffu, best, off);
-    const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-    if (ov > best || (ov == best && oi < bi)) {
-      best = ov;
-      bi = oi;
-    }
-  }
-  const int w = t >> 5, nw = G >> 5;
-  if ((t & 31) == 0) {
-    redv[w] = best;
-    redi[w] = bi;
-  }
-  group_sync(G, g);
-  long long b = redv[0];
-  int r = redi[0];
-  for (int q = 1; q < nw; ++q)
-    if (redv[q] > b || (redv[q] == b && redi[q] < r)) {
-      b = redv[q];
-      r = redi[q];
-    }
-  group_sync(G, g);
-  return r;
-}
+// What the groups of a CTA share.  A group never has fewer threads than its
+// system has rows, so a thread holds a row of the panel in registers, and the
+// arrays are indexed by the CTA's warp or thread.
+constexpr int PBMAX = 16;
+struct Shared {
+  double cand[2][MAXG][PBMAX + 1];  // a warp's pivot candidate: its row of the panel, 1 / its value
+  double row[2][MAXG][PBMAX + 1];   // a group's row k, as above (Cholesky: column k's panel rows)
+  uint4 key[2][MAXG];               // a warp's largest |value| (high word + 1, low word), its row
+  int piv[MAXG][PBMAX];             // the panel's interchanges
+  Divisor dv[BT];                   // a system's diagonal, to divide by
+};
 
 // ---- blocked factorisation pieces -------------------------------------------
 // The factorisations below run in panels of PB columns: pivots inside the
@@ -175,11 +150,32 @@ __device__ void group_trailing(double *A, int lda, int n, int k0, int kb, bool l
   }
 }
 
+// At the top of a loop that rarely runs twice: its invariant loads are not kept
+// in registers across the iterations (whole blocks of L would be).
+__device__ __forceinline__ void reload() { asm volatile("" ::: "memory"); }
+
+// The panel's first `done` interchanges on all columns (a column of the panel
+// takes those after its own) and on the right-hand sides, a column per thread.
+__device__ __forceinline__ void group_swaps(const SystemDesc &S, int k0, int done, const int *piv, int t, int G) {
+  for (int j = t; j < S.n + S.nrhs; j += G) {
+    double *col = j < S.n ? S.a + (int64_t)j * S.lda : S.b + (int64_t)(j - S.n) * S.ldb;
+#pragma unroll 1
+    for (int r = j >= k0 && j < k0 + done ? j - k0 + 1 : 0; r < done; ++r) {
+      const int p = piv[r];
+      if (p == k0 + r) continue;
+      const double x = col[p];
+      col[p] = col[k0 + r];
+      col[k0 + r] = x;
+    }
+  }
+}
+
 // U12 = L11^-1 A12 for the panel rows k0..k0+kb-1 (unit lower L11), a column
 // per thread: row r takes fma(-l_rq, u_q, u_r) for q < r in increasing q.
 template <int PB>
-__device__ void group_u12(double *A, int lda, int n, int k0, int kb, int t, int G) {
+__device__ __forceinline__ void group_u12(double *A, int lda, int n, int k0, int kb, int t, int G) {
   for (int j = k0 + kb + t; j < n; j += G) {
+    reload();
     double u[PB];
 #pragma unroll
     for (int r = 0; r < PB; ++r) u[r] = r < kb ? A[(k0 + r) + (int64_t)j * lda] : 0.0;
@@ -194,208 +190,248 @@ __device__ void group_u12(double *A, int lda, int n, int k0, int kb, int t, int 
   }
 }
 
-// LU with partial pivoting of one system by a group; the row interchanges are
-// applied to B as they happen, then L y = P b and U x = y.
-template <int PB, int TR>
-__device__ int group_lu_solve(const SystemDesc &S, int t, int G, int g, long long *redv, int *redi, double *sinv) {
-  const int n = S.n, lda = S.lda, ldb = S.ldb, nr = S.nrhs;
-  double *A = S.a, *B = S.b;
-  int info = 0;
-  for (int k = 0; k < n; ++k) {
-    const int p = group_argmax(A + (int64_t)k * lda, k, n, t, G, g, redv, redi);
-    const double piv = A[p + (int64_t)k * lda];
-    if (!nonzero64(piv)) {
-      info = k + 1;
-      break;
-    }
-    if (t == 0) *sinv = 1.0 / piv;  // once per group; published by the barrier below
-    if (p != k) {
-      for (int j = t; j < n; j += G) {
-        const double tmp = A[k + (int64_t)j * lda];
-        A[k + (int64_t)j * lda] = A[p + (int64_t)j * lda];
-        A[p + (int64_t)j * lda] = tmp;
-      }
-      for (int c = t; c < nr; c += G) {
-        const double tmp = B[k + (int64_t)c * ldb];
-        B[k + (int64_t)c * ldb] = B[p + (int64_t)c * ldb];
-        B[p + (int64_t)c * ldb] = tmp;
-      }
-    }
-    group_sync(G, g);
-    const double inv = *sinv;
-    for (int i = k + 1 + t; i < n; i += G) A[i + (int64_t)k * lda] *= inv;
-    group_sync(G, g);
-    // the rank-1 update on the rest of this panel's columns; the columns after
-    // the panel get the whole panel at once below
-    const int k0 = k - k % PB, kend = k0 + PB < n ? k0 + PB : n;
-    const int m = n - k - 1, w = kend - k - 1;
-    if (m > 0 && w > 0) {
-      // element e = t, t + G, ... of the m x w block, (i, j) advanced without a
-      // division per element
-      const int dq = G / m, dr = G % m;
-      int i = k + 1 + t % m, j = k + 1 + t / m;
-      for (int e = t; e < m * w; e += G) {
-        A[i + (int64_t)j * lda] = fma(-A[i + (int64_t)k * lda], A[k + (int64_t)j * lda], A[i + (int64_t)j * lda]);
-        i += dr;
-        j += dq;
-        if (i >= n) {
-          i -= m;
-          ++j;
+// Triangular solve of the right-hand sides in blocks of SB rows: a block's own
+// triangle by a thread per right-hand side, then the rows still open take its
+// SB values at once, an element per thread.  Every element receives its
+// fma(-a_ik, x_k, b_i) in the order of the unblocked solve.  UP: from the last
+// row; DIV: by the diagonal (dv); TRANS: element (i, k) of the triangle is A[k, i].
+constexpr int SB = 8;
+template <bool UP, bool DIV, bool TRANS>
+__device__ __forceinline__ void group_trsv(const SystemDesc &S, const Divisor *dv, int t, int G, int g) {
+  const int n = S.n, nr = S.nrhs;
+  const int64_t lda = S.lda, ldb = S.ldb, sr = TRANS ? lda : 1, sc = TRANS ? 1 : lda;
+  const double *A = S.a;
+  double *B = S.b;
+  const int nblk = (n + SB - 1) / SB;
+  for (int s = 0; s < nblk; ++s) {
+    const int k0 = SB * (UP ? nblk - 1 - s : s), kb = n - k0 < SB ? n - k0 : SB;
+    for (int c = t; c < nr; c += G) {
+      reload();
+      double *x = B + k0 + c * ldb;
+      double b[SB];  // the rows in the order of the solve, the current one in slot 0
+      const int q0 = UP ? kb - 1 : 0, dir = UP ? -1 : 1;
+#pragma unroll
+      for (int z = 0; z < SB; ++z) b[z] = z < kb ? x[q0 + dir * z] : 0.0;
+#pragma unroll 1
+      for (int z = 0; z < kb; ++z) {
+        const int q = k0 + q0 + dir * z;
+        const double y = DIV ? div_rn(b[0], dv[q]) : b[0];
+        x[q - k0] = y;
+#pragma unroll
+        for (int r = 1; r < SB; ++r) {
+          if (z + r >= kb) break;
+          b[r - 1] = fma(-A[(q + dir * r) * sr + q * sc], y, b[r]);
         }
       }
     }
     group_sync(G, g);
-    if (k + 1 == kend && kend < n) {  // the panel is done: U12, then A22
-      group_u12<PB>(A, lda, n, k0, kend - k0, t, G);
+    const int i0 = UP ? 0 : k0 + kb, m = UP ? k0 : n - i0;
+    if (m > 0) {
+      const int dq = G / m, dr = G % m;
+      int i = t % m, c = t / m;
+      for (int e = t; e < m * nr; e += G) {
+        reload();
+        const double *x = B + k0 + c * ldb, *a = A + (i0 + i) * sr + k0 * sc;
+        double acc = B[(i0 + i) + c * ldb];
+#pragma unroll
+        for (int z = 0; z < SB; ++z) {
+          const int q = UP ? SB - 1 - z : z;
+          if (q < kb) acc = fma(-a[q * sc], x[q], acc);
+        }
+        B[(i0 + i) + c * ldb] = acc;
+        i += dr;
+        c += dq;
+        if (i >= m) {
+          i -= m;
+          ++c;
+        }
+      }
+    }
+    group_sync(G, g);
+  }
+}
+
+// LU with partial pivoting of one system by a group, then L y = P b and U x = y.
+// A panel stays in registers, a row per thread: per column one barrier, before
+// which every warp leaves its candidate's row (largest |value|, ties to the
+// lowest row, NaN never; compared on the integer pipe) and row k is left for
+// the candidate's place.
+template <int PB, int TR>
+__device__ int group_lu_solve(const SystemDesc &S, int t, int G, int g, Shared &sh) {
+  const unsigned FULL = 0xffffffffu;
+  const int n = S.n, lda = S.lda, nw = G >> 5, w0 = g * nw, warp = w0 + (t >> 5);
+  double *A = S.a;
+  int info = 0;
+  for (int k0 = 0; k0 < n && info == 0; k0 += PB) {
+    const int kb = n - k0 < PB ? n - k0 : PB;
+    const bool in = t >= k0 && t < n;
+    double v[PB];  // this row's columns, the current one in slot 0
+#pragma unroll
+    for (int c = 0; c < PB; ++c) v[c] = c < kb && in ? A[t + (int64_t)(k0 + c) * lda] : 0.0;
+    int done = kb;
+#pragma unroll 1
+    for (int c = 0; c < kb; ++c) {
+      const int k = k0 + c, par = c & 1;
+      const uint32_t hi = (uint32_t)__double2hiint(v[0]) & 0x7fffffffu, lo = (uint32_t)__double2loint(v[0]);
+      const bool valid = t >= k && t < n && (hi < 0x7ff00000u || (hi == 0x7ff00000u && lo == 0));
+      const uint32_t kh = valid ? hi + 1u : 0u;
+      const double inv_own = recip_rn(valid ? v[0] : 1.5);  // (beside the search; 1.5: no special case)
+      const uint32_t mh = __reduce_max_sync(FULL, kh);
+      const uint32_t ml = __reduce_max_sync(FULL, kh == mh ? lo : 0u);
+      const unsigned b = __ballot_sync(FULL, kh == mh && lo == ml);
+      const bool first = (t & 31) == __ffs(b) - 1;
+      if (first) sh.key[par][warp] = make_uint4(mh, ml, (uint32_t)t, 0u);
+      if (first || t == k) {
+#pragma unroll 1
+        for (int two = 0; two < 2; ++two) {
+          if (two ? t != k : !first) continue;
+          double *o = two ? sh.row[par][g] : sh.cand[par][warp];
+#pragma unroll
+          for (int q = 0; q < PB; ++q) o[q] = v[q];
+          o[PBMAX] = inv_own;
+        }
+      }
       group_sync(G, g);
-      group_trailing<TR>(A, lda, n, k0, kend - k0, false, t, G);
+      uint4 best = sh.key[par][w0];
+      int bw = w0;
+      for (int q = 1; q < nw; ++q) {
+        const uint4 o = sh.key[par][w0 + q];
+        if (o.x > best.x || (o.x == best.x && o.y > best.y)) {
+          best = o;
+          bw = w0 + q;
+        }
+      }
+      const double *kr = sh.row[par][g], *pr = best.x != 0u ? sh.cand[par][bw] : kr;
+      const int p = best.x != 0u ? (int)best.z : k;
+      if (!nonzero64(pr[0])) {
+        info = k + 1;
+        done = c;
+        // this column and the panel's others as they stand
+#pragma unroll
+        for (int q = 0; q < PB; ++q)
+          if (c + q < kb && in) A[t + (int64_t)(k + q) * lda] = v[q];
+        break;
+      }
+      if (t == 0) sh.piv[g][c] = p;
+      if (p != k && (t == p || t == k)) {
+        const double *o = t == p ? kr : pr;
+#pragma unroll
+        for (int q = 0; q < PB; ++q) v[q] = o[q];
+      }
+      const double l = t > k ? v[0] * pr[PBMAX] : v[0];
+      if (in) A[t + (int64_t)k * lda] = l;
+#pragma unroll
+      for (int q = 1; q < PB; ++q) {
+        if (c + q >= kb) break;
+        v[q - 1] = t > k ? fma(-l, pr[q], v[q]) : v[q];
+      }
+    }
+    group_sync(G, g);
+    // (a zero pivot ends the factorisation with the interchanges found so far)
+    group_swaps(S, k0, done, sh.piv[g], t, G);
+    group_sync(G, g);
+    if (info == 0 && k0 + kb < n) {
+      group_u12<PB>(A, lda, n, k0, kb, t, G);
+      group_sync(G, g);
+      group_trailing<TR>(A, lda, n, k0, kb, false, t, G);
       group_sync(G, g);
     }
   }
   if (info) return info;
-  // forward: unit lower
-  for (int k = 0; k < n; ++k) {
-    const int m = n - k - 1;
-    if (m > 0) {
-      const int dq = G / m, dr = G % m;
-      int i = k + 1 + t % m, c = t / m;
-      for (int e = t; e < m * nr; e += G) {
-        B[i + (int64_t)c * ldb] = fma(-A[i + (int64_t)k * lda], B[k + (int64_t)c * ldb], B[i + (int64_t)c * ldb]);
-        i += dr;
-        c += dq;
-        if (i >= n) {
-          i -= m;
-          ++c;
-        }
-      }
-    }
-    group_sync(G, g);
-  }
-  // backward: upper
-  for (int k = n - 1; k >= 0; --k) {
-    for (int c = t; c < nr; c += G) B[k + (int64_t)c * ldb] /= A[k + (int64_t)k * lda];
-    group_sync(G, g);
-    if (k > 0) {
-      const int dq = G / k, dr = G % k;
-      int i = t % k, c = t / k;
-      for (int e = t; e < k * nr; e += G) {
-        B[i + (int64_t)c * ldb] = fma(-A[i + (int64_t)k * lda], B[k + (int64_t)c * ldb], B[i + (int64_t)c * ldb]);
-        i += dr;
-        c += dq;
-        if (i >= k) {
-          i -= k;
-          ++c;
-        }
-      }
-    }
-    group_sync(G, g);
-  }
+  Divisor *dv = sh.dv + g * G;
+  if (t < n) dv[t] = divisor(A[t + (int64_t)t * lda]);
+  group_sync(G, g);
+  group_trsv<false, false, false>(S, dv, t, G, g);  // unit lower
+  group_trsv<true, true, false>(S, dv, t, G, g);    // upper
   return 0;
 }
 
 // Cholesky A = L L^T (lower) of one system by a group, then L y = b, L^T x = y.
+// The panel as above; per column one barrier for the pivot's reciprocal root,
+// one for the panel's rows of the scaled column.
 template <int PB, int TR>
-__device__ int group_chol_solve(const SystemDesc &S, int t, int G, int g, double *sinv) {
-  const int n = S.n, lda = S.lda, ldb = S.ldb, nr = S.nrhs;
-  double *A = S.a, *B = S.b;
-  for (int k = 0; k < n; ++k) {
-    const double d = A[k + (int64_t)k * lda];
-    // d > 0 (NaN excluded) on the bits
-    const long long db = __double_as_longlong(d);
-    if (!(db > 0 && db <= 0x7ff0000000000000ll)) return k + 1;
-    // the square root and its reciprocal once per group, not once per thread
-    double r = 0.0;
-    if (t == 0) {
-      r = sqrt(d);
-      *sinv = 1.0 / r;
-    }
-    group_sync(G, g);
-    if (t == 0) A[k + (int64_t)k * lda] = r;
-    const double inv = *sinv;
-    for (int i = k + 1 + t; i < n; i += G) A[i + (int64_t)k * lda] *= inv;
-    group_sync(G, g);
-    // the rank-1 update on the rest of this panel's columns, lower part only,
-    // packed column by column (column jj, global k+1+jj, holds rows jj..m-1):
-    // walking the full square would issue the FP64 update for the upper half
-    // too, predicated off
-    const int k0 = k - k % PB, kend = k0 + PB < n ? k0 + PB : n;
-    const int m = n - k - 1, w = kend - k - 1;
-    if (m > 0 && w > 0) {
-      int ii = t, jj = 0;
-      while (ii >= m && jj < w) {
-        ii -= m - jj - 1;
-        ++jj;
+__device__ int group_chol_solve(const SystemDesc &S, int t, int G, int g, Shared &sh) {
+  const int n = S.n, lda = S.lda;
+  double *A = S.a;
+  int info = 0;
+  for (int k0 = 0; k0 < n && info == 0; k0 += PB) {
+    const int kb = n - k0 < PB ? n - k0 : PB;
+    double v[PB];  // this row's columns, the current one in slot 0
+#pragma unroll
+    for (int c = 0; c < PB; ++c) v[c] = c < kb && t >= k0 + c && t < n ? A[t + (int64_t)(k0 + c) * lda] : 0.0;
+#pragma unroll 1
+    for (int c = 0; c < kb; ++c) {
+      const int k = k0 + c;
+      double *x = sh.row[c & 1][g];
+      if (t == k) {
+        // d > 0 (NaN excluded) on the bits
+        const long long db = __double_as_longlong(v[0]);
+        const bool pos = db > 0 && db <= 0x7ff0000000000000ll;
+        if (pos) {
+          v[0] = sqrt_rn(v[0]);
+          A[k + (int64_t)k * lda] = v[0];
+          x[PBMAX] = recip_rn(v[0]);
+        }
+        sh.piv[g][c] = pos;
       }
-      const int total = w * m - w * (w - 1) / 2;
-      for (int e = t; e < total; e += G) {
-        const int i = k + 1 + ii, j = k + 1 + jj;
-        A[i + (int64_t)j * lda] = fma(-A[i + (int64_t)k * lda], A[j + (int64_t)k * lda], A[i + (int64_t)j * lda]);
-        ii += G;
-        while (ii >= m && jj < w) {
-          ii -= m - jj - 1;
-          ++jj;
+      group_sync(G, g);
+      if (!sh.piv[g][c]) {
+        info = k + 1;
+        // this column and the panel's others as they stand
+#pragma unroll
+        for (int q = 0; q < PB; ++q)
+          if (c + q < kb && t >= k + q && t < n) A[t + (int64_t)(k + q) * lda] = v[q];
+        break;
+      }
+      const bool below = t > k && t < n;
+      if (below) {
+        v[0] *= x[PBMAX];
+        A[t + (int64_t)k * lda] = v[0];
+        if (t < k0 + kb) x[t - k0] = v[0];
+      }
+      group_sync(G, g);
+      if (below) {
+        const double l = v[0];
+#pragma unroll
+        for (int q = 1; q < PB; ++q) {
+          if (c + q >= kb) break;
+          v[q - 1] = fma(-l, x[c + q], v[q]);
         }
       }
     }
     group_sync(G, g);
-    if (k + 1 == kend && kend < n) {  // the panel is done: the trailing lower triangle
-      group_trailing<TR>(A, lda, n, k0, kend - k0, true, t, G);
+    if (info == 0 && k0 + kb < n) {
+      group_trailing<TR>(A, lda, n, k0, kb, true, t, G);
       group_sync(G, g);
     }
   }
-  for (int k = 0; k < n; ++k) {  // L y = b
-    for (int c = t; c < nr; c += G) B[k + (int64_t)c * ldb] /= A[k + (int64_t)k * lda];
-    group_sync(G, g);
-    const int m = n - k - 1;
-    if (m > 0) {
-      const int dq = G / m, dr = G % m;
-      int i = k + 1 + t % m, c = t / m;
-      for (int e = t; e < m * nr; e += G) {
-        B[i + (int64_t)c * ldb] = fma(-A[i + (int64_t)k * lda], B[k + (int64_t)c * ldb], B[i + (int64_t)c * ldb]);
-        i += dr;
-        c += dq;
-        if (i >= n) {
-          i -= m;
-          ++c;
-        }
-      }
-    }
-    group_sync(G, g);
-  }
-  for (int k = n - 1; k >= 0; --k) {  // L^T x = y
-    for (int c = t; c < nr; c += G) B[k + (int64_t)c * ldb] /= A[k + (int64_t)k * lda];
-    group_sync(G, g);
-    if (k > 0) {
-      const int dq = G / k, dr = G % k;
-      int i = t % k, c = t / k;
-      for (int e = t; e < k * nr; e += G) {
-        B[i + (int64_t)c * ldb] = fma(-A[k + (int64_t)i * lda], B[k + (int64_t)c * ldb], B[i + (int64_t)c * ldb]);
-        i += dr;
-        c += dq;
-        if (i >= k) {
-          i -= k;
-          ++c;
-        }
-      }
-    }
-    group_sync(G, g);
-  }
+  if (info) return info;
+  Divisor *dv = sh.dv + g * G;
+  if (t < n) dv[t] = divisor(A[t + (int64_t)t * lda]);
+  group_sync(G, g);
+  group_trsv<false, true, false>(S, dv, t, G, g);  // L y = b
+  group_trsv<true, true, true>(S, dv, t, G, g);    // L^T x = y
   return 0;
 }
 
 template <int PB, int TR>
-__device__ int group_solve(const SystemDesc &S, int t, int G, int g, long long *redv, int *redi, double *sinv) {
-  return S.kind == 1 ? group_chol_solve<PB, TR>(S, t, G, g, sinv) : group_lu_solve<PB, TR>(S, t, G, g, redv, redi, sinv);
+__device__ int group_solve(const SystemDesc &S, int t, int G, int g, Shared &sh) {
+  return S.kind == 1 ? group_chol_solve<PB, TR>(S, t, G, g, sh) : group_lu_solve<PB, TR>(S, t, G, g, sh);
 }
 
+// Bound by FP64 issue (90% of it at orders up to 256) once enough groups share
+// an SM: three CTAs rather than the two that the registers of the trailing
+// update's tile would leave, a few values spilled (with four, whole tiles are:
+// 2% faster at orders up to 256, 20% slower up to 64).  Measured on one GB300,
+// 4000 systems, half LU and half Cholesky: orders 8 to 256, 10.6 ms (13.1 with
+// two CTAs and the panel's columns one after the other through global memory);
+// orders 8 to 64, 0.55 ms (0.64).
 template <int TR>
-__global__ void __launch_bounds__(BT)
+__global__ void __launch_bounds__(BT, 3)
 batched_solve_kernel(const SystemDesc *__restrict__ sys, const int32_t *__restrict__ items, int32_t nitems,
                      int32_t *counter, int32_t *info) {
   __shared__ int32_t cur[ITEM];
-  __shared__ long long redv[MAXG][MAXG];
-  __shared__ double sinv[MAXG];
-  __shared__ int redi[MAXG][MAXG];
+  __shared__ __align__(16) Shared sh;
   const int tid = threadIdx.x;
   for (;;) {
     if (tid == 0) {
@@ -411,9 +447,9 @@ batched_solve_kernel(const SystemDesc *__restrict__ sys, const int32_t *__restri
       const int id = cur[3 + g];
       const SystemDesc S = sys[id];
       const int pb = cur[2];
-      const int r = pb == 16   ? group_solve<16, TR>(S, t, G, g, redv[g], redi[g], &sinv[g])
-                    : pb == 12 ? group_solve<12, TR>(S, t, G, g, redv[g], redi[g], &sinv[g])
-                               : group_solve<8, TR>(S, t, G, g, redv[g], redi[g], &sinv[g]);
+      const int r = pb == 16   ? group_solve<16, TR>(S, t, G, g, sh)
+                    : pb == 12 ? group_solve<12, TR>(S, t, G, g, sh)
+                               : group_solve<8, TR>(S, t, G, g, sh);
       if (t == 0) info[id] = r;
     }
     __syncthreads();
@@ -450,6 +486,7 @@ int batch_items(int32_t count, const int32_t *n, const int32_t *kind, const int3
   for (int b = 0; b < NBUCKET; ++b) {
     int gsz = group_size ? group_size[b] : kDefault[b];
     if (gsz != 32 && gsz != 64 && gsz != 128 && gsz != 256) gsz = kDefault[b];
+    gsz = std::max(gsz, kDefault[b]);  // a thread per row at least
     group[b] = gsz;
     const int pw = panel_width ? panel_width[b] : 8;
     pbw[b] = (pw == 12 || pw == 16) ? pw : 8;

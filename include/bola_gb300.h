@@ -350,7 +350,8 @@ int bola_batch_plan_create(int32_t count, const int32_t *n, const int32_t *kind,
  * rows of the per-thread register tile of the trailing updates (4 or 2,
  * with 4 columns), one value per plan because it sets the kernel's register
  * count.  Zero entries take the built-in defaults (group sizes 32..256 by
- * bucket, panel width 8, tile 4).  None of the three changes any system's
+ * bucket, panel width 8, tile 4); a group smaller than its bucket's order is
+ * widened to the default (a thread per row).  None of the three changes any system's
  * operation order: a tuned plan gives bit-identical results. */
 typedef struct {
   int32_t group_size[8];
