@@ -31,35 +31,49 @@ __global__ void syrk_beta(bool upper, int64_t n, double beta, double *C, int64_t
   c = beta == 0.0 ? 0.0 : __dmul_rn(c, beta);
 }
 
-// Diagonal 32x32 blocks: blockIdx.y = block, blockIdx.x = column jj in the
-// block, threadIdx.x = row ii.  Each element's chain over k keeps BOLA's
-// order exactly and is FP64-latency-bound, so the 32 columns of a block run
-// on 32 SMs.  A arrives in 32-deep chunks staged in shared memory; the next
-// chunk is prefetched into registers while the current one is consumed.
-__global__ void __launch_bounds__(NB)
+// Diagonal 32x32 blocks: blockIdx.y = block.  Each element's chain over k keeps
+// BOLA's order exactly; a warp takes column p's rows and, in the lanes that
+// these leave, column 32 - p's (17 warps per block; 'U' is 'L' turned round),
+// so no lane of the narrow FP64 pipe's 16-cycle instructions is empty, and
+// lanes in a column's unfused tail go through the fused ones' multiply-add.
+// A arrives in 32-deep chunks staged in shared memory; the next chunk is
+// prefetched into registers while the current one is consumed.  SLOTS warps
+// per CTA: one where few blocks leave the chain's latency to bound it (a block
+// then runs on 17 SMs), nine where the blocks fill the chip.  Measured on one
+// GB300, 32 deep, launches serialised: 127 blocks 12 us (23 with a warp per
+// column and the tail's lanes apart), one block 7 (7.9).
+constexpr int SYRK_WARPS = NB / 2 + 1;
+template <int SLOTS>
+__global__ void __launch_bounds__(NB *SLOTS)
 syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const double *__restrict__ A,
           int64_t lda, double *C, int64_t ldc, int lanes, const int32_t *info) {
-  __shared__ double sA[NB][NB + 1];  // 'N': sA[l][r] = A(j0 + r, p0 + l); 'T': sA[r][l] = A(p0 + l, j0 + r)
-  __shared__ double tl[NB];          // 'N': alpha * A(j0 + jj, p0 + l), the column's multipliers
-  if (stop_flag(info)) return;
+  __shared__ double sA[NB][NB + 1];      // 'N': sA[l][r] = A(j0 + r, p0 + l); 'T': sA[r][l] = A(p0 + l, j0 + r)
+  __shared__ double tls[SLOTS][2][NB];   // 'N': alpha * A(j0 + jj, p0 + l), the warp's columns' multipliers
+  if (__syncthreads_or(stop_flag(info))) return;  // (another stream may set it: one answer per CTA)
   const int64_t j0 = (int64_t)blockIdx.y * NB;
   const int jb = (int)imin(NB, n - j0);
-  const int jj = blockIdx.x, ii = threadIdx.x;
-  if (jj >= jb) return;  // uniform over the CTA
-  const bool active = ii < jb && !(upper ? ii > jj : ii < jj);
+  const int w = threadIdx.x / NB, lane = threadIdx.x % NB, p = blockIdx.x * SLOTS + w;
+  const bool second = lane < p;
+  const int r_low = second ? lane + NB - p : lane, c_low = second ? NB - p : p;
+  const int ii = upper ? NB - 1 - r_low : r_low, jj = upper ? NB - 1 - c_low : c_low;
+  const int ja = upper ? NB - 1 - p : p, jz = upper ? p - 1 : NB - p;  // the warp's columns
+  const bool active = p < SYRK_WARPS && !(2 * p == NB && second) && ii < jb && jj < jb;
   // BOLA's daxpy for column jj: the element is in the fused vector body or the unfused tail
   const int64_t len = upper ? jj + 1 : jb - jj;
   const int64_t idx = upper ? ii : ii - jj;
   const bool fz = idx < (len & ~(int64_t)(lanes - 1));
-  double pre[NB];
+  const bool all_fused = __all_sync(0xffffffffu, fz || !active);
+  constexpr int QN = (NB + SLOTS - 1) / SLOTS;  // this thread's part of a chunk: rows (columns) w + SLOTS q
+  double pre[QN];
   auto fetch = [&](int64_t p0) {
     const int pb = (int)imin(NB, k - p0);
 #pragma unroll
-    for (int q = 0; q < NB; ++q) {
-      if (trans_t)  // column q of the block, depth row ii
-        pre[q] = (q < jb && ii < pb) ? A[(p0 + ii) + (j0 + q) * lda] : 0.0;
-      else  // depth column q, block row ii
-        pre[q] = (q < pb && ii < jb) ? A[(j0 + ii) + (p0 + q) * lda] : 0.0;
+    for (int u = 0; u < QN; ++u) {
+      const int q = w + SLOTS * u;
+      if (trans_t)  // column q of the block, depth row `lane`
+        pre[u] = (q < jb && lane < pb) ? A[(p0 + lane) + (j0 + q) * lda] : 0.0;
+      else  // depth column q, block row `lane`
+        pre[u] = (q < pb && lane < jb) ? A[(j0 + lane) + (p0 + q) * lda] : 0.0;
     }
   };
   double *cp = C + (j0 + ii) + (j0 + jj) * ldc;
@@ -69,29 +83,34 @@ syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const do
     const int pb = (int)imin(NB, k - p0);
     __syncthreads();  // the previous chunk is consumed
 #pragma unroll
-    for (int q = 0; q < NB; ++q) sA[q][ii] = pre[q];  // both layouts: q is l ('N') or r ('T')
+    for (int u = 0; u < QN; ++u)
+      if (w + SLOTS * u < NB) sA[w + SLOTS * u][lane] = pre[u];  // both layouts: q is l ('N') or r ('T')
     __syncthreads();
-    // one multiplier per lane, and which are non-zero (BOLA's daxpy skips a
-    // zero scale): the chain below then issues one FP64 instruction per step,
-    // the only one GB300's narrow FP64 pipe must serialise
+    // one multiplier per lane and column, and which are non-zero (BOLA's daxpy
+    // skips a zero scale)
     uint32_t nz = 0;
-    if (!trans_t) {
-      const double tv = ii < pb ? __dmul_rn(alpha, sA[ii][jj]) : 0.0;
-      tl[ii] = tv;
-      nz = __ballot_sync(0xffffffffu, nonzero64(tv));
+    if (!trans_t && p < SYRK_WARPS) {
+      const double ta = lane < pb ? __dmul_rn(alpha, sA[lane][ja]) : 0.0;
+      const double tz = lane < pb && p > 0 ? __dmul_rn(alpha, sA[lane][jz]) : 0.0;
+      tls[w][0][lane] = ta;
+      tls[w][1][lane] = tz;
+      const uint32_t na = __ballot_sync(0xffffffffu, nonzero64(ta)), nl = __ballot_sync(0xffffffffu, nonzero64(tz));
+      nz = second ? nl : na;
     }
-    __syncthreads();
+    __syncwarp();
     if (p0 + NB < k) fetch(p0 + NB);
     if (!active) continue;
     if (!trans_t) {
       // syrk_kernel 'N' (src/syrk.rs:201-222): C(:,jj) += (alpha*A(jj,l)) * A(:,l), BOLA's daxpy
-      if (fz) {
+      const double *tl = tls[w][second];
+      if (all_fused) {
 #pragma unroll 4
         for (int l = 0; l < pb; ++l)
           if ((nz >> l) & 1u) c = fused(tl[l], sA[l][ii], c);
       } else {
+#pragma unroll 4
         for (int l = 0; l < pb; ++l)
-          if ((nz >> l) & 1u) c = add_prod(c, tl[l], sA[l][ii]);
+          if ((nz >> l) & 1u) c = fused_or_unfused2(fz, tl[l], sA[l][ii], c);
       }
     } else {
       // syrk_kernel 'T' (src/syrk.rs:223-247): C(ii,jj) += alpha * dot(A(:,ii), A(:,jj))
@@ -100,6 +119,21 @@ syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const do
     }
   }
   if (active) *cp = c;
+}
+// From this many diagonal blocks on nine warps share a CTA (two CTAs per block).
+constexpr int64_t SYRK_WIDE_BLOCKS = 16;
+int launch_syrk_diag(cudaStream_t s, bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const double *A,
+                     int64_t lda, double *C, int64_t ldc, const int32_t *info) {
+  const int64_t blocks = cdiv(n, NB);
+  ProfScope prof(s, "syrk_diag", (double)imin(n, NB) * (imin(n, NB) + 1) * (double)k * (double)blocks);
+  const int slots = blocks >= SYRK_WIDE_BLOCKS ? 9 : 1;
+  void (*kern)(bool, bool, int64_t, int64_t, double, const double *, int64_t, double *, int64_t, int, const int32_t *) =
+      slots == 9 ? syrk_diag<9> : syrk_diag<1>;
+  BOLA_TRY(roomy(kern));
+  kern<<<dim3((unsigned)cdiv(SYRK_WARPS, slots), (unsigned)blocks), NB * slots, 0, s>>>(
+      upper, trans_t, n, k, alpha, A, lda, C, ldc, lanes(), info);
+  BOLA_CHECK_LAUNCH();
+  return 0;
 }
 
 // ---- potrf2 on one <=32 x 32 block in shared memory (src/potrf2.rs:36-80) ----
@@ -226,8 +260,8 @@ __device__ int p2_walk(bool upper, double *a0, double *rdg, int n, int lanes) {
 // updates of the TRSM of the frame that separates i from j are applied row by
 // row, unfused; then the division by u_ii.
 //
-// Measured on one GB300 at n = 4096, launches serialised: @@L us ('L'),
-// @@U us ('U'), against 50 and 84 for the column sweep on four warps with
+// Measured on one GB300 at n = 4096, launches serialised: 37 us ('L'),
+// 44 us ('U'), against 50 and 84 for the column sweep on four warps with
 // three CTA barriers a column and the recursion.
 constexpr int P2_UPD = 8;                      // update warps
 constexpr int P2_T = 32 * (1 + P2_UPD);
@@ -422,11 +456,7 @@ int syrk_exact(cudaStream_t s, char uplo, char trans, int64_t n, int64_t k, doub
     BOLA_TRY(dgemm_exact(s, tt ? 'T' : 'N', tt ? 'N' : 'T', n, n, k, alpha, A, lda, A, lda, 1.0, C, ldc, NB,
                          info, upper ? 1 : 2));
   }
-  ProfScope prof(s, "syrk_diag", (double)imin(n, NB) * (imin(n, NB) + 1) * (double)k * (double)cdiv(n, NB));
-  BOLA_TRY(roomy(syrk_diag));
-  syrk_diag<<<dim3(NB, (unsigned)cdiv(n, NB)), NB, 0, s>>>(upper, tt, n, k, alpha, A, lda, C, ldc, lanes(), info);
-  BOLA_CHECK_LAUNCH();
-  return 0;
+  return launch_syrk_diag(s, upper, tt, n, k, alpha, A, lda, C, ldc, info);
 }
 
 int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int32_t *info, int32_t col0) {
@@ -457,14 +487,10 @@ namespace {
 // One launch of the diagonal-block chain advance: the diagonal blocks of the
 // nt x nt trailing matrix at C advance over the 32 columns (rows for 'U') at
 // src.
-int advance_diag(cudaStream_t s, bool upper, int64_t nt, const double *src, int64_t lda, double *C, int lan,
+int advance_diag(cudaStream_t s, bool upper, int64_t nt, const double *src, int64_t lda, double *C,
                  const int32_t *info) {
   if (nt <= 0) return 0;
-  ProfScope prof(s, "syrk_diag", (double)NB * (NB + 1) * (double)NB * (double)cdiv(nt, NB));
-  BOLA_TRY(roomy(syrk_diag));
-  syrk_diag<<<dim3(NB, (unsigned)cdiv(nt, NB)), NB, 0, s>>>(upper, upper, nt, NB, -1.0, src, lda, C, lda, lan, info);
-  BOLA_CHECK_LAUNCH();
-  return 0;
+  return launch_syrk_diag(s, upper, upper, nt, NB, -1.0, src, lda, C, lda, info);
 }
 
 // The 64-deep chunk starting at column (row, for 'U') c0 applied to the block
@@ -594,7 +620,6 @@ int potrf_blocked(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, 
     if (NB >= n) return potrf2_rec(s, uplo, n, A, lda, info, 0);
     return potrf_left_looking(s, upper, n, A, lda, info);
   }
-  const int lan = lanes();
   Scratch bk;
   BOLA_TRY(bk.alloc((size_t)n * n * sizeof(double), s));
   LookAhead *la = la_acquire();
@@ -632,7 +657,7 @@ int potrf_blocked(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, 
       if (n_rem <= 0) break;
       if (la && syrk_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(sp, la->ev[2 + ((q - 1) & 1)], 0));
       const double *src_n = upper ? A + j + t * lda : A + t + j * lda;
-      BOLA_TRY(advance_diag(sp, upper, imin(NB, n_rem), src_n, lda, A + t + t * lda, lan, info));
+      BOLA_TRY(advance_diag(sp, upper, imin(NB, n_rem), src_n, lda, A + t + t * lda, info));
       const bool odd = q & 1;
       if (odd) BOLA_TRY(chunk_narrow(sp, upper, n, j - NB, t, A, lda, info));
       syrk_pending = false;
@@ -640,7 +665,7 @@ int potrf_blocked(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, 
         BOLA_TRY(on(la ? la->ev[1] : nullptr, sp, su));
         const int64_t t2 = t + NB;
         const double *src_w = upper ? A + j + t2 * lda : A + t2 + j * lda;
-        BOLA_TRY(advance_diag(su, upper, n_rem - NB, src_w, lda, A + t2 + t2 * lda, lan, info));
+        BOLA_TRY(advance_diag(su, upper, n_rem - NB, src_w, lda, A + t2 + t2 * lda, info));
         if (la) BOLA_TRY_CUDA(cudaEventRecord(la->ev[2 + (q & 1)], su));
         syrk_pending = true;
         if (odd) {
