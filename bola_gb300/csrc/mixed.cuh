@@ -113,7 +113,7 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float(u);
 }
 
-// Writes one 64-wide row of an update operand (K-major, row `r`).
+// Writes columns c .. c + 7 of a 64-wide row of an update operand (K-major, row `r`).
 __device__ __forceinline__ void write_operand_part(int kind, void *op, float *op_lo, int64_t r, int c, const float *v) {
   if (kind == 0) {
     __align__(16) __nv_bfloat16 t[8];
@@ -140,10 +140,6 @@ __device__ __forceinline__ void write_operand_part(int kind, void *op, float *op
       }
     }
   }
-}
-__device__ __forceinline__ void write_operand_row(int kind, void *op, float *op_lo, int64_t r, const float *v) {
-#pragma unroll
-  for (int c = 0; c < 64; c += 8) write_operand_part(kind, op, op_lo, r, c, v + c);
 }
 
 // Columns c .. c + 7 of the exact bf16 slices of 64-wide FP64 row r of a
@@ -255,7 +251,7 @@ struct MixedLU {
   CUtensorMap mapA[2], mapB, mapAlo[2], mapBlo;
   CUtensorMap mapA64[2], mapAlo64[2];  // the A operands in 64-row boxes (the B side of a Cholesky update)
   cudaStream_t sp = nullptr, su = nullptr;
-  cudaEvent_t ev_in = nullptr, ev_sw = nullptr, ev_wide = nullptr, ev_done = nullptr;
+  cudaEvent_t ev_in = nullptr, ev_pan = nullptr, ev_sw = nullptr, ev_wide = nullptr, ev_done = nullptr;
   int reserve(int64_t n, int kind, cudaStream_t s);
   void release(cudaStream_t s);  // frees the buffers (stream-ordered on s)
   void destroy();                // the streams and events too (device idle)

@@ -694,10 +694,30 @@ panel_lu64(double *Wp, int64_t ldw, int64_t mp, int jb, int32_t col0, const int3
   }
 }
 
+// Values `lane` and lane + 32 of row r of an update operand, as write_operand_part rounds them.
+__device__ __forceinline__ void write_operand_pair(int kind, void *op, float *op_lo, int64_t r, int lane, float a,
+                                                   float b) {
+  if (kind == 0) {
+    __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(op) + r * SNB;
+    d[lane] = __float2bfloat16_rn(a);
+    d[lane + 32] = __float2bfloat16_rn(b);
+    return;
+  }
+  float *d = static_cast<float *>(op) + r * SNB;
+  const float ha = tf32_round(a), hb = tf32_round(b);
+  d[lane] = ha;
+  d[lane + 32] = hb;
+  if (kind == 2) {
+    float *dl = op_lo + r * SNB;
+    dl[lane] = tf32_round(a - ha);
+    dl[lane + 32] = tf32_round(b - hb);
+  }
+}
+
 // Rows r0 .. r0 + 63 of the update's K-major A operand (kinds 0-2) from the
 // factored panel: operand row r is row j + 64 + r of W's columns j .. j + 63
 // (final once the panel kernel has written them back), rounded as
-// write_operand_row rounds.  The 64 x 64 tile is read a column at a time and
+// write_operand_part rounds.  The 64 x 64 tile is read a column at a time and
 // written a row at a time, both coalesced, through t (64 x 64, columns
 // XOR-swizzled by the row so that both passes are free of bank conflicts).
 __device__ __forceinline__ void operand_tile(const float *W, int64_t ldw, int64_t j, int64_t m2, int64_t r0,
@@ -721,37 +741,28 @@ __device__ __forceinline__ void operand_tile(const float *W, int64_t ldw, int64_
   for (int r = warp; r < rows; r += 8) {
     const float a = t[r * SNB + (lane ^ (r & 31))], b = t[r * SNB + ((lane + 32) ^ (r & 31))];
     const int64_t orow = r0 + r;
-    if (kind == 0) {
-      __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(op) + orow * SNB;
-      d[lane] = __float2bfloat16_rn(a);
-      d[lane + 32] = __float2bfloat16_rn(b);
-    } else {
-      float *d = static_cast<float *>(op) + orow * SNB;
-      const float ha = tf32_round(a), hb = tf32_round(b);
-      d[lane] = ha;
-      d[lane + 32] = hb;
-      if (kind == 2) {
-        float *dl = op_lo + orow * SNB;
-        dl[lane] = tf32_round(a - ha);
-        dl[lane + 32] = tf32_round(b - hb);
-      }
-    }
+    write_operand_pair(kind, op, op_lo, orow, lane, a, b);
   }
 }
 
-// The panel's interchanges on the columns right of it, U12 = L11^-1 A12 and
-// its K-major B operand: a warp per column, ncta CTAs (the finished columns
+// The panel's interchanges on the columns [w0, w1) right of it, U12 = L11^-1
+// A12 and its K-major B operand: a warp per CPW columns (two share their reads
+// of L11 where there are enough of them), ncta CTAs (the finished columns
 // left of the panel take the interchanges once, when the factorisation is
 // done: apply_left_swaps).  CTA 0 also applies them to the row permutation.
 // The FP32 factors' CTAs from ncta on write the A operand of the update (aop:
-// operand_tile, one 64-row tile each).
-template <typename T>
+// operand_tile, one 64-row tile each).  Bound by the interchanges' scattered
+// rows: measured at n = 8192, launches serialised, 20 us for the 8064 columns
+// after the next panel's (25 with a warp per column and the operand's rows
+// written by one lane), 8 us for the next panel's 64, which alone the critical
+// stream waits for.
+template <typename T, int CPW>
 __global__ void __launch_bounds__(256)
 sswap_trsm(T *W, int64_t ldw, int64_t n, int64_t j, int jb, const int32_t *plan, int kind, void *bop,
-           float *bop_lo, int32_t *bexp, int64_t cap, const int32_t *abort, int ncta, void *aop, float *aop_lo,
-           int32_t *perm) {
+           float *bop_lo, int32_t *bexp, int64_t cap, const int32_t *abort, int64_t w0, int64_t w1, int ncta, void *aop,
+           float *aop_lo, int32_t *perm) {
   sm100::grid_dependency_wait();
-  if (abort != nullptr && *(volatile const int32_t *)abort != 0) return;  // set before this launch (same stream)
+  if (abandoned(abort)) return;
   __shared__ int32_t rows[2 * SNB], src[2 * SNB];
   __shared__ __align__(16) T L[SNB * SNB];
   __shared__ int cnt;
@@ -792,47 +803,62 @@ sswap_trsm(T *W, int64_t ldw, int64_t n, int64_t j, int jb, const int32_t *plan,
     for (int e = 0; e < 4; ++e)
       if (lane + 32 * e < cnt) perm[rows[lane + 32 * e]] = pv[e];
   }
-  const int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (w >= n - j - jb) return;
+  const int64_t w = w0 + ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * CPW;
+  if (w >= w1) return;
   const int64_t col = j + jb + w;
-  T *cp = W + col * ldw;
-  T v[4];
+  T *cp[CPW];
 #pragma unroll
-  for (int e = 0; e < 4; ++e) v[e] = lane + 32 * e < cnt ? cp[src[lane + 32 * e]] : T(0);
+  for (int u = 0; u < CPW; ++u) cp[u] = W + (col + (w + u < w1 ? u : 0)) * ldw;
+  T v[CPW][4];
+#pragma unroll
+  for (int u = 0; u < CPW; ++u)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[u][e] = lane + 32 * e < cnt ? cp[u][src[lane + 32 * e]] : T(0);
   __syncwarp();
 #pragma unroll
-  for (int e = 0; e < 4; ++e)
-    if (lane + 32 * e < cnt) cp[rows[lane + 32 * e]] = v[e];
+  for (int u = 0; u < CPW; ++u)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (w + u < w1 && lane + 32 * e < cnt) cp[u][rows[lane + 32 * e]] = v[u][e];
   __syncwarp();
-  T b0 = lane < jb ? cp[j + lane] : T(0);
-  T b1 = lane + 32 < jb ? cp[j + lane + 32] : T(0);
+  T b0[CPW], b1[CPW];
+#pragma unroll
+  for (int u = 0; u < CPW; ++u) {
+    b0[u] = lane < jb ? cp[u][j + lane] : T(0);
+    b1[u] = lane + 32 < jb ? cp[u][j + lane + 32] : T(0);
+  }
   // rows 0..31 take updates from k < 32 only: two loops, so that no warp
   // instruction runs with every lane idle (an FP64 one costs its full slot)
   const int k0 = jb < 32 ? jb : 32;
   for (int k = 0; k < k0; ++k) {
-    const T bk = __shfl_sync(0xffffffffu, b0, k);
-    if (lane > k) b0 = fmaT(-L[lane + k * SNB], bk, b0);
-    if (lane + 32 < jb) b1 = fmaT(-L[lane + 32 + k * SNB], bk, b1);
+    const T l0 = L[lane + k * SNB], l1 = L[lane + 32 + k * SNB];
+#pragma unroll
+    for (int u = 0; u < CPW; ++u) {
+      const T bk = __shfl_sync(0xffffffffu, b0[u], k);
+      if (lane > k) b0[u] = fmaT(-l0, bk, b0[u]);
+      if (lane + 32 < jb) b1[u] = fmaT(-l1, bk, b1[u]);
+    }
   }
   for (int k = 32; k < jb; ++k) {
-    const T bk = __shfl_sync(0xffffffffu, b1, k - 32);
-    if (lane + 32 > k && lane + 32 < jb) b1 = fmaT(-L[lane + 32 + k * SNB], bk, b1);
-  }
-  if (lane < jb) cp[j + lane] = b0;
-  if (lane + 32 < jb) cp[j + lane + 32] = b1;
-  if (bop != nullptr) {
-    // row (col - j - jb) of the K-major B operand: the 64 values of U12's column
-    if constexpr (std::is_same<T, float>::value) {
-      __shared__ float stage[8][SNB];
-      float *st = stage[threadIdx.x >> 5];
-      st[lane] = lane < jb ? b0 : 0.f;
-      st[lane + 32] = lane + 32 < jb ? b1 : 0.f;
-      __syncwarp();
-      if (lane == 0) write_operand_row(kind, bop, bop_lo, col - j - jb, st);
-    } else {
-      oz_split_pair(lane < jb ? (double)b0 : 0.0, lane + 32 < jb ? (double)b1 : 0.0, lane, col - j - jb, cap,
-                    static_cast<__nv_bfloat16 *>(bop), bexp);
+    const T l1 = L[lane + 32 + k * SNB];
+#pragma unroll
+    for (int u = 0; u < CPW; ++u) {
+      const T bk = __shfl_sync(0xffffffffu, b1[u], k - 32);
+      if (lane + 32 > k && lane + 32 < jb) b1[u] = fmaT(-l1, bk, b1[u]);
     }
+  }
+#pragma unroll
+  for (int u = 0; u < CPW; ++u) {
+    if (w + u >= w1) break;
+    if (lane < jb) cp[u][j + lane] = b0[u];
+    if (lane + 32 < jb) cp[u][j + lane + 32] = b1[u];
+    if (bop == nullptr) continue;
+    // row (col - j - jb) of the K-major B operand: the 64 values of U12's column
+    const T x0 = lane < jb ? b0[u] : T(0), x1 = lane + 32 < jb ? b1[u] : T(0);
+    if constexpr (std::is_same<T, float>::value)
+      write_operand_pair(kind, bop, bop_lo, w + u, lane, x0, x1);
+    else
+      oz_split_pair(x0, x1, lane, w + u, cap, static_cast<__nv_bfloat16 *>(bop), bexp);
   }
 }
 
@@ -911,7 +937,7 @@ int MixedLU::reserve(int64_t n_, int kind_, cudaStream_t s) {
     BOLA_TRY_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
     BOLA_TRY_CUDA(cudaStreamCreateWithPriority(&sp, cudaStreamNonBlocking, greatest));
     BOLA_TRY_CUDA(cudaStreamCreateWithPriority(&su, cudaStreamNonBlocking, least));
-    for (cudaEvent_t *e : {&ev_in, &ev_sw, &ev_wide, &ev_done})
+    for (cudaEvent_t *e : {&ev_in, &ev_pan, &ev_sw, &ev_wide, &ev_done})
       BOLA_TRY_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   }
   if (n_ <= cap_n && kind_ == kind && aop[0]) {
@@ -973,7 +999,7 @@ void MixedLU::release(cudaStream_t s) {
 
 void MixedLU::destroy() {
   release(nullptr);
-  for (cudaEvent_t *e : {&ev_in, &ev_sw, &ev_wide, &ev_done}) {
+  for (cudaEvent_t *e : {&ev_in, &ev_pan, &ev_sw, &ev_wide, &ev_done}) {
     if (*e) cudaEventDestroy(*e);
     *e = nullptr;
   }
@@ -1046,26 +1072,36 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
     } else
       BOLA_TRY(launch_ppanel(lu.sp, W + j + j * ldw, ldw, mp, jb, ipiv + j, (int32_t)j, info, plan_k, track,
                              give_up, lu.err));
-    // the row swaps reach every column: the previous wide update must be done
+    // the row swaps reach the next panel's columns: the previous wide update must be done
     if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(lu.sp, lu.ev_wide, 0));
     wide_pending = false;
-    if (n > jb) {  // (also the last panel: its moves reach the row permutation)
-      ProfScope prof(lu.sp, fp64 ? "sswap_trsm64" : "sswap_trsm", (double)jb * jb * (double)(n - j - jb));
-      // (the FP32 factors: one more CTA per 64 rows below the panel writes
-      // the update's A operand)
-      const int ncta = (int)imax(1, cdiv(n - j - jb, 8));
-      const int nop = (!fp64 && upd) ? (int)cdiv(mp - jb, SNB) : 0;
-      StepLaunch L(dim3((unsigned)(ncta + nop)), dim3(256), 0, lu.sp, true);
-      BOLA_TRY_CUDA(cudaLaunchKernelEx(
-          &L.cfg, sswap_trsm<T>, W, ldw, n, (int64_t)j, jb, (const int32_t *)plan_k, lu.kind,
-          upd ? (void *)lu.bop : nullptr, fp64 ? (float *)nullptr : lu.bop_lo, fp64 ? lu.eb : (int32_t *)nullptr,
-          lu.cap_n, abort, ncta, fp64 ? (void *)nullptr : lu.aop[buf], fp64 ? (float *)nullptr : lu.aop_lo[buf],
-          perm));
-      BOLA_CHECK_LAUNCH();
-    }
-    if (!upd) continue;
     const int64_t m2 = mp - jb, n2 = n - j - jb;
-    const int64_t nb_next = imin((int64_t)panel_width(fp64, n, j + jb), n2);
+    const int64_t nb_next = upd ? imin((int64_t)panel_width(fp64, n, j + jb), n2) : 0;
+    // interchanges, U12 and B operand of the columns [w0, w1) right of the panel
+    auto swap = [&](cudaStream_t st, int64_t w0, int64_t w1) -> int {
+      ProfScope prof(st, fp64 ? "sswap_trsm64" : "sswap_trsm", (double)jb * jb * (double)(w1 - w0));
+      // (on sp also the row permutation and, for the FP32 factors, one more
+      // CTA per 64 rows below the panel that writes the update's A operand)
+      const bool first = st == lu.sp;
+      const bool two = cdiv(w1 - w0, 8) > 2 * (int64_t)num_sms();
+      const int ncta = (int)imax(1, cdiv(w1 - w0, two ? 16 : 8));
+      const int nop = (!fp64 && upd && first) ? (int)cdiv(m2, SNB) : 0;
+      StepLaunch L(dim3((unsigned)(ncta + nop)), dim3(256), 0, st, first);
+      BOLA_TRY_CUDA(cudaLaunchKernelEx(
+          &L.cfg, two ? sswap_trsm<T, 2> : sswap_trsm<T, 1>, W, ldw, n, (int64_t)j, jb, (const int32_t *)plan_k, lu.kind,
+          upd ? (void *)lu.bop : nullptr, fp64 ? (float *)nullptr : lu.bop_lo, fp64 ? lu.eb : (int32_t *)nullptr,
+          lu.cap_n, abort, w0, w1, ncta, fp64 ? (void *)nullptr : lu.aop[buf],
+          fp64 ? (float *)nullptr : lu.aop_lo[buf], first ? perm : nullptr));
+      BOLA_CHECK_LAUNCH();
+      return 0;
+    };
+    if (n2 > nb_next) {  // the columns after the next panel's, beside the critical stream
+      BOLA_TRY_CUDA(cudaEventRecord(lu.ev_pan, lu.sp));
+      BOLA_TRY_CUDA(cudaStreamWaitEvent(lu.su, lu.ev_pan, 0));
+      BOLA_TRY(swap(lu.su, nb_next, n2));
+    }
+    if (n > jb) BOLA_TRY(swap(lu.sp, 0, nb_next));  // (also the last panel: its moves reach the row permutation)
+    if (!upd) continue;
     T *W22 = W + (j + jb) + (j + jb) * ldw;
     // (the next panel's columns follow the swap kernel on sp as its
     // programmatic dependent; the rest go to su)
