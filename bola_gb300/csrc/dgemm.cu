@@ -380,7 +380,10 @@ __global__ void __launch_bounds__(EDGE_T) gemm_edges(const __grid_constant__ Gem
 }
 
 // All of K in one CTA per tile: the first `big` cells of 64x64 as one tile
-// each, the others as 32x32 and, the last of them, 16x16 blocks.
+// each, the others as 32x32 and, the last of them, 16x16 blocks.  104 registers
+// a thread: two CTAs then leave an SM room for one of the small kernels of a
+// factorisation's critical stream (a 32-row solve, a swap), which otherwise
+// waits for a tile to end.
 template <bool TA, bool TB>
 __global__ void __maxnreg__(104) gemm_grid64(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) unsigned char smem[stage_bytes<64, 64>()];

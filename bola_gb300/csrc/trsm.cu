@@ -5,11 +5,13 @@
 // DGEMM for every off-diagonal block, so >97% of the flops run in the GEMM
 // kernel.  The <=64 base cases run on the GPU with BOLA's per-element order:
 //   left, no transpose  — column forward/back substitution with BOLA's daxpy
-//                         (a warp per right-hand side, rows across lanes);
-//   left, transpose     — dot-style substitution, one thread per column;
-//   right               — column sweeps, one thread per row of B; the
-//                         ascending ones (rnu, rtl) for n <= 32
-//                         right-looking, a row over 4 lanes in registers.
+//                         (left_n_base: a warp per right-hand side, rows
+//                         across lanes);
+//   left, transpose, and right — a system is a right-hand side or a row of B:
+//                         a warp per system (tri_warp) while there are few;
+//                         the ascending ones of order <= 32 eight lanes per
+//                         system (tri_asc32); a thread per system for the
+//                         rest (left_t_base, right_base).
 #include "common.cuh"
 
 namespace bola {
@@ -356,7 +358,7 @@ tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *__re
 // Up to how many systems a warp each (tri_warp) beats a thread each: the warps
 // of one SM share its FP64 pipe (n = 64: ~27 cycles of the GPU per ascending
 // system, ~210 per descending one, against 280k cycles for any number of
-// threads; rows of at most 32 columns over 4 lanes take ~24k cycles.
+// threads; tri_asc32 takes ~24k cycles for any number up to its grid's size).
 constexpr int64_t ASC_WARP_MAX = 8192, SEQ_WARP_MAX = 1216, ASC32_WARP_MAX = 912;
 
 struct Ctx {
