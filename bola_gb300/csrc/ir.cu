@@ -129,20 +129,24 @@ convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const doubl
     if (j0 + u < n) W[i + (j0 + u) * ldw] = scaled_pow2<T>(v[u], k, p, 0, 1.0);
 }
 
-// max|u_ii| and min|u_ii| of the low-precision U (one CTA): a cheap lower
-// bound on the conditioning the refinement will face.
+// max|u_ii| and min|u_ii| of the low-precision U (one CTA of at most 32 warps):
+// a cheap lower bound on the conditioning the refinement will face.  Compared
+// as bits; a NaN is passed over.
 template <typename T>
-__global__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, double *out) {
-  __shared__ double mx[32], mn[32];
-  double a = 0.0, b = INFINITY;
+__device__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, double *out) {
+  __shared__ uint64_t mx[32], mn[32];
+  constexpr uint64_t INF = 0x7ff0000000000000ull;
+  uint64_t a = 0, b = INF;
+#pragma unroll 4
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-    const double v = fabs((double)W[i + i * ldw]);
-    a = fmax(a, v);
-    b = fmin(b, v);
+    const uint64_t v = oz_mag((double)W[i + i * ldw]);
+    a = v > a && v <= INF ? v : a;
+    b = v < b ? v : b;
   }
   for (int off = 16; off > 0; off >>= 1) {
-    a = fmax(a, __shfl_xor_sync(0xffffffffu, a, off));
-    b = fmin(b, __shfl_xor_sync(0xffffffffu, b, off));
+    const uint64_t oa = __shfl_xor_sync(0xffffffffu, a, off), ob = __shfl_xor_sync(0xffffffffu, b, off);
+    a = oa > a ? oa : a;
+    b = ob < b ? ob : b;
   }
   if ((threadIdx.x & 31) == 0) {
     mx[threadIdx.x >> 5] = a;
@@ -151,11 +155,11 @@ __global__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, dou
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int w = 1; w < (int)(blockDim.x >> 5); ++w) {
-      a = fmax(a, mx[w]);
-      b = fmin(b, mn[w]);
+      a = mx[w] > a ? mx[w] : a;
+      b = mn[w] < b ? mn[w] : b;
     }
-    out[0] = fmax(a, mx[0]);
-    out[1] = fmin(b, mn[0]);
+    out[0] = __longlong_as_double((long long)a);
+    out[1] = __longlong_as_double((long long)b);
   }
 }
 
@@ -177,37 +181,38 @@ __global__ void compose_perm(int64_t n, const int32_t *ipiv, int32_t *perm) {
   for (int64_t i = threadIdx.x; i < n; i += blockDim.x) perm[i] = p[i];
 }
 
-// max that keeps a NaN (fmax would drop it): the norms below feed the
-// backward-error test, which must fail on a NaN anywhere in x or r
-__device__ __forceinline__ double nan_max(double a, double b) { return (b > a || b != b) ? b : a; }
-
-// Per right-hand side: out[c] = max_i |v[i, c]| (one CTA per column).
-__global__ void col_absmax(int64_t n, const double *__restrict__ v, int64_t ldv, double *out) {
-  __shared__ double red[32];
-  const int c = blockIdx.x;
-  double m = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) m = nan_max(m, fabs(v[i + c * ldv]));
-  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double mm = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mm = nan_max(mm, red[w]);
-    out[c] = mm;
+// max_i |v[i, c]| of up to two groups of columns, a CTA per column.  Compared
+// as bits, in which a NaN exceeds every number: it is kept (fmax would drop
+// it), since the norms feed the backward-error test, which must fail on a NaN
+// anywhere in x or r.
+struct Columns {
+  const double *v;
+  int64_t ld;
+  double *out;
+  int count;
+};
+__global__ void __launch_bounds__(512)
+col_absmax(int64_t n, Columns first, Columns second) {
+  __shared__ uint64_t red[16];
+  const bool two = (int)blockIdx.x >= first.count;
+  const Columns &g = two ? second : first;
+  const int c = (int)blockIdx.x - (two ? first.count : 0);
+  const double *v = g.v + (int64_t)c * g.ld;
+  uint64_t m = 0;
+#pragma unroll 4
+  for (int64_t i = threadIdx.x; i < n; i += 512) {
+    const uint64_t x = oz_mag(v[i]);
+    m = x > m ? x : m;
   }
-}
-
-__global__ void max_of(int64_t n, const double *v, double *out) {
-  __shared__ double red[32];
-  double m = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += blockDim.x) m = nan_max(m, v[i]);
-  for (int off = 16; off > 0; off >>= 1) m = nan_max(m, __shfl_xor_sync(0xffffffffu, m, off));
+  for (int off = 16; off > 0; off >>= 1) {
+    const uint64_t o = __shfl_xor_sync(0xffffffffu, m, off);
+    m = o > m ? o : m;
+  }
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
   __syncthreads();
   if (threadIdx.x == 0) {
-    double mm = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) mm = nan_max(mm, red[w]);
-    *out = mm;
+    for (int w = 1; w < 16; ++w) m = red[w] > m ? red[w] : m;
+    g.out[c] = __longlong_as_double((long long)m);
   }
 }
 
@@ -306,7 +311,11 @@ __device__ __forceinline__ double quotient(double t, double, const Divisor &q) {
 
 template <typename T>
 __global__ void __launch_bounds__(DI_THREADS)
-diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du) {
+diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du, double *extent) {
+  if ((int64_t)blockIdx.x * TB >= n) {  // (the last CTA, beside the others)
+    diag_extent(n, W, ldw, extent);
+    return;
+  }
   __shared__ T B[TB][TB + 1];
   __shared__ Divisor dv[TB];
   const unsigned FULL = 0xffffffffu;
@@ -420,14 +429,16 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned long lon
 // C_d[b] = Dinv_b T[b, k] (column-major 64 x 64), k the block d places
 // before b in solve order (d = blockIdx.y + 1): L[b, b - d] (lower),
 // U[b, b + d] (upper).  C holds C_d for all blocks at C + ((d-1) nb + b) 4096.
-template <bool LOWER>
 __global__ void __launch_bounds__(256)
-couple_blocks(int64_t n, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dinv, float *C) {
+couple_blocks(int64_t n, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dl,
+              const float *__restrict__ Du, float *Cl, float *Cu) {
   __shared__ float D[TB][TB + 1], T[TB][TB + 1];
   const int nb = (int)cdiv(n, TB);
   const int b = blockIdx.x, d = (int)blockIdx.y + 1;
-  float *outp = C + ((int64_t)(d - 1) * nb + b) * TB * TB;
-  const int k = LOWER ? b - d : b + d;
+  const bool lower = blockIdx.z == 0;
+  const float *Dinv = lower ? Dl : Du;
+  float *outp = (lower ? Cl : Cu) + ((int64_t)(d - 1) * nb + b) * TB * TB;
+  const int k = lower ? b - d : b + d;
   if (k < 0 || k >= nb) return;
   const int64_t i0 = (int64_t)b * TB, k0 = (int64_t)k * TB;
   const int kb = (int)imin(TB, n - i0), kbk = (int)imin(TB, n - k0);
@@ -939,10 +950,9 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const float *W, int64_
 // Dinv times the coupling blocks of the FP32 factor's L and U (once per factorisation).
 int couple(cudaStream_t s, int64_t n, const float *W, int64_t ldw, const float *Dl, const float *Du, float *Cl,
            float *Cu) {
-  ProfScope prof(s, "trsv_couple", 2.0 * TNP * 2 * (double)cdiv(n, TB) * TB * TB * TB, 0.0, 2);
+  ProfScope prof(s, "trsv_couple", 2.0 * TNP * 2 * (double)cdiv(n, TB) * TB * TB * TB, 0.0, 1);
   const unsigned nb = (unsigned)cdiv(n, TB);
-  couple_blocks<true><<<dim3(nb, TNP), 256, 0, s>>>(n, W, ldw, Dl, Cl);
-  couple_blocks<false><<<dim3(nb, TNP), 256, 0, s>>>(n, W, ldw, Du, Cu);
+  couple_blocks<<<dim3(nb, TNP, 2), 256, 0, s>>>(n, W, ldw, Dl, Du, Cl, Cu);
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -1167,10 +1177,9 @@ int residual_berr(cudaStream_t s, Workspace &w, int64_t n, int nr, const double 
                   int64_t ldb, const double *x, int64_t ldx, double *berr) {
   double *nrm = w.norms;
   {
-    ProfScope prof(s, "mixed_residual", 2.0 * (double)n * n * nr, 2.0 * OZ_SA * (double)n * n, 4 * (int)cdiv(nr, 16) + 2);
+    ProfScope prof(s, "mixed_residual", 2.0 * (double)n * n * nr, 2.0 * OZ_SA * (double)n * n, 4 * (int)cdiv(nr, 16) + 1);
     BOLA_TRY(w.oz.product(s, nr, x, ldx, b, ldb, w.r, n, w.ts.err));
-    col_absmax<<<nr, 256, 0, s>>>(n, w.r, n, nrm);
-    col_absmax<<<nr, 256, 0, s>>>(n, x, ldx, nrm + nr);
+    col_absmax<<<2 * nr, 512, 0, s>>>(n, Columns{w.r, n, nrm, nr}, Columns{x, ldx, nrm + nr, nr});
   }
   BOLA_CHECK_LAUNCH();
   // through the workspace's pinned staging: both reads are truly asynchronous
@@ -1218,7 +1227,7 @@ int gmres_step(cudaStream_t s, Workspace &w, int64_t n, int nr, const double *a,
   int kk = 0;
   for (int k = 0; k < GM_M; ++k) {
     double *Vk = w.V + (int64_t)k * nr * n, *Zk = w.Z + (int64_t)k * nr * n;
-    col_absmax<<<nr, 256, 0, s>>>(n, Vk, n, beta_d);
+    col_absmax<<<nr, 512, 0, s>>>(n, Columns{Vk, n, beta_d, nr}, Columns{});
     BOLA_CHECK_LAUNCH();
     BOLA_TRY(correction(s, w, n, nr, Vk, n, beta_d, Zk, n, true));
     {
@@ -1406,9 +1415,8 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   // another factor within the same call keeps them)
   if (!w.split_kept) BOLA_TRY(w.oz.split(s, a, lda, w.rowsum));
   {
-    ProfScope prof(s, "mixed_norms", 0.0, 8.0 * (double)n * nr, 2);
-    max_of<<<1, 1024, 0, s>>>(n, w.rowsum, nrm + 3 * nr);
-    col_absmax<<<nr, 256, 0, s>>>(n, b, ldb, nrm + 2 * nr);
+    ProfScope prof(s, "mixed_norms", 0.0, 8.0 * (double)n * nr, 1);
+    col_absmax<<<1 + nr, 512, 0, s>>>(n, Columns{w.rowsum, n, nrm + 3 * nr, 1}, Columns{b, ldb, nrm + 2 * nr, nr});
   }
   BOLA_CHECK_LAUNCH();
   // The spread max|u_ii| / min|u_ii| of the low-precision U is a cheap lower
@@ -1454,13 +1462,13 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
     ProfScope prof(s, "diag_inverses");
     const unsigned nb = (unsigned)cdiv(n, TB);
     if (fp64) {
-      diag_block_inverses<double><<<nb, DI_THREADS, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl, (double *)w.Du);
-      diag_extent<double><<<1, 1024, 0, s>>>(n, (const double *)w.W, ldW, w.norms + 5 * MAXRHS);
+      diag_block_inverses<double><<<nb + 1, DI_THREADS, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl,
+                                                                (double *)w.Du, w.norms + 5 * MAXRHS);
     } else {
-      diag_block_inverses<float><<<nb, DI_THREADS, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du);
+      diag_block_inverses<float><<<nb + 1, DI_THREADS, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du,
+                                                               w.norms + 5 * MAXRHS);
       BOLA_TRY(couple(s, n, (const float *)w.W, n, (const float *)w.Dl, (const float *)w.Du,
                       const_cast<float *>(w.ts.Cl), const_cast<float *>(w.ts.Cu)));
-      diag_extent<float><<<1, 1024, 0, s>>>(n, (const float *)w.W, n, w.norms + 5 * MAXRHS);
     }
   }
   BOLA_CHECK_LAUNCH();
