@@ -129,11 +129,18 @@ convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const doubl
     if (j0 + u < n) W[i + (j0 + u) * ldw] = scaled_pow2<T>(v[u], k, p, 0, 1.0);
 }
 
+// What the host decides on after a factorisation, gathered on the device so that one copy brings it.
+struct FactorEnd {
+  double largest, smallest;  // |u_ii|
+  uint64_t track[3];         // MixedLU::track
+  int32_t info, err;
+};
+
 // max|u_ii| and min|u_ii| of the low-precision U (one CTA of at most 32 warps):
 // a cheap lower bound on the conditioning the refinement will face.  Compared
 // as bits; a NaN is passed over.
 template <typename T>
-__device__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, double *out) {
+__device__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, FactorEnd *out) {
   __shared__ uint64_t mx[32], mn[32];
   constexpr uint64_t INF = 0x7ff0000000000000ull;
   uint64_t a = 0, b = INF;
@@ -158,8 +165,8 @@ __device__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, dou
       a = mx[w] > a ? mx[w] : a;
       b = mn[w] < b ? mn[w] : b;
     }
-    out[0] = __longlong_as_double((long long)a);
-    out[1] = __longlong_as_double((long long)b);
+    out->largest = __longlong_as_double((long long)a);
+    out->smallest = __longlong_as_double((long long)b);
   }
 }
 
@@ -184,7 +191,7 @@ __global__ void compose_perm(int64_t n, const int32_t *ipiv, int32_t *perm) {
 // max_i |v[i, c]| of up to two groups of columns, a CTA per column.  Compared
 // as bits, in which a NaN exceeds every number: it is kept (fmax would drop
 // it), since the norms feed the backward-error test, which must fail on a NaN
-// anywhere in x or r.
+// anywhere in x or r.  flag (optional) is left beside them, as a number.
 struct Columns {
   const double *v;
   int64_t ld;
@@ -192,12 +199,13 @@ struct Columns {
   int count;
 };
 __global__ void __launch_bounds__(512)
-col_absmax(int64_t n, Columns first, Columns second) {
+col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag = nullptr, double *flag_out = nullptr) {
   __shared__ uint64_t red[16];
   const bool two = (int)blockIdx.x >= first.count;
   const Columns &g = two ? second : first;
   const int c = (int)blockIdx.x - (two ? first.count : 0);
   const double *v = g.v + (int64_t)c * g.ld;
+  if (flag != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *flag_out = (double)*flag;
   uint64_t m = 0;
 #pragma unroll 4
   for (int64_t i = threadIdx.x; i < n; i += 512) {
@@ -311,9 +319,13 @@ __device__ __forceinline__ double quotient(double t, double, const Divisor &q) {
 
 template <typename T>
 __global__ void __launch_bounds__(DI_THREADS)
-diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du, double *extent) {
+diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du, FactorEnd *end, const uint64_t *track,
+                    const int32_t *info, const int32_t *err) {
   if ((int64_t)blockIdx.x * TB >= n) {  // (the last CTA, beside the others)
-    diag_extent(n, W, ldw, extent);
+    if (threadIdx.x < 3) end->track[threadIdx.x] = track[threadIdx.x];
+    if (threadIdx.x == 3) end->info = *info;
+    if (threadIdx.x == 4) end->err = *err;
+    diag_extent(n, W, ldw, end);
     return;
   }
   __shared__ T B[TB][TB + 1];
@@ -1179,16 +1191,15 @@ int residual_berr(cudaStream_t s, Workspace &w, int64_t n, int nr, const double 
   {
     ProfScope prof(s, "mixed_residual", 2.0 * (double)n * n * nr, 2.0 * OZ_SA * (double)n * n, 4 * (int)cdiv(nr, 16) + 1);
     BOLA_TRY(w.oz.product(s, nr, x, ldx, b, ldb, w.r, n, w.ts.err));
-    col_absmax<<<2 * nr, 512, 0, s>>>(n, Columns{w.r, n, nrm, nr}, Columns{x, ldx, nrm + nr, nr});
+    col_absmax<<<2 * nr, 512, 0, s>>>(n, Columns{w.r, n, nrm, nr}, Columns{x, ldx, nrm + nr, nr}, w.ts.err,
+                                   nrm + 3 * nr + 1);
   }
   BOLA_CHECK_LAUNCH();
-  // through the workspace's pinned staging: both reads are truly asynchronous
+  // through the workspace's pinned staging: the read is truly asynchronous
   const double *h = w.hpin;
-  int32_t *terr_h = reinterpret_cast<int32_t *>(w.hpin + 3 * MAXRHS + 1);
-  BOLA_TRY_CUDA(cudaMemcpyAsync(w.hpin, nrm, sizeof(double) * (3 * nr + 1), cudaMemcpyDeviceToHost, s));
-  BOLA_TRY_CUDA(cudaMemcpyAsync(terr_h, w.ts.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+  BOLA_TRY_CUDA(cudaMemcpyAsync(w.hpin, nrm, sizeof(double) * (3 * nr + 2), cudaMemcpyDeviceToHost, s));
   BOLA_TRY_CUDA(cudaStreamSynchronize(s));
-  const int32_t terr = *terr_h;
+  const int32_t terr = (int32_t)h[3 * nr + 1];
   if (terr != 0) {
     cudaMemsetAsync(w.ts.err, 0, sizeof(int32_t), s);
     return fail(BOLA_ERR_CUDA, "mixed: a bounded wait expired in the refinement (code %d)", terr);
@@ -1460,26 +1471,26 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   }
   {
     ProfScope prof(s, "diag_inverses");
+    FactorEnd *end = reinterpret_cast<FactorEnd *>(w.norms + 5 * MAXRHS);
     const unsigned nb = (unsigned)cdiv(n, TB);
     if (fp64) {
       diag_block_inverses<double><<<nb + 1, DI_THREADS, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl,
-                                                                (double *)w.Du, w.norms + 5 * MAXRHS);
+                                                                (double *)w.Du, end, w.lu.track, w.info, w.lu.err);
     } else {
       diag_block_inverses<float><<<nb + 1, DI_THREADS, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du,
-                                                               w.norms + 5 * MAXRHS);
+                                                               end, w.lu.track, w.info, w.lu.err);
       BOLA_TRY(couple(s, n, (const float *)w.W, n, (const float *)w.Dl, (const float *)w.Du,
                       const_cast<float *>(w.ts.Cl), const_cast<float *>(w.ts.Cu)));
     }
   }
   BOLA_CHECK_LAUNCH();
-  double ext[2] = {0.0, 0.0};
-  BOLA_TRY_CUDA(cudaMemcpyAsync(ext, w.norms + 5 * MAXRHS, sizeof ext, cudaMemcpyDeviceToHost, s));
-  int32_t finfo = 0, ferr = 0;
-  uint64_t trk[3] = {0, 0, 0};
-  BOLA_TRY_CUDA(cudaMemcpyAsync(trk, w.lu.track, sizeof trk, cudaMemcpyDeviceToHost, s));
-  BOLA_TRY_CUDA(cudaMemcpyAsync(&finfo, w.info, sizeof finfo, cudaMemcpyDeviceToHost, s));
-  BOLA_TRY_CUDA(cudaMemcpyAsync(&ferr, w.lu.err, sizeof ferr, cudaMemcpyDeviceToHost, s));
+  static_assert(sizeof(FactorEnd) <= sizeof(double) * 8, "its room in norms and in the pinned staging");
+  BOLA_TRY_CUDA(cudaMemcpyAsync(w.hpin, w.norms + 5 * MAXRHS, sizeof(FactorEnd), cudaMemcpyDeviceToHost, s));
   BOLA_TRY_CUDA(cudaStreamSynchronize(s));
+  const FactorEnd fin = *reinterpret_cast<const FactorEnd *>(w.hpin);
+  double ext[2] = {fin.largest, fin.smallest};
+  const uint64_t *const trk = fin.track;
+  const int32_t finfo = fin.info, ferr = fin.err;
   info_out.factor_info = finfo;
   info_out.factorization = chol ? 1 : 0;
   // a bounded wait gave up: 5 the panel's candidate exchange, others a
