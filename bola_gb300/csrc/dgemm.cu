@@ -51,6 +51,7 @@ struct GemmArgs {
   int kc;
   const int32_t *info;
   int tri;
+  int first;       // this launch is the product's first
   int edge;        // CTAs that take the edge elements
   int big;         // CTAs with a 64x64 cell, a 32x32 block, a 16x16 block
   int n32, n16;
@@ -367,15 +368,20 @@ __device__ __forceinline__ void cell_at(const GemmArgs &g, int t, int &ci, int &
 // touches other elements of C, lets the next one start as soon as its CTAs are
 // placed, and waits for the one before at its end only, so that what follows on
 // the stream finds all of them done.
+// The first one waits for whatever precedes the product before it lets the
+// others start.
 struct InParallel {
-  __device__ InParallel() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+  __device__ explicit InParallel(const GemmArgs &g) {
+    if (g.first) sm100::grid_dependency_wait();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
   __device__ ~InParallel() { sm100::grid_dependency_wait(); }
 };
 
 template <bool TA, bool TB>
 __global__ void __launch_bounds__(EDGE_T) gemm_edges(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) unsigned char smem[edge_bytes()];
-  InParallel ip;
+  InParallel ip(g);
   if (!stop_flag(g.info)) edge_elements<TA, TB>(g, blockIdx.x, smem);
 }
 
@@ -387,7 +393,7 @@ __global__ void __launch_bounds__(EDGE_T) gemm_edges(const __grid_constant__ Gem
 template <bool TA, bool TB>
 __global__ void __maxnreg__(104) gemm_grid64(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) unsigned char smem[stage_bytes<64, 64>()];
-  InParallel ip;
+  InParallel ip(g);
   if (stop_flag(g.info)) return;
   int b = (int)blockIdx.x, ci, cj;
   if (b < g.big) {
@@ -414,7 +420,7 @@ template <int BT, bool TA, bool TB>
 __global__ void __launch_bounds__(Tile<BT>::NT, BT == 32 ? 5 : BT == 16 ? 10 : 12)
 gemm_grid32(const __grid_constant__ GemmArgs g) {
   __shared__ __align__(16) unsigned char smem[stage_bytes<BT, BT>()];
-  InParallel ip;
+  InParallel ip(g);
   if (stop_flag(g.info)) return;
   const int b = (int)blockIdx.x;
   int ci, cj;
@@ -433,7 +439,7 @@ template <bool TA, bool TB>
 __global__ void __launch_bounds__(Tile<32>::NT, 5) gemm_partial(const __grid_constant__ GemmArgs g) {
   using T = Tile<32>;
   __shared__ __align__(16) unsigned char smem[stage_bytes<32, 32>()];
-  InParallel ip;
+  InParallel ip(g);
   if (stop_flag(g.info)) return;
   const int64_t nchunks = (g.K + g.kc - 1) / g.kc, nsplit = (nchunks + g.cps - 1) / g.cps;
   const int64_t t = blockIdx.x / nsplit, sp = blockIdx.x % nsplit;
@@ -485,7 +491,7 @@ __global__ void __launch_bounds__(Tile<BT>::NT) gemm_split(const __grid_constant
   double *part = reinterpret_cast<double *>(part_raw);  // [cps][TILE], element (i, j) at i + BT j
   cg::cluster_group cluster = cg::this_cluster();
   const int ns = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  InParallel ip;
+  InParallel ip(g);
   int ci, cj;
   cell_at<false>(g, (int)blockIdx.x / ns, ci, cj);
   const int64_t i0 = BT * (int64_t)ci, j0 = BT * (int64_t)cj;
@@ -686,10 +692,9 @@ int launch_plan(cudaStream_t s, TilePlan &p) {
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cfg.attrs = attr;
-    if (beside) {
-      attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-      attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-    }
+    g.first = beside ? 0 : 1;
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     if (cluster > 0) {
       attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
       attr[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;

@@ -318,6 +318,7 @@ template <int RPT>
 __global__ void __launch_bounds__(PAN_T, 1)
 panel_lu_cluster(double *A, int64_t lda, int64_t mp64, int nb, int32_t *ipiv, int32_t *info, int32_t add_on_success,
                  int32_t col0, int lanes, int64_t R64, int32_t *plan, bool fresh) {
+  sm100::grid_dependency_wait();
   cg::cluster_group cluster = cg::this_cluster();
   const int C = (int)cluster.num_blocks();
   const int cr = (int)cluster.block_rank();
@@ -714,6 +715,7 @@ __global__ void plan_from_ipiv(int jb, const int32_t *ipiv, int32_t j, const int
 constexpr int SW_WARPS = 4;
 __global__ void __launch_bounds__(32 * SW_WARPS)
 step_swap_trsm(double *A, int64_t lda, int64_t j, int jb, int64_t c0, int64_t ncols, const int32_t *plan, int lanes) {
+  sm100::grid_dependency_wait();
   __shared__ double L[PNB * PNB];
   if (stop_flag(plan + PLAN_STOP)) return;
   const int lane = threadIdx.x & 31;
@@ -789,7 +791,7 @@ int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int
     cfg.blockDim = dim3(use_smem ? PAN_T : PT, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)C;
     attr[0].val.clusterDim.y = 1;
@@ -812,6 +814,9 @@ int launch_panel(cudaStream_t s, double *A, int64_t lda, int64_t mp, int nb, int
     if (known.load(std::memory_order_relaxed) < 0) continue;
     const int lanes_v = lanes();
     if (use_smem) {
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_after
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.numAttrs = 2;
       BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, cluster_kern, A, lda, mp, nb, ipiv, info, add_on_success, col0, lanes_v, R,
                                        plan, fresh));
       return 0;
@@ -908,7 +913,8 @@ int swap_columns(cudaStream_t s, double *A, int64_t lda, int64_t j, int jb, int6
   if (ncols <= 0) return 0;
   ProfScope prof(s, "getrf_swap_trsm", (double)jb * (jb - 1) * (double)nright, 32.0 * jb * (double)ncols);
   BOLA_TRY(roomy(step_swap_trsm));
-  step_swap_trsm<<<(unsigned)cdiv(ncols, SW_WARPS), 32 * SW_WARPS, 0, s>>>(A, lda, j, jb, c0, ncols, plan, lanes());
+  BOLA_TRY_CUDA(launch_after(step_swap_trsm, dim3((unsigned)cdiv(ncols, SW_WARPS)), 32 * SW_WARPS, 0, s, A, lda, j, jb, c0,
+                             ncols, plan, lanes()));
   BOLA_CHECK_LAUNCH();
   return 0;
 }

@@ -15,6 +15,7 @@
 // 'L' potrf2 block runs column by column with BOLA's fused/unfused pattern
 // per element; 'U' and failing blocks use BOLA's recursion.
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace bola {
 namespace {
@@ -47,6 +48,7 @@ template <int SLOTS>
 __global__ void __launch_bounds__(NB *SLOTS)
 syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const double *__restrict__ A,
           int64_t lda, double *C, int64_t ldc, int lanes, const int32_t *info) {
+  sm100::grid_dependency_wait();
   __shared__ double sA[NB][NB + 1];      // 'N': sA[l][r] = A(j0 + r, p0 + l); 'T': sA[r][l] = A(p0 + l, j0 + r)
   __shared__ double tls[SLOTS][2][NB];   // 'N': alpha * A(j0 + jj, p0 + l), the warp's columns' multipliers
   if (__syncthreads_or(stop_flag(info))) return;  // (another stream may set it: one answer per CTA)
@@ -130,8 +132,8 @@ int launch_syrk_diag(cudaStream_t s, bool upper, bool trans_t, int64_t n, int64_
   void (*kern)(bool, bool, int64_t, int64_t, double, const double *, int64_t, double *, int64_t, int, const int32_t *) =
       slots == 9 ? syrk_diag<9> : syrk_diag<1>;
   BOLA_TRY(roomy(kern));
-  kern<<<dim3((unsigned)cdiv(SYRK_WARPS, slots), (unsigned)blocks), NB * slots, 0, s>>>(
-      upper, trans_t, n, k, alpha, A, lda, C, ldc, lanes(), info);
+  BOLA_TRY_CUDA(launch_after(kern, dim3((unsigned)cdiv(SYRK_WARPS, slots), (unsigned)blocks), NB * slots, 0, s, upper,
+                             trans_t, n, k, alpha, A, lda, C, ldc, lanes(), info));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -406,6 +408,7 @@ __device__ int p2_upper32(double *a, int lanes) {
 
 __global__ void __launch_bounds__(P2_T)
 potrf2_block(bool upper, int n, double *A, int64_t lda, int32_t *info, int32_t col0, int lanes) {
+  sm100::grid_dependency_wait();
   __shared__ double a[NB * P2P];
   __shared__ double a0[LDS * LDS];  // the input, for the recursion: a failing block, a short 'U' one
   __shared__ double rdg[LDS];
@@ -465,7 +468,7 @@ int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int
   if (n <= NB) {
     ProfScope prof(s, "potrf2_block", (double)n * n * n / 3.0);
     BOLA_TRY(roomy(potrf2_block));
-    potrf2_block<<<1, P2_T, 0, s>>>(upper, (int)n, A, lda, info, col0, lanes());
+    BOLA_TRY_CUDA(launch_after(potrf2_block, dim3(1), P2_T, 0, s, upper, (int)n, A, lda, info, col0, lanes()));
     BOLA_CHECK_LAUNCH();
     return 0;
   }

@@ -13,6 +13,7 @@
 //                         system (tri_asc32); a thread per system for the
 //                         rest (left_t_base, right_base).
 #include "common.cuh"
+#include "sm100.cuh"
 
 namespace bola {
 namespace {
@@ -21,6 +22,7 @@ constexpr int STOP = 64;  // TRSM_RECURSION_STOP (src/trsm.rs:8)
 
 __global__ void scale_matrix(int64_t m, int64_t n, double alpha, double *B, int64_t ldb,
                              const int32_t *info) {
+  sm100::grid_dependency_wait();
   if (stop_flag(info)) return;
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= m * n) return;
@@ -45,6 +47,7 @@ template <bool LOWER>
 __global__ void __launch_bounds__(32 * LN_WARPS)
 left_n_base(int m, int64_t n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
             int64_t ldb, int lanes, const int32_t *info) {
+  sm100::grid_dependency_wait();
   __shared__ double sA[STOP * STOP];
   __shared__ Divisor dv[STOP];
   if (stop_flag(info)) return;
@@ -120,6 +123,7 @@ template <bool ASC, bool RIGHT>
 __global__ void __launch_bounds__(32 * TW_WARPS)
 tri_warp(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
          int64_t elem, int64_t sys, const int32_t *info) {
+  sm100::grid_dependency_wait();
   __shared__ double T[STOP * TW_PITCH];
   __shared__ Divisor dv[STOP];
   __shared__ __align__(16) double pbuf[TW_WARPS][2][STOP];
@@ -216,6 +220,7 @@ template <bool LOWER>
 __global__ void __launch_bounds__(TCOLS)
 left_t_base(int m, int64_t n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
             int64_t ldb, const int32_t *info) {
+  sm100::grid_dependency_wait();
   __shared__ double sA[STOP * STOP];
   __shared__ double sB[STOP * TCOLS];
   if (stop_flag(info)) return;
@@ -261,6 +266,7 @@ template <int V>
 __global__ void __launch_bounds__(RB_ROWS)
 right_base(int64_t m, int n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
            int64_t ldb, const int32_t *info) {
+  sm100::grid_dependency_wait();
   extern __shared__ double rb_smem[];
   double *sA = rb_smem;      // n x n, ld n
   double *rd = sA + n * n;   // 1 / a(j, j)
@@ -314,6 +320,7 @@ template <bool RIGHT>
 __global__ void __launch_bounds__(AS_THREADS)
 tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
           int64_t elem, int64_t sys, const int32_t *info) {
+  sm100::grid_dependency_wait();
   __shared__ double T[32 * 33];  // coefficient of x_k in equation j at T[k * 33 + j]
   __shared__ Divisor dv[32];
   if (stop_flag(info)) return;
@@ -374,9 +381,11 @@ int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
   const unsigned g = (unsigned)cdiv(n, LN_WARPS);
   BOLA_TRY(roomy(lower ? left_n_base<true> : left_n_base<false>));
   if (lower)
-    left_n_base<true><<<g, 32 * LN_WARPS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
+    BOLA_TRY_CUDA(launch_after(left_n_base<true>, dim3(g), 32 * LN_WARPS, 0, c.s, (int)m, n, c.unit, A, lda, B, ldb,
+                               c.lanes, c.info));
   else
-    left_n_base<false><<<g, 32 * LN_WARPS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.lanes, c.info);
+    BOLA_TRY_CUDA(launch_after(left_n_base<false>, dim3(g), 32 * LN_WARPS, 0, c.s, (int)m, n, c.unit, A, lda, B, ldb,
+                               c.lanes, c.info));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -386,8 +395,8 @@ int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
   if (!lower && m <= 32 && n > ASC32_WARP_MAX) {
     BOLA_TRY(roomy(tri_asc32<false>));
-    tri_asc32<false><<<(unsigned)cdiv(n, AS_SYS), AS_THREADS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb,
-                                                                        c.info);
+    BOLA_TRY_CUDA(launch_after(tri_asc32<false>, dim3((unsigned)cdiv(n, AS_SYS)), AS_THREADS, 0, c.s, (int)m, n,
+                               c.unit, false, A, lda, B, 1, ldb, c.info));
     BOLA_CHECK_LAUNCH();
     return 0;
   }
@@ -395,17 +404,19 @@ int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
     const unsigned gw = (unsigned)cdiv(n, TW_WARPS);
     BOLA_TRY(roomy(lower ? tri_warp<false, false> : tri_warp<true, false>));
     if (lower)
-      tri_warp<false, false><<<gw, 32 * TW_WARPS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb, c.info);
+      BOLA_TRY_CUDA(launch_after(tri_warp<false, false>, dim3(gw), 32 * TW_WARPS, 0, c.s, (int)m, n, c.unit, false, A,
+                                 lda, B, 1, ldb, c.info));
     else
-      tri_warp<true, false><<<gw, 32 * TW_WARPS, 0, c.s>>>((int)m, n, c.unit, false, A, lda, B, 1, ldb, c.info);
+      BOLA_TRY_CUDA(launch_after(tri_warp<true, false>, dim3(gw), 32 * TW_WARPS, 0, c.s, (int)m, n, c.unit, false, A,
+                                 lda, B, 1, ldb, c.info));
     BOLA_CHECK_LAUNCH();
     return 0;
   }
   const unsigned g = (unsigned)cdiv(n, TCOLS);
   if (lower)
-    left_t_base<true><<<g, TCOLS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.info);
+    BOLA_TRY_CUDA(launch_after(left_t_base<true>, dim3(g), TCOLS, 0, c.s, (int)m, n, c.unit, A, lda, B, ldb, c.info));
   else
-    left_t_base<false><<<g, TCOLS, 0, c.s>>>((int)m, n, c.unit, A, lda, B, ldb, c.info);
+    BOLA_TRY_CUDA(launch_after(left_t_base<false>, dim3(g), TCOLS, 0, c.s, (int)m, n, c.unit, A, lda, B, ldb, c.info));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -415,16 +426,16 @@ int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64
   constexpr bool asc = V == 1 || V == 2;
   if (m <= (!asc ? SEQ_WARP_MAX : n <= 32 ? ASC32_WARP_MAX : ASC_WARP_MAX)) {
     BOLA_TRY(roomy(tri_warp<asc, true>));
-    tri_warp<asc, true><<<(unsigned)cdiv(m, TW_WARPS), 32 * TW_WARPS, 0, c.s>>>((int)n, m, c.unit, V >= 2, A, lda, B, ldb,
-                                                                              1, c.info);
+    BOLA_TRY_CUDA(launch_after(tri_warp<asc, true>, dim3((unsigned)cdiv(m, TW_WARPS)), 32 * TW_WARPS, 0, c.s, (int)n,
+                               m, c.unit, V >= 2, A, lda, B, ldb, 1, c.info));
     BOLA_CHECK_LAUNCH();
     return 0;
   }
   if constexpr (asc) {
     if (n <= 32) {
       BOLA_TRY(roomy(tri_asc32<true>));
-      tri_asc32<true><<<(unsigned)cdiv(m, AS_SYS), AS_THREADS, 0, c.s>>>((int)n, m, c.unit, V >= 2, A, lda, B, ldb, 1,
-                                                                         c.info);
+      BOLA_TRY_CUDA(launch_after(tri_asc32<true>, dim3((unsigned)cdiv(m, AS_SYS)), AS_THREADS, 0, c.s, (int)n, m,
+                                 c.unit, V >= 2, A, lda, B, ldb, 1, c.info));
       BOLA_CHECK_LAUNCH();
       return 0;
     }
@@ -432,7 +443,8 @@ int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64
   const size_t smem = right_base_smem((int)n);
   if (smem > 48 * 1024) BOLA_TRY_CUDA(cudaFuncSetAttribute(right_base<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   BOLA_TRY(roomy(right_base<V>));
-  right_base<V><<<(unsigned)cdiv(m, RB_ROWS), RB_ROWS, smem, c.s>>>(m, (int)n, c.unit, A, lda, B, ldb, c.info);
+  BOLA_TRY_CUDA(launch_after(right_base<V>, dim3((unsigned)cdiv(m, RB_ROWS)), RB_ROWS, smem, c.s, m, (int)n, c.unit,
+                             A, lda, B, ldb, c.info));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -526,7 +538,7 @@ int trsm_exact(cudaStream_t s, char side, char uplo, char transa, char diag, int
   if (m <= 0 || n <= 0) return 0;
   if (alpha != 1.0) {
     ProfScope prof(s, "scale", (double)m * n);
-    scale_matrix<<<(unsigned)cdiv(m * n, 256), 256, 0, s>>>(m, n, alpha, B, ldb, info);
+    BOLA_TRY_CUDA(launch_after(scale_matrix, dim3((unsigned)cdiv(m * n, 256)), 256, 0, s, m, n, alpha, B, ldb, info));
     BOLA_CHECK_LAUNCH();
   }
   Ctx c{s, upc(diag) == 'U', lanes(), info};
