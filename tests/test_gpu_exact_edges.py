@@ -89,3 +89,21 @@ def test_potrf_blocks(both, uplo, n):
     assert o.potrf(uplo, n, A1, n) == 0
     assert g.potrf(uplo, n, A2, n) == 0
     assert same(A1, A2)
+
+
+@pytest.mark.parametrize("n,nrhs", [(32, 3), (33, 1), (200, 3), (257, 300), (1025, 5), (3100, 2)])
+def test_getrs_rows(both, n, nrhs):
+    """Interchanges that move rows anywhere (not only down), the solve after them."""
+    g, o = both
+    rng = np.random.default_rng(n)
+    A = wl.uniform_matrix(n, n, seed=n, lo=-1, hi=1) / n
+    A[np.diag_indices(n)] = 2.0 + rng.random(n)
+    piv = rng.integers(1, n + 1, n).astype(np.int32)
+    piv[::3] = np.arange(1, n + 1)[::3]
+    B = wl.uniform_matrix(n + 3, nrhs, seed=2, lo=-1, hi=1)
+    B1, B2 = B.copy(order="F"), B.copy(order="F")
+    o.laswp(nrhs, B1, n + 3, 1, n, piv, 1)
+    o.trsm("L", "L", "N", "U", n, nrhs, 1.0, A, n, B1, n + 3)
+    o.trsm("L", "U", "N", "N", n, nrhs, 1.0, A, n, B1, n + 3)
+    g.getrs(n, nrhs, A, n, piv, B2, n + 3)
+    assert same(B1, B2)
