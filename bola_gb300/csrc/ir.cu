@@ -200,6 +200,7 @@ struct Columns {
 };
 __global__ void __launch_bounds__(512)
 col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag = nullptr, double *flag_out = nullptr) {
+  sm100::grid_dependency_wait();
   __shared__ uint64_t red[16];
   const bool two = (int)blockIdx.x >= first.count;
   const Columns &g = two ? second : first;
@@ -228,7 +229,10 @@ col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag = nullp
 // scale of a Cholesky's D A D, or none)
 template <typename T>
 __global__ void permute_scale_down(int64_t n, int nrhs, const double *__restrict__ r, int64_t ldr,
-                                   const int32_t *perm, const double *rscale, T *__restrict__ y, const double *pre) {
+                                   const int32_t *perm, const double *rscale, T *__restrict__ y, const double *pre,
+                                   int32_t *tickets) {
+  sm100::grid_dependency_wait();
+  if (blockIdx.x == 0 && threadIdx.x < 2) tickets[threadIdx.x] = 0;  // of the two solves that follow
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n * nrhs) return;
   const int64_t i = e % n, c = e / n;
@@ -244,6 +248,7 @@ __global__ void permute_scale_down(int64_t n, int nrhs, const double *__restrict
 template <typename T>
 __global__ void update_x(int64_t n, int nrhs, const T *__restrict__ y, const double *scale, const double *rscale,
                          double *__restrict__ x, int64_t ldx, int assign, const double *postrow) {
+  sm100::grid_dependency_wait();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= n * nrhs) return;
   const int64_t i = e % n, c = e / n;
@@ -630,6 +635,7 @@ __global__ void __launch_bounds__(256)
 trsv_words(int64_t n, int nrhs, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dinv,
            const float *__restrict__ C, const float *__restrict__ y, float *out, unsigned long long *xw,
            int32_t *ticket, uint32_t epoch, int32_t *err) {
+  sm100::grid_dependency_wait();
   extern __shared__ __align__(128) float tsm[];
   using Tile = float[TB][TB];      // Tile[kk][r] = operand(r, kk), the column-major 64 x 64 block
   using Blk = float[TB][4 * RH];   // Blk[kk][c]
@@ -832,6 +838,7 @@ __global__ void __launch_bounds__(T64_PARTS * TB)
 trsv_dataflow64(int64_t n, int nrhs, const double *__restrict__ W, int64_t ldw, const double *__restrict__ Dinv,
                 const double *__restrict__ y, double *out, int32_t *flags, int32_t *ticket, int32_t epoch,
                 int32_t *err) {
+  sm100::grid_dependency_wait();
   constexpr int PER = TB / T64_PARTS;  // columns of a block per thread
   __shared__ double xs[TB], red[T64_PARTS][TB];
   __shared__ int sb;
@@ -888,7 +895,7 @@ trsv_dataflow64(int64_t n, int nrhs, const double *__restrict__ W, int64_t ldw, 
 }
 
 // Sequencing state of the dataflow solves: flags (one per 64-row block and
-// right-hand side, zeroed once), the ticket, the wait-expiry flag and the
+// right-hand side, zeroed once), the tickets (lower, upper), the wait-expiry flag and the
 // launch epoch.
 struct TrsvSync {
   int32_t *flags = nullptr, *ticket = nullptr, *err = nullptr;
@@ -906,11 +913,13 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const double *W, int64
   ProfScope prof(s, lower ? "trsv64_lower" : "trsv64_upper", (double)n * n * nrhs, 8.0 * (double)n * n / 2, 1);
   const unsigned grid = (unsigned)(cdiv(n, TB) * nrhs);
   const int32_t epoch = ++sync.epoch;
-  BOLA_TRY_CUDA(cudaMemsetAsync(sync.ticket, 0, sizeof(int32_t), s));
+  int32_t *const ticket = sync.ticket + (lower ? 0 : 1);  // (zeroed by permute_scale_down)
   if (lower)
-    trsv_dataflow64<true><<<grid, T64_PARTS * TB, 0, s>>>(n, nrhs, W, ldw, Dinv, y, out, sync.flags, sync.ticket, epoch, sync.err);
+    BOLA_TRY_CUDA(launch_after(trsv_dataflow64<true>, dim3(grid), T64_PARTS * TB, 0, s, n, nrhs, W, ldw, Dinv, y, out,
+                               sync.flags, ticket, epoch, sync.err));
   else
-    trsv_dataflow64<false><<<grid, T64_PARTS * TB, 0, s>>>(n, nrhs, W, ldw, Dinv, y, out, sync.flags, sync.ticket, epoch, sync.err);
+    BOLA_TRY_CUDA(launch_after(trsv_dataflow64<false>, dim3(grid), T64_PARTS * TB, 0, s, n, nrhs, W, ldw, Dinv, y, out,
+                               sync.flags, ticket, epoch, sync.err));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -919,19 +928,21 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const float *W, int64_
   ProfScope prof(s, lower ? "trsv_lower" : "trsv_upper", (double)n * n * nrhs, 4.0 * (double)n * n / 2, 1);
   const unsigned nb = (unsigned)cdiv(n, TB);
   const uint32_t epoch = (uint32_t)++sync.epoch;
-  BOLA_TRY_CUDA(cudaMemsetAsync(sync.ticket, 0, sizeof(int32_t), s));
+  int32_t *const ticket = sync.ticket + (lower ? 0 : 1);  // (zeroed by permute_scale_down)
   const float *C = lower ? sync.Cl : sync.Cu;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(cdiv(nb, TCL) * TCL));
   cfg.blockDim = dim3(256);
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];  // the cluster; as launch_after
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = TCL;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
 #define BOLA_TRSV(LW, RH)                                                                                    \
   do {                                                                                                       \
     static bool attr_set = false;                                                                            \
@@ -945,7 +956,7 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const float *W, int64_
     }                                                                                                        \
     cfg.dynamicSmemBytes = trsv_words_smem<RH>();                                                            \
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, trsv_words<LW, RH>, n, nrhs, W, ldw, Dinv, C, y, out, sync.xw,    \
-                                     sync.ticket, epoch, sync.err));                                         \
+                                     ticket, epoch, sync.err));                                              \
   } while (0)
   if (nrhs <= 16) {
     if (lower) BOLA_TRSV(true, 4);
@@ -1124,16 +1135,16 @@ int ws_reserve(Workspace &w, int64_t n, int64_t nrhs, int kind, cudaStream_t s) 
     BOLA_TRY(alloc(&w.H, sizeof(double) * (GM_M + 2) * MAXRHS * 2));
     BOLA_TRY(alloc(&w.hn, sizeof(double) * MAXRHS));
     BOLA_TRY(alloc(&w.ts.flags, sizeof(int32_t) * cdiv(n, TB) * MAXRHS));
-    BOLA_TRY(alloc(&w.ts.ticket, sizeof(int32_t) * 2));
+    BOLA_TRY(alloc(&w.ts.ticket, sizeof(int32_t) * 3));
     BOLA_TRY(alloc(&w.Mc, sizeof(float) * 2 * TNP * cdiv(n, TB) * TB * TB));
     BOLA_TRY(alloc(&w.ts.xw, sizeof(unsigned long long) * n * MAXRHS));
     // the published words start from epoch 0, which no launch uses
     BOLA_TRY_CUDA(cudaMemset(w.ts.xw, 0, sizeof(unsigned long long) * n * MAXRHS));
     w.ts.Cl = w.Mc;
     w.ts.Cu = w.Mc + TNP * cdiv(n, TB) * TB * TB;
-    w.ts.err = w.ts.ticket + 1;
+    w.ts.err = w.ts.ticket + 2;
     BOLA_TRY_CUDA(cudaMemset(w.ts.flags, 0, sizeof(int32_t) * cdiv(n, TB) * MAXRHS));
-    BOLA_TRY_CUDA(cudaMemset(w.ts.ticket, 0, sizeof(int32_t) * 2));
+    BOLA_TRY_CUDA(cudaMemset(w.ts.ticket, 0, sizeof(int32_t) * 3));
     w.ts.epoch = 0;
     w.n = n;
     w.nrhs = nrhs;
@@ -1166,19 +1177,23 @@ int correction(cudaStream_t s, Workspace &w, int64_t n, int nrhs, const double *
   if (w.fkind == 3) {
     double *y = static_cast<double *>(w.y), *z = static_cast<double *>(w.z);
     const double *W = static_cast<const double *>(w.W);
-    permute_scale_down<double><<<g, 256, 0, s>>>(n, nrhs, r, ldr, w.perm, rs, y, w.chol ? w.dscale : nullptr);
+    BOLA_TRY_CUDA(launch_after(permute_scale_down<double>, dim3(g), 256, 0, s, n, nrhs, r, ldr, w.perm, rs, y,
+                               w.chol ? w.dscale : nullptr, w.ts.ticket));
     BOLA_CHECK_LAUNCH();
     BOLA_TRY(trsv(s, true, n, nrhs, W, w.ldW, static_cast<const double *>(w.Dl), y, z, w.ts));
     BOLA_TRY(trsv(s, false, n, nrhs, W, w.ldW, static_cast<const double *>(w.Du), z, y, w.ts));
-    update_x<double><<<g, 256, 0, s>>>(n, nrhs, y, w.scale, rs, x, ldx, assign ? 1 : 0, w.chol ? w.dscale : nullptr);
+    BOLA_TRY_CUDA(launch_after(update_x<double>, dim3(g), 256, 0, s, n, nrhs, y, w.scale, rs, x, ldx, assign ? 1 : 0,
+                               w.chol ? w.dscale : nullptr));
   } else {
     float *y = static_cast<float *>(w.y), *z = static_cast<float *>(w.z);
     const float *W = static_cast<const float *>(w.W);
-    permute_scale_down<float><<<g, 256, 0, s>>>(n, nrhs, r, ldr, w.perm, rs, y, w.chol ? w.dscale : nullptr);
+    BOLA_TRY_CUDA(launch_after(permute_scale_down<float>, dim3(g), 256, 0, s, n, nrhs, r, ldr, w.perm, rs, y,
+                               w.chol ? w.dscale : nullptr, w.ts.ticket));
     BOLA_CHECK_LAUNCH();
     BOLA_TRY(trsv(s, true, n, nrhs, W, n, static_cast<const float *>(w.Dl), y, z, w.ts));
     BOLA_TRY(trsv(s, false, n, nrhs, W, n, static_cast<const float *>(w.Du), z, y, w.ts));
-    update_x<float><<<g, 256, 0, s>>>(n, nrhs, y, w.scale, rs, x, ldx, assign ? 1 : 0, w.chol ? w.dscale : nullptr);
+    BOLA_TRY_CUDA(launch_after(update_x<float>, dim3(g), 256, 0, s, n, nrhs, y, w.scale, rs, x, ldx, assign ? 1 : 0,
+                               w.chol ? w.dscale : nullptr));
   }
   BOLA_CHECK_LAUNCH();
   return 0;
@@ -1189,10 +1204,10 @@ int residual_berr(cudaStream_t s, Workspace &w, int64_t n, int nr, const double 
                   int64_t ldb, const double *x, int64_t ldx, double *berr) {
   double *nrm = w.norms;
   {
-    ProfScope prof(s, "mixed_residual", 2.0 * (double)n * n * nr, 2.0 * OZ_SA * (double)n * n, 4 * (int)cdiv(nr, 16) + 1);
+    ProfScope prof(s, "mixed_residual", 2.0 * (double)n * n * nr, 2.0 * OZ_SA * (double)n * n, 3 * (int)cdiv(nr, 16) + 1);
     BOLA_TRY(w.oz.product(s, nr, x, ldx, b, ldb, w.r, n, w.ts.err));
-    col_absmax<<<2 * nr, 512, 0, s>>>(n, Columns{w.r, n, nrm, nr}, Columns{x, ldx, nrm + nr, nr}, w.ts.err,
-                                   nrm + 3 * nr + 1);
+    BOLA_TRY_CUDA(launch_after(col_absmax, dim3(2 * nr), 512, 0, s, n, Columns{w.r, n, nrm, nr},
+                               Columns{x, ldx, nrm + nr, nr}, w.ts.err, nrm + 3 * nr + 1));
   }
   BOLA_CHECK_LAUNCH();
   // through the workspace's pinned staging: the read is truly asynchronous

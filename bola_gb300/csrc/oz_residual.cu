@@ -192,11 +192,13 @@ oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int3
 // One CTA per column: its max, then its digits.
 __global__ void __launch_bounds__(1024)
 oz_split_rhs(int64_t n, int nr, const double *__restrict__ x, int64_t ldx, int64_t kp, __nv_bfloat16 *__restrict__ out,
-             int32_t *f) {
+             int32_t *f, unsigned long long *acc) {
+  sm100::grid_dependency_wait();
   __shared__ unsigned long long red[32];
   __shared__ int32_t fe;
   const int c = blockIdx.x;
   const double *xc = x + (int64_t)c * ldx;
+  for (int64_t i = threadIdx.x; i < 2 * n; i += blockDim.x) acc[2 * n * c + i] = 0;  // the product's sums
   uint64_t m = 0;
   if (c < nr)
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
@@ -248,6 +250,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 __global__ void __launch_bounds__(OZR_THREADS, 1)
 oz_product_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapX, int64_t n,
                   int64_t mrows, int chunks_per_cta, unsigned long long *acc, int32_t *err) {
+  sm100::grid_dependency_wait();
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t full[NST], empty[NST], tfull[2], tempty[2];
   __shared__ uint32_t tmem_slot;
@@ -396,6 +399,7 @@ __device__ __forceinline__ double scale2(double v, int k) {
 // out = b - A x (b given) or A x, from the fixed-point sums; columns c < nr.
 __global__ void oz_product_finish(int64_t n, int nr, int c0, const unsigned long long *acc, const int32_t *e,
                                   const int32_t *f, const double *b, int64_t ldb, double *out, int64_t ldo) {
+  sm100::grid_dependency_wait();
   const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n * nr) return;
   const int64_t i = q % n;
@@ -484,12 +488,13 @@ int OzMatrix::product(cudaStream_t s, int nr, const double *x, int64_t ldx, cons
   const int grid_y = (int)cdiv(nchunks, cpc);
   for (int c0 = 0; c0 < nr; c0 += NRB) {
     const int nb = (int)imin(NRB, nr - c0);
-    ProfScope prof(s, "oz_product", 2.0 * (double)n * n * nb, 2.0 * SA * (double)n * n, 4);
-    BOLA_TRY_CUDA(cudaMemsetAsync(acc, 0, sizeof(unsigned long long) * 2 * NRB * n, s));
-    oz_split_rhs<<<NRB, 1024, 0, s>>>(n, nb, x + (int64_t)c0 * ldx, ldx, kp, xplanes, f);
-    oz_product_kernel<<<dim3((unsigned)mt, (unsigned)grid_y), OZR_THREADS, OZR_SMEM, s>>>(mapA, mapX, n, mrows, cpc,
-                                                                                          acc, err);
-    oz_product_finish<<<(unsigned)cdiv(n * nb, 256), 256, 0, s>>>(n, nb, c0, acc, e, f, b, ldb, out, ldo);
+    ProfScope prof(s, "oz_product", 2.0 * (double)n * n * nb, 2.0 * SA * (double)n * n, 3);
+    BOLA_TRY_CUDA(launch_after(oz_split_rhs, dim3(NRB), 1024, 0, s, n, nb, x + (int64_t)c0 * ldx, ldx, kp, xplanes, f,
+                               acc));
+    BOLA_TRY_CUDA(launch_after(oz_product_kernel, dim3((unsigned)mt, (unsigned)grid_y), OZR_THREADS, OZR_SMEM, s, mapA,
+                               mapX, n, mrows, cpc, acc, err));
+    BOLA_TRY_CUDA(launch_after(oz_product_finish, dim3((unsigned)cdiv(n * nb, 256)), 256, 0, s, n, nb, c0, acc, e, f, b,
+                               ldb, out, ldo));
     BOLA_CHECK_LAUNCH();
   }
   return 0;
