@@ -371,6 +371,7 @@ chol_l21(T *W, int64_t ldw, int64_t mp, int jb, int kind, void *aop, float *aop_
 // The diagonal of L, before chol_to_lu overwrites it.
 template <typename T>
 __global__ void chol_diag(int64_t n, const T *W, int64_t ldw, T *dg) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) dg[i] = W[i + i * ldw];
 }
@@ -381,6 +382,7 @@ __global__ void chol_diag(int64_t n, const T *W, int64_t ldw, T *dg) {
 // no other CTA touches.
 template <typename T>
 __global__ void __launch_bounds__(256) chol_to_lu(int64_t n, T *W, int64_t ldw, const T *dg) {
+  sm100::grid_dependency_wait();
   __shared__ T t[32][33];
   const int64_t I = blockIdx.x, J = blockIdx.y;
   if (J > I) return;
@@ -493,9 +495,9 @@ int MixedLU::factor_chol64(cudaStream_t s, double *W, int64_t ldw, int32_t *info
 template <typename T>
 int chol_lu_form(cudaStream_t s, int64_t n, T *W, int64_t ldw, T *dg) {
   ProfScope prof(s, "chol_to_lu", 0.0, 3.0 * sizeof(T) * (double)n * n / 2.0, 2);
-  chol_diag<T><<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, W, ldw, dg);
+  BOLA_TRY_CUDA(launch_after(chol_diag<T>, dim3((unsigned)cdiv(n, 256)), 256, 0, s, n, W, ldw, dg));
   const unsigned nt = (unsigned)cdiv(n, 32);
-  chol_to_lu<T><<<dim3(nt, nt), 256, 0, s>>>(n, W, ldw, dg);
+  BOLA_TRY_CUDA(launch_after(chol_to_lu<T>, dim3(nt, nt), 256, 0, s, n, W, ldw, dg));
   BOLA_CHECK_LAUNCH();
   return 0;
 }

@@ -47,6 +47,7 @@ constexpr int MAXRHS = 32;  // right-hand sides per refinement sweep
 // max|a| in [2^(e-1), 2^e).  A NaN is passed over.
 __global__ void __launch_bounds__(256)
 colblock_max(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *mbits) {
+  sm100::grid_dependency_wait();
   __shared__ uint64_t red[8];
   const int64_t c0 = (int64_t)blockIdx.x * TB, c1 = imin(n, c0 + TB);
   const int64_t rs = cdiv(n, (int64_t)gridDim.y), r0 = (int64_t)blockIdx.y * rs, r1 = imin(n, r0 + rs);
@@ -71,6 +72,7 @@ colblock_max(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long
   }
 }
 __global__ void colblock_finish(int64_t nb, double *scale) {
+  sm100::grid_dependency_wait();
   const int64_t b = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= nb) return;
   const double mm = scale[b];  // (the bits colblock_max left)
@@ -117,6 +119,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const double *scale, T *__restrict__ W,
                int64_t ldw) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
   if (i >= n) return;
   const double p = scale[j0 / TB];
@@ -199,7 +202,7 @@ struct Columns {
   int count;
 };
 __global__ void __launch_bounds__(512)
-col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag = nullptr, double *flag_out = nullptr) {
+col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag, double *flag_out) {
   sm100::grid_dependency_wait();
   __shared__ uint64_t red[16];
   const bool two = (int)blockIdx.x >= first.count;
@@ -269,6 +272,7 @@ __global__ void copy_cols(int64_t n, int nrhs, const double *__restrict__ src, i
 // [0.5, 2), exact, so D A D has an O(1) diagonal.  A diagonal entry that is
 // not positive and finite gets d_i = 1 (the Cholesky then stops at it).
 __global__ void sym_scale(int64_t n, const double *__restrict__ A, int64_t lda, double *d) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double a = A[i + i * lda];
@@ -286,6 +290,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 convert_sym_lower(int64_t n, const double *__restrict__ A, int64_t lda, const double *d, T *__restrict__ W,
                   int64_t ldw) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
   if (i >= n || i < j0) return;
   const double pi = d[i];
@@ -302,6 +307,7 @@ convert_sym_lower(int64_t n, const double *__restrict__ A, int64_t lda, const do
 }
 
 __global__ void iota_perm(int64_t n, int32_t *perm) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) perm[i] = (int32_t)i;
 }
@@ -326,6 +332,7 @@ template <typename T>
 __global__ void __launch_bounds__(DI_THREADS)
 diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du, FactorEnd *end, const uint64_t *track,
                     const int32_t *info, const int32_t *err) {
+  sm100::grid_dependency_wait();
   if ((int64_t)blockIdx.x * TB >= n) {  // (the last CTA, beside the others)
     if (threadIdx.x < 3) end->track[threadIdx.x] = track[threadIdx.x];
     if (threadIdx.x == 3) end->info = *info;
@@ -449,6 +456,7 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned long lon
 __global__ void __launch_bounds__(256)
 couple_blocks(int64_t n, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dl,
               const float *__restrict__ Du, float *Cl, float *Cu) {
+  sm100::grid_dependency_wait();
   __shared__ float D[TB][TB + 1], T[TB][TB + 1];
   const int nb = (int)cdiv(n, TB);
   const int b = blockIdx.x, d = (int)blockIdx.y + 1;
@@ -975,7 +983,7 @@ int couple(cudaStream_t s, int64_t n, const float *W, int64_t ldw, const float *
            float *Cu) {
   ProfScope prof(s, "trsv_couple", 2.0 * TNP * 2 * (double)cdiv(n, TB) * TB * TB * TB, 0.0, 1);
   const unsigned nb = (unsigned)cdiv(n, TB);
-  couple_blocks<<<dim3(nb, TNP, 2), 256, 0, s>>>(n, W, ldw, Dl, Du, Cl, Cu);
+  BOLA_TRY_CUDA(launch_after(couple_blocks, dim3(nb, TNP, 2), 256, 0, s, n, W, ldw, Dl, Du, Cl, Cu));
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -1253,7 +1261,8 @@ int gmres_step(cudaStream_t s, Workspace &w, int64_t n, int nr, const double *a,
   int kk = 0;
   for (int k = 0; k < GM_M; ++k) {
     double *Vk = w.V + (int64_t)k * nr * n, *Zk = w.Z + (int64_t)k * nr * n;
-    col_absmax<<<nr, 512, 0, s>>>(n, Columns{Vk, n, beta_d, nr}, Columns{});
+    BOLA_TRY_CUDA(launch_after(col_absmax, dim3(nr), 512, 0, s, n, Columns{Vk, n, beta_d, nr}, Columns{}, nullptr,
+                               nullptr));
     BOLA_CHECK_LAUNCH();
     BOLA_TRY(correction(s, w, n, nr, Vk, n, beta_d, Zk, n, true));
     {
@@ -1420,21 +1429,22 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   if (chol) {
     // W = D A D (lower triangle), D a power of two per row making the diagonal O(1)
     ProfScope prof(s, "mixed_convert", 0.0, 6.0 * (double)n * n, 2);
-    sym_scale<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, a, lda, w.dscale);
+    BOLA_TRY_CUDA(launch_after(sym_scale, dim3((unsigned)cdiv(n, 256)), 256, 0, s, n, a, lda, w.dscale));
     if (fp64)
-      convert_sym_lower<double><<<cvt, 256, 0, s>>>(n, a, lda, w.dscale, (double *)w.W, ldW);
+      BOLA_TRY_CUDA(launch_after(convert_sym_lower<double>, cvt, 256, 0, s, n, a, lda, w.dscale, (double *)w.W, ldW));
     else
-      convert_sym_lower<float><<<cvt, 256, 0, s>>>(n, a, lda, w.dscale, (float *)w.W, n);
+      BOLA_TRY_CUDA(launch_after(convert_sym_lower<float>, cvt, 256, 0, s, n, a, lda, w.dscale, (float *)w.W, n));
   } else {
     ProfScope prof(s, "mixed_convert", 0.0, 12.0 * (double)n * n, 3);
     BOLA_TRY_CUDA(cudaMemsetAsync(w.scale, 0, sizeof(double) * cdiv(n, TB), s));
-    colblock_max<<<dim3((unsigned)cdiv(n, TB), (unsigned)imin(16, cdiv(n, 256))), 256, 0, s>>>(
-        n, a, lda, reinterpret_cast<unsigned long long *>(w.scale));
-    colblock_finish<<<(unsigned)cdiv(cdiv(n, TB), 256), 256, 0, s>>>(cdiv(n, TB), w.scale);
+    BOLA_TRY_CUDA(launch_after(colblock_max, dim3((unsigned)cdiv(n, TB), (unsigned)imin(16, cdiv(n, 256))), 256, 0, s,
+                               n, a, lda, reinterpret_cast<unsigned long long *>(w.scale)));
+    BOLA_TRY_CUDA(launch_after(colblock_finish, dim3((unsigned)cdiv(cdiv(n, TB), 256)), 256, 0, s, cdiv(n, TB),
+                               w.scale));
     if (fp64)
-      convert_scaled<double><<<cvt, 256, 0, s>>>(n, a, lda, w.scale, (double *)w.W, ldW);
+      BOLA_TRY_CUDA(launch_after(convert_scaled<double>, cvt, 256, 0, s, n, a, lda, w.scale, (double *)w.W, ldW));
     else
-      convert_scaled<float><<<cvt, 256, 0, s>>>(n, a, lda, w.scale, (float *)w.W, n);
+      BOLA_TRY_CUDA(launch_after(convert_scaled<float>, cvt, 256, 0, s, n, a, lda, w.scale, (float *)w.W, n));
   }
   BOLA_CHECK_LAUNCH();
   // A's digit planes and its row sums (once per call: a solve handed on to
@@ -1442,7 +1452,8 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   if (!w.split_kept) BOLA_TRY(w.oz.split(s, a, lda, w.rowsum));
   {
     ProfScope prof(s, "mixed_norms", 0.0, 8.0 * (double)n * nr, 1);
-    col_absmax<<<1 + nr, 512, 0, s>>>(n, Columns{w.rowsum, n, nrm + 3 * nr, 1}, Columns{b, ldb, nrm + 2 * nr, nr});
+    BOLA_TRY_CUDA(launch_after(col_absmax, dim3(1 + nr), 512, 0, s, n, Columns{w.rowsum, n, nrm + 3 * nr, 1},
+                               Columns{b, ldb, nrm + 2 * nr, nr}, nullptr, nullptr));
   }
   BOLA_CHECK_LAUNCH();
   // The spread max|u_ii| / min|u_ii| of the low-precision U is a cheap lower
@@ -1480,7 +1491,7 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
   if (chol || n <= TB) {
     ProfScope prof(s, "mixed_perm");
     if (chol)
-      iota_perm<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, w.perm);
+      BOLA_TRY_CUDA(launch_after(iota_perm, dim3((unsigned)cdiv(n, 256)), 256, 0, s, n, w.perm));
     else
       compose_perm<<<1, 1024, sizeof(int32_t) * n, s>>>(n, w.ipiv, w.perm);
   }
@@ -1489,11 +1500,11 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
     FactorEnd *end = reinterpret_cast<FactorEnd *>(w.norms + 5 * MAXRHS);
     const unsigned nb = (unsigned)cdiv(n, TB);
     if (fp64) {
-      diag_block_inverses<double><<<nb + 1, DI_THREADS, 0, s>>>(n, (const double *)w.W, ldW, (double *)w.Dl,
-                                                                (double *)w.Du, end, w.lu.track, w.info, w.lu.err);
+      BOLA_TRY_CUDA(launch_after(diag_block_inverses<double>, dim3(nb + 1), DI_THREADS, 0, s, n, (const double *)w.W,
+                                 ldW, (double *)w.Dl, (double *)w.Du, end, w.lu.track, w.info, w.lu.err));
     } else {
-      diag_block_inverses<float><<<nb + 1, DI_THREADS, 0, s>>>(n, (const float *)w.W, n, (float *)w.Dl, (float *)w.Du,
-                                                               end, w.lu.track, w.info, w.lu.err);
+      BOLA_TRY_CUDA(launch_after(diag_block_inverses<float>, dim3(nb + 1), DI_THREADS, 0, s, n, (const float *)w.W, n,
+                                 (float *)w.Dl, (float *)w.Du, end, w.lu.track, w.info, w.lu.err));
       BOLA_TRY(couple(s, n, (const float *)w.W, n, (const float *)w.Dl, (const float *)w.Du,
                       const_cast<float *>(w.ts.Cl), const_cast<float *>(w.ts.Cu)));
     }

@@ -100,6 +100,7 @@ __device__ __forceinline__ int32_t exponent_of(uint64_t mag_bits) {
 constexpr int SCH = 128;
 __global__ void __launch_bounds__(256)
 oz_row_stats(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *rmax, double *psum) {
+  sm100::grid_dependency_wait();
   __shared__ double red[128];
   __shared__ unsigned long long mred[128];
   const int r = threadIdx.x & 127, h = threadIdx.x >> 7;
@@ -136,6 +137,7 @@ oz_row_stats(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long
 // rowsum[i] = sum of the partial sums in block order; e[i] from the row max.
 __global__ void oz_row_finish(int64_t n, int nblk, const unsigned long long *rmax, const double *psum, double *rowsum,
                               int32_t *e) {
+  sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   double s = 0.0;
@@ -153,6 +155,7 @@ __global__ void oz_row_finish(int64_t n, int nblk, const unsigned long long *rma
 __global__ void __launch_bounds__(256)
 oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int32_t *__restrict__ e, int64_t mrows,
                 int64_t kp, __nv_bfloat16 *__restrict__ out) {
+  sm100::grid_dependency_wait();
   __shared__ double T[64][65];
   const int64_t i0 = (int64_t)blockIdx.y * 64, j0 = (int64_t)blockIdx.x * 64;
   for (int q = threadIdx.x; q < 64 * 64; q += 256) {
@@ -461,9 +464,11 @@ int OzMatrix::split(cudaStream_t s, const double *A, int64_t lda, double *rowsum
   ProfScope prof(s, "oz_split", 0.0, 8.0 * 2.0 * n * n + 2.0 * SA * n * n, 4);
   const int nblk = (int)cdiv(n, SCH);
   BOLA_TRY_CUDA(cudaMemsetAsync(rmax, 0, sizeof(unsigned long long) * n, s));
-  oz_row_stats<<<dim3((unsigned)cdiv(n, 128), (unsigned)nblk), 256, 0, s>>>(n, A, lda, rmax, psum);
-  oz_row_finish<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, nblk, rmax, psum, rowsum, e);
-  oz_split_matrix<<<dim3((unsigned)cdiv(n, 64), (unsigned)cdiv(n, 64)), 256, 0, s>>>(n, A, lda, e, mrows, kp, planes);
+  BOLA_TRY_CUDA(launch_after(oz_row_stats, dim3((unsigned)cdiv(n, 128), (unsigned)nblk), 256, 0, s, n, A, lda, rmax,
+                             psum));
+  BOLA_TRY_CUDA(launch_after(oz_row_finish, dim3((unsigned)cdiv(n, 256)), 256, 0, s, n, nblk, rmax, psum, rowsum, e));
+  BOLA_TRY_CUDA(launch_after(oz_split_matrix, dim3((unsigned)cdiv(n, 64), (unsigned)cdiv(n, 64)), 256, 0, s, n, A,
+                             lda, e, mrows, kp, planes));
   BOLA_CHECK_LAUNCH();
   BOLA_TRY(make_kmajor_map2(&mapA, planes, n, SA * mrows, kp, RM));
   BOLA_TRY(make_kmajor_map2(&mapX, xplanes, n, SX * NRB, kp, 16));
