@@ -105,34 +105,35 @@ __device__ void group_trailing(double *A, int lda, int n, int k0, int kb, bool l
   const int ntiles = lower ? tr * (tr + 1) / 2 : tr * tc;
   for (int e = t; e < ntiles; e += G) {
     const int i0 = c0 + ti * TR, j0 = c0 + tj * TC;
+    const int nr = n - i0, nc = n - j0;  // rows and columns left: the tile's own where they reach TR and TC
+    double *pc = A + i0 + (int64_t)j0 * lda;
     double acc[TR][TC];
 #pragma unroll
-    for (int r = 0; r < TR; ++r)
+    for (int c = 0; c < TC; ++c)
 #pragma unroll
-      for (int c = 0; c < TC; ++c) {
-        const int i = i0 + r, j = j0 + c;
-        acc[r][c] = (i < n && j < n) ? A[i + (int64_t)j * lda] : 0.0;
-      }
+      for (int r = 0; r < TR; ++r) acc[r][c] = (r < nr && c < nc) ? pc[r + (int64_t)c * lda] : 0.0;
+    const double *pl = A + i0 + (int64_t)k0 * lda;
+    const double *pu = lower ? A + j0 + (int64_t)k0 * lda : A + k0 + (int64_t)j0 * lda;
+    const int64_t su = lower ? 1 : lda, step = lower ? lda : 1;
+#pragma unroll 1
     for (int q = 0; q < kb; ++q) {
-      const int64_t kq = (int64_t)(k0 + q) * lda;
       double l[TR], u[TC];
 #pragma unroll
-      for (int r = 0; r < TR; ++r) l[r] = i0 + r < n ? A[i0 + r + kq] : 0.0;
+      for (int r = 0; r < TR; ++r) l[r] = r < nr ? pl[r] : 0.0;
 #pragma unroll
-      for (int c = 0; c < TC; ++c)
-        u[c] = j0 + c < n ? (lower ? A[j0 + c + kq] : A[(k0 + q) + (int64_t)(j0 + c) * lda]) : 0.0;
+      for (int c = 0; c < TC; ++c) u[c] = c < nc ? pu[c * su] : 0.0;
+      pl += lda;
+      pu += step;
 #pragma unroll
       for (int r = 0; r < TR; ++r)
 #pragma unroll
         for (int c = 0; c < TC; ++c) acc[r][c] = fma(-l[r], u[c], acc[r][c]);
     }
 #pragma unroll
-    for (int r = 0; r < TR; ++r)
+    for (int c = 0; c < TC; ++c)
 #pragma unroll
-      for (int c = 0; c < TC; ++c) {
-        const int i = i0 + r, j = j0 + c;
-        if (i < n && j < n && (!lower || i >= j)) A[i + (int64_t)j * lda] = acc[r][c];
-      }
+      for (int r = 0; r < TR; ++r)
+        if (r < nr && c < nc && (!lower || i0 + r >= j0 + c)) pc[r + (int64_t)c * lda] = acc[r][c];
     if (lower) {
       ti += G;
       while (ti >= tr && tj < tr) {
@@ -420,14 +421,13 @@ __device__ int group_solve(const SystemDesc &S, int t, int G, int g, Shared &sh)
 }
 
 // Bound by FP64 issue (90% of it at orders up to 256) once enough groups share
-// an SM: three CTAs rather than the two that the registers of the trailing
-// update's tile would leave, a few values spilled (with four, whole tiles are:
-// 2% faster at orders up to 256, 20% slower up to 64).  Measured on one GB300,
-// 4000 systems, half LU and half Cholesky: orders 8 to 256, 10.6 ms (13.1 with
-// two CTAs and the panel's columns one after the other through global memory);
-// orders 8 to 64, 0.55 ms (0.64).
-template <int TR>
-__global__ void __launch_bounds__(BT, 3)
+// an SM: CTAS CTAs (batch_ctas), rather than the two that the registers of the
+// trailing update's tile would leave, a few values spilled.  Measured on one
+// GB300, half LU and half Cholesky: 20,000 systems of order 8 to 256 48.4 ms
+// (64.1 with two CTAs and the panel's columns one after the other through global
+// memory, 48.8 with its groups tuned); 4000 of order 8 to 64 0.50 ms (0.62).
+template <int TR, int CTAS>
+__global__ void __launch_bounds__(BT, CTAS)
 batched_solve_kernel(const SystemDesc *__restrict__ sys, const int32_t *__restrict__ items, int32_t nitems,
                      int32_t *counter, int32_t *info) {
   __shared__ int32_t cur[ITEM];
@@ -464,6 +464,7 @@ struct Plan {
   double flops = 0.0;
   int group[NBUCKET];
   int tile = 4;  // register tile rows of the kernel (4 or 2)
+  int ctas = 3;  // per SM (batch_ctas)
   cudaGraphExec_t exec = nullptr;
   const void *g_sys = nullptr;
   const void *g_info = nullptr;
@@ -533,31 +534,46 @@ int batch_items(int32_t count, const int32_t *n, const int32_t *kind, const int3
   return 0;
 }
 
-int batch_grid(int32_t nitems, int tile) {
+// CTAs per SM: four where most of the flops are in systems of order above 128
+// (their barriers and chains need the company), three below, where the values
+// that a fourth CTA spills cost more (3 | 4: 20,000 of order 8 to 256 50.1 |
+// 48.4 ms, 2000 of order 129 to 256 9.4 | 9.1, 4000 of order 8 to 128 1.87 |
+// 2.01, of order 8 to 64 0.50 | 0.65).
+int batch_ctas(int32_t count, const int32_t *n, const int32_t *kind) {
+  double all = 0.0, large = 0.0;
+  for (int i = 0; i < count; ++i) {
+    const double f = (double)n[i] * n[i] * n[i] * (kind && kind[i] == 1 ? 1.0 : 2.0);
+    all += f;
+    if (n[i] > 128) large += f;
+  }
+  return 2.0 * large > all ? 4 : 3;
+}
+
+using BatchKernel = void (*)(const SystemDesc *, const int32_t *, int32_t, int32_t *, int32_t *);
+BatchKernel batch_kernel(int tile, int ctas) {
+  if (tile == 2) return ctas == 4 ? batched_solve_kernel<2, 4> : batched_solve_kernel<2, 3>;
+  return ctas == 4 ? batched_solve_kernel<4, 4> : batched_solve_kernel<4, 3>;
+}
+
+int batch_grid(int32_t nitems, int tile, int ctas) {
   int occ = 0;
-  if (tile == 2)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_solve_kernel<2>, BT, 0);
-  else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batched_solve_kernel<4>, BT, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, batch_kernel(tile, ctas), BT, 0);
   return std::max(1, std::min((int)nitems, num_sms() * std::max(occ, 1)));
 }
 
-void launch_kernel(cudaStream_t s, int tile, int grid, const bola_system *systems, const int32_t *items,
+void launch_kernel(cudaStream_t s, int tile, int ctas, int grid, const bola_system *systems, const int32_t *items,
                    int32_t nitems, int32_t *counter, int32_t *info) {
-  const SystemDesc *sd = reinterpret_cast<const SystemDesc *>(systems);
-  if (tile == 2)
-    batched_solve_kernel<2><<<grid, BT, 0, s>>>(sd, items, nitems, counter, info);
-  else
-    batched_solve_kernel<4><<<grid, BT, 0, s>>>(sd, items, nitems, counter, info);
+  batch_kernel(tile, ctas)<<<grid, BT, 0, s>>>(reinterpret_cast<const SystemDesc *>(systems), items, nitems, counter,
+                                               info);
 }
 
 // One persistent launch over nitems work items (device array); *counter is
 // the work queue's head and is reset here.
 int batch_launch(cudaStream_t s, const bola_system *systems, const int32_t *items, int32_t nitems, int32_t *counter,
-                 int32_t *info, int tile) {
+                 int32_t *info, int tile, int ctas) {
   if (nitems == 0) return 0;
   BOLA_TRY_CUDA(cudaMemsetAsync(counter, 0, sizeof(int32_t), s));
-  launch_kernel(s, tile, batch_grid(nitems, tile), systems, items, nitems, counter, info);
+  launch_kernel(s, tile, ctas, batch_grid(nitems, tile, ctas), systems, items, nitems, counter, info);
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -592,7 +608,8 @@ int bola_batch_plan_create_tuned(int32_t count, const int32_t *n, const int32_t 
     return fail(BOLA_ERR_CUDA, "bola_batch_plan_create: device allocation failed");
   }
   if (!flat.empty()) cudaMemcpy(P->items, flat.data(), sizeof(int32_t) * flat.size(), cudaMemcpyHostToDevice);
-  P->grid = batch_grid(P->nitems, P->tile);
+  P->ctas = batch_ctas(count, n, kind);
+  P->grid = batch_grid(P->nitems, P->tile, P->ctas);
   *plan_out = reinterpret_cast<bola_batch_plan>(P);
   return 0;
 }
@@ -612,7 +629,7 @@ int bola_batch_solve(bola_batch_plan plan, const bola_system *systems, int32_t *
   if (P->nitems == 0) return 0;
   ProfScope prof(s, "batched_solve", P->flops, 0.0, 2);
   BOLA_TRY_CUDA(cudaMemsetAsync(P->counter, 0, sizeof(int32_t), s));
-  launch_kernel(s, P->tile, P->grid, systems, P->items, P->nitems, P->counter, info);
+  launch_kernel(s, P->tile, P->ctas, P->grid, systems, P->items, P->nitems, P->counter, info);
   BOLA_CHECK_LAUNCH();
   return 0;
 }
@@ -632,7 +649,7 @@ int bola_batch_solve_graph(bola_batch_plan plan, const bola_system *systems, int
     cudaGraph_t g;
     BOLA_TRY_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(P->counter, 0, sizeof(int32_t), cap);
-    launch_kernel(cap, P->tile, P->grid, systems, P->items, P->nitems, P->counter, info);
+    launch_kernel(cap, P->tile, P->ctas, P->grid, systems, P->items, P->nitems, P->counter, info);
     BOLA_TRY_CUDA(cudaStreamEndCapture(cap, &g));
     BOLA_TRY_CUDA(cudaGraphInstantiate(&P->exec, g, 0));
     cudaGraphDestroy(g);

@@ -163,8 +163,9 @@ __device__ __forceinline__ double fmaT(double a, double b, double c) { return fm
 int batch_items(int32_t count, const int32_t *n, const int32_t *kind, const int32_t *group_size,
                 std::vector<int32_t> &flat, int32_t *nitems, int *group, double *flops,
                 const int32_t *panel_width = nullptr);
+int batch_ctas(int32_t count, const int32_t *n, const int32_t *kind);
 int batch_launch(cudaStream_t s, const bola_system *systems, const int32_t *items, int32_t nitems, int32_t *counter,
-                 int32_t *info, int tile = 4);
+                 int32_t *info, int tile, int ctas);
 
 // ---- device side -------------------------------------------------------------
 __device__ __forceinline__ double fused(double a, double b, double c) { return __fma_rn(a, b, c); }

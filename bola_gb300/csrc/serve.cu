@@ -409,7 +409,8 @@ struct Server {
     BOLA_TRY_CUDA(cudaMemcpyAsync(A, A0, sizeof(double) * na, cudaMemcpyDeviceToDevice, s));
     BOLA_TRY_CUDA(cudaMemcpyAsync(X, B0, sizeof(double) * nb, cudaMemcpyDeviceToDevice, s));
     BOLA_TRY(batch_launch(s, (const bola_system *)desc.p, (const int32_t *)items.p, nitems, (int32_t *)counter.p,
-                          (int32_t *)info.p, o.tile_rows == 2 ? 2 : 4));
+                          (int32_t *)info.p, o.tile_rows == 2 ? 2 : 4,
+                          batch_ctas(cnt, ns.data(), kinds.data())));
     BOLA_TRY(launch_berr(s, bs, dsys, djobs, dacc, (double *)berr.p));  // synchronises s
     // results back through the same staging buffer
     std::vector<double> hb(cnt);
