@@ -155,13 +155,16 @@ __device__ void group_trailing(double *A, int lda, int n, int k0, int kb, bool l
 // in registers across the iterations (whole blocks of L would be).
 __device__ __forceinline__ void reload() { asm volatile("" ::: "memory"); }
 
-// The panel's first `done` interchanges on all columns (a column of the panel
-// takes those after its own) and on the right-hand sides, a column per thread.
-__device__ __forceinline__ void group_swaps(const SystemDesc &S, int k0, int done, const int *piv, int t, int G) {
+// The first `done` interchanges of the panel of kb columns on all columns and
+// on the right-hand sides, a column per thread.  A column of the panel came out
+// of the registers with those up to its own (all of them from column `done` on,
+// where the panel stopped) and takes the ones after it.
+__device__ __forceinline__ void group_swaps(const SystemDesc &S, int k0, int kb, int done, const int *piv, int t,
+                                            int G) {
   for (int j = t; j < S.n + S.nrhs; j += G) {
     double *col = j < S.n ? S.a + (int64_t)j * S.lda : S.b + (int64_t)(j - S.n) * S.ldb;
 #pragma unroll 1
-    for (int r = j >= k0 && j < k0 + done ? j - k0 + 1 : 0; r < done; ++r) {
+    for (int r = j >= k0 && j < k0 + kb ? j - k0 + 1 : 0; r < done; ++r) {
       const int p = piv[r];
       if (p == k0 + r) continue;
       const double x = col[p];
@@ -329,7 +332,7 @@ __device__ int group_lu_solve(const SystemDesc &S, int t, int G, int g, Shared &
     }
     group_sync(G, g);
     // (a zero pivot ends the factorisation with the interchanges found so far)
-    group_swaps(S, k0, done, sh.piv[g], t, G);
+    group_swaps(S, k0, kb, done, sh.piv[g], t, G);
     group_sync(G, g);
     if (info == 0 && k0 + kb < n) {
       group_u12<PB>(A, lda, n, k0, kb, t, G);
