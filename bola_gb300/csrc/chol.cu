@@ -202,6 +202,7 @@ chol_dblock64(double *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *
     for (int l = 0; l < jb; ++l) {
       const T d = __shfl_sync(0xffffffffu, l < 32 ? c[0] : c[1], l & 31);
       if (!positive(d)) {
+        ch_sync(CH_UPDATED);  // (every update warp has read stop for column l - 1)
         if (lane == 0) {
           stop = 1;
           atomicCAS(info, 0, col0 + l + 1);

@@ -312,6 +312,7 @@ __device__ int p2_lower(double *a, int n, int lanes) {
     for (int l = 0; l < n; ++l) {
       const double d = __shfl_sync(0xffffffffu, c, l);
       if (!positive64(d)) {
+        p2_sync(P2_UPDATED);  // (every update warp has read stop for column l - 1)
         if (lane == 0) stop = l + 1;
         p2_arrive(P2_SCALED);
         break;
@@ -379,6 +380,7 @@ __device__ int p2_upper32(double *a, int lanes) {
     for (int k = 0; k < NB; ++k) {
       const double d = __shfl_sync(0xffffffffu, c, k);
       if (!positive64(d)) {
+        p2_sync(P2_UPDATED);  // (every update warp has read stop for row k - 1)
         if (lane == 0) stop = k + 1;
         p2_arrive(P2_SCALED);
         break;
