@@ -89,6 +89,7 @@ chol_dblock32(float *W, int64_t ldw, int jb, int32_t col0, int64_t n, int32_t *i
         *reinterpret_cast<float4 *>(&D[i & 7][0]) = make_float4(v[0], v[1], v[2], v[3]);
         *reinterpret_cast<float4 *>(&D[i & 7][4]) = make_float4(v[4], v[5], v[6], v[7]);
       }
+      __syncwarp();  // (the barrier counts a warp at its first arrival)
       asm volatile("bar.sync 1, %0;" ::"n"(CNB) : "memory");
       float d[8][8];
 #pragma unroll

@@ -573,6 +573,7 @@ panel_lu64(double *Wp, int64_t ldw, int64_t mp, int jb, int32_t col0, const int3
   for (int k = 0; k < jb; ++k) {
     const int hk = k % PL_LPR;
     // column k's pivot row and reciprocal are final
+    __syncwarp();  // (a barrier counts a warp at its first arrival)
     asm volatile("bar.sync 1, %0;" ::"r"(PL_THREADS) : "memory");
     if (rwarp) {
       // the next pivot, once its row's warp has updated it (named barrier 2:
@@ -580,6 +581,7 @@ panel_lu64(double *Wp, int64_t ldw, int64_t mp, int jb, int32_t col0, const int3
       // updated; the dependent FP64 chain of the reciprocal stays off the
       // row warps
       if (k + 1 < jb) {
+        __syncwarp();
         asm volatile("bar.sync 2, 64;" ::: "memory");
         if (lane == 0) pivot(a[k + 1][k + 1], k + 1);
       }
