@@ -91,7 +91,10 @@ int roomy(void (*kern)(Args...)) {
 
 // Launches a kernel as a programmatic dependent of the one before it on the
 // stream: its CTAs are set up while that one finishes.  Such a kernel calls
-// sm100::grid_dependency_wait() before it touches anything.  (A chain of short
+// sm100::grid_dependency_wait() before it touches anything, and takes what
+// earlier kernels write as plain pointers: it runs before that data is final, so
+// const __restrict__ (data constant while the kernel runs, loads that need not see
+// other kernels' stores) would not be true.  (A chain of short
 // kernels, Cholesky 'U' n = 777: 3218 us against 3474; LU n = 1024: 2403
 // against 2627.)
 template <typename... KArgs, typename... Args>

@@ -771,7 +771,7 @@ __global__ void zero_i32(int32_t *p) { *p = 0; }
 constexpr int GR_T = 256;
 constexpr int64_t GR_MAX = 8192;  // rows: 16 bytes of shared memory each
 __global__ void __launch_bounds__(GR_T)
-getrs_rows(int n, int64_t nrhs, const int32_t *__restrict__ ipiv, double *b, int64_t ldb) {
+getrs_rows(int n, int64_t nrhs, const int32_t *ipiv, double *b, int64_t ldb) {
   sm100::grid_dependency_wait();
   extern __shared__ __align__(16) unsigned char gr_raw[];
   double *x = reinterpret_cast<double *>(gr_raw);

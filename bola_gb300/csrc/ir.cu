@@ -46,7 +46,7 @@ constexpr int MAXRHS = 32;  // right-hand sides per refinement sweep
 // colblock_finish then turns it in place into the block's scale 2^-e with
 // max|a| in [2^(e-1), 2^e).  A NaN is passed over.
 __global__ void __launch_bounds__(256)
-colblock_max(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *mbits) {
+colblock_max(int64_t n, const double *A, int64_t lda, unsigned long long *mbits) {
   sm100::grid_dependency_wait();
   __shared__ uint64_t red[8];
   const int64_t c0 = (int64_t)blockIdx.x * TB, c1 = imin(n, c0 + TB);
@@ -117,7 +117,7 @@ __device__ __forceinline__ T scaled_pow2(double v, int k1, double p1, int k2, do
 constexpr int CVT_COLS = 8;
 template <typename T>
 __global__ void __launch_bounds__(256)
-convert_scaled(int64_t n, const double *__restrict__ A, int64_t lda, const double *scale, T *__restrict__ W,
+convert_scaled(int64_t n, const double *A, int64_t lda, const double *scale, T *__restrict__ W,
                int64_t ldw) {
   sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
@@ -143,7 +143,7 @@ struct FactorEnd {
 // a cheap lower bound on the conditioning the refinement will face.  Compared
 // as bits; a NaN is passed over.
 template <typename T>
-__device__ void diag_extent(int64_t n, const T *__restrict__ W, int64_t ldw, FactorEnd *out) {
+__device__ void diag_extent(int64_t n, const T *W, int64_t ldw, FactorEnd *out) {
   __shared__ uint64_t mx[32], mn[32];
   constexpr uint64_t INF = 0x7ff0000000000000ull;
   uint64_t a = 0, b = INF;
@@ -231,7 +231,7 @@ col_absmax(int64_t n, Columns first, Columns second, const int32_t *flag, double
 // y[i, c] = fl32(pre[p] r[p, c] / rscale[c]), p = perm[i] (pre: the row
 // scale of a Cholesky's D A D, or none)
 template <typename T>
-__global__ void permute_scale_down(int64_t n, int nrhs, const double *__restrict__ r, int64_t ldr,
+__global__ void permute_scale_down(int64_t n, int nrhs, const double *r, int64_t ldr,
                                    const int32_t *perm, const double *rscale, T *__restrict__ y, const double *pre,
                                    int32_t *tickets) {
   sm100::grid_dependency_wait();
@@ -249,7 +249,7 @@ __global__ void permute_scale_down(int64_t n, int nrhs, const double *__restrict
 // the column scale of the LU's 64-column block, or the row scale postrow[i]
 // of a Cholesky
 template <typename T>
-__global__ void update_x(int64_t n, int nrhs, const T *__restrict__ y, const double *scale, const double *rscale,
+__global__ void update_x(int64_t n, int nrhs, const T *y, const double *scale, const double *rscale,
                          double *__restrict__ x, int64_t ldx, int assign, const double *postrow) {
   sm100::grid_dependency_wait();
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,7 +271,7 @@ __global__ void copy_cols(int64_t n, int nrhs, const double *__restrict__ src, i
 // Symmetric scaling of an SPD matrix: d_i = 2^-k with a_ii 2^-2k in
 // [0.5, 2), exact, so D A D has an O(1) diagonal.  A diagonal entry that is
 // not positive and finite gets d_i = 1 (the Cholesky then stops at it).
-__global__ void sym_scale(int64_t n, const double *__restrict__ A, int64_t lda, double *d) {
+__global__ void sym_scale(int64_t n, const double *A, int64_t lda, double *d) {
   sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -288,7 +288,7 @@ __global__ void sym_scale(int64_t n, const double *__restrict__ A, int64_t lda, 
 // W = fl(D A D), lower triangle only (the Cholesky reads no other part).
 template <typename T>
 __global__ void __launch_bounds__(256)
-convert_sym_lower(int64_t n, const double *__restrict__ A, int64_t lda, const double *d, T *__restrict__ W,
+convert_sym_lower(int64_t n, const double *A, int64_t lda, const double *d, T *__restrict__ W,
                   int64_t ldw) {
   sm100::grid_dependency_wait();
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x, j0 = (int64_t)blockIdx.y * CVT_COLS;
@@ -330,7 +330,7 @@ __device__ __forceinline__ double quotient(double t, double, const Divisor &q) {
 
 template <typename T>
 __global__ void __launch_bounds__(DI_THREADS)
-diag_block_inverses(int64_t n, const T *__restrict__ W, int64_t ldw, T *Dl, T *Du, FactorEnd *end, const uint64_t *track,
+diag_block_inverses(int64_t n, const T *W, int64_t ldw, T *Dl, T *Du, FactorEnd *end, const uint64_t *track,
                     const int32_t *info, const int32_t *err) {
   sm100::grid_dependency_wait();
   if ((int64_t)blockIdx.x * TB >= n) {  // (the last CTA, beside the others)
@@ -454,8 +454,8 @@ __device__ __forceinline__ void st_word(unsigned long long *p, unsigned long lon
 // before b in solve order (d = blockIdx.y + 1): L[b, b - d] (lower),
 // U[b, b + d] (upper).  C holds C_d for all blocks at C + ((d-1) nb + b) 4096.
 __global__ void __launch_bounds__(256)
-couple_blocks(int64_t n, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dl,
-              const float *__restrict__ Du, float *Cl, float *Cu) {
+couple_blocks(int64_t n, const float *W, int64_t ldw, const float *Dl,
+              const float *Du, float *Cl, float *Cu) {
   sm100::grid_dependency_wait();
   __shared__ float D[TB][TB + 1], T[TB][TB + 1];
   const int nb = (int)cdiv(n, TB);
@@ -640,8 +640,8 @@ static_assert(trsv_words_smem<8>() + 128 <= 227 * 1024, "trsv_words<RH = 8> shar
 
 template <bool LOWER, int RH>
 __global__ void __launch_bounds__(256)
-trsv_words(int64_t n, int nrhs, const float *__restrict__ W, int64_t ldw, const float *__restrict__ Dinv,
-           const float *__restrict__ C, const float *__restrict__ y, float *out, unsigned long long *xw,
+trsv_words(int64_t n, int nrhs, const float *W, int64_t ldw, const float *Dinv,
+           const float *C, const float *y, float *out, unsigned long long *xw,
            int32_t *ticket, uint32_t epoch, int32_t *err) {
   sm100::grid_dependency_wait();
   extern __shared__ __align__(128) float tsm[];
@@ -843,8 +843,8 @@ constexpr int T64_PARTS = 4;
 // again only waits for CTAs that started before it.
 template <bool LOWER>
 __global__ void __launch_bounds__(T64_PARTS * TB)
-trsv_dataflow64(int64_t n, int nrhs, const double *__restrict__ W, int64_t ldw, const double *__restrict__ Dinv,
-                const double *__restrict__ y, double *out, int32_t *flags, int32_t *ticket, int32_t epoch,
+trsv_dataflow64(int64_t n, int nrhs, const double *W, int64_t ldw, const double *Dinv,
+                const double *y, double *out, int32_t *flags, int32_t *ticket, int32_t epoch,
                 int32_t *err) {
   sm100::grid_dependency_wait();
   constexpr int PER = TB / T64_PARTS;  // columns of a block per thread

@@ -99,7 +99,7 @@ __device__ __forceinline__ int32_t exponent_of(uint64_t mag_bits) {
 // 55 and 275.
 constexpr int SCH = 128;
 __global__ void __launch_bounds__(256)
-oz_row_stats(int64_t n, const double *__restrict__ A, int64_t lda, unsigned long long *rmax, double *psum) {
+oz_row_stats(int64_t n, const double *A, int64_t lda, unsigned long long *rmax, double *psum) {
   sm100::grid_dependency_wait();
   __shared__ double red[128];
   __shared__ unsigned long long mred[128];
@@ -153,7 +153,7 @@ __global__ void oz_row_finish(int64_t n, int nblk, const unsigned long long *rma
 // of which the bytes take 210; with the digits peeled off one after the other
 // and converted one by one, 400.
 __global__ void __launch_bounds__(256)
-oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int32_t *__restrict__ e, int64_t mrows,
+oz_split_matrix(int64_t n, const double *A, int64_t lda, const int32_t *e, int64_t mrows,
                 int64_t kp, __nv_bfloat16 *__restrict__ out) {
   sm100::grid_dependency_wait();
   __shared__ double T[64][65];
@@ -194,7 +194,7 @@ oz_split_matrix(int64_t n, const double *__restrict__ A, int64_t lda, const int3
 // (u * 16 + c) of a row-major array (pitch kp); columns c >= nr are zero.
 // One CTA per column: its max, then its digits.
 __global__ void __launch_bounds__(1024)
-oz_split_rhs(int64_t n, int nr, const double *__restrict__ x, int64_t ldx, int64_t kp, __nv_bfloat16 *__restrict__ out,
+oz_split_rhs(int64_t n, int nr, const double *x, int64_t ldx, int64_t kp, __nv_bfloat16 *__restrict__ out,
              int32_t *f, unsigned long long *acc) {
   sm100::grid_dependency_wait();
   __shared__ unsigned long long red[32];

@@ -113,8 +113,8 @@ __device__ __forceinline__ int small_int(float v) { return __float_as_int(v + 12
 
 __global__ void __launch_bounds__(ZTHREADS, 1)
 oz_update_pipe(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int64_t capA,
-               int64_t capB, int64_t boff, int64_t m, int64_t n, const int32_t *__restrict__ eA,
-               const int32_t *__restrict__ eB, double *__restrict__ W, int64_t ldw, int tpc, int32_t *err,
+               int64_t capB, int64_t boff, int64_t m, int64_t n, const int32_t *eA,
+               const int32_t *eB, double *__restrict__ W, int64_t ldw, int tpc, int32_t *err,
                const int32_t *abort, int lower) {
   sm100::grid_dependency_wait();
   if (abandoned(abort)) return;

@@ -46,7 +46,7 @@ __global__ void syrk_beta(bool upper, int64_t n, double beta, double *C, int64_t
 constexpr int SYRK_WARPS = NB / 2 + 1;
 template <int SLOTS>
 __global__ void __launch_bounds__(NB *SLOTS)
-syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const double *__restrict__ A,
+syrk_diag(bool upper, bool trans_t, int64_t n, int64_t k, double alpha, const double *A,
           int64_t lda, double *C, int64_t ldc, int lanes, const int32_t *info) {
   sm100::grid_dependency_wait();
   __shared__ double sA[NB][NB + 1];      // 'N': sA[l][r] = A(j0 + r, p0 + l); 'T': sA[r][l] = A(p0 + l, j0 + r)

@@ -30,12 +30,31 @@ __global__ void scale_matrix(int64_t m, int64_t n, double alpha, double *B, int6
   B[i + j * ldb] = __dmul_rn(B[i + j * ldb], alpha);
 }
 
+// store(e, load(e)) for e < count, a thread's loads eight at a time in flight
+// (the compiler keeps a load behind the store to shared memory before it).
+template <typename L, typename S>
+__device__ __forceinline__ void copy_in(int count, L &&load, S &&store) {
+  constexpr int U = 8;
+  for (int e0 = threadIdx.x; e0 < count; e0 += U * blockDim.x) {
+    double v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * blockDim.x;
+      v[u] = e < count ? load(e) : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int e = e0 + u * blockDim.x;
+      if (e < count) store(e, v[u]);
+    }
+  }
+}
+
 // Loads the m x m triangle block (column-major, ld = STOP) into shared memory.
 __device__ __forceinline__ void load_tri(double *sA, const double *A, int64_t lda, int m) {
-  for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-    const int i = e % m, k = e / m;
-    sA[i + k * STOP] = A[i + (int64_t)k * lda];
-  }
+  copy_in(
+      m * m, [&](int e) { return A[e % m + (int64_t)(e / m) * lda]; },
+      [&](int e, double v) { sA[e % m + (e / m) * STOP] = v; });
 }
 
 // Left side, op(A) = A: trsm_lnl / trsm_lnu base cases (src/trsm.rs:96-123, 136-163).
@@ -45,7 +64,7 @@ __device__ __forceinline__ void load_tri(double *sA, const double *A, int64_t ld
 constexpr int LN_WARPS = 4;
 template <bool LOWER>
 __global__ void __launch_bounds__(32 * LN_WARPS)
-left_n_base(int m, int64_t n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
+left_n_base(int m, int64_t n, bool unit, const double *A, int64_t lda, double *B,
             int64_t ldb, int lanes, const int32_t *info) {
   sm100::grid_dependency_wait();
   __shared__ double sA[STOP * STOP];
@@ -121,17 +140,19 @@ constexpr int TW_WARPS = 4;
 constexpr int TW_PITCH = STOP + 1;
 template <bool ASC, bool RIGHT>
 __global__ void __launch_bounds__(32 * TW_WARPS)
-tri_warp(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
+tri_warp(int n, int64_t systems, bool unit, bool transposed, const double *A, int64_t lda, double *B,
          int64_t elem, int64_t sys, const int32_t *info) {
   sm100::grid_dependency_wait();
   __shared__ double T[STOP * TW_PITCH];
   __shared__ Divisor dv[STOP];
   __shared__ __align__(16) double pbuf[TW_WARPS][2][STOP];
   if (stop_flag(info)) return;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int r = e % n, c = e / n;  // a(r, c): (k, j), or (j, k) when transposed
-    T[transposed ? c * TW_PITCH + r : r * TW_PITCH + c] = A[r + (int64_t)c * lda];
-  }
+  copy_in(
+      n * n, [&](int e) { return A[e % n + (int64_t)(e / n) * lda]; },
+      [&](int e, double v) {
+        const int r = e % n, c = e / n;  // a(r, c): (k, j), or (j, k) when transposed
+        T[transposed ? c * TW_PITCH + r : r * TW_PITCH + c] = v;
+      });
   __syncthreads();
   if (!unit) {
     if (threadIdx.x < n) dv[threadIdx.x] = divisor(T[threadIdx.x * (TW_PITCH + 1)]);
@@ -218,7 +239,7 @@ constexpr int TCOLS = 32;  // right-hand sides per block in the transposed base 
 
 template <bool LOWER>
 __global__ void __launch_bounds__(TCOLS)
-left_t_base(int m, int64_t n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
+left_t_base(int m, int64_t n, bool unit, const double *A, int64_t lda, double *B,
             int64_t ldb, const int32_t *info) {
   sm100::grid_dependency_wait();
   __shared__ double sA[STOP * STOP];
@@ -264,7 +285,7 @@ inline size_t right_base_smem(int n) { return ((size_t)n * n + n + (size_t)RB_RO
 
 template <int V>
 __global__ void __launch_bounds__(RB_ROWS)
-right_base(int64_t m, int n, bool unit, const double *__restrict__ A, int64_t lda, double *B,
+right_base(int64_t m, int n, bool unit, const double *A, int64_t lda, double *B,
            int64_t ldb, const int32_t *info) {
   sm100::grid_dependency_wait();
   extern __shared__ double rb_smem[];
@@ -318,16 +339,15 @@ constexpr int AS_SYS = AS_THREADS / AL;
 
 template <bool RIGHT>
 __global__ void __launch_bounds__(AS_THREADS)
-tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *__restrict__ A, int64_t lda, double *B,
+tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *A, int64_t lda, double *B,
           int64_t elem, int64_t sys, const int32_t *info) {
   sm100::grid_dependency_wait();
   __shared__ double T[32 * 33];  // coefficient of x_k in equation j at T[k * 33 + j]
   __shared__ Divisor dv[32];
   if (stop_flag(info)) return;
-  for (int e = threadIdx.x; e < n * n; e += AS_THREADS) {
-    const int r = e % n, c = e / n;
-    T[transposed ? c * 33 + r : r * 33 + c] = A[r + (int64_t)c * lda];
-  }
+  copy_in(
+      n * n, [&](int e) { return A[e % n + (int64_t)(e / n) * lda]; },
+      [&](int e, double v) { T[transposed ? e / n * 33 + e % n : e % n * 33 + e / n] = v; });
   __syncthreads();
   if (!unit && threadIdx.x < n) dv[threadIdx.x] = divisor(T[threadIdx.x * 34]);
   __syncthreads();

@@ -3,7 +3,12 @@ and then.
 
 Named barriers: bar.sync and bar.arrive count a warp at its first arrival, so a
 warp that may have diverged is made whole (__syncwarp) in the statement before
-one."""
+one.
+
+Programmatic dependents: a kernel that waits for the one before it
+(griddepcontrol.wait) has started before that one's results are final, so its
+operands are not const __restrict__, which declares them constant during the
+whole kernel and allows loads that need not see another kernel's stores."""
 import glob
 import os
 import re
@@ -27,3 +32,36 @@ def test_warps_are_whole_at_named_barriers(path):
     for m in re.finditer(r'asm volatile\("bar\.(sync|arrive)', text):
         before = text[:m.start()].rstrip()
         assert before.endswith("__syncwarp();"), text[max(0, m.start() - 200):m.end() + 40]
+
+
+def closing(text, at, opening, shutting):
+    """Index of the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] == opening) - (text[i] == shutting)
+        if depth == 0:
+            return i
+    raise ValueError(text[at:at + 80])
+
+
+def kernels(text):
+    """(name, parameters, body) of every kernel defined in `text`."""
+    for m in re.finditer("__global__", text):
+        at = m.end()
+        while True:  # past __launch_bounds__(...) and the like, to the name's parenthesis
+            start = text.index("(", at)
+            name = re.search(r"(\w+)\s*$", text[at:start]).group(1)
+            end = closing(text, start, "(", ")")
+            if not name.startswith("__"):
+                break
+            at = end + 1
+        if text[end + 1:].lstrip().startswith("{"):
+            body = text.index("{", end)
+            yield name, text[start:end], text[body:closing(text, body, "{", "}")]
+
+
+@pytest.mark.parametrize("path", UNITS, ids=os.path.basename)
+def test_programmatic_dependents_take_plain_pointers(path):
+    for name, parameters, body in kernels(source(path)):
+        if re.search(r"grid_dependency_wait|griddepcontrol\.wait|\bInParallel\b", body):
+            assert not re.search(r"const\s+[\w:]+(\s+\w+)?\s*\*\s*__restrict__", parameters), name
