@@ -46,10 +46,10 @@ int num_sms() {
 
 namespace {
 
-// Unique id of the calling thread's current context (0 if none or unknown).
+// The calling thread's current context and its unique id (0 if none or unknown).
 // The driver functions are reached through the runtime's entry-point query,
 // so the library does not link the driver library directly.
-unsigned long long current_context_id() {
+unsigned long long current_context(CUcontext *out) {
   using GetCurrentFn = CUresult (*)(CUcontext *);
   using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
   static GetCurrentFn get_current = nullptr;
@@ -71,17 +71,20 @@ unsigned long long current_context_id() {
   if (get_current == nullptr || get_id == nullptr || get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr ||
       get_id(ctx, &id) != CUDA_SUCCESS)
     return 0;
+  *out = ctx;
   return id;
 }
 
 constexpr int kMaxDevices = 64;
+constexpr int kMaxPools = 8;  // per device: contexts that are served from a pool of their own
 constexpr uint64_t kScratchKept = uint64_t(64) << 20;
 std::mutex g_pool_mu;
 struct PoolSlot {
-  unsigned long long ctx_id = 0;  // the context the pool belongs to: a device reset ends it
+  CUcontext ctx = nullptr;  // the context that the pool belongs to, which ends it (a device reset among others)
+  unsigned long long id = 0;  // and which one at that address
   cudaMemPool_t pool = nullptr;
 };
-PoolSlot g_pool_slot[kMaxDevices];
+PoolSlot g_pool_slot[kMaxDevices][kMaxPools];
 
 }  // namespace
 
@@ -100,11 +103,19 @@ int roomy(const void *kern) {
 cudaMemPool_t scratch_pool() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return nullptr;
-  const unsigned long long id = current_context_id();
+  CUcontext ctx = nullptr;
+  const unsigned long long id = current_context(&ctx);
   if (id == 0) return nullptr;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  PoolSlot &slot = g_pool_slot[dev];
-  if (slot.pool != nullptr && slot.ctx_id == id) return slot.pool;
+  // this context's slot, or a free one, or that of a context that was at this address before
+  PoolSlot *slot = nullptr;
+  for (PoolSlot &s : g_pool_slot[dev]) {
+    if (s.pool != nullptr && s.ctx != ctx) continue;
+    if (s.pool != nullptr && s.id == id) return s.pool;
+    slot = &s;
+    break;
+  }
+  if (slot == nullptr) return nullptr;  // (the default pool serves further contexts)
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -113,11 +124,13 @@ cudaMemPool_t scratch_pool() {
   uint64_t keep = kScratchKept;
   if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
       cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+    if (pool != nullptr) cudaMemPoolDestroy(pool);
     cudaGetLastError();
     return nullptr;
   }
-  slot.pool = pool;
-  slot.ctx_id = id;
+  slot->ctx = ctx;
+  slot->id = id;
+  slot->pool = pool;
   return pool;
 }
 

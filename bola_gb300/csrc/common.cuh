@@ -39,10 +39,11 @@ __host__ __device__ inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 
 __host__ __device__ inline int64_t imin(int64_t a, int64_t b) { return a < b ? a : b; }
 __host__ __device__ inline int64_t imax(int64_t a, int64_t b) { return a > b ? a : b; }
 
-// The library's own stream-ordered memory pool of the current device: keeps
+// The library's own stream-ordered memory pool of the current context: keeps
 // up to 64 MiB of freed memory across synchronisations (the default pool gives
 // everything back at each one, and mapping it again costs ~100 us a call).
-// nullptr when it cannot be created.
+// One for each of a device's first eight contexts; nullptr beyond that or when
+// it cannot be created (the default pool then serves).
 cudaMemPool_t scratch_pool();
 
 // Stream-ordered temporary device memory.
