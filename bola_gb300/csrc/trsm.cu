@@ -461,7 +461,10 @@ int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64
     }
   }
   const size_t smem = right_base_smem((int)n);
-  if (smem > 48 * 1024) BOLA_TRY_CUDA(cudaFuncSetAttribute(right_base<V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // (always the largest order's, so that no thread lowers what another is about to launch with)
+  if (smem > 48 * 1024)
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(right_base<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)right_base_smem(STOP)));
   BOLA_TRY(roomy(right_base<V>));
   BOLA_TRY_CUDA(launch_after(right_base<V>, dim3((unsigned)cdiv(m, RB_ROWS)), RB_ROWS, smem, c.s, m, (int)n, c.unit,
                              A, lda, B, ldb, c.info));
