@@ -75,13 +75,35 @@ unsigned long long current_context(CUcontext *out) {
   return id;
 }
 
+// Whether ctx, which is current, is its device's primary context.
+bool is_primary(CUcontext ctx, int dev) {
+  using RetainFn = CUresult (*)(CUcontext *, CUdevice);
+  using ReleaseFn = CUresult (*)(CUdevice);
+  using StateFn = CUresult (*)(CUdevice, unsigned *, int *);
+  void *state = nullptr, *retain = nullptr, *release = nullptr;
+  cudaDriverEntryPointQueryResult q;
+  if (cudaGetDriverEntryPointByVersion("cuDevicePrimaryCtxGetState", &state, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      cudaGetDriverEntryPointByVersion("cuDevicePrimaryCtxRetain", &retain, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+      cudaGetDriverEntryPointByVersion("cuDevicePrimaryCtxRelease", &release, 12000, cudaEnableDefault, &q) != cudaSuccess)
+    return true;  // (then nothing of its is given back)
+  unsigned flags = 0;
+  int active = 0;
+  CUcontext primary = nullptr;
+  if (reinterpret_cast<StateFn>(state)(dev, &flags, &active) != CUDA_SUCCESS) return true;
+  if (!active) return false;
+  if (reinterpret_cast<RetainFn>(retain)(&primary, dev) != CUDA_SUCCESS) return true;
+  reinterpret_cast<ReleaseFn>(release)(dev);
+  return primary == ctx;
+}
+
 constexpr int kMaxDevices = 64;
 constexpr int kMaxPools = 8;  // per device: contexts that are served from a pool of their own
 constexpr uint64_t kScratchKept = uint64_t(64) << 20;
 std::mutex g_pool_mu;
 struct PoolSlot {
-  CUcontext ctx = nullptr;  // the context that the pool belongs to, which ends it (a device reset among others)
+  CUcontext ctx = nullptr;    // the context that the pool serves
   unsigned long long id = 0;  // and which one at that address
+  bool primary = false;       // the device's primary context: a reset of the device ends the pool with it
   cudaMemPool_t pool = nullptr;
 };
 PoolSlot g_pool_slot[kMaxDevices][kMaxPools];
@@ -107,7 +129,8 @@ cudaMemPool_t scratch_pool() {
   const unsigned long long id = current_context(&ctx);
   if (id == 0) return nullptr;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  // this context's slot, or a free one, or that of a context that was at this address before
+  // this context's slot, or a free one, or that of a context that was at this
+  // address before (whose pool outlives it, and goes back here)
   PoolSlot *slot = nullptr;
   for (PoolSlot &s : g_pool_slot[dev]) {
     if (s.pool != nullptr && s.ctx != ctx) continue;
@@ -116,6 +139,8 @@ cudaMemPool_t scratch_pool() {
     break;
   }
   if (slot == nullptr) return nullptr;  // (the default pool serves further contexts)
+  if (slot->pool != nullptr && !slot->primary) cudaMemPoolDestroy(slot->pool);
+  slot->pool = nullptr;
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
   props.location.type = cudaMemLocationTypeDevice;
@@ -130,6 +155,7 @@ cudaMemPool_t scratch_pool() {
   }
   slot->ctx = ctx;
   slot->id = id;
+  slot->primary = is_primary(ctx, dev);
   slot->pool = pool;
   return pool;
 }

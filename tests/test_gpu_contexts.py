@@ -78,6 +78,33 @@ def test_scratch_stays_bounded_under_two_contexts():
     """)
 
 
+def test_scratch_of_ended_contexts_is_given_back():
+    """The same product in contexts that are destroyed after it, 24 one after the other: no more is kept than for the
+    eight contexts that have a pool of their own."""
+    child("""
+    m, k = 64, 65536
+    a = np.random.default_rng(2).uniform(-1, 1, (k, m))
+    want = a.T @ a
+    free = []
+    f, t = ctypes.c_size_t(), ctypes.c_size_t()
+    for turn in range(24):
+        c = ctypes.c_void_p()
+        ok(cu.cuCtxCreate_v2(ctypes.byref(c), 0, 0))
+        pa, pc = device(a), device(np.zeros((m, m)))
+        st = L.bola_dgemm(b"N", b"T", m, m, k, 1.0, pa, m, pa, m, 0.0, pc, m, None)
+        assert st == 0, (turn, st, L.bola_last_error())
+        ok(cu.cuCtxSynchronize())
+        assert np.abs(host(pc, (m, m)).T - want).max() < 1e-9
+        for p in (pa, pc):
+            ok(cu.cuMemFree_v2(p))
+        ok(cu.cuCtxDestroy_v2(c))
+        ok(cu.cuCtxSetCurrent(ctxs[0]))
+        ok(cu.cuMemGetInfo_v2(ctypes.byref(f), ctypes.byref(t)))
+        free.append(f.value)
+    assert free[0] - free[-1] <= 320 << 20, [(free[0] - v) >> 20 for v in free]
+    """)
+
+
 @pytest.mark.parametrize("kind", [0, 1, 2, 3])
 @pytest.mark.parametrize("spd", [False, True])
 def test_mixed_solve_in_each_context(kind, spd):
