@@ -953,15 +953,10 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const float *W, int64_
   cfg.numAttrs = 2;
 #define BOLA_TRSV(LW, RH)                                                                                    \
   do {                                                                                                       \
-    static bool attr_set = false;                                                                            \
-    if (!attr_set) {                                                                                         \
-      BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                                         (int)trsv_words_smem<RH>()));                                       \
-      if (TCL > 8)                                                                                           \
-        BOLA_TRY_CUDA(                                                                                       \
-            cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));    \
-      attr_set = true;                                                                                       \
-    }                                                                                                        \
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
+                                       (int)trsv_words_smem<RH>()));                                         \
+    if (TCL > 8)                                                                                             \
+      BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)); \
     cfg.dynamicSmemBytes = trsv_words_smem<RH>();                                                            \
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, trsv_words<LW, RH>, n, nrhs, W, ldw, Dinv, C, y, out, sync.xw,    \
                                      ticket, epoch, sync.err));                                              \

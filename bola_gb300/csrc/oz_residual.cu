@@ -481,11 +481,7 @@ int OzMatrix::split(cudaStream_t s, const double *A, int64_t lda, double *rowsum
 int OzMatrix::product(cudaStream_t s, int nr, const double *x, int64_t ldx, const double *b, int64_t ldb, double *out,
                       int64_t ldo, int32_t *err) {
   if (!ready) return fail(BOLA_ERR_CUDA, "oz product: matrix not split");
-  static bool attr = false;
-  if (!attr) {
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZR_SMEM));
-    attr = true;
-  }
+  BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZR_SMEM));
   const int mt = (int)cdiv(n, RM);
   const int nchunks = (int)cdiv(n, KCH);
   const int split = (int)imax(1, imin(nchunks, num_sms() / mt));

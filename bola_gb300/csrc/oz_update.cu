@@ -326,11 +326,7 @@ int oz_update(cudaStream_t s, int64_t m, int64_t n, const CUtensorMap &A, const 
               int64_t capB, const int32_t *eA, const int32_t *eB, double *W, int64_t ldw, int32_t *err, int64_t boff,
               const int32_t *abort, bool lower, bool pdl) {
   if (m <= 0 || n <= 0) return 0;
-  static bool attr = false;
-  if (!attr) {
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_update_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, ZSMEM));
-    attr = true;
-  }
+  BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_update_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, ZSMEM));
   const int64_t tiles = cdiv(m, OBM) * cdiv(n, OBN);
   // runs of up to 8 tiles per CTA, but never fewer CTAs than twice the SMs
   // (a narrow update, on the critical path, keeps one tile per CTA)

@@ -32,6 +32,7 @@ namespace {
 
 constexpr int SNB = 64;   // panel width and update depth
 constexpr int SMAXC = 16;
+constexpr int64_t MAX_N = 8192;  // the largest order (its callers refuse more)
 // a panel's moves of rows for the swap kernels: count, rows[128], src[128] (+ spare)
 constexpr int PLAN_STRIDE = 1 + 4 * SNB;
 
@@ -391,13 +392,9 @@ int launch_ppanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t
   const int64_t R = cdiv(cdiv(mp, C), 4) * 4;
   if (R > PP_MAXR || R < jb)
     return fail(BOLA_ERR_UNSUPPORTED, "mixed LU: panel of %lld x %d not supported", (long long)mp, jb);
-  static bool attr = false;
-  if (!attr) {
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)ppanel_smem(PP_MAXR)));
-    attr = true;
-  }
+  BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)ppanel_smem(PP_MAXR)));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)C, 1, 1);
   cfg.blockDim = dim3((unsigned)imax(64, cdiv(R, 32) * 32), 1, 1);
@@ -1059,11 +1056,7 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
       {
         ProfScope prof(lu.sp, "panel_lu64", (double)jb * jb * jb * 2.0 / 3.0 + (double)(mp - jb) * jb * jb,
                        16.0 * (double)mp * jb);
-        static bool attr = false;
-        if (!attr) {
-          BOLA_TRY_CUDA(cudaFuncSetAttribute(panel_lu64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL_SMEM));
-          attr = true;
-        }
+        BOLA_TRY_CUDA(cudaFuncSetAttribute(panel_lu64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL_SMEM));
         const unsigned nA = mp > PL_SLOTS ? (unsigned)cdiv(mp - PL_SLOTS, PL_SLOTS) : 0u;
         StepLaunch L(dim3(nA + 1), dim3(PL_THREADS), PL_SMEM, lu.sp, true);
         BOLA_TRY_CUDA(cudaLaunchKernelEx(&L.cfg, panel_lu64, Wp, ldw, mp, jb, (int32_t)j, (const int32_t *)win,
@@ -1128,12 +1121,9 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
   // the interchanges on the columns left of each panel, all at once
   if (n > SNB) {
     ProfScope prof(lu.sp, "left_swaps");
+    constexpr size_t most = (sizeof(int32_t) + sizeof(T)) * (size_t)(MAX_N - SNB) + 15;
     const size_t smem = ((sizeof(int32_t) * (size_t)(n - SNB) + 15) & ~(size_t)15) + sizeof(T) * (size_t)(n - SNB);
-    static size_t attr = 0;
-    if (smem > attr) {
-      BOLA_TRY_CUDA(cudaFuncSetAttribute(apply_left_swaps<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      attr = smem;
-    }
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(apply_left_swaps<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     apply_left_swaps<T><<<(unsigned)(cdiv(n, SNB) - 1), 512, smem, lu.sp>>>(W, ldw, n, lu.plan, abort);
     BOLA_CHECK_LAUNCH();
   }

@@ -487,12 +487,8 @@ int tc_update(cudaStream_t s, int kind, int64_t m, int64_t n, const CUtensorMap 
 #define BOLA_TCP(KIND, NPASS)                                                                                   \
   do {                                                                                                          \
     using Cfg = PCfg<KIND, NPASS>;                                                                              \
-    static bool attr = false;                                                                                   \
-    if (!attr) {                                                                                                \
-      BOLA_TRY_CUDA(                                                                                            \
-          cudaFuncSetAttribute(tc_update_pipe<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM)); \
-      attr = true;                                                                                              \
-    }                                                                                                           \
+    BOLA_TRY_CUDA(                                                                                              \
+        cudaFuncSetAttribute(tc_update_pipe<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM)); \
     StepLaunch L(dim3(grid), dim3(PTHREADS), Cfg::SMEM, s, pdl);                                                \
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&L.cfg, tc_update_pipe<KIND, NPASS>, A, B, Alo, Blo, mapW, mapWs, m, n, boff,  \
                                      tpc, err, abort, lower ? 1 : 0, W, ldw));                                  \
@@ -508,12 +504,8 @@ int tc_update(cudaStream_t s, int kind, int64_t m, int64_t n, const CUtensorMap 
 #define BOLA_TC(KIND, NPASS)                                                                              \
   do {                                                                                                    \
     using Cfg = TcCfg<KIND, NPASS>;                                                                       \
-    static bool attr = false;                                                                             \
-    if (!attr) {                                                                                          \
-      BOLA_TRY_CUDA(cudaFuncSetAttribute(tc_update_kernel<KIND, NPASS>,                                   \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_LAUNCH)); \
-      attr = true;                                                                                        \
-    }                                                                                                     \
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(tc_update_kernel<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                       Cfg::SMEM_LAUNCH));                                                \
     tc_update_kernel<KIND, NPASS><<<grid, 128, Cfg::SMEM_LAUNCH, s>>>(A, B, Alo, Blo, m, n, boff, W, ldw, err, abort, lower ? 1 : 0); \
   } while (0)
   if (kind == 0) BOLA_TC(0, 1);

@@ -8,7 +8,12 @@ one.
 Programmatic dependents: a kernel that waits for the one before it
 (griddepcontrol.wait) has started before that one's results are final, so its
 operands are not const __restrict__, which declares them constant during the
-whole kernel and allows loads that need not see another kernel's stores."""
+whole kernel and allows loads that need not see another kernel's stores.
+
+Function attributes: they belong to a device and are shared by its threads, so a
+launch asks for what it needs each time (nothing remembers in a static that it
+has been asked for once) and always for the same shared memory (a size of the
+call's own would lower another thread's limit)."""
 import glob
 import os
 import re
@@ -65,3 +70,14 @@ def test_programmatic_dependents_take_plain_pointers(path):
     for name, parameters, body in kernels(source(path)):
         if re.search(r"grid_dependency_wait|griddepcontrol\.wait|\bInParallel\b", body):
             assert not re.search(r"const\s+[\w:]+(\s+\w+)?\s*\*\s*__restrict__", parameters), name
+
+
+@pytest.mark.parametrize("path", UNITS, ids=os.path.basename)
+def test_function_attributes_are_asked_for_at_each_launch(path):
+    text = source(path)
+    assert not re.search(r"static (bool|size_t|int) \w*attr\w*", text)
+    if os.path.basename(path) == "calibrate.cu":  # (probes, which have the device to themselves)
+        return
+    for m in re.finditer(r"cudaFuncAttributeMaxDynamicSharedMemorySize,", text):
+        size = text[m.end():text.index(";", m.end())]
+        assert not re.search(r"\bsmem\b", size), size
