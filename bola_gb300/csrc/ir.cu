@@ -828,6 +828,10 @@ trsv_words(int64_t n, int nrhs, const float *W, int64_t ldw, const float *Dinv,
 }
 
 constexpr int T64_PARTS = 4;
+// A wait gives up after T64_POLLS polls, T64_SLEEP ns apart at least: long after
+// the chain it waits on, which other work on the GPU may hold up.
+constexpr int T64_POLLS = 7 << 20, T64_SLEEP = 20;
+static_assert((int64_t)T64_POLLS * T64_SLEEP >= ((int64_t)64 << 21), "0.13 s of sleeps at least");
 
 // The FP64 form of the same dataflow, for the FP64-storage factor.  GB300's
 // FP64 pipe retires about two FMAs per clock per SM, so one CTA per block
@@ -873,11 +877,11 @@ trsv_dataflow64(int64_t n, int nrhs, const double *W, int64_t ldw, const double 
     if (tid == 0) {
       int polls = 0;
       while (ld_acquire(flags + (int64_t)k * MAXRHS + c) != epoch) {
-        if (++polls > (1 << 21)) {
+        if (++polls > T64_POLLS) {
           atomicExch(err, 3);
           break;
         }
-        __nanosleep(20);
+        __nanosleep(T64_SLEEP);
       }
     }
     __syncthreads();
