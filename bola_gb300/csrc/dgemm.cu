@@ -459,7 +459,10 @@ __global__ void __launch_bounds__(Tile<32>::NT, 5) gemm_partial(const __grid_con
       });
 }
 
-constexpr int FOLD_T = 128;
+// The fold is a chain of one multiply-add (~65 cycles) per chunk and element; the
+// next FOLD_U chunks' sums are on their way meanwhile (one at a time, a load each:
+// 700 cycles a chunk; 64 x 64 x 100,000: 535 us of 1210).
+constexpr int FOLD_T = 128, FOLD_U = 16;
 __global__ void __launch_bounds__(FOLD_T) gemm_fold(const __grid_constant__ GemmArgs g) {
   if (stop_flag(g.info)) return;
   const int64_t e = (int64_t)blockIdx.x * FOLD_T + threadIdx.x, plane = g.m8 * g.n4;
@@ -472,8 +475,22 @@ __global__ void __launch_bounds__(FOLD_T) gemm_fold(const __grid_constant__ Gemm
     if (g.beta != 1.0) c = __dmul_rn(c, g.beta);
   }
   const int64_t nchunks = (g.K + g.kc - 1) / g.kc;
-#pragma unroll 8
-  for (int64_t ch = 0; ch < nchunks; ++ch) c = fused(g.alpha, g.P[ch * plane + e], c);
+  const double *p = g.P + e;
+  double next[FOLD_U];
+  auto fetch = [&](int64_t ch0) {
+#pragma unroll
+    for (int u = 0; u < FOLD_U; ++u) next[u] = ch0 + u < nchunks ? p[(ch0 + u) * plane] : 0.0;
+  };
+  fetch(0);
+  for (int64_t ch0 = 0; ch0 < nchunks; ch0 += FOLD_U) {
+    double v[FOLD_U];
+#pragma unroll
+    for (int u = 0; u < FOLD_U; ++u) v[u] = next[u];
+    fetch(ch0 + FOLD_U);
+#pragma unroll
+    for (int u = 0; u < FOLD_U; ++u)
+      if (ch0 + u < nchunks) c = fused(g.alpha, v[u], c);
+  }
   g.C[i + j * g.ldc] = c;
 }
 
@@ -566,8 +583,10 @@ __global__ void __launch_bounds__(Tile<BT>::NT) gemm_split(const __grid_constant
 //  - CLUSTER: K over clusters of 2, 4 or 8 CTAs, where that shortens the most
 //    loaded SM's time (a fold costs ~70 cycles a chunk and two barriers);
 //  - MEMORY: K in pieces of `cps` chunks over memory, where many chunks allow
-//    a finer balance than 8 CTAs (two more passes over the partial sums and a
-//    launch), up to SPLIT_BYTES of them.
+//    a finer balance than 8 CTAs (two more passes over the partial sums, a
+//    launch and the fold's chain), up to SPLIT_BYTES of them; beyond what the
+//    pool keeps, mapping them again takes 1.6 us per MiB (512 x 512 x 8192, 256
+//    MiB: 3.62 ms, 4.02 when each call is waited for; 3.93 over clusters).
 // The last four are compared by the cycles they are estimated to take.
 enum Path { GRID64, GRID32, GRID8, CLUSTER, MEMORY };
 struct TilePlan {
@@ -577,7 +596,8 @@ struct TilePlan {
   int rounds = 0;            // GRID32: 32x32 blocks side by side on an SM
   int64_t cells = 0;
 };
-constexpr int64_t SPLIT_BYTES = (int64_t)64 << 20;
+constexpr int64_t SPLIT_BYTES = (int64_t)1 << 30;
+constexpr int64_t KEPT_BYTES = (int64_t)64 << 20;  // what the scratch pool keeps between calls
 constexpr int64_t SM_SMEM = 224 * 1024;  // shared memory of an SM that CTAs can take
 
 // Cells of `t` x `t` that C's main region has: full ones, all, and all that a triangle keeps.
@@ -660,7 +680,7 @@ TilePlan plan_tiles(const GemmArgs &args, int sms, bool may_alloc) {
     if (may_alloc && nch >= 16 && bytes <= SPLIT_BYTES)
       for (int cps = 1; cps <= 4; ++cps) {
         const double cost = per_k(32, cdiv(c.all * cdiv(nch, cps), sms)) * (double)(cps * g.kc) + 10000.0 +
-                            (double)bytes / 1500.0;
+                            (double)bytes / (bytes > KEPT_BYTES ? 255.0 : 1500.0) + 70.0 * (double)nch;
         if (cost < best) {
           best = cost;
           p.path = MEMORY;

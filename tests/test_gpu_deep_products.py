@@ -1,0 +1,48 @@
+"""DGEMM with small outputs and a deep K, where K is split over the GPU: bit for
+bit the oracle's, with and without memory for the partial sums, at the numbers
+of 64-deep chunks where a split's parts, passes and the fold's batches end, and
+with partial sums beyond what the scratch pool keeps."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def both(m, n, k, beta, seed, names, oracle_lib, ta="N", tb="N"):
+    from bola_gb300 import _lib
+    L = _lib.load()
+    rng = np.random.default_rng(seed)
+    a = np.asfortranarray(rng.uniform(-1.0, 1.0, (m, k) if ta == "N" else (k, m)))
+    b = np.asfortranarray(rng.uniform(-1.0, 1.0, (k, n) if tb == "N" else (n, k)))
+    c = np.asfortranarray(rng.uniform(-1.0, 1.0, (m, n)))
+    want = c.copy(order="F")
+    oracle_lib.gemm(ta, tb, m, n, k, -0.75, a, a.shape[0], b, b.shape[0], beta, want, m)
+    ga, gb, gc = (torch.from_numpy(x.ravel(order="F")).cuda() for x in (a, b, c))
+    for name in names:
+        t = gc.clone()
+        st = getattr(L, name)(ta.encode(), tb.encode(), m, n, k, -0.75, ctypes.c_void_p(ga.data_ptr()), a.shape[0],
+                              ctypes.c_void_p(gb.data_ptr()), b.shape[0], beta, ctypes.c_void_p(t.data_ptr()), m,
+                              ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == 0, L.bola_last_error()
+        assert np.array_equal(t.cpu().numpy().reshape(m, n, order="F"), want), (name, m, n, k)
+
+
+@pytest.mark.parametrize("m,n", [(8, 4), (13, 9), (16, 16), (40, 28), (64, 64), (100, 33), (128, 128)])
+@pytest.mark.parametrize("chunks", [9, 15, 16, 17, 32, 33, 64, 65, 127, 129, 300])
+def test_chunks_of_a_split(oracle_lib, m, n, chunks):
+    for k in (64 * chunks - 1, 64 * chunks, 64 * chunks - 55):
+        both(m, n, k, 0.5, m + k, ("bola_dgemm", "bola_dgemm_noalloc"), oracle_lib)
+
+
+@pytest.mark.parametrize("ta,tb", [("N", "T"), ("T", "N"), ("T", "T")])
+@pytest.mark.parametrize("m,n,k", [(21, 18, 2501), (64, 64, 5000), (70, 65, 4097)])
+def test_transposed_operands(oracle_lib, ta, tb, m, n, k):
+    both(m, n, k, 1.0, k, ("bola_dgemm", "bola_dgemm_noalloc"), oracle_lib, ta, tb)
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 64, 140_000), (128, 128, 34_000), (16, 16, 300_000)])
+def test_very_deep(oracle_lib, m, n, k):
+    both(m, n, k, 1.0, k, ("bola_dgemm",), oracle_lib)
