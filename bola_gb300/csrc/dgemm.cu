@@ -92,7 +92,9 @@ __device__ __forceinline__ void copy_async8(double *dst, const double *src, bool
 // STG stages filled by asynchronous copies, three stages (>= 6000 cycles of
 // products) ahead: loads staged through registers, one 16-deep stage ahead,
 // left a CTA that was alone on its SM waiting for memory a quarter of its time.
-template <int BM, int BN, int TM, int TN, int NT, bool TA, bool TB, typename F>
+// Run by the CTA's NT threads, or (TEAM) by one of its teams of NT threads, each
+// with a ring of its own.
+template <int BM, int BN, int TM, int TN, int NT, bool TA, bool TB, bool TEAM = false, typename F>
 __device__ __forceinline__ void tile_chunks(const GemmArgs &g, int64_t i0, int64_t j0, int64_t ch0, int64_t ch1,
                                             unsigned char *smem, F &&chunk_done) {
   constexpr int TX = BM / TM, TY = BN / TN;
@@ -100,7 +102,15 @@ __device__ __forceinline__ void tile_chunks(const GemmArgs &g, int64_t i0, int64
   static_assert(TX * TY == NT, "threads");
   double(*As)[KT][BM + 1] = reinterpret_cast<double(*)[KT][BM + 1]>(smem);
   double(*Bs)[KT][BN + 1] = reinterpret_cast<double(*)[KT][BN + 1]>(smem + sizeof(double) * STG * KT * (BM + 1));
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  const int tid = TEAM ? threadIdx.x % NT : threadIdx.x, tx = tid % TX, ty = tid / TX;
+  auto sync = [] {
+    if constexpr (TEAM) {
+      __syncwarp();
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / NT), "n"(NT) : "memory");
+    } else {
+      __syncthreads();
+    }
+  };
   const int64_t kbeg = ch0 * g.kc, kend = imin(ch1 * g.kc, g.K);
   const int nst = (int)((kend - kbeg + KT - 1) / KT);
   // this thread's elements of a stage: where they are now, and whether their row or column exists
@@ -153,7 +163,7 @@ __device__ __forceinline__ void tile_chunks(const GemmArgs &g, int64_t i0, int64
         for (int q = 0; q < TN; ++q) acc[r][q] = 0.0;
     }
     asm volatile("cp.async.wait_group %0;" ::"n"(STG - 2) : "memory");
-    __syncthreads();  // stage s is there for every thread, and stage s - 1 is used up
+    sync();  // stage s is there for every thread, and stage s - 1 is used up
     fetch(s + STG - 1);
     const int buf = s % STG;
 #pragma unroll
@@ -175,7 +185,7 @@ __device__ __forceinline__ void tile_chunks(const GemmArgs &g, int64_t i0, int64
     }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();  // the ring may be filled again
+  sync();  // the ring may be filled again
 }
 
 // One B x B tile of C over all of K, on NT threads.
@@ -497,15 +507,23 @@ __global__ void __launch_bounds__(FOLD_T) gemm_fold(const __grid_constant__ Gemm
 // K split over the CTAs of a cluster: each leaves its chunks' accumulators in
 // its shared memory, and every CTA then folds its share of the tile's elements
 // over all chunks in order, reading the others' through distributed shared
-// memory (g.cps chunks per CTA at a time).  No CTA may leave the cluster's
+// memory.  A CTA has TEAMS teams of a tile's threads, each with chunks of its own
+// (g.cps at a time): four for 8x8 tiles where K has more chunks than the cluster
+// CTAs, since a team by itself leaves the FP64 pipe waiting for its own chain
+// (without memory, 16 x 16 x 32,768: 112 us with teams, 242 without; 64 x 64 x
+// 16,384: 153 and 226).  Teams of 16x16 tiles want clusters of eight for as many
+// CTAs, and those share SMs: 280 us for the latter.  No CTA may leave the cluster's
 // barriers early, so *info is looked at when C is written.
-template <int BT, bool TA, bool TB>
-__global__ void __launch_bounds__(Tile<BT>::NT) gemm_split(const __grid_constant__ GemmArgs g) {
+constexpr int SPLIT_TEAMS = 4;
+template <int BT, int TEAMS, bool TA, bool TB>
+__global__ void __launch_bounds__(Tile<BT>::NT *TEAMS) gemm_split(const __grid_constant__ GemmArgs g) {
   constexpr int TM = Tile<BT>::TM, TN = Tile<BT>::TN, TX = Tile<BT>::TX, TY = Tile<BT>::TY, NT = Tile<BT>::NT;
-  constexpr int TILE = BT * BT;
-  __shared__ __align__(16) unsigned char smem[stage_bytes<BT, BT>()];
+  constexpr int TILE = BT * BT, RING = (int)stage_bytes<BT, BT>(), T = NT * TEAMS;
+  static_assert(RING % 16 == 0, "the teams' rings");
+  __shared__ __align__(16) unsigned char smem[RING * TEAMS];
   extern __shared__ __align__(16) unsigned char part_raw[];
-  double *part = reinterpret_cast<double *>(part_raw);  // [cps][TILE], element (i, j) at i + BT j
+  double *part = reinterpret_cast<double *>(part_raw);  // [TEAMS][cps][TILE], element (i, j) at i + BT j
+  const int team = threadIdx.x / NT, tid = threadIdx.x % NT;
   cg::cluster_group cluster = cg::this_cluster();
   const int ns = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   InParallel ip(g);
@@ -514,41 +532,44 @@ __global__ void __launch_bounds__(Tile<BT>::NT) gemm_split(const __grid_constant
   const int64_t i0 = BT * (int64_t)ci, j0 = BT * (int64_t)cj;
   const int64_t nchunks = (g.K + g.kc - 1) / g.kc;
   // this thread's elements of the fold
-  constexpr int EP = TILE / 2 > NT ? TILE / 2 / NT : 1;  // clusters of 2 and more
-  const int share = TILE / ns;
+  constexpr int EP = TILE / 2 > T ? TILE / 2 / T : 1;  // clusters of 2 and more
+  const int share = (TILE + ns - 1) / ns;
   double c[EP];
   int el[EP];
   double *cp[EP];
 #pragma unroll
   for (int h = 0; h < EP; ++h) {
-    const int f = (int)threadIdx.x + NT * h;
+    const int f = (int)threadIdx.x + T * h;
     el[h] = rank * share + f;
     const int64_t gi = i0 + el[h] % BT, gj = j0 + el[h] / BT;
-    cp[h] = f < share && gi < g.m8 && gj < g.n4 && tri_keep(g.tri, gi, gj) ? g.C + gi + gj * g.ldc : nullptr;
+    cp[h] = f < share && el[h] < TILE && gi < g.m8 && gj < g.n4 && tri_keep(g.tri, gi, gj) ? g.C + gi + gj * g.ldc : nullptr;
     c[h] = 0.0;
     if (cp[h] != nullptr && g.beta != 0.0) {
       c[h] = *cp[h];
       if (g.beta != 1.0) c[h] = __dmul_rn(c[h], g.beta);
     }
   }
-  for (int64_t base = 0; base < nchunks; base += (int64_t)ns * g.cps) {
-    const int64_t ch0 = imin(nchunks, base + (int64_t)rank * g.cps), ch1 = imin(nchunks, ch0 + g.cps);
-    tile_chunks<BT, BT, TM, TN, NT, TA, TB>(g, i0, j0, ch0, ch1, smem, [&](int64_t ch, double(&acc)[TM][TN]) {
-      double *p = part + (ch - ch0) * TILE + threadIdx.x % TX + BT * (threadIdx.x / TX);
+  const int per = TEAMS * g.cps;  // chunks of a CTA at a time
+  for (int64_t base = 0; base < nchunks; base += (int64_t)ns * per) {
+    const int64_t first = base + (int64_t)rank * per;
+    const int64_t ch0 = imin(nchunks, first + (int64_t)team * g.cps), ch1 = imin(nchunks, ch0 + g.cps);
+    tile_chunks<BT, BT, TM, TN, NT, TA, TB, (TEAMS > 1)>(
+        g, i0, j0, ch0, ch1, smem + RING * team, [&](int64_t ch, double(&acc)[TM][TN]) {
+          double *p = part + (ch - first) * TILE + tid % TX + BT * (tid / TX);
 #pragma unroll
-      for (int r = 0; r < TM; ++r)
+          for (int r = 0; r < TM; ++r)
 #pragma unroll
-        for (int q = 0; q < TN; ++q) p[TX * r + BT * TY * q] = acc[r][q];
-    });
+            for (int q = 0; q < TN; ++q) p[TX * r + BT * TY * q] = acc[r][q];
+        });
     cluster.sync();
-    const int64_t end = imin(nchunks, base + (int64_t)ns * g.cps);
+    const int64_t end = imin(nchunks, base + (int64_t)ns * per);
 #pragma unroll
     for (int h = 0; h < EP; ++h) {
       if (cp[h] == nullptr) continue;
       int64_t ch = base;
       for (int r = 0; r < ns && ch < end; ++r) {
         const double *p = cluster.map_shared_rank(part, r) + el[h];
-        const int cnt = (int)imin(g.cps, end - ch);
+        const int cnt = (int)imin(per, end - ch);
         for (int s0 = 0; s0 < cnt; s0 += 8) {
           double v[8];
 #pragma unroll
@@ -580,8 +601,9 @@ __global__ void __launch_bounds__(Tile<BT>::NT) gemm_split(const __grid_constant
 //    CTA's ~2 us of launch and first loads from a depth of 128 on);
 //  - GRID32, below 2 x SMs cells: 32x32 blocks in full rounds, the rest 16x16;
 //  - GRID8: 8x8 blocks;
-//  - CLUSTER: K over clusters of 2, 4 or 8 CTAs, where that shortens the most
-//    loaded SM's time (a fold costs ~70 cycles a chunk and two barriers);
+//  - CLUSTER: K over clusters of 2, 4 or 8 CTAs (6 with teams), where that
+//    shortens the most loaded SM's time (a fold costs ~70 cycles a chunk and two
+//    barriers), by one team of threads or four in each;
 //  - MEMORY: K in pieces of `cps` chunks over memory, where many chunks allow
 //    a finer balance than 8 CTAs (two more passes over the partial sums, a
 //    launch and the fold's chain), up to SPLIT_BYTES of them; beyond what the
@@ -592,7 +614,7 @@ enum Path { GRID64, GRID32, GRID8, CLUSTER, MEMORY };
 struct TilePlan {
   GemmArgs g;
   Path path = GRID32;
-  int split = 1, tile = 32;  // CLUSTER: CTAs and tile
+  int split = 1, tile = 32, teams = 1;  // CLUSTER: CTAs, tile, teams in a CTA
   int rounds = 0;            // GRID32: 32x32 blocks side by side on an SM
   int64_t cells = 0;
 };
@@ -673,7 +695,30 @@ TilePlan plan_tiles(const GemmArgs &args, int sms, bool may_alloc) {
           p.path = s == 1 ? GRID8 : CLUSTER;
           p.split = s;
           p.tile = t;
+          p.teams = 1;
         }
+      }
+      // The same by teams: 37 to 44 cycles per step of k and team; clusters of s
+      // leave about 4 s SMs over, until there are enough for several rounds.
+      double by_teams = 1e300;
+      int s_teams = 0;
+      for (int s = 2; s <= 8 && t == 8 && nch > 8; s += 2) {
+        const int64_t fit = imax(1, sms - 4 * s);
+        const int64_t ctas = cdiv(T * s, T * s <= 2 * fit ? fit : sms);
+        const double cost = SPLIT_TEAMS * (double)ctas * (ctas == 1 ? 44.0 : 37.0) *
+                                (double)imin(g.K, cdiv(nch, s * SPLIT_TEAMS) * g.kc) +
+                            3000.0 + 70.0 * (double)nch;
+        if (cost < by_teams) {
+          by_teams = cost;
+          s_teams = s;
+        }
+      }
+      if (by_teams < 0.95 * best) {
+        best = by_teams;
+        p.path = CLUSTER;
+        p.split = s_teams;
+        p.tile = t;
+        p.teams = SPLIT_TEAMS;
       }
     }
     const int64_t bytes = 8 * nch * g.m8 * g.n4;
@@ -690,7 +735,8 @@ TilePlan plan_tiles(const GemmArgs &args, int sms, bool may_alloc) {
   }
   if (p.path == CLUSTER || p.path == GRID8) {
     c = count_cells(g.m8, g.n4, p.tile, g.tri, false);
-    g.cps = (int)imin(cdiv(nch, p.split), 8192 / (p.tile * p.tile));  // at most 64 KB
+    // at most 64 KB of partial sums a CTA, 32 of one with teams (which takes up to four an SM)
+    g.cps = (int)imin(cdiv(nch, p.split * p.teams), (p.teams > 1 ? 4096 : 8192) / (p.tile * p.tile * p.teams));
   }
   p.cells = c.all;
   g.fm = c.fm;
@@ -755,14 +801,15 @@ int launch_plan(cudaStream_t s, TilePlan &p) {
     return g.n16 > 0 ? launch(gemm_grid32<16, TA, TB>, g.n16, Tile<16>::NT, 0, pad) : 0;
   }
   if (p.path == CLUSTER) {
-    void (*kern)(const GemmArgs) = p.tile == 32   ? gemm_split<32, TA, TB>
-                                   : p.tile == 16 ? gemm_split<16, TA, TB>
-                                                  : gemm_split<8, TA, TB>;
-    const size_t smem = (size_t)g.cps * p.tile * p.tile * sizeof(double);
+    void (*kern)(const GemmArgs) = p.tile == 32   ? gemm_split<32, 1, TA, TB>
+                                   : p.tile == 16 ? gemm_split<16, 1, TA, TB>
+                                   : p.teams == 1 ? gemm_split<8, 1, TA, TB>
+                                                  : gemm_split<8, SPLIT_TEAMS, TA, TB>;
+    const size_t smem = (size_t)g.cps * p.teams * p.tile * p.tile * sizeof(double);
     if (smem + stage_bytes<32, 32>() > 48 * 1024)
       BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
-    return launch(kern, p.cells * p.split, p.tile == 32 ? Tile<32>::NT : p.tile == 16 ? Tile<16>::NT : Tile<8>::NT,
-                  p.split, smem);
+    return launch(kern, p.cells * p.split,
+                  p.teams * (p.tile == 32 ? Tile<32>::NT : p.tile == 16 ? Tile<16>::NT : Tile<8>::NT), p.split, smem);
   }
   const int64_t nch = (g.K + g.kc - 1) / g.kc;
   Scratch part;
