@@ -9,9 +9,9 @@
 //                         across lanes);
 //   left, transpose, and right — a system is a right-hand side or a row of B:
 //                         a warp per system (tri_warp) while there are few;
-//                         the ascending ones of order <= 32 eight lanes per
-//                         system (tri_asc32); a thread per system for the
-//                         rest (left_t_base, right_base).
+//                         some hundreds to thousands of ascending ones of
+//                         order <= 32 eight lanes per system (tri_asc32); a
+//                         thread per system beyond (left_t_base, right_base).
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -345,9 +345,10 @@ tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *A, i
   __shared__ double T[32 * 33];  // coefficient of x_k in equation j at T[k * 33 + j]
   __shared__ Divisor dv[32];
   if (stop_flag(info)) return;
-  copy_in(
-      n * n, [&](int e) { return A[e % n + (int64_t)(e / n) * lda]; },
-      [&](int e, double v) { T[transposed ? e / n * 33 + e % n : e % n * 33 + e / n] = v; });
+  for (int e = threadIdx.x; e < n * n; e += AS_THREADS) {
+    const int r = e % n, c = e / n;
+    T[transposed ? c * 33 + r : r * 33 + c] = A[r + (int64_t)c * lda];
+  }
   __syncthreads();
   if (!unit && threadIdx.x < n) dv[threadIdx.x] = divisor(T[threadIdx.x * 34]);
   __syncthreads();
@@ -382,11 +383,31 @@ tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *A, i
     if (q + AL * c < n) b[(q + AL * c) * elem] = x[c];
 }
 
-// Up to how many systems a warp each (tri_warp) beats a thread each: the warps
-// of one SM share its FP64 pipe (n = 64: ~27 cycles of the GPU per ascending
-// system, ~210 per descending one, against 280k cycles for any number of
-// threads; tri_asc32 takes ~24k cycles for any number up to its grid's size).
-constexpr int64_t ASC_WARP_MAX = 8192, SEQ_WARP_MAX = 1216, ASC32_WARP_MAX = 912;
+// Which kernel takes a base case of order n, by what each costs.  A thread per
+// system takes its own chain's time (n = 64: ~280k cycles) for any number up to
+// the threads that fit and the fewest instructions per system; a warp per system
+// the shortest chain and the most; tri_asc32 lies between.  Measured crossings
+// (us for n = 8, 16, 32, 64 and a number of systems; 'L' 'U' 'T' 'N' unless said):
+//  - descending: a warp to 1064 systems (64 x 1000: 200 against 214), 608 for
+//    n <= 8 (8 x 1000: 10.7 against 9.8);
+//  - ascending, n > 32: a warp to 100 n systems where each unknown takes a
+//    quotient, 155 n where it takes a product or nothing (64 x 4000: 140 against
+//    207, 64 x 8000: 263 against 207; 'R' 144 to 193 against 250);
+//  - ascending, n <= 32: a warp to 912 systems; then, for n > 8, tri_asc32 to
+//    400 (n - 2) systems (16 x 4000: 18 against 21, 16 x 32,000: 91 against 43), with
+//    a unit diagonal on the left to 700 (n - 6), and always for n > 28 (32 x
+//    100,000: 245 against 315); then a thread (8 x 100,000: 47 against 147).
+enum class Base { WARP, ASC32, THREAD };
+Base descending_base(int64_t n, int64_t systems) {
+  return systems <= (n <= 8 ? 608 : 1064) ? Base::WARP : Base::THREAD;
+}
+Base ascending_base(int64_t n, int64_t systems, bool right, bool unit) {
+  if (n > 32) return systems <= (right || unit ? 155 : 100) * n ? Base::WARP : Base::THREAD;
+  if (systems <= 912) return Base::WARP;
+  if (n <= 8) return Base::THREAD;
+  if (unit && !right) return n > 28 || systems <= 700 * (n - 6) ? Base::ASC32 : Base::THREAD;
+  return systems <= 400 * (n - 2) ? Base::ASC32 : Base::THREAD;
+}
 
 struct Ctx {
   cudaStream_t s;
@@ -413,14 +434,15 @@ int base_left_n(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
 int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A, int64_t lda, double *B,
                 int64_t ldb) {
   ProfScope prof(c.s, "trsm_base", (double)m * m * n);
-  if (!lower && m <= 32 && n > ASC32_WARP_MAX) {
+  const Base base = lower ? descending_base(m, n) : ascending_base(m, n, false, c.unit);
+  if (base == Base::ASC32) {
     BOLA_TRY(roomy(tri_asc32<false>));
     BOLA_TRY_CUDA(launch_after(tri_asc32<false>, dim3((unsigned)cdiv(n, AS_SYS)), AS_THREADS, 0, c.s, (int)m, n,
                                c.unit, false, A, lda, B, 1, ldb, c.info));
     BOLA_CHECK_LAUNCH();
     return 0;
   }
-  if (n <= (lower ? SEQ_WARP_MAX : ASC_WARP_MAX)) {
+  if (base == Base::WARP) {
     const unsigned gw = (unsigned)cdiv(n, TW_WARPS);
     BOLA_TRY(roomy(lower ? tri_warp<false, false> : tri_warp<true, false>));
     if (lower)
@@ -444,7 +466,8 @@ int base_left_t(const Ctx &c, bool lower, int64_t m, int64_t n, const double *A,
 template <int V>
 int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64_t lda, double *B, int64_t ldb) {
   constexpr bool asc = V == 1 || V == 2;
-  if (m <= (!asc ? SEQ_WARP_MAX : n <= 32 ? ASC32_WARP_MAX : ASC_WARP_MAX)) {
+  const Base base = asc ? ascending_base(n, m, true, c.unit) : descending_base(n, m);
+  if (base == Base::WARP) {
     BOLA_TRY(roomy(tri_warp<asc, true>));
     BOLA_TRY_CUDA(launch_after(tri_warp<asc, true>, dim3((unsigned)cdiv(m, TW_WARPS)), 32 * TW_WARPS, 0, c.s, (int)n,
                                m, c.unit, V >= 2, A, lda, B, ldb, 1, c.info));
@@ -452,7 +475,7 @@ int launch_right_base(const Ctx &c, int64_t m, int64_t n, const double *A, int64
     return 0;
   }
   if constexpr (asc) {
-    if (n <= 32) {
+    if (base == Base::ASC32) {
       BOLA_TRY(roomy(tri_asc32<true>));
       BOLA_TRY_CUDA(launch_after(tri_asc32<true>, dim3((unsigned)cdiv(m, AS_SYS)), AS_THREADS, 0, c.s, (int)n, m,
                                  c.unit, V >= 2, A, lda, B, ldb, 1, c.info));
