@@ -31,23 +31,21 @@ __global__ void scale_matrix(int64_t m, int64_t n, double alpha, double *B, int6
 }
 
 // store(e, load(e)) for e < count, a thread's loads eight at a time in flight
-// (the compiler keeps a load behind the store to shared memory before it).
+// while it has that many (the compiler keeps a load behind the store to shared
+// memory before it).
 template <typename L, typename S>
 __device__ __forceinline__ void copy_in(int count, L &&load, S &&store) {
   constexpr int U = 8;
-  for (int e0 = threadIdx.x; e0 < count; e0 += U * blockDim.x) {
+  const int step = blockDim.x;
+  int e = threadIdx.x;
+  for (; e + (U - 1) * step < count; e += U * step) {
     double v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      v[u] = e < count ? load(e) : 0.0;
-    }
+    for (int u = 0; u < U; ++u) v[u] = load(e + u * step);
 #pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e < count) store(e, v[u]);
-    }
+    for (int u = 0; u < U; ++u) store(e + u * step, v[u]);
   }
+  for (; e < count; e += step) store(e, load(e));
 }
 
 // Loads the m x m triangle block (column-major, ld = STOP) into shared memory.
@@ -393,10 +391,11 @@ tri_asc32(int n, int64_t systems, bool unit, bool transposed, const double *A, i
 //  - ascending, n > 32: a warp to 100 n systems where each unknown takes a
 //    quotient, 155 n where it takes a product or nothing (64 x 4000: 140 against
 //    207, 64 x 8000: 263 against 207; 'R' 144 to 193 against 250);
-//  - ascending, n <= 32: a warp to 912 systems; then, for n > 8, tri_asc32 to
-//    400 (n - 2) systems (16 x 4000: 18 against 21, 16 x 32,000: 91 against 43), with
-//    a unit diagonal on the left to 700 (n - 6), and always for n > 28 (32 x
-//    100,000: 245 against 315); then a thread (8 x 100,000: 47 against 147).
+//  - ascending, n <= 32: a warp to 912 systems; a thread beyond for n <= 8 (8 x
+//    100,000: 47 against 147); else tri_asc32, whose time grows with the systems
+//    (32 x 8000: 41 to 43, 32 x 32,000: 143 to 147), or a thread each, whose time
+//    grows by whole rounds of 128 on every SM (62 to 69, 120 to 126), by the
+//    estimates below in us, which follow the measured ones within a tenth.
 enum class Base { WARP, ASC32, THREAD };
 Base descending_base(int64_t n, int64_t systems) {
   return systems <= (n <= 8 ? 608 : 1064) ? Base::WARP : Base::THREAD;
@@ -405,8 +404,11 @@ Base ascending_base(int64_t n, int64_t systems, bool right, bool unit) {
   if (n > 32) return systems <= (right || unit ? 155 : 100) * n ? Base::WARP : Base::THREAD;
   if (systems <= 912) return Base::WARP;
   if (n <= 8) return Base::THREAD;
-  if (unit && !right) return n > 28 || systems <= 700 * (n - 6) ? Base::ASC32 : Base::THREAD;
-  return systems <= 400 * (n - 2) ? Base::ASC32 : Base::THREAD;
+  const double rounds = (double)cdiv(systems, 128 * (int64_t)num_sms()), size = (double)n;
+  const bool less = unit && !right;  // neither a quotient nor a product per unknown, no zero tests
+  const double thread = 5.0 + rounds * (less ? 0.047 : 0.056) * size * size;
+  const double asc32 = 6.0 + 0.001 * (double)systems * (less ? 1.05 + 0.044 * size : 1.25 + 0.095 * size);
+  return asc32 < thread ? Base::ASC32 : Base::THREAD;
 }
 
 struct Ctx {

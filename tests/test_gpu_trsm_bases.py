@@ -7,10 +7,12 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 VARIANTS = [("L", "U", "T"), ("L", "L", "T"), ("R", "U", "N"), ("R", "L", "T"), ("R", "L", "N"), ("R", "U", "T")]
-# (order, numbers of systems): 608 | 1064 descending; 912, 400 (n - 2) and 700 (n - 6) ascending; 100 n and 155 n above 32
-SIZES = [(1, (3, 1000)), (5, (607, 608, 609, 913)), (8, (608, 609, 912, 913, 3001)), (9, (912, 913, 2100, 2101, 2801)),
-         (16, (911, 1064, 1065, 5600, 5601, 7001)), (28, (913, 10401, 15401)), (29, (10800, 10801)), (32, (12000, 12001)),
-         (33, (1065, 3300, 3301, 5115, 5116)), (64, (1064, 1065, 6400, 6401, 9920, 9921))]
+# (order, numbers of systems): 608 | 1064 descending; 912 and estimates ascending, the thread's in rounds of 128 on every
+# SM (19,456); 100 n and 155 n above 32
+SIZES = [(1, (3, 1000)), (5, (607, 608, 609, 913)), (8, (608, 609, 912, 913, 3001)), (9, (912, 913, 2100, 2801)),
+         (16, (911, 1064, 1065, 4000, 5601, 7001)), (28, (913, 8001, 15401)), (31, (11001, 19456, 19457)),
+         (32, (12000, 14001, 19456, 19457, 27001)), (33, (1065, 3300, 3301, 5115, 5116)),
+         (64, (1064, 1065, 6400, 6401, 9920, 9921))]
 
 
 @pytest.mark.parametrize("n,counts", SIZES, ids=[str(n) for n, _ in SIZES])
