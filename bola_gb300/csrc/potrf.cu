@@ -412,7 +412,7 @@ __global__ void __launch_bounds__(P2_T)
 potrf2_block(bool upper, int n, double *A, int64_t lda, int32_t *info, int32_t col0, int lanes) {
   sm100::grid_dependency_wait();
   __shared__ double a[NB * P2P];
-  __shared__ double a0[LDS * LDS];  // the input, for the recursion: a failing block, a short 'U' one
+  __shared__ double a0[LDS * LDS];  // the input, for the recursion: a failing block
   __shared__ double rdg[LDS];
   if (stop_flag(info)) return;
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
@@ -423,8 +423,7 @@ potrf2_block(bool upper, int n, double *A, int64_t lda, int32_t *info, int32_t c
     else a[j * P2P + i] = v;
   }
   __syncthreads();
-  const bool walk = upper && n < NB;
-  int r = walk ? 1 : upper ? p2_upper32(a, lanes) : p2_lower(a, n, lanes);
+  int r = upper ? p2_upper32(a, lanes) : p2_lower(a, n, lanes);  // ('U': n = 32)
   if (r) {  // BOLA's state at a failure is its recursion's: (re)do the block that way
     r = p2_walk(upper, a0, rdg, n, lanes);
     __syncthreads();
@@ -439,6 +438,26 @@ potrf2_block(bool upper, int n, double *A, int64_t lda, int32_t *info, int32_t c
   for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
     const int i = e % n, j = e / n;
     if (upper ? i <= j : i >= j) A[i + (int64_t)j * lda] = upper ? a[i * P2P + j] : a[j * P2P + i];
+  }
+  if (r && threadIdx.x == 0) *info = col0 + r;
+}
+
+// A 'U' block of order below 32: the recursion by itself, on the four warps that
+// it has work for (n = 31, with the copy of a failing block and nine warps: 106 us).
+constexpr int P2_SHORT_T = 128;
+__global__ void __launch_bounds__(P2_SHORT_T)
+potrf2_short_upper(int n, double *A, int64_t lda, int32_t *info, int32_t col0, int lanes) {
+  sm100::grid_dependency_wait();
+  __shared__ double a[LDS * LDS];
+  if (stop_flag(info)) return;
+  for (int e = threadIdx.x; e < n * n; e += P2_SHORT_T) a[e % n + e / n * LDS] = A[e % n + (int64_t)(e / n) * lda];
+  __syncthreads();
+  const int r = p2_walk(true, a, nullptr, n, lanes);
+  __syncthreads();
+  // BOLA stops at the failing column with everything before it written back.
+  for (int e = threadIdx.x; e < n * n; e += P2_SHORT_T) {
+    const int i = e % n, j = e / n;
+    if (i <= j) A[i + (int64_t)j * lda] = a[i + j * LDS];
   }
   if (r && threadIdx.x == 0) *info = col0 + r;
 }
@@ -469,8 +488,13 @@ int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int
   if (n == 0) return 0;
   if (n <= NB) {
     ProfScope prof(s, "potrf2_block", (double)n * n * n / 3.0);
-    BOLA_TRY(roomy(potrf2_block));
-    BOLA_TRY_CUDA(launch_after(potrf2_block, dim3(1), P2_T, 0, s, upper, (int)n, A, lda, info, col0, lanes()));
+    if (upper && n < NB) {
+      BOLA_TRY(roomy(potrf2_short_upper));
+      BOLA_TRY_CUDA(launch_after(potrf2_short_upper, dim3(1), P2_SHORT_T, 0, s, (int)n, A, lda, info, col0, lanes()));
+    } else {
+      BOLA_TRY(roomy(potrf2_block));
+      BOLA_TRY_CUDA(launch_after(potrf2_block, dim3(1), P2_T, 0, s, upper, (int)n, A, lda, info, col0, lanes()));
+    }
     BOLA_CHECK_LAUNCH();
     return 0;
   }
