@@ -160,6 +160,12 @@ def bucket_of(n):
     raise ValueError(n)
 
 
+def group_choices(b):
+    """The group sizes that the library runs as they are for bucket b; a smaller one is widened to the bucket's default
+    (a thread per row at least)."""
+    return tuple(g for g in GROUP_CHOICES if g >= DEFAULT_GROUPS[b])
+
+
 def time_solve(batch, A0, B0, reps, graph=True):
     """Minimum CUDA-event time (ms) of one batched solve over `reps` runs, the
     inputs restored from A0/B0 before each (outside the timed region)."""
@@ -198,7 +204,7 @@ def autotune(batch, reps=3, path=None):
             sub.b_view(j).copy_(batch.b_view(int(i)))
         A0, B0 = sub.A.clone(), sub.B.clone()
         trials[b] = {}
-        for g in GROUP_CHOICES:
+        for g in group_choices(b):
             for pw in PANEL_CHOICES:
                 t = Tuning(best.group_size, best.panel_width, best.tile_rows)
                 t.group_size[b], t.panel_width[b] = g, pw
