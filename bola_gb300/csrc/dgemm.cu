@@ -890,9 +890,10 @@ extern "C" int bola_dgemm(char transa, char transb, int64_t m, int64_t n, int64_
 }
 
 // The allocation-free DGEMM (include/bola_gb300.h): partial sums of a split K
-// stay on chip.  It keeps its documented limit, the scratch that they would
-// take in memory: 64x64 tiles (or the smaller ones with the least tile area on
-// the most loaded SM) fewer than the SMs, K split in 64-deep chunks.
+// stay on chip.  It keeps its documented limit, as callers test for it: outputs
+// of fewer tiles than SMs (64x64, or the smaller ones with the least area on the
+// most loaded SM) whose partial sums, a 64-deep chunk each, would take between
+// 64 MiB and 1 GiB of memory.  (The tiles of the limit are not the plan's.)
 extern "C" int bola_dgemm_noalloc(char transa, char transb, int64_t m, int64_t n, int64_t k, double alpha,
                                   const double *a, int64_t lda, const double *b, int64_t ldb, double beta,
                                   double *c, int64_t ldc, bola_stream_t stream) {
@@ -915,10 +916,10 @@ extern "C" int bola_dgemm_noalloc(char transa, char transb, int64_t m, int64_t n
     const double bytes = 8.0 * (double)nchunks * (double)m8 * (double)n4;
     if (tiles < sms && bytes <= (double)(1u << 30) && bytes > (double)BOLA_NOALLOC_SCRATCH_BYTES)
       return fail(BOLA_ERR_UNSUPPORTED,
-                  "bola_dgemm_noalloc: this shape needs %.0f bytes of split-K scratch, the limit is %llu bytes "
-                  "(%lld chunks x %lld x %lld doubles); use bola_dgemm",
-                  bytes, (unsigned long long)BOLA_NOALLOC_SCRATCH_BYTES, (long long)nchunks, (long long)m8,
-                  (long long)n4);
+                  "bola_dgemm_noalloc: the partial sums of a split K would take %.0f bytes of scratch memory (%lld "
+                  "chunks x %lld x %lld doubles), and this call does not take shapes beyond %llu; use bola_dgemm",
+                  bytes, (long long)nchunks, (long long)m8, (long long)n4,
+                  (unsigned long long)BOLA_NOALLOC_SCRATCH_BYTES);
   }
   return dgemm_body((cudaStream_t)stream, transa, transb, m, n, k, alpha, a, lda, b, ldb, beta, c, ldc, 64, nullptr, 0,
                     false);

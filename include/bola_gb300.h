@@ -151,10 +151,13 @@ int bola_dsyrk(char uplo, char trans, int64_t n, int64_t k, double alpha, const 
  * that must not move).  Same arguments and bit-identical results as
  * bola_dgemm.  Where bola_dgemm may park the partial sums of a split K in
  * temporary device memory, this call keeps them on chip.
- *   - Shapes whose split-K partial sums would need more than 64 MiB in memory
- *     (K/64 chunks x m x n doubles, rounded to BOLA's full 8x4 tiles, for
- *     outputs of fewer 64x64 tiles than the device has SMs) are rejected with
- *     BOLA_ERR_UNSUPPORTED and a message in bola_last_error().
+ *   - A documented limit that callers can rely on, kept from when partial sums
+ *     lay in a fixed array: a shape is rejected with BOLA_ERR_UNSUPPORTED and a
+ *     message in bola_last_error() if its output has fewer tiles than the
+ *     device has SMs (of 64x64, or of 64x32, 32x64, 32x32 or 64x16 where these
+ *     leave less on the most loaded SM) and its partial sums (K/64 chunks x m
+ *     x n doubles, m and n rounded down to BOLA's full 8x4 tiles) would take
+ *     more than 64 MiB and at most 1 GiB.
  *   - Calls keep no state: any number may run at once, on any streams. */
 #define BOLA_NOALLOC_SCRATCH_BYTES (64ull << 20)
 int bola_dgemm_noalloc(char transa, char transb, int64_t m, int64_t n, int64_t k, double alpha,

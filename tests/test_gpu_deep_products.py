@@ -46,3 +46,24 @@ def test_transposed_operands(oracle_lib, ta, tb, m, n, k):
 @pytest.mark.parametrize("m,n,k", [(64, 64, 140_000), (128, 128, 34_000), (16, 16, 300_000)])
 def test_very_deep(oracle_lib, m, n, k):
     both(m, n, k, 1.0, k, ("bola_dgemm",), oracle_lib)
+
+
+def test_the_limit_without_memory():
+    """64 x 64: a chunk's partial sums are 32 KiB, so 2048 chunks (64 MiB) are taken, more are not up to 32,768 (1 GiB),
+    and a refused call leaves C alone."""
+    from bola_gb300 import _lib
+    L = _lib.load()
+    m = n = 64
+    k = 64 * 32768 + 1
+    a = torch.rand(m * k, dtype=torch.float64, device="cuda")
+    c0 = torch.rand(m * n, dtype=torch.float64, device="cuda")
+    for depth, status in [(64 * 2048, 0), (64 * 2048 + 1, -1002), (64 * 32768, -1002), (64 * 32768 + 1, 0)]:
+        c = c0.clone()
+        st = L.bola_dgemm_noalloc(b"N", b"T", m, n, depth, 1.0, ctypes.c_void_p(a.data_ptr()), m,
+                                  ctypes.c_void_p(a.data_ptr()), n, 1.0, ctypes.c_void_p(c.data_ptr()), m,
+                                  ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert st == status, (depth, st)
+        torch.cuda.synchronize()
+        assert torch.equal(c, c0) == (status != 0)
+        if status:
+            assert b"does not take shapes beyond" in L.bola_last_error()
