@@ -470,10 +470,10 @@ int tc_update(cudaStream_t s, int kind, int64_t m, int64_t n, const CUtensorMap 
     // Runs of up to 12 tiles per CTA, never fewer CTAs than twice the SMs (a
     // narrow update, on the critical path, keeps one tile per CTA): the run that
     // takes the fewest tile times in whole rounds of the SMs, a CTA's start and
-    // end counted as 1.7 tiles.  The LU's panel holds 16 SMs meanwhile, the
-    // Cholesky's hardly any.  Against runs of 8: LU n = 8192 16.45 -> 16.25 ms,
-    // Cholesky n = 6000 5.35 -> 5.33.
-    const int64_t sms = num_sms() - (lower ? 0 : 16);
+    // end counted as 1.7 tiles.  The LU's panel holds up to 16 SMs meanwhile (from
+    // 3841 rows on), the Cholesky's hardly any.  Against runs of 8: LU n = 8192
+    // 16.45 -> 16.25 ms, Cholesky n = 6000 5.35 -> 5.33.
+    const int64_t sms = imax(1, num_sms() - (lower ? 0 : 16));  // (a slice of a GPU may have no more)
     int tpc = 1;
     double least = 1e30;
     for (int t = 1; t <= 12 && (t == 1 || tiles / t >= 2 * (int64_t)num_sms()); ++t) {
