@@ -581,9 +581,6 @@ int batch_launch(cudaStream_t s, const bola_system *systems, const int32_t *item
   return 0;
 }
 
-namespace {
-
-}  // namespace
 }  // namespace bola
 
 using namespace bola;

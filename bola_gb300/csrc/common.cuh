@@ -180,15 +180,6 @@ __device__ __forceinline__ double add_prod(double c, double t, double x) {
 __device__ __forceinline__ double sub_prod(double c, double t, double x) {
   return __dsub_rn(c, __dmul_rn(t, x));
 }
-// Split cluster barrier: ARRIVE (release) and WAIT (acquire), so that work
-// between them overlaps the other CTAs' arrival.
-__device__ __forceinline__ void cluster_arrive() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void cluster_wait() {
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // x != 0.0 (NaN included) on the integer pipe.  GB300 retires ~2 FP64
 // operations per clock per SM and a comparison takes a slot like an FMA, so
 // the zero tests inside BOLA's update loops are done on the bits.
@@ -378,13 +369,6 @@ __device__ __forceinline__ Cand cand_none() {
   c.key = INT64_MAX;
   c.idx = 0;
   return c;
-}
-__device__ __forceinline__ Cand shfl_cand(const Cand &c, int src) {
-  Cand o;
-  o.v = __shfl_sync(0xffffffffu, c.v, src);
-  o.key = __shfl_sync(0xffffffffu, c.key, src);
-  o.idx = __shfl_sync(0xffffffffu, c.idx, src);
-  return o;
 }
 __device__ __forceinline__ Cand warp_best(Cand c) {
   for (int off = 16; off > 0; off >>= 1) {

@@ -103,11 +103,9 @@ __device__ __forceinline__ int32_t interchange_step(int j, int x, int jb, int32_
 // From the final state of the interchange steps (no replay of the swaps):
 // position q < jb takes its pivot pivl[q], and each of the first jb rows
 // that is not a pivot goes to the position posin[x] >= jb it was displaced
-// to.  One warp; entries are compacted with ballots.  With rows_s != nullptr
-// the list also goes to shared memory, as panel rows (rows_s, src_s, *cnt_s).
+// to.  One warp; entries are compacted with ballots.
 __device__ __forceinline__ void list_panel_moves(const int32_t *pivl, const int32_t *posin, int jb, int32_t col0,
-                                                 int32_t *plan, int32_t *rows_s = nullptr, int32_t *src_s = nullptr,
-                                                 int *cnt_s = nullptr) {
+                                                 int32_t *plan) {
   const unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   int base = 0;
@@ -119,10 +117,6 @@ __device__ __forceinline__ void list_panel_moves(const int32_t *pivl, const int3
       const int slot = base + __popc(m & ((1u << lane) - 1u));
       plan[1 + slot] = col0 + q;
       plan[1 + 2 * SNB + slot] = col0 + pivl[q];
-      if (rows_s != nullptr) {
-        rows_s[slot] = q;
-        src_s[slot] = pivl[q];
-      }
     }
     base += __popc(m);
   }
@@ -134,17 +128,10 @@ __device__ __forceinline__ void list_panel_moves(const int32_t *pivl, const int3
       const int slot = base + __popc(m & ((1u << lane) - 1u));
       plan[1 + slot] = col0 + posin[x];
       plan[1 + 2 * SNB + slot] = col0 + x;
-      if (rows_s != nullptr) {
-        rows_s[slot] = posin[x];
-        src_s[slot] = x;
-      }
     }
     base += __popc(m);
   }
-  if (lane == 0) {
-    plan[0] = base;
-    if (cnt_s != nullptr) *cnt_s = base;
-  }
+  if (lane == 0) plan[0] = base;
 }
 
 // Dynamic shared memory of the panel: the rows' finished values (column-major,
@@ -447,7 +434,7 @@ __device__ __forceinline__ double recip64(double p) {
 
 // Steps 2 and 3 of the panel above in one launch (Wp: the panel's top-left,
 // rows col0.. of W).  The selection has fixed the pivot order (row win[q]
-// is the pivot of column q, chosen by partial pivoting among the nominees),
+// is the pivot of column q, chosen by partial pivoting on the FP32 copies),
 // so the panel is factored without further pivoting, as CALU's last step
 // does: the selected block and every row below it go through the same 64
 // right-looking steps.  CTA i < nA takes the panel's rows at positions
@@ -492,7 +479,7 @@ panel_lu64(double *Wp, int64_t ldw, int64_t mp, int jb, int32_t col0, const int3
   }
   extern __shared__ __align__(16) double pl_raw[];
   double(*a)[SNB + 1] = reinterpret_cast<double(*)[SNB + 1]>(pl_raw);  // rows 0..63: the block; 64 + i: slot i
-  __shared__ int32_t win[SNB], pivl[SNB], posin[SNB], at_[SNB], rows_s[2 * SNB], src_s[2 * SNB];
+  __shared__ int32_t win[SNB], pivl[SNB], posin[SNB], at_[SNB];
   __shared__ int32_t slot[PL_SLOTS];  // panel position of slot i's row (-1: none)
   __shared__ double rinv_s[2];   // 1 / the pivot of column k (k & 1)
   __shared__ int bad;
@@ -633,7 +620,7 @@ panel_lu64(double *Wp, int64_t ldw, int64_t mp, int jb, int32_t col0, const int3
       ipiv[jdone] = interchange_step(jdone, win[jdone], jb, col0, posin, at_);
     }
   __syncthreads();
-  if (top && warp == 0) list_panel_moves(pivl, posin, jb, col0, plan, rows_s, src_s);
+  if (top && warp == 0) list_panel_moves(pivl, posin, jb, col0, plan);
   // -- this CTA's rows: L21 to their final positions (the last CTA's to
   // where the interchanges put them) and their exact bf16 slices, one
   // exponent per row
@@ -1011,7 +998,7 @@ void MixedLU::destroy() {
 namespace {
 
 // Width of the panel starting at j.
-int panel_width(bool, int64_t n, int64_t j) { return (int)imin(SNB, n - j); }
+int panel_width(int64_t n, int64_t j) { return (int)imin(SNB, n - j); }
 
 }  // namespace
 
@@ -1041,7 +1028,7 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
   int jb = 0;
   bool wide_pending = false;
   for (int64_t j = 0, k = 0; j < n; j += jb, ++k) {
-    jb = panel_width(fp64, n, j);
+    jb = panel_width(n, j);
     const int64_t mp = n - j;
     const bool upd = j + jb < n;
     const int buf = (int)(k & 1);
@@ -1071,7 +1058,7 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
     if (wide_pending) BOLA_TRY_CUDA(cudaStreamWaitEvent(lu.sp, lu.ev_wide, 0));
     wide_pending = false;
     const int64_t m2 = mp - jb, n2 = n - j - jb;
-    const int64_t nb_next = upd ? imin((int64_t)panel_width(fp64, n, j + jb), n2) : 0;
+    const int64_t nb_next = upd ? imin((int64_t)panel_width(n, j + jb), n2) : 0;
     // interchanges, U12 and B operand of the columns [w0, w1) right of the panel
     auto swap = [&](cudaStream_t st, int64_t w0, int64_t w1) -> int {
       ProfScope prof(st, fp64 ? "sswap_trsm64" : "sswap_trsm", (double)jb * jb * (double)(w1 - w0));

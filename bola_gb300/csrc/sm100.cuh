@@ -85,16 +85,6 @@ __device__ __forceinline__ uint32_t cluster_addr(const void *local, int rank) {
 // Asynchronous stores into another CTA's shared memory that complete by
 // adding their byte count to that CTA's mbarrier (st.async): the receiver
 // waits on its own mbarrier instead of a cluster-wide barrier.
-__device__ __forceinline__ void st_async(uint32_t addr, double v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
-               "l"(__double_as_longlong(v)), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void st_async(uint32_t addr, long long v, uint32_t bar) {
-  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr), "l"(v),
-               "r"(bar)
-               : "memory");
-}
 __device__ __forceinline__ void st_async4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d,
                                           uint32_t bar) {
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
