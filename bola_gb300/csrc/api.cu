@@ -5,6 +5,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <set>
 #include <utility>
 
@@ -108,7 +109,95 @@ struct PoolSlot {
 };
 PoolSlot g_pool_slot[kMaxDevices][kMaxPools];
 
+// Memory that graphs use: a block goes to one captured graph at a time and back
+// to this list when CUDA says that the graph is gone (on a thread of its own,
+// where no CUDA call may be made).  Blocks beyond MAX_FREE are given back to the
+// device at the next capture that finds them.
+struct GraphBlock {
+  void *ptr = nullptr;
+  size_t bytes = 0;
+  unsigned long long ctx_id = 0;
+  GraphBlock *next = nullptr;
+};
+constexpr int kMaxFreeBlocks = 16;
+std::mutex g_graph_mu;
+GraphBlock *g_graph_free = nullptr;
+void CUDART_CB graph_gone(void *block) {
+  std::lock_guard<std::mutex> lk(g_graph_mu);
+  static_cast<GraphBlock *>(block)->next = g_graph_free;
+  g_graph_free = static_cast<GraphBlock *>(block);
+}
+// Calls that allocate are allowed on this thread while one of its streams is captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 }  // namespace
+
+int graph_memory(cudaStream_t s, size_t bytes, void **out) {
+  *out = nullptr;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  cudaGraph_t graph = nullptr;
+  BOLA_TRY_CUDA(cudaStreamGetCaptureInfo(s, &status, nullptr, &graph));
+  if (status != cudaStreamCaptureStatusActive) return fail(BOLA_ERR_CUDA, "graph_memory: the stream is not being captured");
+  size_t size = (size_t)64 << 10;
+  while (size < bytes) size *= 2;
+  CUcontext ctx = nullptr;
+  const unsigned long long id = current_context(&ctx);
+  RelaxedCapture relaxed;
+  GraphBlock *block = nullptr, *extra = nullptr;
+  {
+    std::lock_guard<std::mutex> lk(g_graph_mu);
+    int kept = 0;
+    for (GraphBlock **at = &g_graph_free; *at != nullptr;) {
+      GraphBlock *b = *at;
+      const bool take = block == nullptr && b->ctx_id == id && b->bytes == size;
+      if (!take && (b->ctx_id != id || ++kept <= kMaxFreeBlocks)) {
+        at = &b->next;
+        continue;
+      }
+      *at = b->next;
+      if (take) {
+        block = b;
+      } else {
+        b->next = extra;
+        extra = b;
+      }
+    }
+  }
+  while (extra != nullptr) {
+    GraphBlock *b = extra;
+    extra = b->next;
+    cudaFree(b->ptr);
+    delete b;
+  }
+  if (block == nullptr) {
+    block = new (std::nothrow) GraphBlock();
+    if (block == nullptr) return fail(BOLA_ERR_CUDA, "graph_memory: out of host memory");
+    const cudaError_t e = cudaMalloc(&block->ptr, size);
+    if (e != cudaSuccess) {
+      delete block;
+      return cuda_fail(e, "cudaMalloc(graph memory)");
+    }
+    block->bytes = size;
+    block->ctx_id = id;
+  }
+  cudaUserObject_t owner = nullptr;
+  cudaError_t e = cudaUserObjectCreate(&owner, block, graph_gone, 1, cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    graph_gone(block);
+    return cuda_fail(e, "cudaUserObjectCreate");
+  }
+  e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(owner, 1);
+    return cuda_fail(e, "cudaGraphRetainUserObject");
+  }
+  *out = block->ptr;
+  return 0;
+}
 
 int roomy(const void *kern) {
   int dev = 0;

@@ -46,6 +46,12 @@ __host__ __device__ inline int64_t imax(int64_t a, int64_t b) { return a > b ? a
 // it cannot be created (the default pool then serves).
 cudaMemPool_t scratch_pool();
 
+// `bytes` of device memory for the graph that stream s is being captured into: it
+// belongs to the graph and its copies and executables, and comes back to the
+// library when the last of them is destroyed.  Unlike memory nodes it leaves the
+// graph free to be cloned, nested and instantiated several times.
+int graph_memory(cudaStream_t s, size_t bytes, void **out);
+
 // Stream-ordered temporary device memory.
 class Scratch {
  public:
@@ -53,12 +59,17 @@ class Scratch {
   Scratch(const Scratch &) = delete;
   Scratch &operator=(const Scratch &) = delete;
   ~Scratch() { release(); }
-  int alloc(size_t bytes, cudaStream_t s) {
+  // in_graph: no memory nodes while s is captured (graph_memory instead).
+  int alloc(size_t bytes, cudaStream_t s, bool in_graph = false) {
     release();
     stream_ = s;
     if (bytes == 0) return 0;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;  // a captured allocation belongs to its graph
     cudaStreamIsCapturing(s, &cap);
+    if (in_graph && cap == cudaStreamCaptureStatusActive) {
+      borrowed_ = true;
+      return graph_memory(s, bytes, &ptr_);
+    }
     cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool() : nullptr;
     cudaError_t e = pool != nullptr ? cudaMallocFromPoolAsync(&ptr_, bytes, pool, s) : cudaMallocAsync(&ptr_, bytes, s);
     if (e != cudaSuccess) {
@@ -68,8 +79,9 @@ class Scratch {
     return 0;
   }
   void release() {
-    if (ptr_) cudaFreeAsync(ptr_, stream_);
+    if (ptr_ && !borrowed_) cudaFreeAsync(ptr_, stream_);
     ptr_ = nullptr;
+    borrowed_ = false;
   }
   template <class T>
   T *as() const { return static_cast<T *>(ptr_); }
@@ -77,6 +89,7 @@ class Scratch {
  private:
   void *ptr_ = nullptr;
   cudaStream_t stream_ = nullptr;
+  bool borrowed_ = false;  // the memory of a graph
 };
 
 // Asks for all of an SM's shared memory as such for a kernel of the FP64 path

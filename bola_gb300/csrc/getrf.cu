@@ -981,7 +981,7 @@ int getrf_blocked(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, 
     return m == 0 || n == 0 ? 0 : getrf2_rec(s, m, n, A, lda, ipiv, info, 0);
   }
   Scratch plans;
-  BOLA_TRY(plans.alloc((size_t)cdiv(min_mn, PNB) * PLAN_INTS * sizeof(int32_t), s));
+  BOLA_TRY(plans.alloc((size_t)cdiv(min_mn, PNB) * PLAN_INTS * sizeof(int32_t), s, true));
   // look-ahead pays from a few hundred columns on; below that its events and
   // the extra launches cost more than the overlap saves
   LookAhead *la = min_mn >= LOOK_AHEAD_MIN ? la_acquire() : nullptr;
