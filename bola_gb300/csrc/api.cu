@@ -136,6 +136,11 @@ struct RelaxedCapture {
 
 }  // namespace
 
+unsigned long long context_id() {
+  CUcontext ctx = nullptr;
+  return current_context(&ctx);
+}
+
 int graph_memory(cudaStream_t s, size_t bytes, void **out) {
   *out = nullptr;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;

@@ -957,10 +957,15 @@ int trsv(cudaStream_t s, bool lower, int64_t n, int nrhs, const float *W, int64_
   cfg.numAttrs = 2;
 #define BOLA_TRSV(LW, RH)                                                                                    \
   do {                                                                                                       \
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize,      \
-                                       (int)trsv_words_smem<RH>()));                                         \
-    if (TCL > 8)                                                                                             \
-      BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)); \
+    static PerContext asked;                                                                                 \
+    BOLA_TRY(asked([]() -> int {                                                                             \
+      BOLA_TRY_CUDA(cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+                                         (int)trsv_words_smem<RH>()));                                       \
+      if (TCL > 8)                                                                                           \
+        BOLA_TRY_CUDA(                                                                                       \
+            cudaFuncSetAttribute(trsv_words<LW, RH>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));    \
+      return 0;                                                                                              \
+    }));                                                                                                     \
     cfg.dynamicSmemBytes = trsv_words_smem<RH>();                                                            \
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&cfg, trsv_words<LW, RH>, n, nrhs, W, ldw, Dinv, C, y, out, sync.xw,    \
                                      ticket, epoch, sync.err));                                              \

@@ -481,7 +481,11 @@ int OzMatrix::split(cudaStream_t s, const double *A, int64_t lda, double *rowsum
 int OzMatrix::product(cudaStream_t s, int nr, const double *x, int64_t ldx, const double *b, int64_t ldb, double *out,
                       int64_t ldo, int32_t *err) {
   if (!ready) return fail(BOLA_ERR_CUDA, "oz product: matrix not split");
-  BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZR_SMEM));
+  static PerContext asked;
+  BOLA_TRY(asked([]() -> int {
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_product_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, OZR_SMEM));
+    return 0;
+  }));
   const int mt = (int)cdiv(n, RM);
   const int nchunks = (int)cdiv(n, KCH);
   const int split = (int)imax(1, imin(nchunks, num_sms() / mt));

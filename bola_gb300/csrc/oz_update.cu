@@ -326,7 +326,11 @@ int oz_update(cudaStream_t s, int64_t m, int64_t n, const CUtensorMap &A, const 
               int64_t capB, const int32_t *eA, const int32_t *eB, double *W, int64_t ldw, int32_t *err, int64_t boff,
               const int32_t *abort, bool lower, bool pdl) {
   if (m <= 0 || n <= 0) return 0;
-  BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_update_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, ZSMEM));
+  static PerContext asked;
+  BOLA_TRY(asked([]() -> int {
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(oz_update_pipe, cudaFuncAttributeMaxDynamicSharedMemorySize, ZSMEM));
+    return 0;
+  }));
   const int64_t tiles = cdiv(m, OBM) * cdiv(n, OBN);
   // runs of up to 8 tiles per CTA, but never fewer CTAs than twice the SMs
   // (a narrow update, on the critical path, keeps one tile per CTA)

@@ -379,9 +379,13 @@ int launch_ppanel(cudaStream_t s, G *W, int64_t ldw, int64_t mp, int jb, int32_t
   const int64_t R = cdiv(cdiv(mp, C), 4) * 4;
   if (R > PP_MAXR || R < jb)
     return fail(BOLA_ERR_UNSUPPORTED, "mixed LU: panel of %lld x %d not supported", (long long)mp, jb);
-  BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)ppanel_smem(PP_MAXR)));
+  static PerContext asked;
+  BOLA_TRY(asked([]() -> int {
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    BOLA_TRY_CUDA(cudaFuncSetAttribute(ppanel_kernel<G>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)ppanel_smem(PP_MAXR)));
+    return 0;
+  }));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)C, 1, 1);
   cfg.blockDim = dim3((unsigned)imax(64, cdiv(R, 32) * 32), 1, 1);
@@ -1043,7 +1047,11 @@ static int factor_lookahead(MixedLU &lu, cudaStream_t s, T *W, int64_t ldw, int3
       {
         ProfScope prof(lu.sp, "panel_lu64", (double)jb * jb * jb * 2.0 / 3.0 + (double)(mp - jb) * jb * jb,
                        16.0 * (double)mp * jb);
-        BOLA_TRY_CUDA(cudaFuncSetAttribute(panel_lu64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL_SMEM));
+        static PerContext asked;
+        BOLA_TRY(asked([]() -> int {
+          BOLA_TRY_CUDA(cudaFuncSetAttribute(panel_lu64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PL_SMEM));
+          return 0;
+        }));
         const unsigned nA = mp > PL_SLOTS ? (unsigned)cdiv(mp - PL_SLOTS, PL_SLOTS) : 0u;
         StepLaunch L(dim3(nA + 1), dim3(PL_THREADS), PL_SMEM, lu.sp, true);
         BOLA_TRY_CUDA(cudaLaunchKernelEx(&L.cfg, panel_lu64, Wp, ldw, mp, jb, (int32_t)j, (const int32_t *)win,

@@ -487,8 +487,12 @@ int tc_update(cudaStream_t s, int kind, int64_t m, int64_t n, const CUtensorMap 
 #define BOLA_TCP(KIND, NPASS)                                                                                   \
   do {                                                                                                          \
     using Cfg = PCfg<KIND, NPASS>;                                                                              \
-    BOLA_TRY_CUDA(                                                                                              \
-        cudaFuncSetAttribute(tc_update_pipe<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM)); \
+    static PerContext asked;                                                                                    \
+    BOLA_TRY(asked([]() -> int {                                                                                \
+      BOLA_TRY_CUDA(                                                                                            \
+          cudaFuncSetAttribute(tc_update_pipe<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM)); \
+      return 0;                                                                                                 \
+    }));                                                                                                        \
     StepLaunch L(dim3(grid), dim3(PTHREADS), Cfg::SMEM, s, pdl);                                                \
     BOLA_TRY_CUDA(cudaLaunchKernelEx(&L.cfg, tc_update_pipe<KIND, NPASS>, A, B, Alo, Blo, mapW, mapWs, m, n, boff,  \
                                      tpc, err, abort, lower ? 1 : 0, W, ldw));                                  \
@@ -504,8 +508,12 @@ int tc_update(cudaStream_t s, int kind, int64_t m, int64_t n, const CUtensorMap 
 #define BOLA_TC(KIND, NPASS)                                                                              \
   do {                                                                                                    \
     using Cfg = TcCfg<KIND, NPASS>;                                                                       \
-    BOLA_TRY_CUDA(cudaFuncSetAttribute(tc_update_kernel<KIND, NPASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                       Cfg::SMEM_LAUNCH));                                                \
+    static PerContext asked;                                                                              \
+    BOLA_TRY(asked([]() -> int {                                                                          \
+      BOLA_TRY_CUDA(cudaFuncSetAttribute(tc_update_kernel<KIND, NPASS>,                                   \
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::SMEM_LAUNCH)); \
+      return 0;                                                                                           \
+    }));                                                                                                  \
     tc_update_kernel<KIND, NPASS><<<grid, 128, Cfg::SMEM_LAUNCH, s>>>(A, B, Alo, Blo, m, n, boff, W, ldw, err, abort, lower ? 1 : 0); \
   } while (0)
   if (kind == 0) BOLA_TC(0, 1);

@@ -98,7 +98,7 @@ def case_mixed(n, kind, kappa_exp=None):
 
 
 def case_batched(count):
-    from .batch import Batch, config4_batch
+    from bola_gb300.batch import Batch, config4_batch
     ns, nrhs, kinds, fill = config4_batch(count, seed=4)
     b = Batch(ns, nrhs, kinds)
     fill(b)
@@ -112,7 +112,7 @@ def case_batched(count):
 
 
 def _print_scopes():
-    from . import api
+    from bola_gb300 import api
     prof = api.profile_read()
     total = sum(v["ms"] for v in prof.values()) or 1.0
     for name, v in sorted(prof.items(), key=lambda kv: -kv[1]["ms"]):
@@ -128,7 +128,7 @@ def main(argv):
     case, args = argv[0], [int(a) for a in argv[1:]]
     fn = {"getrf": case_getrf, "potrf": case_potrf, "mixed": case_mixed, "batched": case_batched}[case]
     if scopes:
-        from . import api
+        from bola_gb300 import api
         fn(*args)  # warm
         api.profile_reset()
         api.profile_enable(True)

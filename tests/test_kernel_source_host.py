@@ -10,10 +10,10 @@ Programmatic dependents: a kernel that waits for the one before it
 operands are not const __restrict__, which declares them constant during the
 whole kernel and allows loads that need not see another kernel's stores.
 
-Function attributes: they belong to a device and are shared by its threads, so a
-launch asks for what it needs each time (nothing remembers in a static that it
-has been asked for once) and always for the same shared memory (a size of the
-call's own would lower another thread's limit)."""
+Function attributes: they belong to a context and are shared by its threads, so
+no static of the process remembers that they have been asked for once (PerContext
+remembers for which context), and the same shared memory is asked for always (a
+size of the call's own would lower another thread's limit)."""
 import glob
 import os
 import re
@@ -73,7 +73,7 @@ def test_programmatic_dependents_take_plain_pointers(path):
 
 
 @pytest.mark.parametrize("path", UNITS, ids=os.path.basename)
-def test_function_attributes_are_asked_for_at_each_launch(path):
+def test_function_attributes_belong_to_a_context(path):
     text = source(path)
     assert not re.search(r"static (bool|size_t|int) \w*attr\w*", text)
     if os.path.basename(path) == "calibrate.cu":  # (probes, which have the device to themselves)
