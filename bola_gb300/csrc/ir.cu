@@ -1234,7 +1234,8 @@ int residual_berr(cudaStream_t s, Workspace &w, int64_t n, int nr, const double 
   double e = 0.0;
   for (int c = 0; c < nr; ++c) {
     const double den = h[3 * nr] * h[nr + c] + h[2 * nr + c];
-    const double v = den > 0.0 ? h[c] / den : (h[c] > 0.0 ? INFINITY : 0.0);
+    // (a NaN in A, x or b makes den one, and is no answer)
+    const double v = den > 0.0 ? h[c] / den : h[c] == 0.0 && den == 0.0 ? 0.0 : INFINITY;
     e = std::isnan(v) ? INFINITY : fmax(e, v);
   }
   *berr = e;

@@ -124,7 +124,7 @@ __global__ void berr_finish(const BerrSys *__restrict__ sys, int32_t count, cons
   double e = 0.0;
   for (int c = 0; c < sys[s].nrhs; ++c) {
     const double r = v[1 + c], den = v[0] * v[33 + c] + v[65 + c];
-    const double q = den > 0.0 ? r / den : (r > 0.0 ? INFINITY : 0.0);
+    const double q = den > 0.0 ? r / den : r == 0.0 && den == 0.0 ? 0.0 : INFINITY;  // (den: NaN as x or b may be)
     e = isnan(q) ? INFINITY : fmax(e, q);
   }
   berr[s] = e;
