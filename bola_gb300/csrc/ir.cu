@@ -312,6 +312,12 @@ __global__ void iota_perm(int64_t n, int32_t *perm) {
   if (i < n) perm[i] = (int32_t)i;
 }
 
+// "No interchange" for every row.
+__global__ void identity_ipiv(int64_t n, int32_t *ipiv) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) ipiv[i] = (int32_t)i + 1;
+}
+
 // Inverses of the 64x64 diagonal blocks of L (unit lower) and U, once per
 // factorisation: block b -> Dl[b], Du[b] (column-major 64x64).  Substitution
 // down (L) or up (U) the block, four threads per column of the inverse (rows
@@ -1630,6 +1636,10 @@ int dgesv_mixed_ws(Workspace &w, bool chol, int64_t n, int64_t nrhs, const doubl
                                       cudaMemcpyDeviceToDevice, s));
       copy_cols<<<(unsigned)cdiv(n * nr, 256), 256, 0, s>>>(n, nr, b, ldb, x, ldx);
     }
+    // (a singular A leaves the entries after its panel as they are, and after a
+    // Cholesky that gave up they have never been written)
+    identity_ipiv<<<(unsigned)cdiv(n, 256), 256, 0, s>>>(n, w.ipiv);
+    BOLA_CHECK_LAUNCH();
     int st = bola_dgetrf(n, n, acopy, n, w.ipiv, w.info, (bola_stream_t)s);
     if (st == 0) st = bola_dgetrs(n, nr, acopy, n, w.ipiv, x, ldx, (bola_stream_t)s);
     cudaFreeAsync(acopy, s);
