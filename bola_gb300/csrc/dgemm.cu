@@ -746,8 +746,9 @@ TilePlan plan_tiles(const GemmArgs &args, int sms, bool may_alloc) {
   return p;
 }
 
+// partial: the memory of a MEMORY plan.
 template <bool TA, bool TB>
-int launch_plan(cudaStream_t s, TilePlan &p) {
+int launch_plan(cudaStream_t s, TilePlan &p, double *partial) {
   GemmArgs &g = p.g;
   bool beside = false;  // a launch of this product precedes
   auto launch = [&](void (*kern)(const GemmArgs), int64_t ctas, int threads, int cluster = 0, size_t smem = 0) -> int {
@@ -812,9 +813,7 @@ int launch_plan(cudaStream_t s, TilePlan &p) {
                   p.teams * (p.tile == 32 ? Tile<32>::NT : p.tile == 16 ? Tile<16>::NT : Tile<8>::NT), p.split, smem);
   }
   const int64_t nch = (g.K + g.kc - 1) / g.kc;
-  Scratch part;
-  BOLA_TRY(part.alloc((size_t)(8 * nch * g.m8 * g.n4), s));
-  g.P = part.as<double>();
+  g.P = partial;
   BOLA_TRY(launch(gemm_partial<TA, TB>, p.cells * cdiv(nch, g.cps), Tile<32>::NT));
   gemm_fold<<<(unsigned)cdiv(g.m8 * g.n4, FOLD_T), FOLD_T, 0, s>>>(g);
   BOLA_CHECK_LAUNCH();
@@ -845,10 +844,16 @@ int dgemm_body(cudaStream_t s, char ta, char tb, int64_t m, int64_t n, int64_t k
   g.info = info;
   g.tri = tri;
   TilePlan p = plan_tiles(g, num_sms(), may_alloc);
-  if (!TA && !TB) return launch_plan<false, false>(s, p);
-  if (!TA && TB) return launch_plan<false, true>(s, p);
-  if (TA && !TB) return launch_plan<true, false>(s, p);
-  return launch_plan<true, true>(s, p);
+  Scratch part;
+  if (p.path == MEMORY && part.alloc((size_t)(8 * cdiv(g.K, kc) * g.m8 * g.n4), s) != 0) {
+    cudaGetLastError();  // (there is a plan that needs no memory)
+    p = plan_tiles(g, num_sms(), false);
+  }
+  double *const P = part.as<double>();
+  if (!TA && !TB) return launch_plan<false, false>(s, p, P);
+  if (!TA && TB) return launch_plan<false, true>(s, p, P);
+  if (TA && !TB) return launch_plan<true, false>(s, p, P);
+  return launch_plan<true, true>(s, p, P);
 }
 
 }  // namespace

@@ -67,3 +67,37 @@ def test_the_limit_without_memory():
         assert torch.equal(c, c0) == (status != 0)
         if status:
             assert b"does not take shapes beyond" in L.bola_last_error()
+
+
+def test_deep_product_when_memory_is_short():
+    """Partial sums of a gigabyte where 0.6 GB are free: the product is formed without them, with the same bits."""
+    from bola_gb300 import _lib
+    L = _lib.load()
+    m = n = 128
+    k = 500_000
+
+    def product(c):
+        return L.bola_dgemm(b"N", b"T", m, n, k, 1.0, ctypes.c_void_p(a.data_ptr()), m, ctypes.c_void_p(b.data_ptr()), n,
+                            1.0, ctypes.c_void_p(c.data_ptr()), m,
+                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+
+    a, b = (torch.rand(m * k, dtype=torch.float64, device="cuda") - 0.5 for _ in range(2))
+    c0 = torch.rand(m * n, dtype=torch.float64, device="cuda")
+    c1, c2 = c0.clone(), c0.clone()
+    assert product(c1) == 0, L.bola_last_error()
+    # the plan without memory, once before memory is short (its kernels are loaded then)
+    warm = c0.clone()
+    assert L.bola_dgemm_noalloc(b"N", b"T", m, n, 30_000, 1.0, ctypes.c_void_p(a.data_ptr()), m,
+                                ctypes.c_void_p(b.data_ptr()), n, 1.0, ctypes.c_void_p(warm.data_ptr()), m,
+                                ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hold = torch.empty(torch.cuda.mem_get_info()[0] - 600_000_000, dtype=torch.uint8, device="cuda")
+    try:
+        status = product(c2)
+        torch.cuda.synchronize()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert status == 0, L.bola_last_error()
+    assert torch.equal(c1, c2) and not torch.equal(c1, c0)
