@@ -212,7 +212,10 @@ int roomy(const void *kern) {
   std::lock_guard<std::mutex> lk(mu);
   if (done.count({dev, kern})) return 0;
   BOLA_TRY_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-  done.insert({dev, kern});
+  try {
+    done.insert({dev, kern});
+  } catch (...) {  // (out of host memory: asked for again next time, and no exception leaves a C entry)
+  }
   return 0;
 }
 
