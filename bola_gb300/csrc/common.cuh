@@ -176,8 +176,10 @@ int getrf2_rec(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, int
 // Look-ahead resources of one blocked factorisation: a high-priority stream
 // for the critical path (panels, the next block's columns), a low-priority
 // stream for the rest of each trailing update, and events.
-// Pooled per device, so concurrent callers each take their own set.
+// Pooled per device, so concurrent callers each take their own set, and used in
+// the context that they were made in only.
 struct LookAhead {
+  unsigned long long ctx_id = 0;
   cudaStream_t sp = nullptr, su = nullptr;
   cudaEvent_t ev[8] = {};
 };

@@ -924,16 +924,19 @@ std::vector<LookAhead *> g_la_pool[64];
 LookAhead *la_acquire() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  const unsigned long long id = context_id();
   {
     std::lock_guard<std::mutex> lk(g_la_mu);
     auto &pool = g_la_pool[dev & 63];
-    if (!pool.empty()) {
-      LookAhead *la = pool.back();
-      pool.pop_back();
-      return la;
-    }
+    for (size_t i = pool.size(); i-- > 0;)
+      if (pool[i]->ctx_id == id) {
+        LookAhead *la = pool[i];
+        pool.erase(pool.begin() + (std::ptrdiff_t)i);
+        return la;
+      }
   }
   LookAhead *la = new LookAhead();
+  la->ctx_id = id;
   int least = 0, greatest = 0;
   bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess &&
             cudaStreamCreateWithPriority(&la->sp, cudaStreamNonBlocking, greatest) == cudaSuccess &&

@@ -135,6 +135,32 @@ def test_mixed_solve_in_each_context(kind, spd):
     """)
 
 
+def test_look_ahead_in_each_context():
+    """The streams that a large factorisation overlaps on belong to a context: each has its own."""
+    child("""
+    n = 600
+    rng = np.random.default_rng(3)
+    a = rng.uniform(-1, 1, (n, n))
+    s = a @ a.T / n + np.eye(n)
+    first = None
+    for c in ctxs + ctxs:
+        ok(cu.cuCtxSetCurrent(c))
+        pa, ps = device(a), device(s)
+        piv, info = device(np.zeros(n, np.int32)), device(np.ones(2, np.int32))
+        st = L.bola_dgetrf(n, n, pa, n, piv, info, None)
+        assert st == 0, (st, L.bola_last_error())
+        st = L.bola_dpotrf(b"L", n, ps, n, ctypes.c_void_p(info.value + 4), None)
+        assert st == 0, (st, L.bola_last_error())
+        ok(cu.cuCtxSynchronize())
+        got = host(pa, (n, n)).tobytes(), host(ps, (n, n)).tobytes(), host(info, (1,)).tobytes()
+        assert got[2] == bytes(8)
+        assert first is None or got == first
+        first = got
+        for p in (pa, ps, piv, info):
+            ok(cu.cuMemFree_v2(p))
+    """)
+
+
 def test_right_solves_from_two_threads():
     """Base cases of different orders from two host threads: neither's launch loses the shared memory that the other's
     set."""
