@@ -177,13 +177,14 @@ int getrf2_rec(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, int
 // for the critical path (panels, the next block's columns), a low-priority
 // stream for the rest of each trailing update, and events.
 // Pooled per device, so concurrent callers each take their own set, and used in
-// the context that they were made in only.
+// the context that they were made in only.  A set that a captured call has used
+// is part of that capture until it ends, and is not given to calls outside it.
 struct LookAhead {
   unsigned long long ctx_id = 0;
   cudaStream_t sp = nullptr, su = nullptr;
   cudaEvent_t ev[8] = {};
 };
-LookAhead *la_acquire();  // nullptr if the resources cannot be created
+LookAhead *la_acquire(cudaStream_t s);  // for a call on stream s; nullptr if the resources cannot be created
 void la_release(LookAhead *la);
 
 int potrf2_rec(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, int32_t *info,

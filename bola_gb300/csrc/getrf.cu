@@ -919,17 +919,28 @@ int getrf2_rec(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, int
 namespace {
 std::mutex g_la_mu;
 std::vector<LookAhead *> g_la_pool[64];
+
+// The capture that stream s is part of (0: none).
+unsigned long long capture_of(cudaStream_t s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(s, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusNone ? 0 : id;
+}
 }  // namespace
 
-LookAhead *la_acquire() {
+LookAhead *la_acquire(cudaStream_t s) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  const unsigned long long id = context_id();
+  const unsigned long long id = context_id(), capture = capture_of(s);
   {
     std::lock_guard<std::mutex> lk(g_la_mu);
     auto &pool = g_la_pool[dev & 63];
     for (size_t i = pool.size(); i-- > 0;)
-      if (pool[i]->ctx_id == id) {
+      if (pool[i]->ctx_id == id && capture_of(pool[i]->sp) == capture && capture_of(pool[i]->su) == capture) {
         LookAhead *la = pool[i];
         pool.erase(pool.begin() + (std::ptrdiff_t)i);
         return la;
@@ -987,7 +998,7 @@ int getrf_blocked(cudaStream_t s, int64_t m, int64_t n, double *A, int64_t lda, 
   BOLA_TRY(plans.alloc((size_t)cdiv(min_mn, PNB) * PLAN_INTS * sizeof(int32_t), s, true));
   // look-ahead pays from a few hundred columns on; below that its events and
   // the extra launches cost more than the overlap saves
-  LookAhead *la = min_mn >= LOOK_AHEAD_MIN ? la_acquire() : nullptr;
+  LookAhead *la = min_mn >= LOOK_AHEAD_MIN ? la_acquire(s) : nullptr;
   cudaStream_t sp = la ? la->sp : s, su = la ? la->su : s;
   auto run = [&]() -> int {
     if (la) {

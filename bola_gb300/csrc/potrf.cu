@@ -651,7 +651,7 @@ int potrf_blocked(cudaStream_t s, char uplo, int64_t n, double *A, int64_t lda, 
   }
   Scratch bk;
   BOLA_TRY(bk.alloc((size_t)n * n * sizeof(double), s));
-  LookAhead *la = la_acquire();
+  LookAhead *la = la_acquire(s);
   cudaStream_t sp = la ? la->sp : s, su = la ? la->su : s;
   auto on = [&](cudaEvent_t e, cudaStream_t from, cudaStream_t to) -> int {
     if (!la || from == to) return 0;

@@ -93,3 +93,46 @@ def test_memory_of_graphs_comes_back():
         torch.cuda.synchronize()
         free.append(torch.cuda.mem_get_info()[0])
     assert free[0] - free[-1] <= 8 << 20, free
+
+
+def test_direct_calls_beside_a_capture():
+    """While one stream is being captured, a call on another runs at once, and neither disturbs the other (a captured
+    call's streams stay part of the capture until it ends)."""
+    d, L = Driver(), _lib.load()
+    n = 600
+    a0 = torch.from_numpy(wl.uniform_matrix(n, n, seed=9, lo=-1, hi=1).ravel(order="F").copy()).cuda()
+    s0 = torch.from_numpy(wl.spd_matrix(n, seed=9).ravel(order="F").copy()).cuda()
+    bufs = [(a0.clone(), s0.clone(), torch.zeros(n, dtype=torch.int32, device="cuda"),
+             torch.ones(2, dtype=torch.int32, device="cuda")) for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def calls(stream, a, sp, piv, info):
+        s = ctypes.c_void_p(stream.cuda_stream)
+        assert L.bola_dgetrf(n, n, _p(a), n, _p(piv), _p(info), s) == 0, L.bola_last_error()
+        assert L.bola_dpotrf(b"L", n, _p(sp), n, _p(info[1:]), s) == 0, L.bola_last_error()
+
+    calls(streams[1], *bufs[1])  # (attributes, pools)
+    torch.cuda.synchronize()
+    want = [t.clone() for t in bufs[1]]
+    g, x = ctypes.c_void_p(), ctypes.c_void_p()
+    s = ctypes.c_void_p(streams[0].cuda_stream)
+    d.cuStreamBeginCapture_v2(s, 2)  # (relaxed: other streams' calls are allowed)
+    calls(streams[0], *bufs[0])
+    bufs[1][0].copy_(a0)
+    bufs[1][1].copy_(s0)
+    torch.cuda.default_stream().synchronize()
+    calls(streams[1], *bufs[1])
+    calls_again = [t.clone() for t in (a0, s0)] + [torch.zeros_like(want[2]), torch.ones_like(want[3])]
+    torch.cuda.default_stream().synchronize()
+    calls(streams[1], *calls_again)
+    d.cuStreamEndCapture(s, ctypes.byref(g))
+    torch.cuda.synchronize()
+    for got in (bufs[1], calls_again):
+        assert all(torch.equal(t, w) for t, w in zip(got, want))
+    d.cuGraphInstantiateWithFlags(ctypes.byref(x), g, ctypes.c_ulonglong(0))
+    d.cuGraphLaunch(x, s)
+    torch.cuda.synchronize()
+    assert all(torch.equal(t, w) for t, w in zip(bufs[0], want))
+    d.cuGraphExecDestroy(x)
+    d.cuGraphDestroy(g)
